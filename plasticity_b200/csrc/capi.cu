@@ -56,8 +56,17 @@ struct CgGraph {
   cudaStream_t body_stream = nullptr;
   long long amg_version = -1;
   double* ctl = nullptr;   // device: [0] rtol, [1] itmax, [2] absolute threshold (set on the device)
-  int* state = nullptr;    // device: [0] iterations, [1] converged
+  int* state = nullptr;    // device (in ReadBack): [0] iterations, [1] converged
   long long prefix_kernels = 0, body_kernels = 0;
+};
+
+// What the host reads back after a residual or a linear solve, in one copy to a
+// page-locked mirror (each small copy to pageable memory costs about 9 us).
+struct ReadBack {
+  DevStatus status;      // first inverted Gauss point of the last assembly
+  int waits;             // set by a solver kernel whose bounded wait ran out
+  int cg[2][2];          // [precision]: iterations, converged
+  double scal[2];        // [0] |R|
 };
 
 struct HostLevel {
@@ -112,7 +121,7 @@ struct pfem_ctx {
   double *dU = nullptr, *dR = nullptr, *dDg = nullptr, *dUprev = nullptr, *dUprev2 = nullptr;
   double* dUprev3 = nullptr;
   double bbox_lo[3] = {0, 0, 0}, bbox_ext[3] = {1, 1, 1};
-  double *dUtmp = nullptr, *dScal = nullptr, *dPart = nullptr;
+  double *dUtmp = nullptr, *dPart = nullptr;
   double* dK64 = nullptr;
   float* dK32 = nullptr;
   double* dDenseWork = nullptr;  // FP64 work matrix of the coarse dense inverse (both precisions)
@@ -125,7 +134,7 @@ struct pfem_ctx {
   float* dKbuf32 = nullptr;
   double* dKbuf64 = nullptr;
   double* dFbuf = nullptr;
-  DevStatus* dStatus = nullptr;
+  ReadBack *dBack = nullptr, *hBack = nullptr;
   // boundary conditions
   bool bcs_set = false;
   BcDev bc;
@@ -179,11 +188,14 @@ int cuda_fail(pfem_ctx* c) {
     }                                                         \
   } while (0)
 
+// Slack at the end of the matrix arrays, whose bulk copies are rounded out to 16 bytes
+// (spmv_pipe.cuh).
+constexpr size_t kCopySlack = 16;
 template <typename T>
-cudaError_t dalloc(pfem_ctx* ctx, T** p, size_t n) {
+cudaError_t dalloc(pfem_ctx* ctx, T** p, size_t n, size_t slack = 0) {
   *p = nullptr;
   if (n == 0) n = 1;
-  cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+  cudaError_t e = cudaMalloc((void**)p, n * sizeof(T) + slack);
   if (e == cudaSuccess) ctx->allocs.push_back((void*)*p);
   return e;
 }
@@ -200,8 +212,8 @@ cudaError_t d2h(const pfem_ctx* ctx, void* dst, const void* src, size_t bytes) {
   return e == cudaSuccess ? cudaStreamSynchronize(ctx->st) : e;
 }
 template <typename T>
-cudaError_t upload(pfem_ctx* ctx, T** p, const std::vector<T>& h) {
-  cudaError_t e = dalloc(ctx, p, h.size());
+cudaError_t upload(pfem_ctx* ctx, T** p, const std::vector<T>& h, size_t slack = 0) {
+  cudaError_t e = dalloc(ctx, p, h.size(), slack);
   if (e != cudaSuccess) return e;
   if (!h.empty()) e = h2d(ctx, *p, h.data(), h.size() * sizeof(T));
   return e;
@@ -671,14 +683,17 @@ int amg_alloc(pfem_ctx* ctx) {
     v.A.nbrow = h.nbrow;
     v.A.bs = h.bs;
     v.A.nnzb = l == 0 ? ctx->nnzb : h.rowptr[h.nbrow];
+    v.A.err = &ctx->dBack->waits;
     if (l == 0) {
+      v.A.max_row = ctx->max_row;
       v.A.rowptr = ctx->dBrowptr;
       v.A.col = ctx->dBcol;
       v.A.col16 = ctx->dBcol16;
     } else {
-      CK(upload(ctx, &v.A.rowptr, h.rowptr));
-      CK(upload(ctx, &v.A.col, h.col));
-      CK(dalloc(ctx, &v.A.val, (size_t)v.A.nnzb * h.bs * h.bs));
+      for (int n = 0; n < h.nbrow; ++n) v.A.max_row = std::max(v.A.max_row, h.rowptr[n + 1] - h.rowptr[n]);
+      CK(upload(ctx, &v.A.rowptr, h.rowptr, kCopySlack));
+      CK(upload(ctx, &v.A.col, h.col, kCopySlack));
+      CK(dalloc(ctx, &v.A.val, (size_t)v.A.nnzb * h.bs * h.bs, kCopySlack));
     }
     CK(dalloc(ctx, &v.dinv, (size_t)h.nbrow * h.bs * h.bs));
     v.nagg = h.nagg;
@@ -994,7 +1009,7 @@ int cg_graph_build(pfem_ctx* ctx) {
   if (G.graph) { cudaGraphDestroy(G.graph); G.graph = nullptr; }
   if (!G.ctl) {
     CK(dalloc(ctx, &G.ctl, 4));
-    CK(dalloc(ctx, &G.state, 4));
+    G.state = ctx->dBack->cg[std::is_same<T, double>::value ? 1 : 0];
     CK(cudaStreamCreateWithFlags(&G.body_stream, cudaStreamNonBlocking));
   }
   KrylovWork<T>& w = kw_of<T>(ctx);
@@ -1083,6 +1098,16 @@ int cg_graph_build(pfem_ctx* ctx) {
   return PFEM_OK;
 }
 
+// Bring ReadBack to the host (synchronizes); an error when a solver kernel gave up
+// waiting for its own copies.
+int read_back(pfem_ctx* ctx) {
+  CK(cudaMemcpyAsync(ctx->hBack, ctx->dBack, sizeof(ReadBack), cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  if (!ctx->hBack->waits) return PFEM_OK;
+  CK(cudaMemsetAsync(&ctx->dBack->waits, 0, sizeof(int), ctx->st));
+  return fail(ctx, PFEM_ERR_CUDA, "a solver kernel's wait for its copies timed out");
+}
+
 // Preconditioned CG / BiCGStab on level-0 operator with the AMG V-cycle.
 // b and the result x live in kw.b / kw.x.  Returns iterations (>=0) or <0.
 template <typename T>
@@ -1107,9 +1132,9 @@ int krylov_inner(pfem_ctx* ctx, int method, double rtol, int itmax, int* iters, 
     const double ctl[2] = {rtol, (double)std::max(itmax, 1)};
     CK(cudaMemcpyAsync(G.ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
     CK(cudaGraphLaunch(G.exec, st));
-    int sh[2] = {0, 0};
-    CK(cudaMemcpyAsync(sh, G.state, sizeof(sh), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    rc = read_back(ctx);
+    if (rc) return rc;
+    const int* sh = ctx->hBack->cg[std::is_same<T, double>::value ? 1 : 0];
     *iters = sh[0];
     *conv = sh[1] != 0;
     pfem::launch_counter() += G.prefix_kernels + (long long)sh[0] * G.body_kernels;
@@ -1152,7 +1177,7 @@ int krylov_inner(pfem_ctx* ctx, int method, double rtol, int itmax, int* iters, 
     }
   }
   CKL();
-  return PFEM_OK;
+  return read_back(ctx);
 }
 
 // Solve K x = b (kw.b -> kw.x) to relative tolerance rtol.  Below the level a
@@ -1219,13 +1244,13 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
   cudaStream_t st = ctx->st;
   const bool fbar = ctx->kind == PFEM_HEX8_FINITE_FBAR;
   const bool small = ctx->kind == PFEM_HEX8_SMALL;
-  CK(cudaMemsetAsync(ctx->dStatus, 0, sizeof(DevStatus), st));
+  CK(cudaMemsetAsync(&ctx->dBack->status, 0, sizeof(DevStatus), st));
   if (commit) {
     ElemArgs<double> a{};
     a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
     a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
     a.R = ctx->dR; a.Kval = ctx->dK64; a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
-    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = ctx->dStatus;
+    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
     if (small) launch_element_small<double>(a, ctx->dAllElems, (int)ctx->ne, true, ctx->hard, st);
     else launch_element_color<double>(a, ctx->dAllElems, (int)ctx->ne, true, fbar, ctx->hard, st);
     CKL();
@@ -1241,7 +1266,7 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
       a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
       a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
       a.R = ctx->dR; a.Kval = ctx->dK64; a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
-      a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = ctx->dStatus;
+      a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
       a.Kbuf = ctx->dKbuf64; a.Fbuf = ctx->dFbuf;
       if (small) launch_element_small<double>(a, ctx->dAllElems, (int)ctx->ne, false, ctx->hard, st);
       else launch_element_color<double>(a, ctx->dAllElems, (int)ctx->ne, false, fbar, ctx->hard, st);
@@ -1253,7 +1278,7 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
       a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
       a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
       a.R = ctx->dR; a.Kval = ctx->dK32; a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
-      a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = ctx->dStatus;
+      a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
       a.Kbuf = ctx->dKbuf32; a.Fbuf = ctx->dFbuf;
       if (small) launch_element_small<float>(a, ctx->dAllElems, (int)ctx->ne, false, ctx->hard, st);
       else launch_element_color<float>(a, ctx->dAllElems, (int)ctx->ne, false, fbar, ctx->hard, st);
@@ -1271,7 +1296,7 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
     a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
     a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
     a.R = ctx->dR; a.Kval = ctx->dK64; a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
-    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = ctx->dStatus;
+    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
     for (int c = 0; c < nc; ++c) {
       const int* cl = ctx->dColorList + ctx->color_ptr[c];
       const int cn = ctx->color_ptr[c + 1] - ctx->color_ptr[c];
@@ -1284,7 +1309,7 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
     a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
     a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
     a.R = ctx->dR; a.Kval = ctx->dK32; a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
-    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = ctx->dStatus;
+    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
     for (int c = 0; c < nc; ++c) {
       const int* cl = ctx->dColorList + ctx->color_ptr[c];
       const int cn = ctx->color_ptr[c + 1] - ctx->color_ptr[c];
@@ -1297,15 +1322,15 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
 }
 
 int ensure_tangent(pfem_ctx* ctx, int prec) {
-  if (prec == PFEM_FP64 && !ctx->dK64) CK(dalloc(ctx, &ctx->dK64, (size_t)ctx->nnzb * 9));
-  if (prec == PFEM_MIXED && !ctx->dK32) CK(dalloc(ctx, &ctx->dK32, (size_t)ctx->nnzb * 9));
+  if (prec == PFEM_FP64 && !ctx->dK64) CK(dalloc(ctx, &ctx->dK64, (size_t)ctx->nnzb * 9, kCopySlack));
+  if (prec == PFEM_MIXED && !ctx->dK32) CK(dalloc(ctx, &ctx->dK32, (size_t)ctx->nnzb * 9, kCopySlack));
   return PFEM_OK;
 }
 
 int check_status(pfem_ctx* ctx) {
-  DevStatus s;
-  CK(cudaMemcpyAsync(&s, ctx->dStatus, sizeof(s), cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
+  int rc = read_back(ctx);
+  if (rc) return rc;
+  const DevStatus& s = ctx->hBack->status;
   if (s.code) {
     char buf[256];
     snprintf(buf, sizeof(buf),
@@ -1327,10 +1352,10 @@ int residual_system(pfem_ctx* ctx, int prec, double lam, double* rnorm, double* 
   if (prec == PFEM_FP64) impose_dirichlet<double>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK64, ctx->dR, ctx->dDg, ctx->st);
   else impose_dirichlet<float>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK32, ctx->dR, ctx->dDg, ctx->st);
   CKL();
-  dot<double>(ctx->ndof, ctx->dR, ctx->dR, ctx->dScal, ctx->dPart, ctx->st, true);
+  dot<double>(ctx->ndof, ctx->dR, ctx->dR, ctx->dBack->scal, ctx->dPart, ctx->st, true);
   CKL();
-  CK(cudaMemcpyAsync(rnorm, ctx->dScal, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   rc = check_status(ctx);  // synchronizes
+  *rnorm = ctx->hBack->scal[0];
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx->e0, ctx->e1);
   if (t_asm) *t_asm += ms;
@@ -1694,8 +1719,8 @@ int device_pattern(pfem_ctx* ctx, const std::vector<int>& nptr, const std::vecto
     if (acc * 9 >= (1ll << 31)) return fail(ctx, PFEM_ERR_BAD_ARG, "pattern too large for 32-bit indices");
     ctx->browptr[n + 1] = (int)acc;
   }
-  CK(upload(ctx, &ctx->dBrowptr, ctx->browptr));
-  CK(dalloc(ctx, &ctx->dBcol, (size_t)acc));
+  CK(upload(ctx, &ctx->dBrowptr, ctx->browptr, kCopySlack));
+  CK(dalloc(ctx, &ctx->dBcol, (size_t)acc, kCopySlack));
   launch_node_rows((int)nn, dnptr, dnel, ctx->dElem, ctx->dBrowptr, nullptr, ctx->dBcol, derr, st);
   CKL();
   CK(dalloc(ctx, &ctx->dRank, (size_t)ne * 64));
@@ -1884,14 +1909,14 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
   }
   // ---- device upload ----
   cudaError_t ce;
-#define UP(ptr, vec) if ((ce = upload(ctx, &ptr, vec)) != cudaSuccess) { pfem_set_cuda_error(ce, #ptr, __FILE__, __LINE__); return bail(PFEM_ERR_CUDA); }
+#define UP(ptr, vec, ...) if ((ce = upload(ctx, &ptr, vec, ##__VA_ARGS__)) != cudaSuccess) { pfem_set_cuda_error(ce, #ptr, __FILE__, __LINE__); return bail(PFEM_ERR_CUDA); }
 #define AL(ptr, n) if ((ce = dalloc(ctx, &ptr, n)) != cudaSuccess) { pfem_set_cuda_error(ce, #ptr, __FILE__, __LINE__); return bail(PFEM_ERR_CUDA); }
   UP(ctx->dX, ctx->X);
   if (!dev_pattern) {
     UP(ctx->dElem, ctx->elem);
     UP(ctx->dRank, rank);
-    UP(ctx->dBrowptr, ctx->browptr);
-    UP(ctx->dBcol, ctx->bcol);
+    UP(ctx->dBrowptr, ctx->browptr, kCopySlack);
+    UP(ctx->dBcol, ctx->bcol, kCopySlack);
   }
   UP(ctx->dColorList, clist);
   UP(ctx->dAllElems, all);
@@ -1922,7 +1947,7 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
           else c16[k] = (int16_t)d;
         }
       });
-      if (fits) UP(ctx->dBcol16, c16);
+      if (fits) UP(ctx->dBcol16, c16, kCopySlack);
     }
     const char* am = getenv("PFEM_ASSEMBLY");
     ctx->colored_assembly = am && std::string(am) == "colored";
@@ -1944,9 +1969,13 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
   AL(ctx->dUprev2, ctx->ndof);
   AL(ctx->dUprev3, ctx->ndof);
   AL(ctx->dUtmp, ctx->ndof);
-  AL(ctx->dScal, 16);
   AL(ctx->dPart, 2048);
-  AL(ctx->dStatus, 1);
+  AL(ctx->dBack, 1);
+  if ((ce = cudaMallocHost((void**)&ctx->hBack, sizeof(ReadBack))) != cudaSuccess ||
+      (ce = cudaMemsetAsync(ctx->dBack, 0, sizeof(ReadBack), ctx->st)) != cudaSuccess) {
+    pfem_set_cuda_error(ce, "ReadBack", __FILE__, __LINE__);
+    return bail(PFEM_ERR_CUDA);
+  }
 #undef UP
 #undef AL
   int rc = pfem_reset(ctx);
@@ -1969,6 +1998,7 @@ void pfem_destroy(pfem_ctx* ctx) {
     if (g->body_stream) cudaStreamDestroy(g->body_stream);
   }
   for (void* p : ctx->allocs) cudaFree(p);
+  if (ctx->hBack) cudaFreeHost(ctx->hBack);
   if (ctx->e0) cudaEventDestroy(ctx->e0);
   if (ctx->e1) cudaEventDestroy(ctx->e1);
   if (ctx->t0) cudaEventDestroy(ctx->t0);
@@ -1981,7 +2011,7 @@ int pfem_inversion_info(const pfem_ctx* ctx, int64_t* e, int32_t* g, double* J) 
   if (!ctx) return PFEM_ERR_BAD_ARG;
   if (ctx->device < 0) return PFEM_ERR_STATE;
   DevStatus s;
-  if (d2h(ctx, &s, ctx->dStatus, sizeof(s)) != cudaSuccess) return PFEM_ERR_CUDA;
+  if (d2h(ctx, &s, &ctx->dBack->status, sizeof(s)) != cudaSuccess) return PFEM_ERR_CUDA;
   if (e) *e = s.code ? s.e : 0;
   if (g) *g = s.code ? s.g : 0;
   if (J) *J = s.code ? s.J : 0.0;
@@ -2581,7 +2611,7 @@ int pfem_amg_apply(pfem_ctx* ctx, const double* r, double* z) {
   } else {
     return fail(ctx, PFEM_ERR_STATE, "no AMG hierarchy built for the resident tangent");
   }
-  return PFEM_OK;
+  return read_back(ctx);
 }
 
 int pfem_amg_dense(pfem_ctx* ctx, int32_t level, int32_t what, double* out, int64_t* dims) {
@@ -2782,7 +2812,7 @@ int pfem_profile(pfem_ctx* ctx, int32_t what, int32_t reps, double* ms) {
   float t = 0;
   CK(cudaEventElapsedTime(&t, ctx->e0, ctx->e1));
   *ms = t / reps;
-  return PFEM_OK;
+  return read_back(ctx);
 }
 
 int64_t pfem_kernel_launches(void) { return (int64_t)g_launches; }

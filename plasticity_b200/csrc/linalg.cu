@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "linalg.cuh"
+#include "spmv_pipe.cuh"
 
 namespace pfem {
 
@@ -117,9 +118,47 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
   }
 }
 
+template <typename T, int BS, int MODE, bool C16>
+static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, T c1, T c2,
+                          cudaStream_t st) {
+  auto* kern = bsr_spmv_pipe_kernel<T, BS, MODE, C16>;
+  const int sm = pipe_smem_bytes<T, BS>(A.max_row, C16);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  int dev = 0, sms = 148, per = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32, sm);
+  constexpr int R = PipeShape<T, BS>::ROWS;
+  const int tiles = (A.nbrow + R - 1) / R;
+  const int grid = std::min(tiles, sms * std::max(per, 1));
+  pfem::count_launch();
+  kern<<<grid, 32, sm, st>>>(A.nbrow, tiles, A.max_row, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, c1, c2,
+                             A.err);
+}
+// The streamed kernel takes a matrix whose rows have at most 32 blocks and whose
+// arrays start on 16 bytes, from as many rows on as keep most warps of the chip busy:
+// below, one row per half-warp (or warp) has less latency per launch.  The cycle,
+// register / streamed: 20.6 / 22.6 us at 8^3 (729 rows), 26.4 / 26.7 at 16^3 (4,913),
+// 54 / 51 at 24^3 (15,625), 117 / 100 at 40^3.  6 x 6 levels, with the finest level
+// streamed: 152 / 146 us at 48^3 (4,913 rows of 6 x 6), 647 / 603 at 80^3 (19,683).
+constexpr int kPipeRows3 = 8192, kPipeRows6 = 4096;
+template <typename T, int MODE>
+static bool spmv_pipe_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, T c1, T c2,
+                             cudaStream_t st) {
+  const bool c16 = A.bs == 3 && A.col16;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(A.val) | reinterpret_cast<uintptr_t>(A.rowptr) |
+                       (c16 ? reinterpret_cast<uintptr_t>(A.col16) : reinterpret_cast<uintptr_t>(A.col));
+  if (A.nbrow < (A.bs == 3 ? kPipeRows3 : kPipeRows6) || A.max_row < 1 || A.max_row > 32 || !A.err || (at & 15)) return false;
+  if (c16) pipe_launch_t<T, 3, MODE, true>(A, x, y, b, dinv, xo, c1, c2, st);
+  else if (A.bs == 3) pipe_launch_t<T, 3, MODE, false>(A, x, y, b, dinv, xo, c1, c2, st);
+  else pipe_launch_t<T, 6, MODE, false>(A, x, y, b, dinv, xo, c1, c2, st);
+  return true;
+}
+
 template <typename T, int MODE>
 static void spmv_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, T c1, T c2,
                         cudaStream_t st) {
+  if (spmv_pipe_launch<T, MODE>(A, x, y, b, dinv, xo, c1, c2, st)) return;
   // 6 x 6 levels of fewer than kWarpRowsBelow rows fill too few warp slots with half
   // a warp per row: give each row a whole warp there (measured at 64^3: level 2,
   // 512 rows, 7.4 -> 6.5 us per pass; level 1, 10,648 rows, 14.3 -> 18.2 us)

@@ -73,6 +73,8 @@ struct BsrMat {
   // optional, device: col[k] - row as 16-bit offsets (set when every offset fits),
   // read by the SpMV in place of col
   const int16_t* col16 = nullptr;
+  int max_row = 0;        // blocks of the longest row (0: unknown)
+  int* err = nullptr;     // device flag that a kernel sets when a bounded wait ran out
 };
 
 // One level of smoothed-aggregation AMG.  Every fine block row n belongs to

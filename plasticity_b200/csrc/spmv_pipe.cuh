@@ -1,0 +1,358 @@
+// spmv_pipe.cuh -- block-CSR SpMV with the matrix streamed through shared memory.
+//
+// What bounds it: the matrix is read once (HBM, or L2 when it fits).  Read straight
+// into registers, a lane's 36-byte block is nine loads whose 32 addresses lie 36
+// bytes apart, each of them touching every 128-byte line of the warp's kilobyte, and
+// the gathered vector entries cost another line per neighbour: the kernel then runs
+// at the L1's rate of lines, 4.6 TB/s from HBM and no faster from L2 (3.65 TB/s at
+// 40^3).  Here every warp copies its tile of rows (contiguous in the value, column
+// and row-pointer arrays) with cp.async.bulk into shared memory of its own, so the
+// bytes in flight cost no registers and no warp waits for another one.
+//
+// 3 x 3 blocks: eight rows per tile, four lanes per row.  A lane takes every fourth
+// block of its row; the lanes of a warp read shared memory at the rows' stride (27
+// blocks = 243 words, odd: few bank conflicts), and in a node-ordered mesh the rows'
+// k-th neighbours are consecutive nodes, so the gathers of x fall into a few lines.
+// Each component has seven partial sums, one block of a 27-block row each, added as a
+// tree: no deeper than the register kernel's two blocks per lane and four shuffles.
+// 6 x 6 blocks: half a warp per row, lane k takes blocks k and k + 16, 16-byte reads
+// at a stride of 36 words (no conflicts).
+#pragma once
+#include <cstdint>
+
+#include "linalg.cuh"
+
+namespace pfem {
+
+constexpr long long kPipeWaitLimit = 1ll << 20;  // polls of a barrier before a kernel gives up
+
+__device__ __forceinline__ uint32_t pipe_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void pipe_bar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ bool pipe_bar_wait(uint32_t bar, uint32_t phase) {
+  for (long long it = 0; it < kPipeWaitLimit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(phase)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void pipe_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void pipe_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Both addresses and the size are multiples of 16 bytes.
+__device__ __forceinline__ void pipe_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+// The same, with the lines marked for early eviction: a matrix that is streamed once
+// per pass should not push the gathered vector out of L2.
+__device__ __forceinline__ void pipe_copy_first(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], pol;\n\t}\n" ::
+          "r"(dst), "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
+// LANES lanes per row and ROWS rows per tile; a CTA is one warp with one tile in shared
+// memory (8 rows of 27 blocks: 8 KB float, 16 KB double; 4 rows of 6 x 6: 15 KB), so
+// that 13 to 24 of them share an SM and the copies of some overlap the arithmetic of
+// the others.  Measured at 64^3, FP32, per pass over 281 MB: 44.0 us (6.4 TB/s; the
+// register kernel 59.8); one warp with two stages 49.2, two warps with two stages
+// 50.5, a producer lane feeding eight half-warp-per-row warps through four stages
+// 51.4.  FP64 79.0 us (103.1).  Two lanes per row: the same at 64^3, 14 % slower at
+// 40^3 (16.5 against 14.4 us).  The cycle in its graph: 431 -> 342 us at 64^3.
+template <typename T, int BS>
+struct PipeShape {
+  static constexpr int LANES = BS == 3 ? 4 : 16;
+  static constexpr int ROWS = BS == 3 ? 32 / LANES : 4;
+  static_assert(ROWS % 4 == 0, "a tile's row pointers start on 16 bytes");
+};
+
+// Byte layout of a tile: values, column ids, row pointers; each region starts on 16
+// bytes and has room for the slack of copies whose ends are rounded out to 16 bytes.
+struct PipeLay {
+  int cols, rows, bytes;
+};
+template <typename T, int BS>
+__host__ __device__ inline PipeLay pipe_lay(int max_row, bool c16) {
+  constexpr int R = PipeShape<T, BS>::ROWS;
+  PipeLay l;
+  l.cols = (R * max_row * BS * BS * (int)sizeof(T) + 32 + 15) & ~15;
+  l.rows = l.cols + ((R * max_row * (c16 ? 2 : 4) + 32 + 15) & ~15);
+  l.bytes = l.rows + R * 4 + 16;
+  return l;
+}
+constexpr int kPipeHead = 16;  // the barrier, in front of the tile
+template <typename T, int BS>
+inline int pipe_smem_bytes(int max_row, bool c16) {
+  return kPipeHead + pipe_lay<T, BS>(max_row, c16).bytes;
+}
+
+// Start the copies of tile t (rows t R .., blocks s0 .. s1); one lane.
+template <typename T, int BS, bool C16>
+__device__ __forceinline__ void pipe_issue(unsigned char* stage, const PipeLay& lay, uint32_t bar, int t, int nbrow, int s0,
+                                           int s1, const int* rowptr, const int* col, const int16_t* col16, const T* val) {
+  constexpr int R = PipeShape<T, BS>::ROWS, VB = BS * BS * (int)sizeof(T), CB = C16 ? 2 : 4;
+  const int r0 = t * R, rows = min(R, nbrow - r0);
+  const long long va = ((long long)s0 * VB) & ~15ll, ca = ((long long)s0 * CB) & ~15ll;
+  const uint32_t vb = (uint32_t)((((long long)s1 * VB + 15) & ~15ll) - va);
+  const uint32_t cb = (uint32_t)((((long long)s1 * CB + 15) & ~15ll) - ca);
+  const uint32_t rb = (uint32_t)(((rows + 1) * 4 + 15) & ~15);
+  const uint32_t dst = pipe_smem(stage);
+  pipe_expect(bar, vb + cb + rb);
+  pipe_copy(dst + lay.rows, rowptr + r0, rb, bar);
+  if (cb) pipe_copy(dst + lay.cols, (C16 ? (const char*)col16 : (const char*)col) + ca, cb, bar);
+  if (vb) pipe_copy_first(dst, (const char*)val + va, vb, bar);
+}
+
+// What the modes do with a row's sum v (A x), row by row:
+//   0: y = v   1: y = b - v   2: y -= Dinv v, xo += x   3: xo = c2 x + c1 (y - Dinv v)
+//   4: as 3, added to xo      5: y = Dinv (b - v), xo = c1 y
+template <typename T, int BS, int MODE, bool C16>
+__global__ void __launch_bounds__(32)
+bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__ rowptr, const int* __restrict__ col,
+                     const int16_t* __restrict__ col16, const T* __restrict__ val, const T* x, T* y, const T* b,
+                     const T* __restrict__ dinv, T* xo, T c1, T c2, int* err) {
+  using SH = PipeShape<T, BS>;
+  constexpr int R = SH::ROWS, BB = BS * BS;
+  extern __shared__ __align__(128) unsigned char psm[];
+  const PipeLay lay = pipe_lay<T, BS>(max_row, C16);
+  const int lane = threadIdx.x;
+  unsigned char* const st = psm + kPipeHead;
+  const uint32_t bar = pipe_smem(psm);
+  int n0 = 0, n1 = 0;  // block range of the next tile to copy (lane 0)
+  if (lane == 0) {
+    pipe_bar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    const int t = blockIdx.x, tn = t + gridDim.x;
+    const int s0 = rowptr[t * R], s1 = rowptr[min(t * R + R, nbrow)];
+    if (tn < ntiles) {
+      n0 = rowptr[tn * R];
+      n1 = rowptr[min(tn * R + R, nbrow)];
+    }
+    pipe_issue<T, BS, C16>(st, lay, bar, t, nbrow, s0, s1, rowptr, col, col16, val);
+  }
+  __syncwarp();
+  uint32_t phase = 0;
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
+    // a lane's row(s) of the tile and the epilogue's operands, in flight while the tile arrives
+    if constexpr (BS == 3) {
+      constexpr int LN = SH::LANES;  // par: which of the row's lanes this one is
+      const int rl = lane & (R - 1), par = lane / R;
+      const int row = t * R + rl;
+      const bool ok = row < nbrow, own = ok && par == 0;
+      const long long at = (long long)row * 3;
+      T bi[3], yi[3], xi[3], oi[3], D[9];
+      if (own) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          if (MODE == 1 || MODE == 5) bi[i] = b[at + i];
+          if (MODE == 2 || MODE == 3 || MODE == 4) { yi[i] = y[at + i]; xi[i] = x[at + i]; }
+          if (MODE == 2 || MODE == 4) oi[i] = xo[at + i];
+        }
+        if (MODE >= 2) {
+#pragma unroll
+          for (int i = 0; i < 9; ++i) D[i] = dinv[(long long)row * 9 + i];
+        }
+      }
+      if (!__all_sync(0xffffffffu, pipe_bar_wait(bar, phase))) {
+        if (lane == 0) atomicExch(err, 1);
+        return;
+      }
+      const int* rp = reinterpret_cast<const int*>(st + lay.rows);
+      const int s0 = rp[0];
+      const int b0 = ok ? rp[rl] - s0 : 0, len = ok ? rp[rl + 1] - s0 - b0 : 0;
+      const T* vs = reinterpret_cast<const T*>(st + (((long long)s0 * (9 * (int)sizeof(T))) & 15)) + (long long)b0 * 9;
+      const int* cs = reinterpret_cast<const int*>(st + lay.cols + (((long long)s0 * 4) & 15)) + b0;
+      const int16_t* cs16 = reinterpret_cast<const int16_t*>(st + lay.cols + (((long long)s0 * 2) & 15)) + b0;
+      // seven partial sums per component, each of every seventh of the lane's blocks
+      constexpr int NP = 7;
+      T acc[NP][3];
+#pragma unroll
+      for (int m = 0; m < NP; ++m) acc[m][0] = acc[m][1] = acc[m][2] = T(0);
+      const int most = __reduce_max_sync(0xffffffffu, len);
+      for (int base = par; base < most; base += LN * NP) {
+        T xv[NP][3];
+#pragma unroll
+        for (int m = 0; m < NP; ++m) {
+          const int q = base + LN * m;
+          const bool in = q < len;
+          const long long c = in ? (C16 ? row + (int)cs16[q] : cs[q]) : 0;
+#pragma unroll
+          for (int j = 0; j < 3; ++j) xv[m][j] = in ? x[c * 3 + j] : T(0);
+        }
+#pragma unroll
+        for (int m = 0; m < NP; ++m) {
+          const int q = base + LN * m;
+          if (q < len) {
+            const T* B = vs + q * 9;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+              for (int j = 0; j < 3; ++j) acc[m][i] += B[i * 3 + j] * xv[m][j];
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0 && t + (int)gridDim.x < ntiles) {
+        const int tn = t + gridDim.x, tf = tn + gridDim.x;
+        pipe_issue<T, BS, C16>(st, lay, bar, tn, nbrow, n0, n1, rowptr, col, col16, val);
+        n0 = tf < ntiles ? rowptr[tf * R] : 0;
+        n1 = tf < ntiles ? rowptr[min(tf * R + R, nbrow)] : 0;
+      }
+      T v[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        v[i] = ((acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i])) + ((acc[4][i] + acc[5][i]) + acc[6][i]);
+#pragma unroll
+        for (int o = 16; o >= R; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+      }
+      if (own) {
+        if (MODE == 0) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i) y[at + i] = v[i];
+        } else if (MODE == 1) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i) y[at + i] = bi[i] - v[i];
+        } else {
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            T w = T(0);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) w += D[i * 3 + j] * (MODE == 5 ? bi[j] - v[j] : v[j]);
+            if (MODE == 2) {
+              y[at + i] = yi[i] - w;
+              xo[at + i] = oi[i] + xi[i];
+            } else if (MODE == 5) {
+              y[at + i] = w;
+              xo[at + i] = c1 * w;
+            } else {
+              const T upd = c2 * xi[i] + c1 * (yi[i] - w);
+              xo[at + i] = MODE == 3 ? upd : oi[i] + upd;
+            }
+          }
+        }
+      }
+    } else {
+      const int hl = lane & 15;
+      bool waited = false;
+#pragma unroll 1
+      for (int r2 = 0; r2 < R / 2; ++r2) {
+        const int rl = 2 * r2 + (lane >> 4);
+        const int row = t * R + rl;
+        const bool ok = row < nbrow, own = ok && hl < BS;
+        const long long at = (long long)row * BS + hl;
+        T bi = T(0), yi = T(0), xi = T(0), oi = T(0), D[BS];
+#pragma unroll
+        for (int j = 0; j < BS; ++j) D[j] = T(0);
+        if (own) {
+          if (MODE == 1 || MODE == 5) bi = b[at];
+          if (MODE == 2 || MODE == 3 || MODE == 4) { yi = y[at]; xi = x[at]; }
+          if (MODE == 2 || MODE == 4) oi = xo[at];
+          if (MODE >= 2) {
+#pragma unroll
+            for (int j = 0; j < BS; ++j) D[j] = dinv[(long long)row * BB + hl * BS + j];
+          }
+        }
+        if (!waited) {
+          waited = __all_sync(0xffffffffu, pipe_bar_wait(bar, phase));
+          if (!waited) break;
+        }
+        const int* rp = reinterpret_cast<const int*>(st + lay.rows);
+        const int s0 = rp[0];
+        const int b0 = ok ? rp[rl] - s0 : 0, b1 = ok ? rp[rl + 1] - s0 : 0;
+        const T* vs = reinterpret_cast<const T*>(st);
+        const int* cs = reinterpret_cast<const int*>(st + lay.cols + (((long long)s0 * 4) & 15));
+        T xv[2][BS];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int q = b0 + hl + 16 * h;
+          const bool in = q < b1;
+          const long long c = in ? cs[q] : 0;
+#pragma unroll
+          for (int j = 0; j < BS; ++j) xv[h][j] = in ? x[c * BS + j] : T(0);
+        }
+        T acc[BS];
+#pragma unroll
+        for (int i = 0; i < BS; ++i) acc[i] = T(0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int q = b0 + hl + 16 * h;
+          if (q < b1) {
+            using V = typename std::conditional<std::is_same<T, float>::value, float4, double2>::type;
+            constexpr int PER = 16 / (int)sizeof(T);
+            const V* B4 = reinterpret_cast<const V*>(vs + (long long)q * BB);
+            T bv[BB];
+#pragma unroll
+            for (int m = 0; m < BB / PER; ++m) {
+              const V u = B4[m];
+              const T* ut = reinterpret_cast<const T*>(&u);
+#pragma unroll
+              for (int j = 0; j < PER; ++j) bv[m * PER + j] = ut[j];
+            }
+#pragma unroll
+            for (int i = 0; i < BS; ++i)
+#pragma unroll
+              for (int j = 0; j < BS; ++j) acc[i] += bv[i * BS + j] * xv[h][j];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < BS; ++i) {
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        }
+        T v = acc[0];
+#pragma unroll
+        for (int i = 1; i < BS; ++i)
+          if (hl == i) v = acc[i];
+        T w = T(0);
+        if (MODE >= 2) {
+          const T e = MODE == 5 ? bi - v : v;
+#pragma unroll
+          for (int j = 0; j < BS; ++j) w += D[j] * __shfl_sync(0xffffffffu, e, (lane & 16) + j);
+        }
+        if (!own) continue;
+        if (MODE == 0) {
+          y[at] = v;
+        } else if (MODE == 1) {
+          y[at] = bi - v;
+        } else if (MODE == 2) {
+          y[at] = yi - w;
+          xo[at] = oi + xi;
+        } else if (MODE == 5) {
+          y[at] = w;
+          xo[at] = c1 * w;
+        } else {
+          const T upd = c2 * xi + c1 * (yi - w);
+          xo[at] = MODE == 3 ? upd : oi + upd;
+        }
+      }
+      if (!waited) {
+        if (lane == 0) atomicExch(err, 1);
+        return;
+      }
+      __syncwarp();
+      if (lane == 0 && t + (int)gridDim.x < ntiles) {
+        const int tn = t + gridDim.x, tf = tn + gridDim.x;
+        pipe_issue<T, BS, C16>(st, lay, bar, tn, nbrow, n0, n1, rowptr, col, col16, val);
+        n0 = tf < ntiles ? rowptr[tf * R] : 0;
+        n1 = tf < ntiles ? rowptr[min(tf * R + R, nbrow)] : 0;
+      }
+    }
+  }
+}
+
+}  // namespace pfem
