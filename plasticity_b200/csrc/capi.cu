@@ -476,21 +476,16 @@ void mgs_qr(int m, std::vector<double>& A, double R[36]) {
 // of the Galerkin operator P^T A P of every level.  Level 0 uses the
 // tangent's block pattern in place (its rowptr/col stay empty).
 // The hierarchy stops at the first level with at most this many unknowns; that
-// level is inverted densely (dense.cu on the device, or on the host when small)
+// level is inverted densely (dense.cu; with partial pivoting when small, where partly
+// constrained aggregates leave coarse rows that are nearly dependent)
 // and applied as one dense matrix-vector product per cycle.  The inverse costs
 // n^3 at every rebuild: at 64^3 a 3,072-unknown dense level 2 saves a W-cycle's
 // two visits to it (about 100 us per cycle) but adds about 11 ms per rebuild,
 // so by default the hierarchy goes one level further there (162 unknowns).
 // PFEM_COARSE_DENSE_MAX overrides the bound.
 constexpr long long kCoarseDenseMax = 1500;
-// Coarsest levels up to this size are inverted on the host with partial pivoting
-// (n^3 <= 2.7e7 multiply-adds: 1.3 ms at 162 unknowns, but 16 ms at 384); larger
-// ones on the device without row exchanges (about 1.4 ms at 384), which the
-// coarse operators of all but the smallest meshes (full aggregates, every rigid
-// mode present) do not need.
 // The adaptive AMG policy charges a rebuild this many Krylov iterations.
 constexpr double kRebuildCostIters = 12.0;
-constexpr int kCoarseHostMax = 300;
 
 void build_amg_structure(pfem_ctx* c) {
   long long dense_max = kCoarseDenseMax;
@@ -748,47 +743,6 @@ int krylov_alloc(pfem_ctx* ctx) {
   return PFEM_OK;
 }
 
-// Gauss-Jordan inverse of a dense n x n matrix (row-major, double) with
-// partial pivoting; near-singular pivots are regularised.  Used for small
-// coarsest levels (at most kCoarseHostMax unknowns), where a pivot-free
-// elimination can meet tiny pivots: partially constrained aggregates leave
-// coarse rows that are nearly dependent.
-void dense_inverse_host(int n, std::vector<double>& a, std::vector<double>& inv) {
-  // In-place Gauss-Jordan with partial pivoting (n^3 multiply-adds): column c of the
-  // identity is never stored, the pivot row's slot c takes 1 / pivot, and the row
-  // exchanges are undone on the columns at the end.
-  double scl = 0;
-  for (int i = 0; i < n; ++i) scl = std::max(scl, std::fabs(a[(size_t)i * n + i]));
-  std::vector<int> perm(n);
-  for (int c = 0; c < n; ++c) {
-    int piv = c;
-    double best = std::fabs(a[(size_t)c * n + c]);
-    for (int r = c + 1; r < n; ++r)
-      if (std::fabs(a[(size_t)r * n + c]) > best) { best = std::fabs(a[(size_t)r * n + c]); piv = r; }
-    perm[c] = piv;
-    if (piv != c)
-      for (int j = 0; j < n; ++j) std::swap(a[(size_t)c * n + j], a[(size_t)piv * n + j]);
-    double* rc = a.data() + (size_t)c * n;
-    double pv = rc[c];
-    if (std::fabs(pv) < 1e-14 * std::max(scl, 1e-300)) pv = (pv >= 0 ? 1.0 : -1.0) * 1e-14 * std::max(scl, 1e-300);
-    const double ip = 1.0 / pv;
-    rc[c] = 1.0;
-    for (int j = 0; j < n; ++j) rc[j] *= ip;
-    for (int r = 0; r < n; ++r) {
-      if (r == c) continue;
-      double* rr = a.data() + (size_t)r * n;
-      const double f = rr[c];
-      if (f == 0.0) continue;
-      rr[c] = 0.0;
-      for (int j = 0; j < n; ++j) rr[j] -= f * rc[j];
-    }
-  }
-  for (int c = n - 1; c >= 0; --c)
-    if (perm[c] != c)
-      for (int i = 0; i < n; ++i) std::swap(a[(size_t)i * n + c], a[(size_t)i * n + perm[c]]);
-  inv.swap(a);
-}
-
 // Numeric AMG set-up on the current (Dirichlet-imposed) tangent of precision T:
 // block-Jacobi inverses, Chebyshev bounds by power iteration, Galerkin
 // coarse operators, dense coarse inverse -- all on the device.  Rebuilt per load step by default
@@ -838,35 +792,14 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
   }
   if (dbg) cudaStreamSynchronize(ctx->st);
   auto tl = std::chrono::steady_clock::now();
-  // coarsest operator: dense inverse, on the device (blocked Gauss-Jordan) for
-  // large coarsest levels, on the host with partial pivoting for small ones
-  if (A.coarse_n > kCoarseHostMax) {
+  // coarsest operator: dense inverse
+  if (A.coarse_n > pfem::kPivotMax) {
     pfem::dense_coarse_inverse<T>(ctx->hl[L].nbrow, A.coarse_rp, A.coarse_cl, A.coarse_val, A.coarse_n,
                                   ctx->dDenseWork, A.coarse_inv, ctx->st);
     CKL();
   } else {
-    const HostLevel& hc = ctx->hl[L];
-    std::vector<T> hv((size_t)A.coarse_nnzb * 36);
-    CK(cudaMemcpyAsync(hv.data(), A.coarse_val, hv.size() * sizeof(T), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    const int n = A.coarse_n;
-    std::vector<double> dense((size_t)n * n, 0.0), inv;
-    for (int I = 0; I < hc.nbrow; ++I)
-      for (int k = hc.rowptr[I]; k < hc.rowptr[I + 1]; ++k) {
-        const int J = hc.col[k];
-        for (int r = 0; r < 6; ++r)
-          for (int c = 0; c < 6; ++c) dense[(size_t)(I * 6 + r) * n + J * 6 + c] = (double)hv[(size_t)k * 36 + r * 6 + c];
-      }
-    // rigid modes absent from an aggregate leave zero rows: put 1 on their diagonal
-    for (int i = 0; i < n; ++i) {
-      bool zero = true;
-      for (int j = 0; j < n && zero; ++j) zero = dense[(size_t)i * n + j] == 0.0;
-      if (zero) dense[(size_t)i * n + i] = 1.0;
-    }
-    dense_inverse_host(n, dense, inv);
-    std::vector<T> invT(inv.begin(), inv.end());
-    CK(cudaMemcpyAsync(A.coarse_inv, invT.data(), invT.size() * sizeof(T), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
+    CK(pfem::pivot_inverse<T>((int)A.coarse_nnzb, A.lv[L - 1].c_row, A.coarse_cl, A.coarse_val, A.coarse_n, A.coarse_inv,
+                              ctx->st));
   }
   A.built = true;
   A.version++;

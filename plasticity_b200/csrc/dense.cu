@@ -16,9 +16,9 @@
 // Every kernel reads only what the previous one finished writing, and A[K,K] is
 // read only by the diagonal kernel, so no CTA sees a block half replaced.
 // No row exchanges: the Galerkin operator of the (Dirichlet-imposed) tangent of a
-// large mesh is close to symmetric positive definite (small coarsest levels are
-// inverted on the host with partial pivoting instead); a pivot below 1e-14 of the
-// largest diagonal entry is replaced by that floor.
+// large mesh is close to symmetric positive definite; a pivot below 1e-14 of the
+// largest diagonal entry is replaced by that floor.  Coarsest levels of up to
+// kPivotMax unknowns take pivot_inverse_kernel, which chooses its pivots.
 #include <cstdint>
 
 #include "linalg.cuh"
@@ -212,6 +212,209 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(int n, int kb, double
   }
 }
 
+// Inverse with partial pivoting of up to kPivotMax unknowns, in one launch: a cluster
+// of eight CTAs holds the matrix in registers, CTA k a panel of columns, a warp up to
+// CPW of them, lane l the rows l, l + 32, ...
+//
+// In-place Gauss-Jordan: column c of the identity is never stored.  Rows are not
+// exchanged: step c takes the unused row with the largest |a[., c]| (the lowest such
+// row when equal) and remembers it, and the inverse is written through that
+// permutation.  A pivot row is not divided by its pivot until the end (its later
+// updates are linear in it), so an update is one fused multiply-add per entry, with a
+// multiplier of 0 in the pivot row.  What bounds it is the chain of n steps and their
+// instructions.  A pivot search needs one column only, so the CTA that owns a panel
+// runs the panel's steps by itself (one __syncthreads each), keeping the multipliers
+// of every step in shared memory; one cluster barrier later the other CTAs copy them
+// and apply the whole panel to their own columns without any barrier.  Measured at
+// 162 unknowns (the coarsest level at 8^3 and 64^3): 215 us; with a barrier of
+// the cluster per step 551 us, dividing at once and selecting the pivot row in every
+// update 286 us; the host's inverse with its two copies took 600-750 us.
+constexpr int PC = 8, PT = 512;  // CTAs of the cluster, threads of a CTA
+
+inline int pivot_cols(int n) { return (n + PC - 1) / PC; }
+inline size_t pivot_smem(int n) { return (size_t)2 * pivot_cols(n) * n * sizeof(double); }
+
+template <typename T, int RR, int CPW>
+__global__ void __cluster_dims__(PC, 1, 1) __launch_bounds__(PT)
+pivot_inverse_kernel(int cp, int nnzb, const int* __restrict__ br, const int* __restrict__ cl, const T* __restrict__ val,
+                     int n, T* __restrict__ inv) {
+  constexpr int NW = PT / 32, CMAX = NW * CPW;
+  extern __shared__ __align__(16) double pvm[];
+  __shared__ double ipv[2][CMAX];  // 1 / pivot of the own panel's steps, of a copied panel's
+  __shared__ int prow[2][CMAX];    // and their rows
+  __shared__ double wmax[NW];      // largest diagonal entry that a warp has seen
+  __shared__ double rowip[32 * RR];  // 1 / pivot of each row
+  __shared__ int perm[32 * RR], pos[32 * RR];
+  const int rank = (int)(blockIdx.x % PC), t = threadIdx.x, w = t >> 5, lane = t & 31;
+  double* const F = pvm;                   // multipliers of the own panel, [step][row]
+  double* const G = pvm + (size_t)cp * n;  // a copied panel's
+  const int j0 = rank * cp, ncol = max(0, min(cp, n - j0));
+  auto barrier = []() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  };
+  auto remote = [](const void* p, int cta) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
+    return r;
+  };
+  // ordered with the barriers (both volatile), free to be in flight together
+  auto get = [](uint32_t a) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+  };
+  // ---- own columns from the 6 x 6 blocks (br, cl: row and column of each), through
+  // shared memory; a row with no entry gets a unit diagonal ----
+  for (int e = t; e < ncol * n; e += PT) F[e] = 0.0;
+  for (int i = t; i < n; i += PT) pos[i] = 0;  // until the elimination: whether row i has an entry
+  __syncthreads();
+  double dm = 0.0;
+#pragma unroll 4
+  for (int e = t; e < nnzb * 36; e += PT) {
+    const int k = e / 36, rc = e - 36 * k, i = br[k] * 6 + rc / 6, j = cl[k] * 6 + rc % 6;
+    const double v = (double)val[e];
+    if (v != 0.0) pos[i] = 1;
+    if (j == i) dm = fmax(dm, fabs(v));
+    if (j >= j0 && j < j0 + ncol) F[(size_t)(j - j0) * n + i] = v;
+  }
+  __syncthreads();
+  for (int i = t; i < n; i += PT)
+    if (!pos[i]) {
+      dm = fmax(dm, 1.0);
+      if (i >= j0 && i < j0 + ncol) F[(size_t)(i - j0) * n + i] = 1.0;
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
+  if (lane == 0) wmax[w] = dm;
+  __syncthreads();
+  double a[CPW][RR];
+#pragma unroll
+  for (int m = 0; m < CPW; ++m)
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const int q = w + NW * m, i = lane + 32 * r;
+      a[m][r] = (q < ncol && i < n) ? F[(size_t)q * n + i] : 0.0;
+    }
+  double scl = 0.0;
+  for (int q = 0; q < NW; ++q) scl = fmax(scl, wmax[q]);
+  const double floor_abs = 1e-14 * fmax(scl, 1e-300);
+  unsigned used = 0;  // of this lane's rows, bit r
+  // Step with multipliers f, pivot row p, 1 / pivot ip on the warp's columns but `skip`.
+  auto apply = [&](const double* f, int p, double ip, int skip) {
+    const int pr = p >> 5, pl = p & 31;
+    double fr[RR], x[CPW];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) fr[r] = lane + 32 * r < n ? f[lane + 32 * r] : 0.0;
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if (r == pr) {  // the whole CTA takes the same branch
+#pragma unroll
+        for (int m = 0; m < CPW; ++m) x[m] = __shfl_sync(0xffffffffu, a[m][r], pl) * ip;
+      }
+#pragma unroll
+    for (int m = 0; m < CPW; ++m)
+      if (m != skip) {
+#pragma unroll
+        for (int r = 0; r < RR; ++r) a[m][r] = fma(-fr[r], x[m], a[m][r]);
+      }
+    if (lane == pl) used |= 1u << pr;
+  };
+  // The warp that holds step s's column (its m-th) searches it and publishes the step;
+  // the column becomes that of the inverse.
+  auto publish = [&](double (&v)[RR], int s) {
+    // the largest |v| as two 32-bit words (ordered like the number; a NaN is above
+    // all), then the lowest row that has it
+    unsigned hw[RR], hm = 0u, lm = 0u, im = 0xffffffffu;
+    bool on[RR];
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      on[r] = lane + 32 * r < n && !((used >> r) & 1u);
+      hw[r] = (unsigned)__double2hiint(v[r]) & 0x7fffffffu;
+      if (on[r]) hm = max(hm, hw[r]);
+    }
+    hm = __reduce_max_sync(0xffffffffu, hm);
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if (on[r] && hw[r] == hm) lm = max(lm, (unsigned)__double2loint(v[r]));
+    lm = __reduce_max_sync(0xffffffffu, lm);
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if (on[r] && hw[r] == hm && (unsigned)__double2loint(v[r]) == lm) im = min(im, (unsigned)(lane + 32 * r));
+    const int p = (int)__reduce_min_sync(0xffffffffu, im), pr = p >> 5, pl = p & 31;
+    double pv = 0.0;
+#pragma unroll
+    for (int r = 0; r < RR; ++r)
+      if (r == pr) pv = __shfl_sync(0xffffffffu, v[r], pl);
+    if (fabs(pv) < floor_abs) pv = (pv >= 0 ? 1.0 : -1.0) * floor_abs;
+    const double ip = 1.0 / pv;
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const bool here = r == pr && lane == pl;
+      const double f = here ? 0.0 : v[r];
+      if (lane + 32 * r < n) F[(size_t)s * n + lane + 32 * r] = f;
+      v[r] = here ? 1.0 : -f * ip;
+    }
+    if (lane == 0) {
+      ipv[0][s] = ip;
+      prow[0][s] = p;
+    }
+  };
+  __syncthreads();  // F and pos have been read
+  for (int k = 0; k < PC; ++k) {
+    const int steps = max(0, min(cp, n - k * cp));
+    if (k == rank) {
+      for (int s = 0; s < steps; ++s) {
+        int skip = -1;
+        if (w == s % NW) {
+          skip = s / NW;
+#pragma unroll
+          for (int m = 0; m < CPW; ++m)
+            if (m == skip) publish(a[m], s);
+        }
+        __syncthreads();
+        apply(F + (size_t)s * n, prow[0][s], ipv[0][s], skip);
+      }
+    }
+    barrier();  // the panel's steps are in its CTA's shared memory
+    if (k != rank) {
+      const uint32_t f = remote(F, k), ip = remote(ipv[0], k), pr = remote(prow[0], k);
+      for (int e0 = t; e0 < steps * n; e0 += 8 * PT) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (e0 + u * PT < steps * n) v[u] = get(f + 8u * (uint32_t)(e0 + u * PT));
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (e0 + u * PT < steps * n) G[e0 + u * PT] = v[u];
+      }
+      if (t < steps) {
+        ipv[1][t] = get(ip + 8u * (uint32_t)t);
+        int v;
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(pr + 4u * (uint32_t)t));
+        prow[1][t] = v;
+      }
+      __syncthreads();
+      for (int s = 0; s < steps; ++s) apply(G + (size_t)s * n, prow[1][s], ipv[1][s], -1);
+    }
+    if (t < steps) {
+      const int o = k == rank ? 0 : 1, p = prow[o][t];
+      perm[k * cp + t] = p;
+      pos[p] = k * cp + t;
+      rowip[p] = ipv[o][t];
+    }
+    __syncthreads();  // G and prow[1] may be overwritten
+  }
+#pragma unroll
+  for (int m = 0; m < CPW; ++m)
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const int q = w + NW * m, i = lane + 32 * r;
+      if (q < ncol && i < n) inv[(long long)pos[i] * n + perm[j0 + q]] = (T)(a[m][r] * rowip[i]);
+    }
+  barrier();  // no CTA leaves while another may read its shared memory
+}
+
 // out (n x n, stride n) = the leading n x n block of A (stride np), in precision T.
 template <typename T>
 __global__ void dense_out_kernel(int n, int np, const double* __restrict__ A, T* __restrict__ out) {
@@ -267,6 +470,27 @@ void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val,
   count_launch();
   dense_out_kernel<T><<<2048, 256, 0, st>>>(n, np, A, inv);
 }
+
+template <typename T, int RR, int CPW>
+static cudaError_t pivot_launch(int nnzb, const int* br, const int* cl, const T* val, int n, T* inv, cudaStream_t st) {
+  auto* kern = pivot_inverse_kernel<T, RR, CPW>;
+  const size_t sm = pivot_smem(n);
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  count_launch();
+  kern<<<PC, PT, sm, st>>>(pivot_cols(n), nnzb, br, cl, val, n, inv);
+  return cudaGetLastError();
+}
+// Six rows per lane and two columns per warp up to 192 unknowns, ten and three up to
+// kPivotMax.
+template <typename T>
+cudaError_t pivot_inverse(int nnzb, const int* br, const int* cl, const T* val, int n, T* inv, cudaStream_t st) {
+  static_assert(kPivotMax <= 32 * 10 && (kPivotMax + PC - 1) / PC <= 3 * (PT / 32), "rows and columns fit");
+  return n <= 192 ? pivot_launch<T, 6, 2>(nnzb, br, cl, val, n, inv, st)
+                  : pivot_launch<T, 10, 3>(nnzb, br, cl, val, n, inv, st);
+}
+template cudaError_t pivot_inverse<float>(int, const int*, const int*, const float*, int, float*, cudaStream_t);
+template cudaError_t pivot_inverse<double>(int, const int*, const int*, const double*, int, double*, cudaStream_t);
 
 template void dense_coarse_inverse<float>(int, const int*, const int*, const float*, int, double*, float*,
                                           cudaStream_t);
