@@ -48,13 +48,16 @@ struct KrylovWork {
 // (V-cycle, two dot products, the p / x / r updates, |r|) ending in a
 // one-thread kernel that sets the loop condition from the device-resident
 // residual.  One launch and one host synchronisation per linear solve.
-// Re-captured when the AMG hierarchy is rebuilt (its Chebyshev coefficients
-// are kernel arguments); the tolerance and iteration cap are read from ctl.
+// A set-up writes into the same device arrays, so the graph outlives it; it is
+// captured again when the smoother's degree changes (and, for other degrees than 2,
+// whose coefficients are kernel arguments, after every set-up).  The tolerance and
+// iteration cap are read from ctl.
 struct CgGraph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t body_stream = nullptr;
-  long long amg_version = -1;
+  int degree = -1;              // the captured smoother's degree, and for other degrees than
+  long long amg_version = -1;   // 2 the set-up
   double* ctl = nullptr;   // device: [0] rtol, [1] itmax, [2] absolute threshold (set on the device)
   int* state = nullptr;    // device (in ReadBack): [0] iterations, [1] converged
   long long prefix_kernels = 0, body_kernels = 0;
@@ -148,7 +151,7 @@ struct pfem_ctx {
   KrylovWork<double> kw64;
   CgGraph cg32, cg64;
   int tangent_prec = -1;  // precision of the last imposed tangent
-  cudaEvent_t e0 = nullptr, e1 = nullptr, t0 = nullptr, t1 = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr, t0 = nullptr, t1 = nullptr, a0 = nullptr, a1 = nullptr;
   // learned predictor
   pfem::MlpState mlp;
   int steps_taken = 0;
@@ -648,12 +651,6 @@ __global__ void hash_fill_kernel(long long n, float* xf, double* xd) {
   }
 }
 template <typename T>
-__global__ void scale_by_inv_kernel(long long n, const T* __restrict__ s, const T* __restrict__ w, T* __restrict__ v) {
-  const T inv = T(1) / *s;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    v[i] = w[i] * inv;
-}
-template <typename T>
 __global__ void bicg_finish_kernel(T* sc) {
   sc[2] = sc[0] / sc[4];
   sc[3] = sc[5] / sc[6];
@@ -691,6 +688,7 @@ int amg_alloc(pfem_ctx* ctx) {
       CK(dalloc(ctx, &v.A.val, (size_t)v.A.nnzb * h.bs * h.bs, kCopySlack));
     }
     CK(dalloc(ctx, &v.dinv, (size_t)h.nbrow * h.bs * h.bs));
+    CK(dalloc(ctx, &v.co, (size_t)CO_COUNT));
     v.nagg = h.nagg;
     CK(upload(ctx, &v.agg, h.agg));
     std::vector<T> Th(h.T.begin(), h.T.end());
@@ -743,10 +741,23 @@ int krylov_alloc(pfem_ctx* ctx) {
   return PFEM_OK;
 }
 
+// The levels' lmax on the host, for smoothing of another degree than 2 (whose
+// coefficients are kernel arguments); waits for the set-up the first time after it.
+template <typename T>
+int host_lmax(pfem_ctx* ctx) {
+  Amg<T>& A = amg_of<T>(ctx);
+  if (A.lmax_version == A.version) return PFEM_OK;
+  for (AmgLevel<T>& v : A.lv)
+    CK(cudaMemcpyAsync(&v.lmax, v.co + CO_LMAX, sizeof(T), cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  A.lmax_version = A.version;
+  return PFEM_OK;
+}
+
 // Numeric AMG set-up on the current (Dirichlet-imposed) tangent of precision T:
 // block-Jacobi inverses, Chebyshev bounds by power iteration, Galerkin
-// coarse operators, dense coarse inverse -- all on the device.  Rebuilt per load step by default
-// (the reference's reuse policy, Solver.jl:243-245).
+// coarse operators, dense coarse inverse -- all on the device, without a wait: the
+// scalars that one kernel finds and the next ones need stay there (AmgLevel::co).
 template <typename T>
 int amg_setup(pfem_ctx* ctx, int cheb_degree) {
   const bool dbg = getenv("PFEM_DEBUG_AMG") != nullptr;
@@ -757,7 +768,6 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
   rc = krylov_alloc<T>(ctx);
   if (rc) return rc;
   Amg<T>& A = amg_of<T>(ctx);
-  KrylovWork<T>& w = kw_of<T>(ctx);
   A.cheb_degree = cheb_degree;
   A.lv[0].A.val = K_of<T>(ctx);
   const int L = (int)A.lv.size();
@@ -765,33 +775,31 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
     AmgLevel<T>& v = A.lv[l];
     blockdiag_invert<T>(v.A, v.dinv, ctx->st);
     CKL();
-    // power iteration on D^-1 A
+    // Power iteration on D^-1 A, 12 steps, each one pass over the matrix; the iterate is
+    // rescaled every second step only (a spectral radius of 1e18 still fits single
+    // precision), and the estimate is the ratio of the last two norms.
     const long long n = (long long)v.A.nbrow * v.A.bs;
     pfem::count_launch(); hash_fill_kernel<<<256, 256, 0, ctx->st>>>(n, std::is_same<T, float>::value ? (float*)v.d : nullptr,
                                                std::is_same<T, double>::value ? (double*)v.d : nullptr);
-    for (int it = 0; it < 12; ++it) {
-      bsr_spmv<T>(v.A, v.d, v.t, ctx->st);
-      blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, v.t, v.r, T(1), nullptr, ctx->st);
-      dot<T>(n, v.r, v.r, w.sc + 8, w.part, ctx->st, true);
-      pfem::count_launch(); scale_by_inv_kernel<T><<<256, 256, 0, ctx->st>>>(n, w.sc + 8, v.r, v.d);
+    for (int it = 1; it <= 12; ++it) {
+      const T* from = it % 2 ? v.d : v.r;
+      T* to = it % 2 ? v.r : v.d;
+      bsr_power_step<T>(v.A, v.dinv, from, to, ctx->st);
+      if (it % 2 == 0 && it < 12) {
+        const int np = norm2_partials<T>(n, to, ctx->dPart, ctx->st);
+        scale_by_norm<T>(n, ctx->dPart, np, to, ctx->st);
+      }
     }
+    const int np = norm2_partials<T>(n, v.r, ctx->dPart, ctx->st);
+    norm2_partials<T>(n, v.d, ctx->dPart + 1024, ctx->st);
+    power_finish<T>(np, ctx->dPart, ctx->dPart + 1024, v.co, ctx->st);
     CKL();
-    T lm = 0;
-    CK(cudaMemcpyAsync(&lm, w.sc + 8, sizeof(T), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    v.lmax = (T)(1.1 * (double)lm);
-    if (getenv("PFEM_DEBUG_AMG"))
-      fprintf(stderr, "amg level %d: block rows %d bs %d nnzb %lld aggregates %d P blocks %d lmax %.4g\n", l,
-              v.A.nbrow, v.A.bs, v.A.nnzb, v.nagg, v.nnzP, (double)v.lmax);
     // smoothed prolongator and Galerkin operator of the next level
-    const T omega = (T)(4.0 / (3.0 * (double)lm));
     T* cval = (l + 1 < L) ? A.lv[l + 1].A.val : A.coarse_val;
     const int nnzC = (int)ctx->hl[l + 1].rowptr[ctx->hl[l + 1].nbrow];
-    sa_setup_level<T>(v, omega, cval, nnzC, ctx->st);
+    sa_setup_level<T>(v, cval, nnzC, ctx->st);
     CKL();
   }
-  if (dbg) cudaStreamSynchronize(ctx->st);
-  auto tl = std::chrono::steady_clock::now();
   // coarsest operator: dense inverse
   if (A.coarse_n > pfem::kPivotMax) {
     pfem::dense_coarse_inverse<T>(ctx->hl[L].nbrow, A.coarse_rp, A.coarse_cl, A.coarse_val, A.coarse_n,
@@ -803,13 +811,20 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
   }
   A.built = true;
   A.version++;
+  if (cheb_degree != 2) {
+    rc = host_lmax<T>(ctx);
+    if (rc) return rc;
+  }
   if (dbg) {
-    cudaStreamSynchronize(ctx->st);
-    auto te = std::chrono::steady_clock::now();
-    fprintf(stderr, "amg set-up %.3f ms: levels %.3f ms, coarse inverse (%d unknowns) %.3f ms\n",
-            std::chrono::duration<double, std::milli>(te - ts).count(),
-            std::chrono::duration<double, std::milli>(tl - ts).count(), A.coarse_n,
-            std::chrono::duration<double, std::milli>(te - tl).count());
+    rc = host_lmax<T>(ctx);
+    if (rc) return rc;
+    for (int l = 0; l < L; ++l) {
+      const AmgLevel<T>& v = A.lv[l];
+      fprintf(stderr, "amg level %d: block rows %d bs %d nnzb %lld aggregates %d P blocks %d lmax %.4g\n", l,
+              v.A.nbrow, v.A.bs, v.A.nnzb, v.nagg, v.nnzP, (double)v.lmax);
+    }
+    fprintf(stderr, "amg set-up %.3f ms (coarse inverse of %d unknowns)\n",
+            std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - ts).count(), A.coarse_n);
   }
   return PFEM_OK;
 }
@@ -817,41 +832,29 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
 // Chebyshev smoothing (block-Jacobi preconditioned) on level l:
 // x <- x + p(D^-1 A) D^-1 (b - A x), degree A.cheb_degree, interval
 // [lmax/30, lmax].  zero: x enters as 0.
-// Degree-2 coefficients on [lmax/30, lmax]: x2 = x0 + d0 + d1 with d0 = r0 / th,
-// r0 = Dinv (b - A x0), r1 = r0 - Dinv A d0, d1 = c1 r1 + (c2 - 1) d0.
-template <typename T>
-void cheb2_coeffs(const AmgLevel<T>& v, T* inv_th, T* c1, T* c2) {
-  const double lmx = (double)v.lmax, lmn = lmx / 30.0;
-  const double th = 0.5 * (lmx + lmn), de = 0.5 * (lmx - lmn);
-  const double sg = th / de, rho = 1.0 / sg;
-  const double rn = 1.0 / (2.0 * sg - rho);
-  *inv_th = T(1.0 / th);
-  *c1 = T(2.0 * rn / de);
-  *c2 = T(1.0 + rn * rho);
-}
-
+// Degree 2: x2 = x0 + d0 + d1 with d0 = r0 / th, r0 = Dinv (b - A x0), r1 = r0 - Dinv A d0,
+// d1 = c1 r1 + (c2 - 1) d0; the set-up leaves 1 / th, c1 and c2 in v.co.
 template <typename T>
 void cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero) {
   const long long n = (long long)v.A.nbrow * v.A.bs;
+  const T* const ith = v.co + CO_ITH;
+  if (degree == 2) {
+    // one block-Jacobi pass (or a fused residual pass) and one fused SpMV pass
+    if (zero) blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, ith, v.d, ctx->st);
+    else bsr_residual_precond<T>(v.A, v.dinv, x, b, v.r, v.d, v.co, ctx->st);
+    bsr_cheb2<T>(v.A, v.dinv, v.d, v.r, x, zero, v.co, ctx->st);
+    return;
+  }
   const double lmx = (double)v.lmax, lmn = lmx / 30.0;
   const double th = 0.5 * (lmx + lmn), de = 0.5 * (lmx - lmn);
   const double sg = th / de;
   double rho = 1.0 / sg;
-  if (degree == 2) {
-    // one block-Jacobi pass (or a fused residual pass) and one fused SpMV pass
-    T inv_th, c1, c2;
-    cheb2_coeffs<T>(v, &inv_th, &c1, &c2);
-    if (zero) blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, inv_th, v.d, ctx->st);
-    else bsr_residual_precond<T>(v.A, v.dinv, x, b, v.r, v.d, inv_th, ctx->st);
-    bsr_cheb2<T>(v.A, v.dinv, v.d, v.r, x, zero, c1, c2, ctx->st);
-    return;
-  }
   if (zero) {
     fill<T>(n, x, T(0), ctx->st);
-    blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, T(1.0 / th), v.d, ctx->st);
+    blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, ith, v.d, ctx->st);
   } else {
     bsr_residual<T>(v.A, x, b, v.t, ctx->st);
-    blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, v.t, v.r, T(1.0 / th), v.d, ctx->st);
+    blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, v.t, v.r, ith, v.d, ctx->st);
   }
   for (int k = 1; k <= degree; ++k) {
     if (k < degree) {
@@ -937,7 +940,8 @@ template <typename T>
 int cg_graph_build(pfem_ctx* ctx) {
   CgGraph& G = cg_of<T>(ctx);
   Amg<T>& A = amg_of<T>(ctx);
-  if (G.exec && G.amg_version == A.version) return PFEM_OK;
+  const long long version = A.cheb_degree == 2 ? 0 : A.version;
+  if (G.exec && G.degree == A.cheb_degree && G.amg_version == version) return PFEM_OK;
   if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
   if (G.graph) { cudaGraphDestroy(G.graph); G.graph = nullptr; }
   if (!G.ctl) {
@@ -1027,7 +1031,8 @@ int cg_graph_build(pfem_ctx* ctx) {
   G.prefix_kernels = c1 - c0 + 1;
   G.body_kernels = c2 - c1 + 1;
   pfem::launch_counter() = c0;
-  G.amg_version = A.version;
+  G.degree = A.cheb_degree;
+  G.amg_version = version;
   return PFEM_OK;
 }
 
@@ -1304,27 +1309,21 @@ int newton_correction(pfem_ctx* ctx, const pfem_solve_opts* o, double rtol, bool
   const int prec = o->precision;
   int rc;
   auto t0 = std::chrono::steady_clock::now();
-  if (prec == PFEM_FP64) {
-    if (rebuild || !ctx->amg64.built) {
-      rc = amg_setup<double>(ctx, o->cheb_degree);
-      if (rc) return rc;
-    } else {
-      // reused hierarchy: the level-0 operator is the current tangent; the
-      // smoother keeps the block-Jacobi inverse its Chebyshev interval was
-      // estimated with (a fresh inverse under the old interval can diverge)
-      ctx->amg64.lv[0].A.val = ctx->dK64;
-    }
+  const bool setup = rebuild || !(prec == PFEM_FP64 ? ctx->amg64.built : ctx->amg32.built);
+  if (setup) {
+    CK(cudaEventRecord(ctx->a0, ctx->st));
+    rc = prec == PFEM_FP64 ? amg_setup<double>(ctx, o->cheb_degree) : amg_setup<float>(ctx, o->cheb_degree);
+    if (rc) return rc;
+    CK(cudaEventRecord(ctx->a1, ctx->st));
+  } else if (prec == PFEM_FP64) {
+    // reused hierarchy: the level-0 operator is the current tangent; the
+    // smoother keeps the block-Jacobi inverse its Chebyshev interval was
+    // estimated with (a fresh inverse under the old interval can diverge)
+    ctx->amg64.lv[0].A.val = ctx->dK64;
   } else {
-    if (rebuild || !ctx->amg32.built) {
-      rc = amg_setup<float>(ctx, o->cheb_degree);
-      if (rc) return rc;
-    } else {
-      ctx->amg32.lv[0].A.val = ctx->dK32;
-    }
+    ctx->amg32.lv[0].A.val = ctx->dK32;
   }
-  CK(cudaStreamSynchronize(ctx->st));
   auto t1 = std::chrono::steady_clock::now();
-  *t_amg += std::chrono::duration<double, std::milli>(t1 - t0).count();
   bool conv = false;
   if (prec == PFEM_FP64) {
     convert<double, double>(ctx->ndof, ctx->dR, ctx->kw64.b, -1.0, ctx->st);
@@ -1335,9 +1334,17 @@ int newton_correction(pfem_ctx* ctx, const pfem_solve_opts* o, double rtol, bool
   }
   if (rc) return rc;
   CKL();
-  CK(cudaStreamSynchronize(ctx->st));
+  // the solve has waited for the set-up, which ran ahead of the host: its time is its
+  // host part (structure, first allocations) or its device part, the longer
   auto t2 = std::chrono::steady_clock::now();
-  *t_kry += std::chrono::duration<double, std::milli>(t2 - t1).count();
+  double amg_ms = 0.0;
+  if (setup) {
+    float dev_ms = 0;
+    cudaEventElapsedTime(&dev_ms, ctx->a0, ctx->a1);
+    amg_ms = std::max((double)dev_ms, std::chrono::duration<double, std::milli>(t1 - t0).count());
+  }
+  *t_amg += amg_ms;
+  *t_kry += std::max(0.0, std::chrono::duration<double, std::milli>(t2 - t0).count() - amg_ms);
   // an inexact inner solve is still a descent step; Newton judges it
   if (converged) *converged = conv;
   return PFEM_OK;
@@ -1524,6 +1531,10 @@ static int smooth_prediction(pfem_ctx* ctx, double lam, int degree) {
   if (!A.built || degree <= 0) return PFEM_OK;
   KrylovWork<T>& w = kw_of<T>(ctx);
   AmgLevel<T>& v = A.lv[0];
+  if (degree != 2) {
+    const int rc = host_lmax<T>(ctx);
+    if (rc) return rc;
+  }
   v.A.val = K_of<T>(ctx);
   blockdiag_invert<T>(v.A, v.dinv, ctx->st);
   convert<double, T>(ctx->ndof, ctx->dR, w.b, -1.0, ctx->st);
@@ -1732,6 +1743,8 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
     cudaEventCreate(&ctx->e1);
     cudaEventCreate(&ctx->t0);
     cudaEventCreate(&ctx->t1);
+    cudaEventCreate(&ctx->a0);
+    cudaEventCreate(&ctx->a1);
   }
   if ((long long)ctx->ndof >= (1ll << 31)) return bail(fail(ctx, PFEM_ERR_BAD_ARG, "mesh too large for 32-bit dof indices"));
   // ---- host topology ----
@@ -1936,6 +1949,8 @@ void pfem_destroy(pfem_ctx* ctx) {
   if (ctx->e1) cudaEventDestroy(ctx->e1);
   if (ctx->t0) cudaEventDestroy(ctx->t0);
   if (ctx->t1) cudaEventDestroy(ctx->t1);
+  if (ctx->a0) cudaEventDestroy(ctx->a0);
+  if (ctx->a1) cudaEventDestroy(ctx->a1);
   if (ctx->st) cudaStreamDestroy(ctx->st);
   delete ctx;
 }

@@ -19,7 +19,9 @@ namespace pfem {
 //   2: r -= Dinv (A x); xo += x             (Chebyshev step on x = d)
 //   3: xo = c2 x + c1 (y - Dinv A x)        (fused degree-2 Chebyshev, x = d0, y = r0)
 //   4: as 3, added to xo
-//   5: y = Dinv (b - A x), xo = c1 y        (preconditioned residual + first direction)
+//   5: y = Dinv (b - A x), xo = y / th      (preconditioned residual + first direction)
+//   6: y = Dinv A x                         (a step of the power iteration)
+// with 1 / th, c1 and c2 from the level's scalars co.
 template <typename T, int BS, int MODE, bool VEC = false, int LANES = 16, bool C16 = false>
 __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __restrict__ rowptr,
                                                        const int* __restrict__ col,
@@ -28,7 +30,7 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
                                                        const T* __restrict__ x, T* __restrict__ y,
                                                        const T* __restrict__ b,
                                                        const T* __restrict__ dinv, T* __restrict__ xo,
-                                                       T c1, T c2) {
+                                                       const T* __restrict__ co) {
   // LANES lanes per block row: half a warp for 3 x 3 blocks (a level-0 row has at
   // most 27 blocks: two per lane), a warp for 6 x 6 blocks (one 144-byte block
   // per lane); values and column ids are read once, through the streaming
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
 #pragma unroll
       for (int j = 0; j < BS; ++j) t += D[lane * BS + j] * (b[base + j] - acc[j]);
       y[base + lane] = t;
-      xo[base + lane] = c1 * t;
+      xo[base + lane] = co[CO_ITH] * t;
       return;
     }
     T v = acc[0];
@@ -104,13 +106,15 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
       T t = T(0);
 #pragma unroll
       for (int j = 0; j < BS; ++j) t += D[lane * BS + j] * acc[j];
-      if (MODE == 2) {
+      if (MODE == 6) {
+        y[base + lane] = t;
+      } else if (MODE == 2) {
         y[base + lane] -= t;
         xo[base + lane] += x[base + lane];
       } else {
         // degree-2 Chebyshev in one pass: r1 = r0 - Dinv A d0,
         // x2 = x0 + c2 d0 + c1 r1 (c2 = 1 + rn rho, c1 = 2 rn / delta)
-        const T upd = c2 * x[base + lane] + c1 * (y[base + lane] - t);
+        const T upd = co[CO_C2] * x[base + lane] + co[CO_C1] * (y[base + lane] - t);
         if (MODE == 3) xo[base + lane] = upd;
         else xo[base + lane] += upd;
       }
@@ -119,7 +123,7 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
 }
 
 template <typename T, int BS, int MODE, bool C16>
-static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, T c1, T c2,
+static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, const T* co,
                           cudaStream_t st) {
   auto* kern = bsr_spmv_pipe_kernel<T, BS, MODE, C16>;
   const int sm = pipe_smem_bytes<T, BS>(A.max_row, C16);
@@ -132,7 +136,7 @@ static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, cons
   const int tiles = (A.nbrow + R - 1) / R;
   const int grid = std::min(tiles, sms * std::max(per, 1));
   pfem::count_launch();
-  kern<<<grid, 32, sm, st>>>(A.nbrow, tiles, A.max_row, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, c1, c2,
+  kern<<<grid, 32, sm, st>>>(A.nbrow, tiles, A.max_row, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, co,
                              A.err);
 }
 // The streamed kernel takes a matrix whose rows have at most 32 blocks and whose
@@ -143,22 +147,22 @@ static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, cons
 // streamed: 152 / 146 us at 48^3 (4,913 rows of 6 x 6), 647 / 603 at 80^3 (19,683).
 constexpr int kPipeRows3 = 8192, kPipeRows6 = 4096;
 template <typename T, int MODE>
-static bool spmv_pipe_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, T c1, T c2,
+static bool spmv_pipe_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, const T* co,
                              cudaStream_t st) {
   const bool c16 = A.bs == 3 && A.col16;
   const uintptr_t at = reinterpret_cast<uintptr_t>(A.val) | reinterpret_cast<uintptr_t>(A.rowptr) |
                        (c16 ? reinterpret_cast<uintptr_t>(A.col16) : reinterpret_cast<uintptr_t>(A.col));
   if (A.nbrow < (A.bs == 3 ? kPipeRows3 : kPipeRows6) || A.max_row < 1 || A.max_row > 32 || !A.err || (at & 15)) return false;
-  if (c16) pipe_launch_t<T, 3, MODE, true>(A, x, y, b, dinv, xo, c1, c2, st);
-  else if (A.bs == 3) pipe_launch_t<T, 3, MODE, false>(A, x, y, b, dinv, xo, c1, c2, st);
-  else pipe_launch_t<T, 6, MODE, false>(A, x, y, b, dinv, xo, c1, c2, st);
+  if (c16) pipe_launch_t<T, 3, MODE, true>(A, x, y, b, dinv, xo, co, st);
+  else if (A.bs == 3) pipe_launch_t<T, 3, MODE, false>(A, x, y, b, dinv, xo, co, st);
+  else pipe_launch_t<T, 6, MODE, false>(A, x, y, b, dinv, xo, co, st);
   return true;
 }
 
 template <typename T, int MODE>
-static void spmv_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, T c1, T c2,
+static void spmv_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, const T* co,
                         cudaStream_t st) {
-  if (spmv_pipe_launch<T, MODE>(A, x, y, b, dinv, xo, c1, c2, st)) return;
+  if (spmv_pipe_launch<T, MODE>(A, x, y, b, dinv, xo, co, st)) return;
   // 6 x 6 levels of fewer than kWarpRowsBelow rows fill too few warp slots with half
   // a warp per row: give each row a whole warp there (measured at 64^3: level 2,
   // 512 rows, 7.4 -> 6.5 us per pass; level 1, 10,648 rows, 14.3 -> 18.2 us)
@@ -173,48 +177,53 @@ static void spmv_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const 
   pfem::count_launch();
   if (A.bs == 3 && A.col16)
     bsr_spmv_kernel<T, 3, MODE, false, 16, true><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16,
-                                                                              A.val, x, y, b, dinv, xo, c1, c2);
+                                                                              A.val, x, y, b, dinv, xo, co);
   else if (A.bs == 3)
-    bsr_spmv_kernel<T, 3, MODE><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, c1, c2);
+    bsr_spmv_kernel<T, 3, MODE><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, co);
   else if (aligned && wide)
     bsr_spmv_kernel<T, 6, MODE, true, 32><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo,
-                                                                  c1, c2);
+                                                                  co);
   else if (aligned)
-    bsr_spmv_kernel<T, 6, MODE, true><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, c1,
-                                                              c2);
+    bsr_spmv_kernel<T, 6, MODE, true><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo,
+                                                              co);
   else
-    bsr_spmv_kernel<T, 6, MODE><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, c1, c2);
+    bsr_spmv_kernel<T, 6, MODE><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, co);
 }
 
 template <typename T>
 void bsr_spmv(const BsrMat<T>& A, const T* x, T* y, cudaStream_t st) {
-  spmv_launch<T, 0>(A, x, y, nullptr, nullptr, nullptr, T(0), T(0), st);
+  spmv_launch<T, 0>(A, x, y, nullptr, nullptr, nullptr, nullptr, st);
 }
 template <typename T>
 void bsr_residual(const BsrMat<T>& A, const T* x, const T* b, T* r, cudaStream_t st) {
-  spmv_launch<T, 1>(A, x, r, b, nullptr, nullptr, T(0), T(0), st);
+  spmv_launch<T, 1>(A, x, r, b, nullptr, nullptr, nullptr, st);
 }
 template <typename T>
 void bsr_cheb_step(const BsrMat<T>& A, const T* dinv, const T* d, T* r, T* x, cudaStream_t st) {
-  spmv_launch<T, 2>(A, d, r, nullptr, dinv, x, T(0), T(0), st);
+  spmv_launch<T, 2>(A, d, r, nullptr, dinv, x, nullptr, st);
 }
 template <typename T>
-void bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero, T c1, T c2,
+void bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero, const T* co,
                cudaStream_t st) {
-  if (zero) spmv_launch<T, 3>(A, d0, const_cast<T*>(r0), nullptr, dinv, x, c1, c2, st);
-  else spmv_launch<T, 4>(A, d0, const_cast<T*>(r0), nullptr, dinv, x, c1, c2, st);
+  if (zero) spmv_launch<T, 3>(A, d0, const_cast<T*>(r0), nullptr, dinv, x, co, st);
+  else spmv_launch<T, 4>(A, d0, const_cast<T*>(r0), nullptr, dinv, x, co, st);
 }
 template <typename T>
-void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r, T* d, T scale,
+void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r, T* d, const T* co,
                           cudaStream_t st) {
-  spmv_launch<T, 5>(A, x, r, b, dinv, d, scale, T(0), st);
+  spmv_launch<T, 5>(A, x, r, b, dinv, d, co, st);
+}
+template <typename T>
+void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, cudaStream_t st) {
+  spmv_launch<T, 6>(A, x, y, nullptr, dinv, nullptr, nullptr, st);
 }
 
 // ------------------------------------------------------------------ block diagonal
-// r = Dinv * v per block row (one thread per scalar row); optional scale.
+// r = Dinv * v per block row (one thread per scalar row), d = *scale r.
 template <typename T, int BS>
 __global__ void blockdiag_apply_kernel(int nbrow, const T* __restrict__ dinv, const T* __restrict__ v,
-                                       T* __restrict__ r, T scale, T* __restrict__ d) {
+                                       T* __restrict__ r, const T* __restrict__ scale,
+                                       T* __restrict__ d) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= (long long)nbrow * BS) return;
   const long long row = i / BS;
@@ -225,10 +234,10 @@ __global__ void blockdiag_apply_kernel(int nbrow, const T* __restrict__ dinv, co
 #pragma unroll
   for (int j = 0; j < BS; ++j) t += D[j] * vv[j];
   r[i] = t;
-  if (d) d[i] = scale * t;
+  d[i] = *scale * t;
 }
 template <typename T>
-void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, T scale, T* d, cudaStream_t st) {
+void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, const T* scale, T* d, cudaStream_t st) {
   const long long n = (long long)nbrow * bs;
   const int blocks = (int)((n + 255) / 256);
   if (bs == 3) { pfem::count_launch(); blockdiag_apply_kernel<T, 3><<<blocks, 256, 0, st>>>(nbrow, dinv, v, r, scale, d); }
@@ -433,6 +442,67 @@ __global__ void cg_xr_fused_kernel(long long n, const T* __restrict__ part_pq, i
   if (threadIdx.x == 0) part_rr[blockIdx.x] = acc;
   if (blockIdx.x == 0 && threadIdx.x == 0) sc[0] = sc[2];
 }
+// ---- power iteration: squared norms in double (an iterate may be as large as its type
+// allows), kNormBlocks partials at most ----
+constexpr int kNormBlocks = 1024;
+static int norm_blocks(long long n) {
+  return (int)std::min<long long>(std::max<long long>((n + RED_THREADS - 1) / RED_THREADS, 1), kNormBlocks);
+}
+template <typename T>
+__global__ void norm2_partials_kernel(long long n, const T* __restrict__ v, double* __restrict__ part) {
+  __shared__ double sh[32];
+  double s = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    s += (double)v[i] * (double)v[i];
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+template <typename T>
+int norm2_partials(long long n, const T* v, double* part, cudaStream_t st) {
+  const int blocks = norm_blocks(n);
+  pfem::count_launch();
+  norm2_partials_kernel<T><<<blocks, RED_THREADS, 0, st>>>(n, v, part);
+  return blocks;
+}
+// v /= sqrt(sum(part))
+template <typename T>
+__global__ void scale_by_norm_kernel(long long n, const double* __restrict__ part, int np, T* __restrict__ v) {
+  __shared__ double sh[33];
+  const double inv = 1.0 / sqrt(all_sum_partials(part, np, sh));
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    v[i] = (T)((double)v[i] * inv);
+}
+template <typename T>
+void scale_by_norm(long long n, const double* part, int np, T* v, cudaStream_t st) {
+  pfem::count_launch();
+  scale_by_norm_kernel<T><<<norm_blocks(n), RED_THREADS, 0, st>>>(n, part, np, v);
+}
+// A level's scalars from the last two iterates' squared norms (np partials each).
+template <typename T>
+__global__ void power_finish_kernel(int np, const double* __restrict__ prev, const double* __restrict__ last,
+                                    T* __restrict__ co) {
+  __shared__ double sh[33];
+  const double a = all_sum_partials(prev, np, sh);
+  __syncthreads();
+  const double b = all_sum_partials(last, np, sh);
+  if (threadIdx.x != 0) return;
+  const double lm = sqrt(b / a);
+  const T lmax = (T)(1.1 * lm);
+  const double lmx = (double)lmax, lmn = lmx / 30.0;
+  const double th = 0.5 * (lmx + lmn), de = 0.5 * (lmx - lmn);
+  const double sg = th / de, rho = 1.0 / sg;
+  const double rn = 1.0 / (2.0 * sg - rho);
+  co[CO_LMAX] = lmax;
+  co[CO_ITH] = T(1.0 / th);
+  co[CO_C1] = T(2.0 * rn / de);
+  co[CO_C2] = T(1.0 + rn * rho);
+  co[CO_OMEGA] = T(4.0 / (3.0 * lm));
+}
+template <typename T>
+void power_finish(int np, const double* prev, const double* last, T* co, cudaStream_t st) {
+  pfem::count_launch();
+  power_finish_kernel<T><<<1, 1024, 0, st>>>(np, prev, last, co);
+}
 template <typename T>
 int dot_partials(long long n, const T* a, const T* b, T* part, cudaStream_t st) {
   long long nb = (n + RED_THREADS - 1) / RED_THREADS;
@@ -636,7 +706,8 @@ __global__ void sa_prolongator_kernel(int nnzP, const int* __restrict__ p_row, c
                                       const int* __restrict__ rowptr, const int* __restrict__ col,
                                       const T* __restrict__ val, const int* __restrict__ pslot,
                                       const int* __restrict__ agg, const T* __restrict__ Tb,
-                                      const T* __restrict__ dinv, T w, T* __restrict__ pval) {
+                                      const T* __restrict__ dinv, const T* __restrict__ omega,
+                                      T* __restrict__ pval) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nnzP) return;
   const int n = p_row[p];
@@ -662,6 +733,7 @@ __global__ void sa_prolongator_kernel(int nnzP, const int* __restrict__ p_row, c
   const bool own = p_cl[p] == agg[n];
   const T* Tn = Tb + (long long)n * BS * 6;
   T* P = pval + (long long)p * BS * 6;
+  const T w = *omega;
 #pragma unroll
   for (int i = 0; i < BS; ++i)
 #pragma unroll
@@ -864,12 +936,12 @@ __global__ void sa_prolong_kernel(int nbrow, const int* __restrict__ p_rp, const
 }
 
 template <typename T>
-void sa_setup_level(const AmgLevel<T>& v, T w, T* cval, int nnzC, cudaStream_t st) {
+void sa_setup_level(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st) {
   const int BSs = v.A.bs;
   if (BSs == 3) {
     pfem::count_launch();
     sa_prolongator_kernel<T, 3><<<(v.nnzP + 127) / 128, 128, 0, st>>>(v.nnzP, v.p_row, v.p_cl, v.A.rowptr, v.A.col,
-                                                                     v.A.val, v.pslot, v.agg, v.T, v.dinv, w, v.p_val);
+                                                                     v.A.val, v.pslot, v.agg, v.T, v.dinv, v.co + CO_OMEGA, v.p_val);
     pfem::count_launch();
     sa_ap_kernel<T, 3><<<(v.nnzAP + 127) / 128, 128, 0, st>>>(v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
                                                              v.p_rp, v.p_cl, v.p_val, v.ap_val);
@@ -882,7 +954,7 @@ void sa_setup_level(const AmgLevel<T>& v, T w, T* cval, int nnzC, cudaStream_t s
   } else {
     pfem::count_launch();
     sa_prolongator_kernel<T, 6><<<(v.nnzP + 127) / 128, 128, 0, st>>>(v.nnzP, v.p_row, v.p_cl, v.A.rowptr, v.A.col,
-                                                                     v.A.val, v.pslot, v.agg, v.T, v.dinv, w, v.p_val);
+                                                                     v.A.val, v.pslot, v.agg, v.T, v.dinv, v.co + CO_OMEGA, v.p_val);
     pfem::count_launch();
     sa_ap_kernel<T, 6><<<(v.nnzAP + 127) / 128, 128, 0, st>>>(v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
                                                              v.p_rp, v.p_cl, v.p_val, v.ap_val);
@@ -938,10 +1010,14 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, cudaStre
   template void bsr_spmv<T>(const BsrMat<T>&, const T*, T*, cudaStream_t);                         \
   template void bsr_residual<T>(const BsrMat<T>&, const T*, const T*, T*, cudaStream_t);           \
   template void bsr_cheb_step<T>(const BsrMat<T>&, const T*, const T*, T*, T*, cudaStream_t);      \
-  template void bsr_cheb2<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, bool, T, T, cudaStream_t); \
-  template void bsr_residual_precond<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, T,    \
+  template void bsr_cheb2<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, bool, const T*, cudaStream_t); \
+  template void bsr_residual_precond<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, const T*, \
                                         cudaStream_t);                                             \
-  template void blockdiag_apply<T>(int, int, const T*, const T*, T*, T, T*, cudaStream_t);         \
+  template void bsr_power_step<T>(const BsrMat<T>&, const T*, const T*, T*, cudaStream_t);         \
+  template int norm2_partials<T>(long long, const T*, double*, cudaStream_t);                      \
+  template void scale_by_norm<T>(long long, const double*, int, T*, cudaStream_t);                 \
+  template void power_finish<T>(int, const double*, const double*, T*, cudaStream_t);              \
+  template void blockdiag_apply<T>(int, int, const T*, const T*, T*, const T*, T*, cudaStream_t);  \
   template void blockdiag_invert<T>(const BsrMat<T>&, T*, cudaStream_t);                           \
   template void dot<T>(long long, const T*, const T*, T*, T*, cudaStream_t, bool);                 \
   template void fill<T>(long long, T*, T, cudaStream_t);                                           \
@@ -961,7 +1037,7 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, cudaStre
   template void impose_dirichlet<T>(const BcDev&, long long, double, const double*, T*, double*,   \
                                     double*, cudaStream_t);                                        \
   template void dense_mv<T>(int, const T*, const T*, T*, cudaStream_t);                            \
-  template void sa_setup_level<T>(const AmgLevel<T>&, T, T*, int, cudaStream_t);                   \
+  template void sa_setup_level<T>(const AmgLevel<T>&, T*, int, cudaStream_t);                   \
   template void sa_restrict<T>(const AmgLevel<T>&, const T*, T*, cudaStream_t);                    \
   template void sa_prolong<T>(const AmgLevel<T>&, const T*, T*, cudaStream_t);                     \
   template void sa_prolong2<T>(const AmgLevel<T>&, const T*, const T*, T*, cudaStream_t);

@@ -26,13 +26,21 @@ struct BcDev {
 template <typename T> void bsr_spmv(const BsrMat<T>& A, const T* x, T* y, cudaStream_t st);
 template <typename T> void bsr_residual(const BsrMat<T>& A, const T* x, const T* b, T* r, cudaStream_t st);
 template <typename T> void bsr_cheb_step(const BsrMat<T>& A, const T* dinv, const T* d, T* r, T* x, cudaStream_t st);
-// Degree-2 Chebyshev in one pass: x (=, or += unless zero) c2 d0 + c1 (r0 - Dinv A d0).
+// Degree-2 Chebyshev in one pass: x (=, or += unless zero) c2 d0 + c1 (r0 - Dinv A d0);
+// co holds the level's scalars on the device.
 template <typename T> void bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero,
-                                     T c1, T c2, cudaStream_t st);
-// r = Dinv (b - A x), d = scale r.
+                                     const T* co, cudaStream_t st);
+// r = Dinv (b - A x), d = co[CO_ITH] r.
 template <typename T> void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r,
-                                                T* d, T scale, cudaStream_t st);
-template <typename T> void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, T scale, T* d, cudaStream_t st);
+                                                T* d, const T* co, cudaStream_t st);
+// Power iteration: y = Dinv A x; the partials of |v|^2 (at most 1024, count returned);
+// v /= sqrt(sum(part)); a level's scalars from the last two iterates' squared norms.
+template <typename T> void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, cudaStream_t st);
+template <typename T> int norm2_partials(long long n, const T* v, double* part, cudaStream_t st);
+template <typename T> void scale_by_norm(long long n, const double* part, int np, T* v, cudaStream_t st);
+template <typename T> void power_finish(int np, const double* prev, const double* last, T* co, cudaStream_t st);
+// r = Dinv v, d = *scale r (scale on the device).
+template <typename T> void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, const T* scale, T* d, cudaStream_t st);
 template <typename T> void blockdiag_invert(const BsrMat<T>& A, T* dinv, cudaStream_t st);
 template <typename T> void dot(long long n, const T* a, const T* b, T* out, T* part, cudaStream_t st, bool take_sqrt);
 template <typename T> void fill(long long n, T* x, T v, cudaStream_t st);
@@ -57,7 +65,7 @@ template <typename T> void add_to_double(long long n, const T* x, double* U, cud
 template <typename KT> void impose_dirichlet(const BcDev& bc, long long ndof, double lam, const double* U, KT* K, double* R, double* dg, cudaStream_t st);
 void bc_apply(const BcDev& bc, double lam, double* U, cudaStream_t st);
 template <typename T> void dense_mv(int n, const T* M, const T* b, T* y, cudaStream_t st);
-template <typename T> void sa_setup_level(const AmgLevel<T>& v, T w, T* cval, int nnzC, cudaStream_t st);
+template <typename T> void sa_setup_level(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st);
 template <typename T> void sa_restrict(const AmgLevel<T>& v, const T* r, T* bc, cudaStream_t st);
 template <typename T> void sa_prolong(const AmgLevel<T>& v, const T* xc, T* x, cudaStream_t st);
 template <typename T> void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, cudaStream_t st);

@@ -77,6 +77,11 @@ struct BsrMat {
   int* err = nullptr;     // device flag that a kernel sets when a bounded wait ran out
 };
 
+// Scalars of a level's set-up: the spectral radius estimate of D^-1 A (x 1.1); of the
+// degree-2 Chebyshev smoother on [lmax/30, lmax]: 1 / th (th the interval's centre, the
+// first step of any degree), c1, c2; the prolongator's 4 / (3 rho).
+enum : int { CO_LMAX = 0, CO_ITH = 1, CO_C1 = 2, CO_C2 = 3, CO_OMEGA = 4, CO_COUNT = 8 };
+
 // One level of smoothed-aggregation AMG.  Every fine block row n belongs to
 // one aggregate agg[n] and carries the tentative bs x 6 block T_n (the six
 // rigid-body modes, orthonormalised per aggregate).  The prolongator is
@@ -86,7 +91,8 @@ template <typename VT>
 struct AmgLevel {
   BsrMat<VT> A;
   VT* dinv = nullptr;     // nbrow x bs x bs inverse diagonal blocks
-  VT lmax = 0;            // spectral radius estimate of D^-1 A (x 1.1)
+  VT* co = nullptr;       // device: the set-up's scalars (CO_*), so that nothing waits for them
+  VT lmax = 0;            // host copy of co[CO_LMAX], brought over when a caller needs it
   int nagg = 0;
   int* agg = nullptr;     // nbrow aggregate of each block row
   VT* T = nullptr;        // nbrow x bs x 6
@@ -118,7 +124,8 @@ struct Amg {
   VT *cx = nullptr, *cb = nullptr;
   bool built = false;
   int cheb_degree = 2;
-  long long version = 0;     // bumped by every numeric set-up (captured solver graphs key on it)
+  long long version = 0;     // bumped by every numeric set-up
+  long long lmax_version = 0;  // the set-up that the levels' host lmax belong to
 };
 
 }  // namespace pfem

@@ -119,12 +119,13 @@ __device__ __forceinline__ void pipe_issue(unsigned char* stage, const PipeLay& 
 
 // What the modes do with a row's sum v (A x), row by row:
 //   0: y = v   1: y = b - v   2: y -= Dinv v, xo += x   3: xo = c2 x + c1 (y - Dinv v)
-//   4: as 3, added to xo      5: y = Dinv (b - v), xo = c1 y
+//   4: as 3, added to xo      5: y = Dinv (b - v), xo = y / th      6: y = Dinv v
+// (1 / th, c1, c2 from co)
 template <typename T, int BS, int MODE, bool C16>
 __global__ void __launch_bounds__(32)
 bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__ rowptr, const int* __restrict__ col,
                      const int16_t* __restrict__ col16, const T* __restrict__ val, const T* x, T* y, const T* b,
-                     const T* __restrict__ dinv, T* xo, T c1, T c2, int* err) {
+                     const T* __restrict__ dinv, T* xo, const T* co, int* err) {
   using SH = PipeShape<T, BS>;
   constexpr int R = SH::ROWS, BB = BS * BS;
   extern __shared__ __align__(128) unsigned char psm[];
@@ -147,6 +148,8 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
   }
   __syncwarp();
   uint32_t phase = 0;
+  const T c1 = MODE == 3 || MODE == 4 ? co[CO_C1] : MODE == 5 ? co[CO_ITH] : T(0);
+  const T c2 = MODE == 3 || MODE == 4 ? co[CO_C2] : T(0);
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
     // a lane's row(s) of the tile and the epilogue's operands, in flight while the tile arrives
     if constexpr (BS == 3) {
@@ -239,6 +242,8 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
             } else if (MODE == 5) {
               y[at + i] = w;
               xo[at + i] = c1 * w;
+            } else if (MODE == 6) {
+              y[at + i] = w;
             } else {
               const T upd = c2 * xi[i] + c1 * (yi[i] - w);
               xo[at + i] = MODE == 3 ? upd : oi[i] + upd;
@@ -335,6 +340,8 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
         } else if (MODE == 5) {
           y[at] = w;
           xo[at] = c1 * w;
+        } else if (MODE == 6) {
+          y[at] = w;
         } else {
           const T upd = c2 * xi + c1 * (yi - w);
           xo[at] = MODE == 3 ? upd : oi + upd;
