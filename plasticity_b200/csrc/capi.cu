@@ -39,15 +39,16 @@ struct KrylovWork {
   T *rh = nullptr, *v = nullptr, *s = nullptr, *t = nullptr, *ph = nullptr, *sh = nullptr;
   T* sc = nullptr;    // device scalars
   T* part = nullptr;  // reduction partials
+  double* dpart = nullptr;     // the fused PCG body's: r.z, p.q and r.r, kMaxPartials each
+  unsigned* ticket = nullptr;  // zero between launches of cg_xr_fused
   T* b = nullptr;
   T *xa = nullptr, *b0 = nullptr;  // iterative refinement: accumulated solution, saved right-hand side
 };
 
 // The preconditioned-CG loop captured as one CUDA graph: a prefix (x = 0,
 // r = b, |b|) and a conditional WHILE node whose body is one iteration
-// (V-cycle, two dot products, the p / x / r updates, |r|) ending in a
-// one-thread kernel that sets the loop condition from the device-resident
-// residual.  One launch and one host synchronisation per linear solve.
+// (V-cycle, the p / x / r updates with the dot products inside, |r|); the last kernel's
+// last CTA sets the loop condition from the device-resident residual.  One launch and one host synchronisation per linear solve.
 // A set-up writes into the same device arrays, so the graph outlives it; it is
 // captured again when the smoother's degree changes (and, for other degrees than 2,
 // whose coefficients are kernel arguments, after every set-up).  The tolerance and
@@ -151,6 +152,8 @@ struct pfem_ctx {
   KrylovWork<double> kw64;
   CgGraph cg32, cg64;
   int tangent_prec = -1;  // precision of the last imposed tangent
+  int chain_len = 0;      // the cycle's kernels are being captured as a programmatic
+  int* chain = nullptr;   // launch chain: &chain_len meanwhile
   cudaEvent_t e0 = nullptr, e1 = nullptr, t0 = nullptr, t1 = nullptr, a0 = nullptr, a1 = nullptr;
   // learned predictor
   pfem::MlpState mlp;
@@ -737,7 +740,10 @@ int krylov_alloc(pfem_ctx* ctx) {
   CK(dalloc(ctx, &w.v, n)); CK(dalloc(ctx, &w.s, n)); CK(dalloc(ctx, &w.t, n));
   CK(dalloc(ctx, &w.ph, n)); CK(dalloc(ctx, &w.sh, n)); CK(dalloc(ctx, &w.b, n));
   CK(dalloc(ctx, &w.xa, n)); CK(dalloc(ctx, &w.b0, n));
-  CK(dalloc(ctx, &w.sc, 16)); CK(dalloc(ctx, &w.part, 3 * 2048));  // three partial sets of the fused PCG body
+  CK(dalloc(ctx, &w.sc, 16)); CK(dalloc(ctx, &w.part, 2048));
+  CK(dalloc(ctx, &w.dpart, 3 * (size_t)pfem::kMaxPartials));
+  CK(dalloc(ctx, &w.ticket, 1));
+  CK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned), ctx->st));
   return PFEM_OK;
 }
 
@@ -834,16 +840,19 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
 // [lmax/30, lmax].  zero: x enters as 0.
 // Degree 2: x2 = x0 + d0 + d1 with d0 = r0 / th, r0 = Dinv (b - A x0), r1 = r0 - Dinv A d0,
 // d1 = c1 r1 + (c2 - 1) d0; the set-up leaves 1 / th, c1 and c2 in v.co.
+// started: with a zero x, v.r = Dinv b and v.d = v.r / th are there already.  part:
+// receives the partials of b.x (only degree 2, nonzero x); their count is returned.
 template <typename T>
-void cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero) {
+int cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero, bool started = false,
+         double* part = nullptr) {
   const long long n = (long long)v.A.nbrow * v.A.bs;
   const T* const ith = v.co + CO_ITH;
   if (degree == 2) {
     // one block-Jacobi pass (or a fused residual pass) and one fused SpMV pass
-    if (zero) blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, ith, v.d, ctx->st);
-    else bsr_residual_precond<T>(v.A, v.dinv, x, b, v.r, v.d, v.co, ctx->st);
-    bsr_cheb2<T>(v.A, v.dinv, v.d, v.r, x, zero, v.co, ctx->st);
-    return;
+    const Queue q(ctx->st, ctx->chain);
+    if (!zero) bsr_residual_precond<T>(v.A, v.dinv, x, b, v.r, v.d, v.co, q);
+    else if (!started) blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, ith, v.d, q);
+    return bsr_cheb2<T>(v.A, v.dinv, v.d, v.r, x, zero, v.co, q, b, part);
   }
   const double lmx = (double)v.lmax, lmn = lmx / 30.0;
   const double th = 0.5 * (lmx + lmn), de = 0.5 * (lmx - lmn);
@@ -851,7 +860,7 @@ void cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero
   double rho = 1.0 / sg;
   if (zero) {
     fill<T>(n, x, T(0), ctx->st);
-    blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, ith, v.d, ctx->st);
+    if (!started) blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, b, v.r, ith, v.d, ctx->st);
   } else {
     bsr_residual<T>(v.A, x, b, v.t, ctx->st);
     blockdiag_apply<T>(v.A.nbrow, v.A.bs, v.dinv, v.t, v.r, ith, v.d, ctx->st);
@@ -866,20 +875,24 @@ void cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero
       axpby<T>(n, T(1), v.d, T(1), x, ctx->st);
     }
   }
+  return 0;
 }
 
+// started: v.r and v.d hold the smoother's start on b (the kernel that made b wrote
+// them as well).  part: partials of b.x, as cheb.
 template <typename T>
-void vcycle(pfem_ctx* ctx, int l, const T* b, T* x) {
+int vcycle(pfem_ctx* ctx, int l, const T* b, T* x, bool started = false, double* part = nullptr) {
   Amg<T>& A = amg_of<T>(ctx);
   const int L = (int)A.lv.size();
   AmgLevel<T>& v = A.lv[l];
-  cheb<T>(ctx, v, A.cheb_degree, b, x, true);
-  bsr_residual<T>(v.A, x, b, v.t, ctx->st);
+  const Queue q(ctx->st, ctx->chain);
+  cheb<T>(ctx, v, A.cheb_degree, b, x, true, started);
+  bsr_residual<T>(v.A, x, b, v.t, q);
   T* bn = (l + 1 < L) ? A.lv[l + 1].b : A.cb;
   T* xn = (l + 1 < L) ? A.lv[l + 1].x : A.cx;
-  sa_restrict<T>(v, v.t, bn, ctx->st);
-  if (l + 1 < L) vcycle<T>(ctx, l + 1, bn, xn);
-  else dense_mv<T>(A.coarse_n, A.coarse_inv, bn, xn, ctx->st);
+  sa_restrict<T>(v, v.t, bn, l + 1 < L ? &A.lv[l + 1] : nullptr, q);
+  if (l + 1 < L) vcycle<T>(ctx, l + 1, bn, xn, true);
+  else dense_mv<T>(A.coarse_n, A.coarse_inv, bn, xn, q);
   if (l >= 1 && l + 1 < L) {
     // Below the finest level the cycle is a W: two iterations on the coarse
     // problem.  The second starts from the coarse residual bn - A_c xn, which
@@ -888,13 +901,13 @@ void vcycle(pfem_ctx* ctx, int l, const T* b, T* x) {
     // corrections are prolonged in one pass.  The coarse levels cost a small
     // fraction of level 0, and the stronger coarse solve cuts the CG iterations.
     AmgLevel<T>& c = A.lv[l + 1];
-    bsr_residual<T>(c.A, xn, bn, c.b2, ctx->st);
-    vcycle<T>(ctx, l + 1, c.b2, c.x2);
-    sa_prolong2<T>(v, xn, c.x2, x, ctx->st);
+    bsr_residual_start<T>(c.A, c.dinv, xn, bn, c.b2, c.r, c.d, c.co, q);
+    vcycle<T>(ctx, l + 1, c.b2, c.x2, true);
+    sa_prolong2<T>(v, xn, c.x2, x, q);
   } else {
-    sa_prolong<T>(v, xn, x, ctx->st);
+    sa_prolong<T>(v, xn, x, q);
   }
-  cheb<T>(ctx, v, A.cheb_degree, b, x, false);
+  return cheb<T>(ctx, v, A.cheb_degree, b, x, false, false, part);
 }
 
 template <typename T>
@@ -907,34 +920,6 @@ __global__ void cg_graph_init_kernel(cudaGraphConditionalHandle h, const T* __re
   *sc0 = T(1);                  // with p = 0, the first update p = z + (r.z / 1) p gives p = z
   cudaGraphSetConditional(h, (b > 0.0 && isfinite(b)) ? 1u : 0u);
 }
-// End of a PCG iteration: |r| from the np partials of r.r (fixed order, one
-// CTA of 1024 threads), into sc_rn, then the loop condition.
-template <typename T>
-__global__ void cg_graph_check_kernel(cudaGraphConditionalHandle h, const T* __restrict__ part, int np,
-                                      T* __restrict__ sc_rn, const double* __restrict__ ctl,
-                                      int* __restrict__ state) {
-  __shared__ T sh[32];
-  T v = T(0);
-  for (int i = threadIdx.x; i < np; i += blockDim.x) v += part[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x >= 32) return;
-  v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : T(0);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (threadIdx.x != 0) return;
-  const T rn = sqrt(v);
-  *sc_rn = rn;
-  const int it = state[0] + 1;
-  state[0] = it;
-  const double r = (double)rn;
-  const bool conv = r <= ctl[2];
-  state[1] = conv ? 1 : 0;
-  cudaGraphSetConditional(h, (!conv && isfinite(r) && it < (int)ctl[1]) ? 1u : 0u);
-}
-
 // Capture (or reuse) the device-side CG loop for the current hierarchy.
 template <typename T>
 int cg_graph_build(pfem_ctx* ctx) {
@@ -956,11 +941,13 @@ int cg_graph_build(pfem_ctx* ctx) {
   const long long c0 = pfem::launch_counter();
   cudaGraph_t g = nullptr;
   cudaGraph_t body = nullptr;
+  AmgLevel<T>& v0 = A.lv[0];
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return fail(ctx, PFEM_ERR_CUDA, std::string("CG graph capture: ") + cudaGetErrorString(e));
   auto abort_capture = [&](cudaError_t err, const char* what) {
     cudaGraph_t junk = nullptr;
     ctx->st = st;
+    ctx->chain = nullptr;
     cudaStreamEndCapture(G.body_stream, &junk);
     cudaStreamEndCapture(st, &junk);
     if (junk) cudaGraphDestroy(junk);
@@ -972,6 +959,7 @@ int cg_graph_build(pfem_ctx* ctx) {
   e = cudaMemcpyAsync(w.r, w.b, n * sizeof(T), cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) return abort_capture(e, "r = b");
   dot<T>(n, w.b, w.b, w.sc + 10, w.part, st, true);
+  blockdiag_apply<T>(K.nbrow, 3, v0.dinv, w.r, v0.r, v0.co + CO_ITH, v0.d, st);
   cudaStreamCaptureStatus cs;
   const cudaGraphNode_t* deps = nullptr;
   size_t nd = 0;
@@ -999,20 +987,29 @@ int cg_graph_build(pfem_ctx* ctx) {
   e = cudaStreamBeginCaptureToGraph(G.body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return abort_capture(e, "body capture");
   cudaStream_t bs = G.body_stream;
+  // Programmatic launches (degree 2 only: the others' vector kernels do not wait): a
+  // kernel's matrix, prolongator or inverse is on its way while its predecessor ends.
   ctx->st = bs;  // the V-cycle launches on ctx->st
-  vcycle<T>(ctx, 0, w.r, w.z);
+  ctx->chain_len = 0;
+  ctx->chain = A.cheb_degree == 2 ? &ctx->chain_len : nullptr;
+  const Queue q(bs, ctx->chain);
+  // sc[0] = r.z of the previous iteration, sc[2] = r.z; the dot products are summed
+  // by the kernels whose results they are made of, their final sums by their users
+  double* const part_rz = w.dpart;
+  double* const part_pq = w.dpart + pfem::kMaxPartials;
+  int np_rz = vcycle<T>(ctx, 0, w.r, w.z, true, ctx->chain ? part_rz : nullptr);
   ctx->st = st;
-  // sc[0] = r.z of the previous iteration, sc[2] = r.z; the final sums of the
-  // three dot products happen inside the kernels that use them
-  T* const part_rz = w.part;
-  T* const part_pq = w.part + 2048;
-  T* const part_rr = w.part + 4096;
-  const int np_rz = dot_partials<T>(n, w.r, w.z, part_rz, bs);
-  cg_p_fused<T>(n, part_rz, np_rz, w.sc, w.z, w.p, bs);
-  bsr_spmv<T>(K, w.p, w.q, bs);
-  const int np_pq = dot_partials<T>(n, w.p, w.q, part_pq, bs);
-  const int np_rr = cg_xr_fused<T>(n, part_pq, np_pq, w.sc, w.p, w.q, w.x, w.r, part_rr, bs);
-  cg_graph_check_kernel<T><<<1, 1024, 0, bs>>>(h, part_rr, np_rr, w.sc + 3, G.ctl, G.state);
+  ctx->chain = nullptr;
+  if (np_rz == 0) np_rz = dot_partials_double<T>(n, w.r, w.z, part_rz, q);
+  cg_p_fused<T>(n, part_rz, np_rz, w.sc, w.z, w.p, q);
+  const int np_pq = bsr_spmv<T>(K, w.p, w.q, q, part_pq);
+  CgLoop loop;
+  loop.h = h;
+  loop.ctl = G.ctl;
+  loop.state = G.state;
+  loop.ticket = w.ticket;
+  loop.part_rr = w.dpart + 2 * pfem::kMaxPartials;
+  cg_xr_fused<T>(K.nbrow, part_pq, np_pq, w.sc, w.p, w.q, w.x, w.r, v0.dinv, v0.co, v0.r, v0.d, loop, q);
   e = cudaStreamEndCapture(bs, &body);
   if (e != cudaSuccess) return abort_capture(e, "body end");
   const long long c2 = pfem::launch_counter();
@@ -1029,7 +1026,7 @@ int cg_graph_build(pfem_ctx* ctx) {
   }
   // launches are counted when the graph runs, not when it is captured
   G.prefix_kernels = c1 - c0 + 1;
-  G.body_kernels = c2 - c1 + 1;
+  G.body_kernels = c2 - c1;
   pfem::launch_counter() = c0;
   G.degree = A.cheb_degree;
   G.amg_version = version;
@@ -2732,7 +2729,10 @@ int pfem_profile(pfem_ctx* ctx, int32_t what, int32_t reps, double* ms) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
+    ctx->chain_len = 0;
+    ctx->chain = ctx->amg32.cheb_degree == 2 ? &ctx->chain_len : nullptr;
     vcycle<float>(ctx, 0, w.r, w.z);
+    ctx->chain = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
     pfem::launch_counter() = c0;  // counted when replayed below, not when captured
     if (e != cudaSuccess) return fail(ctx, PFEM_ERR_CUDA, std::string("cycle capture: ") + cudaGetErrorString(e));

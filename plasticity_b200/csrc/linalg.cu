@@ -10,43 +10,72 @@
 
 namespace pfem {
 
+// ------------------------------------------------------------------ reductions
+// Deterministic two-pass dot product: per-block partials, then one block.
+constexpr int RED_THREADS = 256;
+constexpr int RED_BLOCKS = 1184;  // 148 SMs x 8
+
+template <typename T>
+__device__ __forceinline__ T block_sum(T v, T* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) sh[w] = v;
+  __syncthreads();
+  v = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : T(0);
+  if (w == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  return v;
+}
+
+// Partials of a.b summed in double, at most kMaxPartials (count returned).
+template <typename T>
+__global__ void dot_partial_double_kernel(long long n, const T* a, const T* b, double* part) {
+  __shared__ double sh[32];
+  pdl_go();
+  pdl_wait();
+  double v = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    v += (double)a[i] * (double)b[i];
+  v = block_sum(v, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = v;
+}
+template <typename T>
+int dot_partials_double(long long n, const T* a, const T* b, double* part, const Queue& q) {
+  const int blocks = (int)std::min<long long>(std::max<long long>((n + RED_THREADS - 1) / RED_THREADS, 1), RED_BLOCKS);
+  launch(q, dot_partial_double_kernel<T>, blocks, RED_THREADS, 0, n, a, b, part);
+  return blocks;
+}
+
 // ------------------------------------------------------------------ SpMV
 // Half a warp per block row; lane k holds block rowptr[i]+k (+16, ...), loads
 // the whole bs x bs block and the matching bs entries of x, and the half-warp
-// reduces the bs partial sums by a fixed xor tree.  Mode selects the epilogue:
-//   0: y = A x
-//   1: y = b - A x                          (residual)
-//   2: r -= Dinv (A x); xo += x             (Chebyshev step on x = d)
-//   3: xo = c2 x + c1 (y - Dinv A x)        (fused degree-2 Chebyshev, x = d0, y = r0)
-//   4: as 3, added to xo
-//   5: y = Dinv (b - A x), xo = y / th      (preconditioned residual + first direction)
-//   6: y = Dinv A x                         (a step of the power iteration)
-// with 1 / th, c1 and c2 from the level's scalars co.
-template <typename T, int BS, int MODE, bool VEC = false, int LANES = 16, bool C16 = false>
-__global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __restrict__ rowptr,
+// reduces the bs partial sums by a fixed xor tree.  The modes are SpmvVec's.  DOT: the
+// row's share of x.y (mode 0) or b.xo (mode 4) is summed per CTA into part.
+template <typename T, int BS, int MODE, bool VEC = false, int LANES = 16, bool C16 = false, bool DOT = false>
+__global__ void __launch_bounds__(128) bsr_spmv_kernel(int nbrow, const int* __restrict__ rowptr,
                                                        const int* __restrict__ col,
                                                        const int16_t* __restrict__ col16,
-                                                       const T* __restrict__ val,
-                                                       const T* __restrict__ x, T* __restrict__ y,
-                                                       const T* __restrict__ b,
-                                                       const T* __restrict__ dinv, T* __restrict__ xo,
-                                                       const T* __restrict__ co) {
+                                                       const T* __restrict__ val, SpmvVec<T> a) {
   // LANES lanes per block row: half a warp for 3 x 3 blocks (a level-0 row has at
   // most 27 blocks: two per lane), a warp for 6 x 6 blocks (one 144-byte block
   // per lane); values and column ids are read once, through the streaming
-  // (evict-first) path so they do not push the gathered x out of the caches.
+  // (evict-first) path so they do not push the gathered x out of the caches.  The
+  // first block and the block inverse are in flight before the wait for the vectors.
   static_assert(LANES == 16 || LANES == 32, "half or whole warps per row");
+  pdl_go();
   const int row = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) / LANES);
   const int lane = threadIdx.x & (LANES - 1);
-  const bool ok = row < nbrow;
+  const bool ok = row < nbrow, own = ok && lane < BS;
+  const long long at = (long long)row * BS + lane;
   const int s = ok ? rowptr[row] : 0, e = ok ? rowptr[row + 1] : 0;
-  T acc[BS];
-#pragma unroll
-  for (int i = 0; i < BS; ++i) acc[i] = T(0);
-  for (int k = s + lane; k < e; k += LANES) {
-    const int c = C16 ? row + (int)__ldcs(col16 + k) : __ldcs(col + k);
+  T bv[BS * BS], D[BS];
+  int c = 0;
+  auto block = [&](int k) {
+    c = C16 ? row + (int)__ldcs(col16 + k) : __ldcs(col + k);
     const T* B = val + (long long)k * (BS * BS);
-    T bv[BS * BS];
     if constexpr (VEC) {
       // 16-byte streaming loads (a 6 x 6 block is 144 / 288 bytes; the launcher
       // checks that val is 16-byte aligned, so every block is)
@@ -65,13 +94,34 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
 #pragma unroll
       for (int q = 0; q < BS * BS; ++q) bv[q] = __ldcs(B + q);
     }
+  };
+  int k = s + lane;
+  if (k < e) block(k);
+#pragma unroll
+  for (int j = 0; j < BS; ++j) D[j] = (MODE >= 2 && own) ? a.dinv[(long long)row * (BS * BS) + lane * BS + j] : T(0);
+  const T c1 = MODE == 3 || MODE == 4 ? a.co[CO_C1] : MODE == 5 || MODE == 7 ? a.co[CO_ITH] : T(0);
+  const T c2 = MODE == 3 || MODE == 4 ? a.co[CO_C2] : T(0);
+  pdl_wait();
+  T bi = T(0), yi = T(0), xi = T(0), oi = T(0);
+  if (own) {
+    if (MODE == 1 || MODE == 5 || MODE == 7 || (DOT && MODE == 4)) bi = a.b[at];
+    if (MODE == 2 || MODE == 3 || MODE == 4) yi = a.y[at];
+    if (MODE == 2 || MODE == 3 || MODE == 4 || (DOT && MODE == 0)) xi = a.x[at];
+    if (MODE == 2 || MODE == 4) oi = a.xo[at];
+  }
+  T acc[BS];
+#pragma unroll
+  for (int i = 0; i < BS; ++i) acc[i] = T(0);
+  while (k < e) {
     T xv[BS];
 #pragma unroll
-    for (int j = 0; j < BS; ++j) xv[j] = x[(long long)c * BS + j];
+    for (int j = 0; j < BS; ++j) xv[j] = a.x[(long long)c * BS + j];
 #pragma unroll
     for (int i = 0; i < BS; ++i)
 #pragma unroll
       for (int j = 0; j < BS; ++j) acc[i] += bv[i * BS + j] * xv[j];
+    k += LANES;
+    if (k < e) block(k);
   }
 #pragma unroll
   for (int i = 0; i < BS; ++i) {
@@ -80,52 +130,54 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int nbrow, const int* __r
     for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     acc[i] = v;
   }
-  if (ok && lane < BS) {
-    const long long base = (long long)row * BS;
-    if (MODE == 5) {
-      // r = Dinv (b - A x) (into y), d = c1 r (into xo)
-      const T* D = dinv + (long long)row * (BS * BS);
-      T t = T(0);
+  T v = acc[0];
 #pragma unroll
-      for (int j = 0; j < BS; ++j) t += D[lane * BS + j] * (b[base + j] - acc[j]);
-      y[base + lane] = t;
-      xo[base + lane] = co[CO_ITH] * t;
-      return;
-    }
-    T v = acc[0];
+  for (int i = 1; i < BS; ++i)
+    if (lane == i) v = acc[i];
+  T w = T(0);
+  if (MODE == 5 || MODE == 7) {
+    v = bi - v;
 #pragma unroll
-    for (int i = 1; i < BS; ++i)
-      if (lane == i) v = acc[i];
+    for (int j = 0; j < BS; ++j) w += D[j] * __shfl_sync(0xffffffffu, v, (threadIdx.x & 31 & ~(LANES - 1)) + j);
+  } else if (MODE >= 2) {
+#pragma unroll
+    for (int j = 0; j < BS; ++j) w += D[j] * acc[j];
+  }
+  double dot = 0.0;
+  if (own) {
     if (MODE == 0) {
-      y[base + lane] = v;
+      a.y[at] = v;
+      if (DOT) dot = (double)xi * (double)v;
     } else if (MODE == 1) {
-      y[base + lane] = b[base + lane] - v;
+      a.y[at] = bi - v;
+    } else if (MODE == 2) {
+      a.y[at] = yi - w;
+      a.xo[at] = oi + xi;
+    } else if (MODE == 5 || MODE == 7) {
+      if (MODE == 7) a.z[at] = v;
+      a.y[at] = w;
+      a.xo[at] = c1 * w;
+    } else if (MODE == 6) {
+      a.y[at] = w;
     } else {
-      // t = (Dinv A d)_lane with d = x (the gathered vector)
-      const T* D = dinv + (long long)row * (BS * BS);
-      T t = T(0);
-#pragma unroll
-      for (int j = 0; j < BS; ++j) t += D[lane * BS + j] * acc[j];
-      if (MODE == 6) {
-        y[base + lane] = t;
-      } else if (MODE == 2) {
-        y[base + lane] -= t;
-        xo[base + lane] += x[base + lane];
-      } else {
-        // degree-2 Chebyshev in one pass: r1 = r0 - Dinv A d0,
-        // x2 = x0 + c2 d0 + c1 r1 (c2 = 1 + rn rho, c1 = 2 rn / delta)
-        const T upd = co[CO_C2] * x[base + lane] + co[CO_C1] * (y[base + lane] - t);
-        if (MODE == 3) xo[base + lane] = upd;
-        else xo[base + lane] += upd;
-      }
+      // degree-2 Chebyshev in one pass: r1 = r0 - Dinv A d0,
+      // x2 = x0 + c2 d0 + c1 r1 (c2 = 1 + rn rho, c1 = 2 rn / delta)
+      T upd = c2 * xi + c1 * (yi - w);
+      if (MODE == 4) upd = oi + upd;
+      a.xo[at] = upd;
+      if (DOT) dot = (double)bi * (double)upd;
     }
+  }
+  if constexpr (DOT) {
+    __shared__ double sh[32];
+    dot = block_sum(dot, sh);
+    if (threadIdx.x == 0) a.part[blockIdx.x] = dot;
   }
 }
 
-template <typename T, int BS, int MODE, bool C16>
-static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, const T* co,
-                          cudaStream_t st) {
-  auto* kern = bsr_spmv_pipe_kernel<T, BS, MODE, C16>;
+template <typename T, int BS, int MODE, bool C16, bool DOT>
+static int pipe_launch_t(const BsrMat<T>& A, const SpmvVec<T>& a, const Queue& qu) {
+  auto* kern = bsr_spmv_pipe_kernel<T, BS, MODE, C16, DOT>;
   const int sm = pipe_smem_bytes<T, BS>(A.max_row, C16);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   int dev = 0, sms = 148, per = 1;
@@ -134,10 +186,9 @@ static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, cons
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32, sm);
   constexpr int R = PipeShape<T, BS>::ROWS;
   const int tiles = (A.nbrow + R - 1) / R;
-  const int grid = std::min(tiles, sms * std::max(per, 1));
-  pfem::count_launch();
-  kern<<<grid, 32, sm, st>>>(A.nbrow, tiles, A.max_row, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, co,
-                             A.err);
+  const int grid = std::min(std::min(tiles, sms * std::max(per, 1)), kMaxPartials);
+  launch(qu, kern, grid, 32, sm, A.nbrow, tiles, A.max_row, A.rowptr, A.col, A.col16, A.val, a, A.err);
+  return grid;
 }
 // The streamed kernel takes a matrix whose rows have at most 32 blocks and whose
 // arrays start on 16 bytes, from as many rows on as keep most warps of the chip busy:
@@ -146,23 +197,21 @@ static void pipe_launch_t(const BsrMat<T>& A, const T* x, T* y, const T* b, cons
 // 54 / 51 at 24^3 (15,625), 117 / 100 at 40^3.  6 x 6 levels, with the finest level
 // streamed: 152 / 146 us at 48^3 (4,913 rows of 6 x 6), 647 / 603 at 80^3 (19,683).
 constexpr int kPipeRows3 = 8192, kPipeRows6 = 4096;
-template <typename T, int MODE>
-static bool spmv_pipe_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, const T* co,
-                             cudaStream_t st) {
-  const bool c16 = A.bs == 3 && A.col16;
+template <typename T>
+static bool spmv_streams(const BsrMat<T>& A) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(A.val) | reinterpret_cast<uintptr_t>(A.rowptr) |
-                       (c16 ? reinterpret_cast<uintptr_t>(A.col16) : reinterpret_cast<uintptr_t>(A.col));
-  if (A.nbrow < (A.bs == 3 ? kPipeRows3 : kPipeRows6) || A.max_row < 1 || A.max_row > 32 || !A.err || (at & 15)) return false;
-  if (c16) pipe_launch_t<T, 3, MODE, true>(A, x, y, b, dinv, xo, co, st);
-  else if (A.bs == 3) pipe_launch_t<T, 3, MODE, false>(A, x, y, b, dinv, xo, co, st);
-  else pipe_launch_t<T, 6, MODE, false>(A, x, y, b, dinv, xo, co, st);
-  return true;
+                       (A.bs == 3 && A.col16 ? reinterpret_cast<uintptr_t>(A.col16) : reinterpret_cast<uintptr_t>(A.col));
+  return A.nbrow >= (A.bs == 3 ? kPipeRows3 : kPipeRows6) && A.max_row >= 1 && A.max_row <= 32 && A.err && !(at & 15);
 }
 
-template <typename T, int MODE>
-static void spmv_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const T* dinv, T* xo, const T* co,
-                        cudaStream_t st) {
-  if (spmv_pipe_launch<T, MODE>(A, x, y, b, dinv, xo, co, st)) return;
+// DOT (3 x 3 blocks): returns the number of partials, 0 when there would be too many.
+template <typename T, int MODE, bool DOT = false>
+static int spmv_launch(const BsrMat<T>& A, const SpmvVec<T>& a, const Queue& qu) {
+  if (spmv_streams(A)) {
+    if (A.bs == 3 && A.col16) return pipe_launch_t<T, 3, MODE, true, DOT>(A, a, qu);
+    if (A.bs == 3) return pipe_launch_t<T, 3, MODE, false, DOT>(A, a, qu);
+    if constexpr (!DOT) return pipe_launch_t<T, 6, MODE, false, false>(A, a, qu);
+  }
   // 6 x 6 levels of fewer than kWarpRowsBelow rows fill too few warp slots with half
   // a warp per row: give each row a whole warp there (measured at 64^3: level 2,
   // 512 rows, 7.4 -> 6.5 us per pass; level 1, 10,648 rows, 14.3 -> 18.2 us)
@@ -174,74 +223,102 @@ static void spmv_launch(const BsrMat<T>& A, const T* x, T* y, const T* b, const 
   const long long threads = (long long)A.nbrow * (wide ? 32 : 16);
   const int blocks = (int)((threads + kThreads - 1) / kThreads);
   const bool aligned = (reinterpret_cast<uintptr_t>(A.val) & 15) == 0;
-  pfem::count_launch();
-  if (A.bs == 3 && A.col16)
-    bsr_spmv_kernel<T, 3, MODE, false, 16, true><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16,
-                                                                              A.val, x, y, b, dinv, xo, co);
-  else if (A.bs == 3)
-    bsr_spmv_kernel<T, 3, MODE><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, co);
-  else if (aligned && wide)
-    bsr_spmv_kernel<T, 6, MODE, true, 32><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo,
-                                                                  co);
-  else if (aligned)
-    bsr_spmv_kernel<T, 6, MODE, true><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo,
-                                                              co);
-  else
-    bsr_spmv_kernel<T, 6, MODE><<<blocks, kThreads, 0, st>>>(A.nbrow, A.rowptr, A.col, A.col16, A.val, x, y, b, dinv, xo, co);
+  if constexpr (DOT) {
+    if (blocks > kMaxPartials) return 0;
+    if (A.col16) launch(qu, bsr_spmv_kernel<T, 3, MODE, false, 16, true, true>, blocks, kThreads, 0, A.nbrow, A.rowptr, A.col, A.col16, A.val, a);
+    else launch(qu, bsr_spmv_kernel<T, 3, MODE, false, 16, false, true>, blocks, kThreads, 0, A.nbrow, A.rowptr, A.col, A.col16, A.val, a);
+    return blocks;
+  } else {
+    auto* kern = A.bs == 3 ? (A.col16 ? bsr_spmv_kernel<T, 3, MODE, false, 16, true> : bsr_spmv_kernel<T, 3, MODE>)
+                 : aligned ? (wide ? bsr_spmv_kernel<T, 6, MODE, true, 32> : bsr_spmv_kernel<T, 6, MODE, true>)
+                           : bsr_spmv_kernel<T, 6, MODE>;
+    launch(qu, kern, blocks, kThreads, 0, A.nbrow, A.rowptr, A.col, A.col16, A.val, a);
+    return 0;
+  }
 }
 
 template <typename T>
-void bsr_spmv(const BsrMat<T>& A, const T* x, T* y, cudaStream_t st) {
-  spmv_launch<T, 0>(A, x, y, nullptr, nullptr, nullptr, nullptr, st);
+int bsr_spmv(const BsrMat<T>& A, const T* x, T* y, Queue q, double* part) {
+  SpmvVec<T> a;
+  a.x = x; a.y = y; a.part = part;
+  if (!part) return spmv_launch<T, 0>(A, a, q);
+  const int np = spmv_launch<T, 0, true>(A, a, q);
+  if (np > 0) return np;
+  spmv_launch<T, 0>(A, a, q);
+  return dot_partials_double<T>((long long)A.nbrow * A.bs, x, y, part, q);
 }
 template <typename T>
-void bsr_residual(const BsrMat<T>& A, const T* x, const T* b, T* r, cudaStream_t st) {
-  spmv_launch<T, 1>(A, x, r, b, nullptr, nullptr, nullptr, st);
+void bsr_residual(const BsrMat<T>& A, const T* x, const T* b, T* r, Queue q) {
+  SpmvVec<T> a;
+  a.x = x; a.y = r; a.b = b;
+  spmv_launch<T, 1>(A, a, q);
 }
 template <typename T>
 void bsr_cheb_step(const BsrMat<T>& A, const T* dinv, const T* d, T* r, T* x, cudaStream_t st) {
-  spmv_launch<T, 2>(A, d, r, nullptr, dinv, x, nullptr, st);
+  SpmvVec<T> a;
+  a.x = d; a.y = r; a.dinv = dinv; a.xo = x;
+  spmv_launch<T, 2>(A, a, st);
 }
 template <typename T>
-void bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero, const T* co,
-               cudaStream_t st) {
-  if (zero) spmv_launch<T, 3>(A, d0, const_cast<T*>(r0), nullptr, dinv, x, co, st);
-  else spmv_launch<T, 4>(A, d0, const_cast<T*>(r0), nullptr, dinv, x, co, st);
+int bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero, const T* co, Queue q,
+              const T* b, double* part) {
+  SpmvVec<T> a;
+  a.x = d0; a.y = const_cast<T*>(r0); a.dinv = dinv; a.xo = x; a.co = co; a.b = b; a.part = part;
+  if (zero) return spmv_launch<T, 3>(A, a, q);
+  if (!part) return spmv_launch<T, 4>(A, a, q);
+  const int np = spmv_launch<T, 4, true>(A, a, q);
+  if (np > 0) return np;
+  spmv_launch<T, 4>(A, a, q);
+  return dot_partials_double<T>((long long)A.nbrow * A.bs, b, x, part, q);
 }
 template <typename T>
-void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r, T* d, const T* co,
-                          cudaStream_t st) {
-  spmv_launch<T, 5>(A, x, r, b, dinv, d, co, st);
+void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r, T* d, const T* co, Queue q) {
+  SpmvVec<T> a;
+  a.x = x; a.y = r; a.b = b; a.dinv = dinv; a.xo = d; a.co = co;
+  spmv_launch<T, 5>(A, a, q);
+}
+template <typename T>
+void bsr_residual_start(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* res, T* r, T* d, const T* co,
+                        Queue q) {
+  SpmvVec<T> a;
+  a.x = x; a.y = r; a.b = b; a.dinv = dinv; a.xo = d; a.co = co; a.z = res;
+  spmv_launch<T, 7>(A, a, q);
 }
 template <typename T>
 void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, cudaStream_t st) {
-  spmv_launch<T, 6>(A, x, y, nullptr, dinv, nullptr, nullptr, st);
+  SpmvVec<T> a;
+  a.x = x; a.y = y; a.dinv = dinv;
+  spmv_launch<T, 6>(A, a, st);
 }
 
 // ------------------------------------------------------------------ block diagonal
 // r = Dinv * v per block row (one thread per scalar row), d = *scale r.
 template <typename T, int BS>
-__global__ void blockdiag_apply_kernel(int nbrow, const T* __restrict__ dinv, const T* __restrict__ v,
-                                       T* __restrict__ r, const T* __restrict__ scale,
-                                       T* __restrict__ d) {
+__global__ void blockdiag_apply_kernel(int nbrow, const T* __restrict__ dinv, const T* v, T* r,
+                                       const T* __restrict__ scale, T* d) {
+  pdl_go();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)nbrow * BS) return;
+  const bool in = i < (long long)nbrow * BS;
   const long long row = i / BS;
   const int li = (int)(i - row * BS);
-  const T* D = dinv + row * (BS * BS) + li * BS;
+  T D[BS];
+#pragma unroll
+  for (int j = 0; j < BS; ++j) D[j] = in ? dinv[row * (BS * BS) + li * BS + j] : T(0);
+  const T s = *scale;
+  pdl_wait();
+  if (!in) return;
   const T* vv = v + row * BS;
   T t = T(0);
 #pragma unroll
   for (int j = 0; j < BS; ++j) t += D[j] * vv[j];
   r[i] = t;
-  d[i] = *scale * t;
+  d[i] = s * t;
 }
 template <typename T>
-void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, const T* scale, T* d, cudaStream_t st) {
+void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, const T* scale, T* d, Queue q) {
   const long long n = (long long)nbrow * bs;
-  const int blocks = (int)((n + 255) / 256);
-  if (bs == 3) { pfem::count_launch(); blockdiag_apply_kernel<T, 3><<<blocks, 256, 0, st>>>(nbrow, dinv, v, r, scale, d); }
-  else { pfem::count_launch(); blockdiag_apply_kernel<T, 6><<<blocks, 256, 0, st>>>(nbrow, dinv, v, r, scale, d); }
+  launch(q, bs == 3 ? blockdiag_apply_kernel<T, 3> : blockdiag_apply_kernel<T, 6>, (int)((n + 255) / 256), 256, 0, nbrow,
+         dinv, v, r, scale, d);
 }
 
 // Invert the diagonal blocks (Gauss-Jordan with partial pivoting in double).
@@ -300,26 +377,7 @@ void blockdiag_invert(const BsrMat<T>& A, T* dinv, cudaStream_t st) {
   else { pfem::count_launch(); blockdiag_invert_kernel<T, 6><<<blocks, 128, 0, st>>>(A.nbrow, A.rowptr, A.col, A.val, dinv); }
 }
 
-// ------------------------------------------------------------------ reductions
-// Deterministic two-pass dot product: per-block partials, then one block.
-constexpr int RED_THREADS = 256;
-constexpr int RED_BLOCKS = 1184;  // 148 SMs x 8
-
-template <typename T>
-__device__ __forceinline__ T block_sum(T v, T* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  v = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : T(0);
-  if (w == 0) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  }
-  return v;
-}
-
+// ------------------------------------------------------------------ dot products
 template <typename T>
 __global__ void dot_partial_kernel(long long n, const T* __restrict__ a, const T* __restrict__ b,
                                    T* __restrict__ part) {
@@ -398,11 +456,15 @@ void cg_p(long long n, const T* num, const T* den, const T* z, T* p, cudaStream_
   const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
   pfem::count_launch(); cg_p_kernel<T><<<blocks, 256, 0, st>>>(n, num, den, z, p);
 }
+static int fused_update_blocks(long long n) {
+  const long long nb = (n + RED_THREADS - 1) / RED_THREADS;
+  return (int)(nb < RED_BLOCKS ? (nb > 0 ? nb : 1) : RED_BLOCKS);
+}
 // ---- PCG updates with the final reduction fused in ----
 // Every CTA sums the same np partials in the same order (a strided pass and a
 // fixed tree), so all CTAs see the same scalar and the result is deterministic.
 template <typename T>
-__device__ __forceinline__ T all_sum_partials(const T* __restrict__ part, int np, T* sh) {
+__device__ __forceinline__ T all_sum_partials(const T* part, int np, T* sh) {
   T v = T(0);
   for (int i = threadIdx.x; i < np; i += blockDim.x) v += part[i];
   v = block_sum(v, sh);
@@ -413,35 +475,82 @@ __device__ __forceinline__ T all_sum_partials(const T* __restrict__ part, int np
 }
 // rz = sum(part_rz);  p = z + (rz / sc[0]) p;  sc[2] = rz
 template <typename T>
-__global__ void cg_p_fused_kernel(long long n, const T* __restrict__ part, int np, T* __restrict__ sc,
-                                  const T* __restrict__ z, T* __restrict__ p) {
-  __shared__ T sh[33];
-  const T rz = all_sum_partials(part, np, sh);
+__global__ void cg_p_fused_kernel(long long n, const double* part, int np, T* sc, const T* z, T* p) {
+  __shared__ double sh[33];
+  pdl_go();
+  pdl_wait();
+  const T rz = (T)all_sum_partials(part, np, sh);
   const T be = rz / sc[0];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     p[i] = z[i] + be * p[i];
   if (blockIdx.x == 0 && threadIdx.x == 0) sc[2] = rz;
 }
-// pq = sum(part_pq);  alpha = sc[2] / pq;  x += alpha p;  r -= alpha q;
-// part_rr[cta] = this CTA's share of r.r;  sc[0] = sc[2] (r.z of the next beta)
+// pq = sum(part_pq);  alpha = sc[2] / pq;  x += alpha p;  r -= alpha q;  the smoother's
+// start on the new r;  sc[0] = sc[2] (r.z of the next beta).  A thread per node.  The
+// CTA that finishes last adds the CTAs' shares of r.r in their order and sets the
+// loop's condition.
 template <typename T>
-__global__ void cg_xr_fused_kernel(long long n, const T* __restrict__ part_pq, int np, T* __restrict__ sc,
-                                   const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ x,
-                                   T* __restrict__ r, T* __restrict__ part_rr) {
-  __shared__ T sh[33];
-  const T pq = all_sum_partials(part_pq, np, sh);
+__global__ void __launch_bounds__(256) cg_xr_fused_kernel(int nbrow, const double* part_pq, int np, T* sc, const T* p,
+                                                          const T* q, T* x, T* r, const T* __restrict__ dinv,
+                                                          const T* __restrict__ co, T* sr, T* sd, CgLoop loop) {
+  __shared__ double sh[33];
+  __shared__ bool last;
+  pdl_go();
+  const T ith = co[CO_ITH];
+  pdl_wait();
+  const T pq = (T)all_sum_partials(part_pq, np, sh);
   const T al = sc[2] / pq;
-  T acc = T(0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    x[i] += al * p[i];
-    const T ri = r[i] - al * q[i];
-    r[i] = ri;
-    acc += ri * ri;
+  double acc = 0.0;
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nbrow; n += gridDim.x * blockDim.x) {
+    const long long at = (long long)n * 3;
+    T ri[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      x[at + j] += al * p[at + j];
+      ri[j] = r[at + j] - al * q[at + j];
+      r[at + j] = ri[j];
+      acc += (double)ri[j] * (double)ri[j];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      T t = T(0);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) t += dinv[(long long)n * 9 + i * 3 + j] * ri[j];
+      sr[at + i] = t;
+      sd[at + i] = ith * t;
+    }
   }
+  __syncthreads();  // sh is free again
   acc = block_sum(acc, sh);
-  if (threadIdx.x == 0) part_rr[blockIdx.x] = acc;
-  if (blockIdx.x == 0 && threadIdx.x == 0) sc[0] = sc[2];
+  if (threadIdx.x == 0) {
+    loop.part_rr[blockIdx.x] = acc;
+    __threadfence();
+    last = atomicInc(loop.ticket, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const double rr = all_sum_partials(loop.part_rr, (int)gridDim.x, sh);
+  if (threadIdx.x != 0) return;
+  sc[0] = sc[2];
+  const double rn = sqrt(rr);
+  const int it = loop.state[0] + 1;
+  const bool conv = rn <= loop.ctl[2];
+  loop.state[0] = it;
+  loop.state[1] = conv ? 1 : 0;
+  cudaGraphSetConditional(loop.h, (!conv && isfinite(rn) && it < (int)loop.ctl[1]) ? 1u : 0u);
 }
+template <typename T>
+void cg_p_fused(long long n, const double* part, int np, T* sc, const T* z, T* p, Queue q) {
+  launch(q, cg_p_fused_kernel<T>, fused_update_blocks(n), RED_THREADS, 0, n, part, np, sc, z, p);
+}
+template <typename T>
+void cg_xr_fused(int nbrow, const double* part_pq, int np, T* sc, const T* p, const T* q, T* x, T* r, const T* dinv,
+                 const T* co, T* sr, T* sd, const CgLoop& loop, Queue qu) {
+  launch(qu, cg_xr_fused_kernel<T>, fused_update_blocks(nbrow), RED_THREADS, 0, nbrow, part_pq, np, sc, p, q, x, r, dinv,
+         co, sr, sd, loop);
+}
+
 // ---- power iteration: squared norms in double (an iterate may be as large as its type
 // allows), kNormBlocks partials at most ----
 constexpr int kNormBlocks = 1024;
@@ -503,31 +612,6 @@ void power_finish(int np, const double* prev, const double* last, T* co, cudaStr
   pfem::count_launch();
   power_finish_kernel<T><<<1, 1024, 0, st>>>(np, prev, last, co);
 }
-template <typename T>
-int dot_partials(long long n, const T* a, const T* b, T* part, cudaStream_t st) {
-  long long nb = (n + RED_THREADS - 1) / RED_THREADS;
-  const int blocks = (int)(nb < RED_BLOCKS ? (nb > 0 ? nb : 1) : RED_BLOCKS);
-  pfem::count_launch(); dot_partial_kernel<T><<<blocks, RED_THREADS, 0, st>>>(n, a, b, part);
-  return blocks;
-}
-int fused_update_blocks(long long n) {
-  const long long nb = (n + RED_THREADS - 1) / RED_THREADS;
-  return (int)(nb < RED_BLOCKS ? (nb > 0 ? nb : 1) : RED_BLOCKS);
-}
-template <typename T>
-void cg_p_fused(long long n, const T* part, int np, T* sc, const T* z, T* p, cudaStream_t st) {
-  pfem::count_launch();
-  cg_p_fused_kernel<T><<<fused_update_blocks(n), RED_THREADS, 0, st>>>(n, part, np, sc, z, p);
-}
-template <typename T>
-int cg_xr_fused(long long n, const T* part_pq, int np, T* sc, const T* p, const T* q, T* x, T* r, T* part_rr,
-                cudaStream_t st) {
-  const int blocks = fused_update_blocks(n);
-  pfem::count_launch();
-  cg_xr_fused_kernel<T><<<blocks, RED_THREADS, 0, st>>>(n, part_pq, np, sc, p, q, x, r, part_rr);
-  return blocks;
-}
-
 // BiCGStab helpers with device scalars s[0..]: see krylov code for layout.
 template <typename T>
 __global__ void bicg_p_kernel(long long n, const T* __restrict__ sc, const T* __restrict__ r,
@@ -678,22 +762,32 @@ void bc_apply(const BcDev& bc, double lam, double* U, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ coarse solve
-// Dense coarse solve y = Ainv b (one warp per row).
+// Dense coarse solve y = Ainv b (one warp per row; the row's first entries are in
+// flight before the wait for b).
 template <typename T>
-__global__ void dense_mv_kernel(int n, const T* __restrict__ M, const T* __restrict__ b, T* __restrict__ y) {
+__global__ void dense_mv_kernel(int n, const T* __restrict__ M, const T* b, T* y) {
+  pdl_go();
   const int row = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
+  constexpr int AHEAD = 6;
+  const T* m = M + (long long)row * n;
+  T a[AHEAD];
+#pragma unroll
+  for (int u = 0; u < AHEAD; ++u) a[u] = (row < n && lane + 32 * u < n) ? m[lane + 32 * u] : T(0);
+  pdl_wait();
   if (row >= n) return;
   T s = T(0);
-  for (int j = lane; j < n; j += 32) s += M[(long long)row * n + j] * b[j];
+#pragma unroll
+  for (int u = 0; u < AHEAD; ++u)
+    if (lane + 32 * u < n) s += a[u] * b[lane + 32 * u];
+  for (int j = lane + 32 * AHEAD; j < n; j += 32) s += m[j] * b[j];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) y[row] = s;
 }
 template <typename T>
-void dense_mv(int n, const T* M, const T* b, T* y, cudaStream_t st) {
-  const int blocks = (int)(((long long)n * 32 + 255) / 256);
-  pfem::count_launch(); dense_mv_kernel<T><<<blocks, 256, 0, st>>>(n, M, b, y);
+void dense_mv(int n, const T* M, const T* b, T* y, Queue q) {
+  launch(q, dense_mv_kernel<T>, (int)(((long long)n * 32 + 255) / 256), 256, 0, n, M, b, y);
 }
 
 // ------------------------------------------------------------------ smoothed aggregation
@@ -844,12 +938,12 @@ __global__ void sa_transpose_copy_kernel(int nnzP, const int* __restrict__ pt_bl
 // 16-byte aligned (double), as three 8- or 16-byte loads: every 6-value row of a
 // bs x 6 transfer block and every 6-vector of a coarse level is.
 template <typename T, bool STREAM>
-__device__ __forceinline__ void load6(const T* __restrict__ p, T* v) {
+__device__ __forceinline__ void load6(const T* p, T* v) {
   using V2 = typename std::conditional<std::is_same<T, float>::value, float2, double2>::type;
   const V2* q = reinterpret_cast<const V2*>(p);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const V2 w = STREAM ? __ldcs(q + k) : __ldg(q + k);
+    const V2 w = STREAM ? __ldcs(q + k) : q[k];
     v[2 * k] = w.x;
     v[2 * k + 1] = w.y;
   }
@@ -861,30 +955,51 @@ __device__ __forceinline__ void load6(const T* __restrict__ p, T* v) {
 // tree and the WPA warp sums are added in warp order, so the result is
 // deterministic.  Coarse levels have few aggregates of many blocks each; there
 // WPA = 4 spreads an aggregate over 128 lanes.
-template <typename T, int BS, int WPA>
+// START: the smoother's start on bc at the next level (block size 6) as well, sr =
+// Dinv bc and sd = co[CO_ITH] sr, from the six sums that the last warp holds.
+template <typename T, int BS, int WPA, bool START>
 __global__ void __launch_bounds__(256) sa_restrict_kernel(int nagg, const int* __restrict__ pt_rp,
                                                           const int* __restrict__ pt_row,
-                                                          const T* __restrict__ ptval, const T* __restrict__ r,
-                                                          T* __restrict__ bc) {
+                                                          const T* __restrict__ ptval, const T* r, T* bc,
+                                                          const T* __restrict__ dinv, const T* __restrict__ co, T* sr,
+                                                          T* sd) {
   __shared__ T part[8][6];
+  pdl_go();
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int I = blockIdx.x * (8 / WPA) + wid / WPA;
   const int w = wid % WPA;
   T s[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-  if (I < nagg) {
-    const int t1 = pt_rp[I + 1];
-    for (int t = pt_rp[I] + w * 32 + lane; t < t1; t += 32 * WPA) {
-      const T* P = ptval + (long long)t * BS * 6;
-      const T* rv = r + (long long)pt_row[t] * BS;
+  const bool in = I < nagg;
+  const int t1 = in ? pt_rp[I + 1] : 0;
+  int t = in ? pt_rp[I] + w * 32 + lane : 0;
+  // the first block of each lane is in flight before the wait for r
+  T pv[BS][6];
+  long long n = 0;
+  auto block = [&]() {
+    const T* P = ptval + (long long)t * BS * 6;
+    n = pt_row[t];
 #pragma unroll
-      for (int j = 0; j < BS; ++j) {
-        const T rj = rv[j];
-        T pv[6];
-        load6<T, false>(P + j * 6, pv);
+    for (int j = 0; j < BS; ++j) load6<T, false>(P + j * 6, pv[j]);
+  };
+  if (t < t1) block();
+  T D[6], ith = T(0);
+  const bool own = in && w == 0 && lane < 6;
+  if constexpr (START) {
 #pragma unroll
-        for (int c = 0; c < 6; ++c) s[c] += pv[c] * rj;
-      }
+    for (int j = 0; j < 6; ++j) D[j] = own ? dinv[(long long)I * 36 + lane * 6 + j] : T(0);
+    ith = co[CO_ITH];
+  }
+  pdl_wait();
+  while (t < t1) {
+    const T* rv = r + n * BS;
+#pragma unroll
+    for (int j = 0; j < BS; ++j) {
+      const T rj = rv[j];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) s[c] += pv[j][c] * rj;
     }
+    t += 32 * WPA;
+    if (t < t1) block();
   }
 #pragma unroll
   for (int c = 0; c < 6; ++c)
@@ -894,34 +1009,48 @@ __global__ void __launch_bounds__(256) sa_restrict_kernel(int nagg, const int* _
 #pragma unroll
   for (int c = 1; c < 6; ++c)
     if (lane == c) out = s[c];
-  if constexpr (WPA == 1) {
-    if (I < nagg && lane < 6) bc[(long long)I * 6 + lane] = out;
-  } else {
+  if constexpr (WPA > 1) {
     if (lane < 6) part[wid][lane] = out;
     __syncthreads();
-    if (w == 0 && I < nagg && lane < 6) {
-      T v = part[wid][lane];
+    if (w == 0 && lane < 6) {
 #pragma unroll
-      for (int q = 1; q < WPA; ++q) v += part[wid + q][lane];
-      bc[(long long)I * 6 + lane] = v;
+      for (int q = 1; q < WPA; ++q) out += part[wid + q][lane];
     }
   }
+  if constexpr (START) {
+    T v = T(0);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) v += D[j] * __shfl_sync(0xffffffffu, out, j);
+    if (own) {
+      sr[(long long)I * 6 + lane] = v;
+      sd[(long long)I * 6 + lane] = ith * v;
+    }
+  }
+  if (own) bc[(long long)I * 6 + lane] = out;
 }
 // Prolongation x[n*BS+j] += sum_{p in P row n} (P_p xc[col(p)])_j
 // (TWO: x += P (xc + xc2), the two corrections of a W-cycle visit).
 template <typename T, int BS, bool TWO = false>
 __global__ void sa_prolong_kernel(int nbrow, const int* __restrict__ p_rp, const int* __restrict__ p_cl,
-                                  const T* __restrict__ pval, const T* __restrict__ xc, const T* __restrict__ xc2,
-                                  T* __restrict__ x) {
+                                  const T* __restrict__ pval, const T* xc, const T* xc2, T* x) {
+  pdl_go();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)nbrow * BS) return;
+  const bool in = i < (long long)nbrow * BS;
   const int n = (int)(i / BS), j = (int)(i % BS);
+  int p = in ? p_rp[n] : 0;
+  const int p1 = in ? p_rp[n + 1] : 0;
+  // the first block's row is in flight before the wait for the corrections
+  T pv[6];
+  long long a = 0;
+  auto block = [&]() {
+    load6<T, true>(pval + (long long)p * BS * 6 + j * 6, pv);
+    a = (long long)p_cl[p] * 6;
+  };
+  if (p < p1) block();
+  pdl_wait();
   T s = T(0);
-  for (int p = p_rp[n]; p < p_rp[n + 1]; ++p) {
-    const T* P = pval + (long long)p * BS * 6 + j * 6;
-    const long long a = (long long)p_cl[p] * 6;
-    T pv[6], xv[6];
-    load6<T, true>(P, pv);
+  while (p < p1) {
+    T xv[6];
     load6<T, false>(xc + a, xv);
     if (TWO) {
       T x2v[6];
@@ -931,8 +1060,9 @@ __global__ void sa_prolong_kernel(int nbrow, const int* __restrict__ p_rp, const
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c) s += pv[c] * xv[c];
+    if (++p < p1) block();
   }
-  x[i] += s;
+  if (in) x[i] += s;
 }
 
 template <typename T>
@@ -970,54 +1100,47 @@ void sa_setup_level(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st) {
 constexpr int kRestrictWideBelow = 4096;
 
 template <typename T>
-void sa_restrict(const AmgLevel<T>& v, const T* r, T* bc, cudaStream_t st) {
+void sa_restrict(const AmgLevel<T>& v, const T* r, T* bc, const AmgLevel<T>* next, Queue q) {
   const bool wide = v.nagg < kRestrictWideBelow;
   const long long warps = (long long)v.nagg * (wide ? 4 : 1);
   const int blocks = (int)((warps + 7) / 8);
-  pfem::count_launch();
-  if (v.A.bs == 3) {
-    if (wide) sa_restrict_kernel<T, 3, 4><<<blocks, 256, 0, st>>>(v.nagg, v.pt_rp, v.pt_row, v.pt_val, r, bc);
-    else sa_restrict_kernel<T, 3, 1><<<blocks, 256, 0, st>>>(v.nagg, v.pt_rp, v.pt_row, v.pt_val, r, bc);
-  } else {
-    if (wide) sa_restrict_kernel<T, 6, 4><<<blocks, 256, 0, st>>>(v.nagg, v.pt_rp, v.pt_row, v.pt_val, r, bc);
-    else sa_restrict_kernel<T, 6, 1><<<blocks, 256, 0, st>>>(v.nagg, v.pt_rp, v.pt_row, v.pt_val, r, bc);
-  }
+  auto* kern = v.A.bs == 3 ? (wide ? (next ? sa_restrict_kernel<T, 3, 4, true> : sa_restrict_kernel<T, 3, 4, false>)
+                                   : (next ? sa_restrict_kernel<T, 3, 1, true> : sa_restrict_kernel<T, 3, 1, false>))
+                           : (wide ? (next ? sa_restrict_kernel<T, 6, 4, true> : sa_restrict_kernel<T, 6, 4, false>)
+                                   : (next ? sa_restrict_kernel<T, 6, 1, true> : sa_restrict_kernel<T, 6, 1, false>));
+  launch(q, kern, blocks, 256, 0, v.nagg, v.pt_rp, v.pt_row, v.pt_val, r, bc, next ? next->dinv : nullptr,
+         next ? next->co : nullptr, next ? next->r : nullptr, next ? next->d : nullptr);
 }
 template <typename T>
-static void prolong_launch(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, cudaStream_t st) {
+static void prolong_launch(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, const Queue& q) {
   const long long n = (long long)v.A.nbrow * v.A.bs;
-  const int blocks = (int)((n + 255) / 256);
-  pfem::count_launch();
-  if (v.A.bs == 3) {
-    if (xc2) sa_prolong_kernel<T, 3, true><<<blocks, 256, 0, st>>>(v.A.nbrow, v.p_rp, v.p_cl, v.p_val, xc, xc2, x);
-    else sa_prolong_kernel<T, 3><<<blocks, 256, 0, st>>>(v.A.nbrow, v.p_rp, v.p_cl, v.p_val, xc, xc, x);
-  } else {
-    if (xc2) sa_prolong_kernel<T, 6, true><<<blocks, 256, 0, st>>>(v.A.nbrow, v.p_rp, v.p_cl, v.p_val, xc, xc2, x);
-    else sa_prolong_kernel<T, 6><<<blocks, 256, 0, st>>>(v.A.nbrow, v.p_rp, v.p_cl, v.p_val, xc, xc, x);
-  }
+  auto* kern = v.A.bs == 3 ? (xc2 ? sa_prolong_kernel<T, 3, true> : sa_prolong_kernel<T, 3>)
+                           : (xc2 ? sa_prolong_kernel<T, 6, true> : sa_prolong_kernel<T, 6>);
+  launch(q, kern, (int)((n + 255) / 256), 256, 0, v.A.nbrow, v.p_rp, v.p_cl, v.p_val, xc, xc2, x);
 }
 template <typename T>
-void sa_prolong(const AmgLevel<T>& v, const T* xc, T* x, cudaStream_t st) {
-  prolong_launch<T>(v, xc, nullptr, x, st);
+void sa_prolong(const AmgLevel<T>& v, const T* xc, T* x, Queue q) {
+  prolong_launch<T>(v, xc, nullptr, x, q);
 }
 template <typename T>
-void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, cudaStream_t st) {
-  prolong_launch<T>(v, xc, xc2, x, st);
+void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, Queue q) {
+  prolong_launch<T>(v, xc, xc2, x, q);
 }
 
 // ------------------------------------------------------------------ instantiations
 #define PFEM_INST(T)                                                                               \
-  template void bsr_spmv<T>(const BsrMat<T>&, const T*, T*, cudaStream_t);                         \
-  template void bsr_residual<T>(const BsrMat<T>&, const T*, const T*, T*, cudaStream_t);           \
+  template int bsr_spmv<T>(const BsrMat<T>&, const T*, T*, Queue, double*);                        \
+  template void bsr_residual<T>(const BsrMat<T>&, const T*, const T*, T*, Queue);                  \
   template void bsr_cheb_step<T>(const BsrMat<T>&, const T*, const T*, T*, T*, cudaStream_t);      \
-  template void bsr_cheb2<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, bool, const T*, cudaStream_t); \
-  template void bsr_residual_precond<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, const T*, \
-                                        cudaStream_t);                                             \
+  template int bsr_cheb2<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, bool, const T*, Queue, const T*, \
+                            double*);                                                              \
+  template void bsr_residual_precond<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, const T*, Queue); \
+  template void bsr_residual_start<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, T*, const T*, Queue); \
   template void bsr_power_step<T>(const BsrMat<T>&, const T*, const T*, T*, cudaStream_t);         \
   template int norm2_partials<T>(long long, const T*, double*, cudaStream_t);                      \
   template void scale_by_norm<T>(long long, const double*, int, T*, cudaStream_t);                 \
   template void power_finish<T>(int, const double*, const double*, T*, cudaStream_t);              \
-  template void blockdiag_apply<T>(int, int, const T*, const T*, T*, const T*, T*, cudaStream_t);  \
+  template void blockdiag_apply<T>(int, int, const T*, const T*, T*, const T*, T*, Queue);         \
   template void blockdiag_invert<T>(const BsrMat<T>&, T*, cudaStream_t);                           \
   template void dot<T>(long long, const T*, const T*, T*, T*, cudaStream_t, bool);                 \
   template void fill<T>(long long, T*, T, cudaStream_t);                                           \
@@ -1029,18 +1152,18 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, cudaStre
   template void bicg_xr<T>(long long, const T*, const T*, const T*, const T*, const T*, T*, T*,    \
                            cudaStream_t);                                                          \
   template void scalar_copy<T>(T*, const T*, cudaStream_t);                                        \
-  template int dot_partials<T>(long long, const T*, const T*, T*, cudaStream_t);                   \
-  template void cg_p_fused<T>(long long, const T*, int, T*, const T*, T*, cudaStream_t);           \
-  template int cg_xr_fused<T>(long long, const T*, int, T*, const T*, const T*, T*, T*, T*,         \
-                              cudaStream_t);                                                       \
+  template int dot_partials_double<T>(long long, const T*, const T*, double*, const Queue&);       \
+  template void cg_p_fused<T>(long long, const double*, int, T*, const T*, T*, Queue);             \
+  template void cg_xr_fused<T>(int, const double*, int, T*, const T*, const T*, T*, T*, const T*, const T*, T*, T*, \
+                               const CgLoop&, Queue);                                              \
   template void add_to_double<T>(long long, const T*, double*, cudaStream_t);                      \
   template void impose_dirichlet<T>(const BcDev&, long long, double, const double*, T*, double*,   \
                                     double*, cudaStream_t);                                        \
-  template void dense_mv<T>(int, const T*, const T*, T*, cudaStream_t);                            \
+  template void dense_mv<T>(int, const T*, const T*, T*, Queue);                            \
   template void sa_setup_level<T>(const AmgLevel<T>&, T*, int, cudaStream_t);                   \
-  template void sa_restrict<T>(const AmgLevel<T>&, const T*, T*, cudaStream_t);                    \
-  template void sa_prolong<T>(const AmgLevel<T>&, const T*, T*, cudaStream_t);                     \
-  template void sa_prolong2<T>(const AmgLevel<T>&, const T*, const T*, T*, cudaStream_t);
+  template void sa_restrict<T>(const AmgLevel<T>&, const T*, T*, const AmgLevel<T>*, Queue);       \
+  template void sa_prolong<T>(const AmgLevel<T>&, const T*, T*, Queue);                     \
+  template void sa_prolong2<T>(const AmgLevel<T>&, const T*, const T*, T*, Queue);
 PFEM_INST(float)
 PFEM_INST(double)
 template void convert<double, float>(long long, const double*, float*, double, cudaStream_t);

@@ -24,6 +24,27 @@
 
 namespace pfem {
 
+// What an SpMV works on, and what it does with a row's sum v = (A x), by mode:
+//   0: y = v   1: y = b - v   2: y -= Dinv v, xo += x   3: xo = c2 x + c1 (y - Dinv v)
+//   4: as 3, added to xo      5: y = Dinv (b - v), xo = y / th      6: y = Dinv v
+//   7: z = b - v, y = Dinv z, xo = y / th
+// 2 is a Chebyshev step on x = d; 3 and 4 the degree-2 smoother in one pass (x = d0,
+// y = r0); 5 its start on a residual, 7 the same with the residual kept; 6 a step of
+// the power iteration.  1 / th, c1 and c2 are the level's scalars co.  Vectors that
+// earlier kernels of a programmatic launch chain write are not __restrict__ const: such
+// a load could be served by the read-only path while they are still being written.
+template <typename T>
+struct SpmvVec {
+  const T* x = nullptr;
+  T* y = nullptr;
+  const T* b = nullptr;
+  const T* dinv = nullptr;
+  T* xo = nullptr;
+  const T* co = nullptr;
+  T* z = nullptr;
+  double* part = nullptr;  // partials of x.y (mode 0) or b.xo (mode 4), one per CTA
+};
+
 constexpr long long kPipeWaitLimit = 1ll << 20;  // polls of a barrier before a kernel gives up
 
 __device__ __forceinline__ uint32_t pipe_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -117,20 +138,16 @@ __device__ __forceinline__ void pipe_issue(unsigned char* stage, const PipeLay& 
   if (vb) pipe_copy_first(dst, (const char*)val + va, vb, bar);
 }
 
-// What the modes do with a row's sum v (A x), row by row:
-//   0: y = v   1: y = b - v   2: y -= Dinv v, xo += x   3: xo = c2 x + c1 (y - Dinv v)
-//   4: as 3, added to xo      5: y = Dinv (b - v), xo = y / th      6: y = Dinv v
-// (1 / th, c1, c2 from co)
-template <typename T, int BS, int MODE, bool C16>
+template <typename T, int BS, int MODE, bool C16, bool DOT>
 __global__ void __launch_bounds__(32)
 bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__ rowptr, const int* __restrict__ col,
-                     const int16_t* __restrict__ col16, const T* __restrict__ val, const T* x, T* y, const T* b,
-                     const T* __restrict__ dinv, T* xo, const T* co, int* err) {
+                     const int16_t* __restrict__ col16, const T* __restrict__ val, SpmvVec<T> a, int* err) {
   using SH = PipeShape<T, BS>;
   constexpr int R = SH::ROWS, BB = BS * BS;
   extern __shared__ __align__(128) unsigned char psm[];
   const PipeLay lay = pipe_lay<T, BS>(max_row, C16);
   const int lane = threadIdx.x;
+  pdl_go();
   unsigned char* const st = psm + kPipeHead;
   const uint32_t bar = pipe_smem(psm);
   int n0 = 0, n1 = 0;  // block range of the next tile to copy (lane 0)
@@ -148,8 +165,10 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
   }
   __syncwarp();
   uint32_t phase = 0;
-  const T c1 = MODE == 3 || MODE == 4 ? co[CO_C1] : MODE == 5 ? co[CO_ITH] : T(0);
-  const T c2 = MODE == 3 || MODE == 4 ? co[CO_C2] : T(0);
+  const T c1 = MODE == 3 || MODE == 4 ? a.co[CO_C1] : MODE == 5 || MODE == 7 ? a.co[CO_ITH] : T(0);
+  const T c2 = MODE == 3 || MODE == 4 ? a.co[CO_C2] : T(0);
+  double dot = 0.0;
+  pdl_wait();  // the first tile is on its way
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
     // a lane's row(s) of the tile and the epilogue's operands, in flight while the tile arrives
     if constexpr (BS == 3) {
@@ -162,13 +181,14 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
       if (own) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-          if (MODE == 1 || MODE == 5) bi[i] = b[at + i];
-          if (MODE == 2 || MODE == 3 || MODE == 4) { yi[i] = y[at + i]; xi[i] = x[at + i]; }
-          if (MODE == 2 || MODE == 4) oi[i] = xo[at + i];
+          if (MODE == 1 || MODE == 5 || MODE == 7 || (DOT && MODE == 4)) bi[i] = a.b[at + i];
+          if (MODE == 2 || MODE == 3 || MODE == 4) yi[i] = a.y[at + i];
+          if (MODE == 2 || MODE == 3 || MODE == 4 || (DOT && MODE == 0)) xi[i] = a.x[at + i];
+          if (MODE == 2 || MODE == 4) oi[i] = a.xo[at + i];
         }
         if (MODE >= 2) {
 #pragma unroll
-          for (int i = 0; i < 9; ++i) D[i] = dinv[(long long)row * 9 + i];
+          for (int i = 0; i < 9; ++i) D[i] = a.dinv[(long long)row * 9 + i];
         }
       }
       if (!__all_sync(0xffffffffu, pipe_bar_wait(bar, phase))) {
@@ -195,7 +215,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           const bool in = q < len;
           const long long c = in ? (C16 ? row + (int)cs16[q] : cs[q]) : 0;
 #pragma unroll
-          for (int j = 0; j < 3; ++j) xv[m][j] = in ? x[c * 3 + j] : T(0);
+          for (int j = 0; j < 3; ++j) xv[m][j] = in ? a.x[c * 3 + j] : T(0);
         }
 #pragma unroll
         for (int m = 0; m < NP; ++m) {
@@ -226,27 +246,37 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
       if (own) {
         if (MODE == 0) {
 #pragma unroll
-          for (int i = 0; i < 3; ++i) y[at + i] = v[i];
+          for (int i = 0; i < 3; ++i) {
+            a.y[at + i] = v[i];
+            if (DOT) dot += (double)xi[i] * (double)v[i];
+          }
         } else if (MODE == 1) {
 #pragma unroll
-          for (int i = 0; i < 3; ++i) y[at + i] = bi[i] - v[i];
+          for (int i = 0; i < 3; ++i) a.y[at + i] = bi[i] - v[i];
         } else {
+          if (MODE == 5 || MODE == 7) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) v[i] = bi[i] - v[i];
+          }
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             T w = T(0);
 #pragma unroll
-            for (int j = 0; j < 3; ++j) w += D[i * 3 + j] * (MODE == 5 ? bi[j] - v[j] : v[j]);
+            for (int j = 0; j < 3; ++j) w += D[i * 3 + j] * v[j];
             if (MODE == 2) {
-              y[at + i] = yi[i] - w;
-              xo[at + i] = oi[i] + xi[i];
-            } else if (MODE == 5) {
-              y[at + i] = w;
-              xo[at + i] = c1 * w;
+              a.y[at + i] = yi[i] - w;
+              a.xo[at + i] = oi[i] + xi[i];
+            } else if (MODE == 5 || MODE == 7) {
+              if (MODE == 7) a.z[at + i] = v[i];
+              a.y[at + i] = w;
+              a.xo[at + i] = c1 * w;
             } else if (MODE == 6) {
-              y[at + i] = w;
+              a.y[at + i] = w;
             } else {
-              const T upd = c2 * xi[i] + c1 * (yi[i] - w);
-              xo[at + i] = MODE == 3 ? upd : oi[i] + upd;
+              T upd = c2 * xi[i] + c1 * (yi[i] - w);
+              if (MODE == 4) upd = oi[i] + upd;
+              a.xo[at + i] = upd;
+              if (DOT) dot += (double)bi[i] * (double)upd;
             }
           }
         }
@@ -264,12 +294,12 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
 #pragma unroll
         for (int j = 0; j < BS; ++j) D[j] = T(0);
         if (own) {
-          if (MODE == 1 || MODE == 5) bi = b[at];
-          if (MODE == 2 || MODE == 3 || MODE == 4) { yi = y[at]; xi = x[at]; }
-          if (MODE == 2 || MODE == 4) oi = xo[at];
+          if (MODE == 1 || MODE == 5 || MODE == 7) bi = a.b[at];
+          if (MODE == 2 || MODE == 3 || MODE == 4) { yi = a.y[at]; xi = a.x[at]; }
+          if (MODE == 2 || MODE == 4) oi = a.xo[at];
           if (MODE >= 2) {
 #pragma unroll
-            for (int j = 0; j < BS; ++j) D[j] = dinv[(long long)row * BB + hl * BS + j];
+            for (int j = 0; j < BS; ++j) D[j] = a.dinv[(long long)row * BB + hl * BS + j];
           }
         }
         if (!waited) {
@@ -288,7 +318,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           const bool in = q < b1;
           const long long c = in ? cs[q] : 0;
 #pragma unroll
-          for (int j = 0; j < BS; ++j) xv[h][j] = in ? x[c * BS + j] : T(0);
+          for (int j = 0; j < BS; ++j) xv[h][j] = in ? a.x[c * BS + j] : T(0);
         }
         T acc[BS];
 #pragma unroll
@@ -325,26 +355,27 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           if (hl == i) v = acc[i];
         T w = T(0);
         if (MODE >= 2) {
-          const T e = MODE == 5 ? bi - v : v;
+          if (MODE == 5 || MODE == 7) v = bi - v;
 #pragma unroll
-          for (int j = 0; j < BS; ++j) w += D[j] * __shfl_sync(0xffffffffu, e, (lane & 16) + j);
+          for (int j = 0; j < BS; ++j) w += D[j] * __shfl_sync(0xffffffffu, v, (lane & 16) + j);
         }
         if (!own) continue;
         if (MODE == 0) {
-          y[at] = v;
+          a.y[at] = v;
         } else if (MODE == 1) {
-          y[at] = bi - v;
+          a.y[at] = bi - v;
         } else if (MODE == 2) {
-          y[at] = yi - w;
-          xo[at] = oi + xi;
-        } else if (MODE == 5) {
-          y[at] = w;
-          xo[at] = c1 * w;
+          a.y[at] = yi - w;
+          a.xo[at] = oi + xi;
+        } else if (MODE == 5 || MODE == 7) {
+          if (MODE == 7) a.z[at] = v;
+          a.y[at] = w;
+          a.xo[at] = c1 * w;
         } else if (MODE == 6) {
-          y[at] = w;
+          a.y[at] = w;
         } else {
           const T upd = c2 * xi + c1 * (yi - w);
-          xo[at] = MODE == 3 ? upd : oi + upd;
+          a.xo[at] = MODE == 3 ? upd : oi + upd;
         }
       }
       if (!waited) {
@@ -359,6 +390,11 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
         n1 = tf < ntiles ? rowptr[min(tf * R + R, nbrow)] : 0;
       }
     }
+  }
+  if constexpr (DOT) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    if (lane == 0) a.part[blockIdx.x] = dot;
   }
 }
 
