@@ -133,6 +133,7 @@ struct pfem_ctx {
   // in each, the longest block row, element-ordered tangents and forces (lazy)
   int *dNptr = nullptr, *dNel = nullptr;
   uint8_t* dNloc = nullptr;
+  unsigned* dWords = nullptr;  // sources of every block of K (nodes in at most eight elements)
   int max_row = 0;
   bool colored_assembly = false;
   float* dKbuf32 = nullptr;
@@ -1206,7 +1207,8 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
       if (small) launch_element_small<double>(a, ctx->dAllElems, (int)ctx->ne, false, ctx->hard, st);
       else launch_element_color<double>(a, ctx->dAllElems, (int)ctx->ne, false, fbar, ctx->hard, st);
       launch_gather_rows<double>((int)ctx->nn, ctx->dNptr, ctx->dNel, ctx->dNloc, ctx->dBrowptr, ctx->dRank,
-                                 ctx->dKbuf64, ctx->dFbuf, ctx->dK64, ctx->dR, ctx->max_row, st);
+                                 ctx->dWords, ctx->dKbuf64, ctx->dFbuf, ctx->dK64, ctx->dR, ctx->max_row,
+                                 &ctx->dBack->waits, st);
     } else {
       if (!ctx->dKbuf32) CK(dalloc(ctx, &ctx->dKbuf32, (size_t)ctx->ne * 576));
       ElemArgs<float> a{};
@@ -1218,7 +1220,8 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
       if (small) launch_element_small<float>(a, ctx->dAllElems, (int)ctx->ne, false, ctx->hard, st);
       else launch_element_color<float>(a, ctx->dAllElems, (int)ctx->ne, false, fbar, ctx->hard, st);
       launch_gather_rows<float>((int)ctx->nn, ctx->dNptr, ctx->dNel, ctx->dNloc, ctx->dBrowptr, ctx->dRank,
-                                ctx->dKbuf32, ctx->dFbuf, ctx->dK32, ctx->dR, ctx->max_row, st);
+                                ctx->dWords, ctx->dKbuf32, ctx->dFbuf, ctx->dK32, ctx->dR, ctx->max_row,
+                                &ctx->dBack->waits, st);
     }
     CKL();
     return PFEM_OK;
@@ -1891,6 +1894,16 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
         }
       });
       if (fits) UP(ctx->dBcol16, c16, kCopySlack);
+    }
+    bool eight = ctx->max_row <= 32;
+    for (int64_t n = 0; n < nn && eight; ++n) eight = nptr[n + 1] - nptr[n] <= 8;
+    if (eight) {
+      AL(ctx->dWords, (size_t)ctx->nnzb);
+      launch_gather_words((int)nn, ctx->dNptr, ctx->dNel, ctx->dNloc, ctx->dBrowptr, ctx->dRank, ctx->dWords, ctx->st);
+      if ((ce = cudaGetLastError()) != cudaSuccess) {
+        pfem_set_cuda_error(ce, "gather words", __FILE__, __LINE__);
+        return bail(PFEM_ERR_CUDA);
+      }
     }
     const char* am = getenv("PFEM_ASSEMBLY");
     ctx->colored_assembly = am && std::string(am) == "colored";

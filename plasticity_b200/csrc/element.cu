@@ -27,8 +27,10 @@
 // on principal values: the trial stress is an isotropic function of b^e, so
 // its deviator and the flow direction share b^e's eigenbasis, and the
 // reference's global-Voigt formulas reduce to these principal ones exactly.
+#include <algorithm>
 #include <type_traits>
 
+#include "bulk_copy.cuh"
 #include "common.cuh"
 #include "pfem_internal.h"
 
@@ -1112,79 +1114,172 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(int nn, const int* __r
   if (lane < 3) R[(long long)a * 3 + lane] = fr;
 }
 
-// Rows of at most 32 blocks (every hex mesh: 27): lane p of the node's warp owns
-// block p of the row in registers.  The node's element ids, positions and rank
-// bytes are loaded once, one element per lane; then, element by element in
-// increasing order, the lane whose position appears among the element's eight
-// rank bytes (at most one does, per column node b) adds that 3 x 3 block.  The
-// value loads of different elements do not depend on each other, nothing goes
-// through shared memory, and each lane sums in the same element order as the
-// shared-memory gather above.
+// A node's sources, one word per block of its row: nibble j is 1 + the column node's
+// position in the node's j-th incident element, 0 where it is not in it (the first
+// position where an element names a node twice).  For nodes in at most eight elements.
+__global__ void __launch_bounds__(256) gather_words_kernel(int nn, const int* __restrict__ nptr,
+                                                           const int* __restrict__ nel,
+                                                           const uint8_t* __restrict__ nloc,
+                                                           const int* __restrict__ browptr,
+                                                           const uint8_t* __restrict__ rank,
+                                                           unsigned* __restrict__ words) {
+  const int a = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (a >= nn) return;
+  const int r0 = browptr[a], len = browptr[a + 1] - r0, q0 = nptr[a], nq = nptr[a + 1] - q0;
+  for (int p = lane; p < len; p += 32) {
+    unsigned w = 0u;
+    for (int j = 0; j < nq && j < 8; ++j) {
+      const uint8_t* rk = rank + (long long)nel[q0 + j] * 64 + nloc[q0 + j] * 8;
+      for (int b = 7; b >= 0; --b)
+        if (rk[b] == p) w = (w & ~(15u << (4 * j))) | ((unsigned)(b + 1) << (4 * j));
+    }
+    words[r0 + p] = w;
+  }
+}
+void launch_gather_words(int nn, const int* nptr, const int* nel, const uint8_t* nloc, const int* browptr,
+                         const uint8_t* rank, unsigned* words, cudaStream_t st) {
+  pfem::count_launch();
+  gather_words_kernel<<<(nn + 7) / 8, 256, 0, st>>>(nn, nptr, nel, nloc, browptr, rank, words);
+}
+
+// Rows of at most 32 blocks whose nodes are in at most eight elements (every box of
+// hexes).  What bounds it is HBM: every K_e value once in, every K value once out (948 MB
+// at 64^3, FP32: 145 us at the copy bandwidth).  A warp per node that matched rank
+// bytes and loaded its slices into registers took 402 us: 900 instructions per node and
+// a chain of dependent loads too long for the warps its registers left; staging those
+// slices in shared memory with 16-byte loads took 485 us.  This takes 165 us (FP64 650
+// -> 315 us).  Here a warp goes through its nodes with the
+// next one's slices (288 or 576 bytes per element, cp.async.bulk by one lane each)
+// already on their way to the other half of its shared memory, the indices of the two
+// after that in flight, and the matches read from the precomputed words.  Lane p owns
+// block p and adds in element order, as above; the finished row leaves through shared
+// memory in consecutive stores.
+constexpr int GS_WARPS = 4;
 template <typename KT>
-__global__ void __launch_bounds__(256) gather_rows_lane_kernel(int nn, const int* __restrict__ nptr,
-                                                               const int* __restrict__ nel,
-                                                               const uint8_t* __restrict__ nloc,
-                                                               const int* __restrict__ browptr,
-                                                               const uint8_t* __restrict__ rank,
-                                                               const KT* __restrict__ Kbuf,
-                                                               const double* __restrict__ Fbuf,
-                                                               KT* __restrict__ Kval, double* __restrict__ R) {
+struct GatherStage {
+  KT k[8 * 72];
+  double f[24];
+};
+template <typename KT>
+__global__ void __launch_bounds__(32 * GS_WARPS) gather_rows_stream_kernel(
+    int nn, const int* __restrict__ nptr, const int* __restrict__ nel, const uint8_t* __restrict__ nloc,
+    const int* __restrict__ browptr, const unsigned* __restrict__ words, const KT* __restrict__ Kbuf,
+    const double* __restrict__ Fbuf, KT* __restrict__ Kval, double* __restrict__ R, int* err) {
+  __shared__ __align__(16) GatherStage<KT> stage[GS_WARPS][2];
+  __shared__ __align__(8) uint64_t bars[GS_WARPS][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int a = (int)blockIdx.x * (int)(blockDim.x >> 5) + warp;
-  if (a >= nn) return;  // whole warps
-  const int r0 = browptr[a], len = browptr[a + 1] - r0;
-  const int q0 = nptr[a], nq = nptr[a + 1] - q0;
-  const unsigned key = (unsigned)lane * 0x01010101u;
-  KT acc[9];
+  const int step = (int)gridDim.x * GS_WARPS, first = (int)blockIdx.x * GS_WARPS + warp;
+  if (first >= nn) return;  // whole warps; nothing below is block-wide
+  const uint32_t bar = bulk_smem(bars[warp]);
+  if (lane == 0) {
+    bulk_bar_init(bar, 1);
+    bulk_bar_init(bar + 8, 1);
+    bulk_init_fence();
+  }
+  __syncwarp();
+  constexpr uint32_t SLICE = 72 * sizeof(KT);
+  // node n: its incidence range; the lane's element and position in it
+  auto range = [&](int n, int& q0, int& nq) {
+    q0 = n < nn ? nptr[n] : 0;
+    nq = n < nn ? nptr[n + 1] - q0 : 0;
+  };
+  auto entry = [&](int q0, int nq, int& e, int& al) {
+    e = lane < nq ? nel[q0 + lane] : 0;
+    al = lane < nq ? nloc[q0 + lane] : 0;
+  };
+  auto issue = [&](int s, int nq, int e, int al) {
+    if (nq == 0) return;
+    bulk_fence();  // the row that left through this half before the copies into it
+    if (lane == 0) bulk_expect(bar + 8 * s, (uint32_t)nq * SLICE);
+    __syncwarp();
+    if (lane < nq)
+      bulk_copy_first(bulk_smem(stage[warp][s].k) + lane * SLICE, Kbuf + (long long)e * 576 + al * 72, SLICE, bar + 8 * s);
+  };
+  int q0a, nqa, q0b, nqb, ea, ala, eb, alb;  // a: the current node's, b: the next one's
+  range(first, q0a, nqa);
+  range(first + step, q0b, nqb);
+  entry(q0a, nqa, ea, ala);
+  issue(0, nqa, ea, ala);
+  entry(q0b, nqb, eb, alb);
+  int q0c, nqc;
+  range(first + 2 * step, q0c, nqc);
+  int s = 0;
+  uint32_t phase = 0;  // bit s: the phase that half s waits for next
+  for (int a = first; a < nn; a += step) {
+    const int r0 = browptr[a], len = browptr[a + 1] - r0;
+    const unsigned w = lane < len ? words[r0 + lane] : 0u;
+    // force rows of the node, lane 3 j + d
+    const int fj = lane / 3;
+    const int fe = __shfl_sync(0xffffffffu, ea, fj), fa = __shfl_sync(0xffffffffu, ala, fj);
+    const double fv = fj < nqa ? Fbuf[(long long)fe * 24 + fa * 3 + (lane - 3 * fj)] : 0.0;
+    if (a + step < nn) issue(s ^ 1, nqb, eb, alb);
+    int ec, alc, q0d, nqd;
+    entry(q0c, nqc, ec, alc);
+    range(a + 3 * step, q0d, nqd);
+    KT acc[9];
 #pragma unroll
-  for (int v = 0; v < 9; ++v) acc[v] = KT(0);
-  double fr = 0.0;
-  for (int base = 0; base < nq; base += 32) {
-    const int cnt = min(32, nq - base);
-    int e_l = 0, al_l = 0;
-    unsigned lo_l = 0xFFFFFFFFu, hi_l = 0xFFFFFFFFu;
-    if (lane < cnt) {
-      e_l = nel[q0 + base + lane];
-      al_l = nloc[q0 + base + lane];
-      const uint2 rk = *reinterpret_cast<const uint2*>(rank + (long long)e_l * 64 + al_l * 8);
-      lo_l = rk.x;
-      hi_l = rk.y;
-    }
-#pragma unroll 4
-    for (int j = 0; j < cnt; ++j) {
-      const int e = __shfl_sync(0xffffffffu, e_l, j), al = __shfl_sync(0xffffffffu, al_l, j);
-      const unsigned lo = __shfl_sync(0xffffffffu, lo_l, j), hi = __shfl_sync(0xffffffffu, hi_l, j);
-      const unsigned ml = __vcmpeq4(lo, key), mh = __vcmpeq4(hi, key);
-      const int b = ml ? ((__ffs(ml) - 1) >> 3) : (mh ? 4 + ((__ffs(mh) - 1) >> 3) : -1);
-      if (b >= 0) {
-        const KT* src = Kbuf + (long long)e * 576 + al * 72 + b * 3;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) acc[i * 3 + k] += __ldcs(src + i * 24 + k);
+    for (int v = 0; v < 9; ++v) acc[v] = KT(0);
+    GatherStage<KT>& S = stage[warp][s];
+    if (lane < 24) S.f[lane] = fv;
+    if (nqa > 0) {
+      if (!__all_sync(0xffffffffu, bulk_bar_wait(bar + 8 * s, (phase >> s) & 1u))) {
+        // report it, and leave only when the other half's copies have landed as well
+        if (lane == 0) atomicExch(err, 1);
+        if (a + step < nn && nqb > 0) bulk_bar_wait(bar + 8 * (s ^ 1), (phase >> (s ^ 1)) & 1u);
+        return;
       }
-      if (lane < 3) fr += Fbuf[(long long)e * 24 + al * 3 + lane];
+      phase ^= 1u << s;
     }
-  }
-  if (lane < len) {
-    KT* dst = Kval + (long long)(r0 + lane) * 9;
+    __syncwarp();
+    double fr = 0.0;
 #pragma unroll
-    for (int v = 0; v < 9; ++v) dst[v] = acc[v];
+    for (int j = 0; j < 8; ++j) {
+      if (j < nqa) {
+        const unsigned b = (w >> (4 * j)) & 15u;
+        if (b) {
+          const KT* src = S.k + j * 72 + (int)b * 3 - 3;
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc[i * 3 + k] += src[i * 24 + k];
+        }
+        if (lane < 3) fr += S.f[3 * j + lane];
+      }
+    }
+    __syncwarp();
+    if (lane < len) {
+#pragma unroll
+      for (int v = 0; v < 9; ++v) S.k[lane * 9 + v] = acc[v];
+    }
+    __syncwarp();
+    KT* const dst = Kval + (long long)r0 * 9;
+    for (int v = lane; v < len * 9; v += 32) dst[v] = S.k[v];
+    if (lane < 3) R[(long long)a * 3 + lane] = fr;
+    __syncwarp();
+    nqa = nqb; ea = eb; ala = alb;
+    nqb = nqc; eb = ec; alb = alc;
+    q0c = q0d; nqc = nqd;
+    s ^= 1;
   }
-  if (lane < 3) R[(long long)a * 3 + lane] = fr;
 }
 
 template <typename KT>
 void launch_gather_rows(int nn, const int* nptr, const int* nel, const uint8_t* nloc, const int* browptr,
-                        const uint8_t* rank, const KT* Kbuf, const double* Fbuf, KT* Kval, double* R, int maxlen,
-                        cudaStream_t st) {
+                        const uint8_t* rank, const unsigned* words, const KT* Kbuf, const double* Fbuf, KT* Kval, double* R,
+                        int maxlen, int* err, cudaStream_t st) {
   constexpr int WARPS = 8;
   const size_t sm = (size_t)WARPS * maxlen * 9 * sizeof(KT);
   const int blocks = (nn + WARPS - 1) / WARPS;
   if (blocks <= 0) return;
-  if (maxlen <= 32) {
+  if (words && maxlen <= 32) {
+    int dev = 0, sms = 148, per = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, gather_rows_stream_kernel<KT>, 32 * GS_WARPS, 0);
+    const int grid = std::min((nn + GS_WARPS - 1) / GS_WARPS, sms * std::max(per, 1));
     pfem::count_launch();
-    gather_rows_lane_kernel<KT><<<blocks, 32 * WARPS, 0, st>>>(nn, nptr, nel, nloc, browptr, rank, Kbuf, Fbuf, Kval, R);
+    gather_rows_stream_kernel<KT><<<grid, 32 * GS_WARPS, 0, st>>>(nn, nptr, nel, nloc, browptr, words, Kbuf, Fbuf, Kval, R,
+                                                                  err);
     return;
   }
   if (sm > 48 * 1024)  // rows longer than a hex mesh's 27 blocks (the 8-bit rank table caps them at 256)
@@ -1194,9 +1289,11 @@ void launch_gather_rows(int nn, const int* nptr, const int* nel, const uint8_t* 
                                                         maxlen);
 }
 template void launch_gather_rows<double>(int, const int*, const int*, const uint8_t*, const int*, const uint8_t*,
-                                         const double*, const double*, double*, double*, int, cudaStream_t);
+                                         const unsigned*, const double*, const double*, double*, double*, int, int*,
+                                         cudaStream_t);
 template void launch_gather_rows<float>(int, const int*, const int*, const uint8_t*, const int*, const uint8_t*,
-                                        const float*, const double*, float*, double*, int, cudaStream_t);
+                                        const unsigned*, const float*, const double*, float*, double*, int, int*,
+                                        cudaStream_t);
 
 template void launch_element_color<double>(const ElemArgs<double>&, const int*, int, bool, bool, int, cudaStream_t);
 template void launch_element_color<float>(const ElemArgs<float>&, const int*, int, bool, bool, int, cudaStream_t);

@@ -49,10 +49,14 @@ void launch_element_small(const ElemArgs<KT>& a, const int* elist, int n, bool c
 // the elements incident to node a in increasing element order (nptr/nel, with
 // nloc the node's position in the element), of the element buffers' (a, b)
 // blocks and force rows.  Every block of K and every entry of R is written once.
+// words (launch_gather_words; null when a node is in more than eight elements) names
+// the sources of every block of K; err: see BsrMat.
 template <typename KT>
 void launch_gather_rows(int nn, const int* nptr, const int* nel, const uint8_t* nloc, const int* browptr,
-                        const uint8_t* rank, const KT* Kbuf, const double* Fbuf, KT* Kval, double* R, int maxlen,
-                        cudaStream_t st);
+                        const uint8_t* rank, const unsigned* words, const KT* Kbuf, const double* Fbuf, KT* Kval, double* R,
+                        int maxlen, int* err, cudaStream_t st);
+void launch_gather_words(int nn, const int* nptr, const int* nel, const uint8_t* nloc, const int* browptr,
+                         const uint8_t* rank, unsigned* words, cudaStream_t st);
 
 // One-time topology on the device (topology.cu): per-node block rows
 // (count pass with col = null, fill pass with rowptr) and the rank table.

@@ -20,6 +20,7 @@
 #pragma once
 #include <cstdint>
 
+#include "bulk_copy.cuh"
 #include "linalg.cuh"
 
 namespace pfem {
@@ -44,47 +45,6 @@ struct SpmvVec {
   T* z = nullptr;
   double* part = nullptr;  // partials of x.y (mode 0) or b.xo (mode 4), one per CTA
 };
-
-constexpr long long kPipeWaitLimit = 1ll << 20;  // polls of a barrier before a kernel gives up
-
-__device__ __forceinline__ uint32_t pipe_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void pipe_bar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ bool pipe_bar_wait(uint32_t bar, uint32_t phase) {
-  for (long long it = 0; it < kPipeWaitLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(phase)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void pipe_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void pipe_expect(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Both addresses and the size are multiples of 16 bytes.
-__device__ __forceinline__ void pipe_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-// The same, with the lines marked for early eviction: a matrix that is streamed once
-// per pass should not push the gathered vector out of L2.
-__device__ __forceinline__ void pipe_copy_first(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], pol;\n\t}\n" ::
-          "r"(dst), "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
 
 // LANES lanes per row and ROWS rows per tile; a CTA is one warp with one tile in shared
 // memory (8 rows of 27 blocks: 8 KB float, 16 KB double; 4 rows of 6 x 6: 15 KB), so
@@ -131,11 +91,11 @@ __device__ __forceinline__ void pipe_issue(unsigned char* stage, const PipeLay& 
   const uint32_t vb = (uint32_t)((((long long)s1 * VB + 15) & ~15ll) - va);
   const uint32_t cb = (uint32_t)((((long long)s1 * CB + 15) & ~15ll) - ca);
   const uint32_t rb = (uint32_t)(((rows + 1) * 4 + 15) & ~15);
-  const uint32_t dst = pipe_smem(stage);
-  pipe_expect(bar, vb + cb + rb);
-  pipe_copy(dst + lay.rows, rowptr + r0, rb, bar);
-  if (cb) pipe_copy(dst + lay.cols, (C16 ? (const char*)col16 : (const char*)col) + ca, cb, bar);
-  if (vb) pipe_copy_first(dst, (const char*)val + va, vb, bar);
+  const uint32_t dst = bulk_smem(stage);
+  bulk_expect(bar, vb + cb + rb);
+  bulk_copy(dst + lay.rows, rowptr + r0, rb, bar);
+  if (cb) bulk_copy(dst + lay.cols, (C16 ? (const char*)col16 : (const char*)col) + ca, cb, bar);
+  if (vb) bulk_copy_first(dst, (const char*)val + va, vb, bar);
 }
 
 template <typename T, int BS, int MODE, bool C16, bool DOT>
@@ -149,12 +109,11 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
   const int lane = threadIdx.x;
   pdl_go();
   unsigned char* const st = psm + kPipeHead;
-  const uint32_t bar = pipe_smem(psm);
+  const uint32_t bar = bulk_smem(psm);
   int n0 = 0, n1 = 0;  // block range of the next tile to copy (lane 0)
   if (lane == 0) {
-    pipe_bar_init(bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    bulk_bar_init(bar, 1);
+    bulk_init_fence();
     const int t = blockIdx.x, tn = t + gridDim.x;
     const int s0 = rowptr[t * R], s1 = rowptr[min(t * R + R, nbrow)];
     if (tn < ntiles) {
@@ -191,7 +150,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           for (int i = 0; i < 9; ++i) D[i] = a.dinv[(long long)row * 9 + i];
         }
       }
-      if (!__all_sync(0xffffffffu, pipe_bar_wait(bar, phase))) {
+      if (!__all_sync(0xffffffffu, bulk_bar_wait(bar, phase))) {
         if (lane == 0) atomicExch(err, 1);
         return;
       }
@@ -303,7 +262,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           }
         }
         if (!waited) {
-          waited = __all_sync(0xffffffffu, pipe_bar_wait(bar, phase));
+          waited = __all_sync(0xffffffffu, bulk_bar_wait(bar, phase));
           if (!waited) break;
         }
         const int* rp = reinterpret_cast<const int*>(st + lay.rows);
