@@ -85,10 +85,13 @@ __device__ __forceinline__ void eig3_jacobi(double* a, double* w, double* V) {
       const int o = 3 - p - q;
       const double apq = a[3 * p + q];
       if (apq != 0.0) {
-        const double theta = (a[3 * q + q] - a[3 * p + p]) / (2.0 * apq);
-        double t;
-        if (fabs(theta) > 1e150) t = 0.5 / theta;
-        else t = copysign(1.0, theta) / (fabs(theta) + sqrt(theta * theta + 1.0));
+        // t = sign(theta) / (|theta| + sqrt(theta^2 + 1)), theta = d / h, without the
+        // quotient: two divisions and two square roots per rotation
+        const double d = a[3 * q + q] - a[3 * p + p], h = 2.0 * apq;
+        const double den = fabs(d) + sqrt(d * d + h * h);
+        const double t = den > 0.0 ? copysign(1.0, d) * h / den : 1.0;  // 0: h^2 underflows beside d = 0
+        // not rsqrt: it makes the rotations less orthogonal (the residual's error against
+        // 64 bits grows by an eighth) for 2.5 % of the element kernel
         const double c = 1.0 / sqrt(t * t + 1.0);
         const double s = t * c;
         a[3 * p + p] -= t * apq;

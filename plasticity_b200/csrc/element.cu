@@ -1,22 +1,27 @@
-// element.cu -- K1: fused per-color F-bar Hex8 element kernel + colored scatter.
+// element.cu -- K1: fused F-bar Hex8 element kernel, and the row gather that forms K and R.
 //
-// One warp owns four elements of one color.  Phase A: lane (slot, g) evaluates
+// One warp owns four elements.  Phase A: lane (slot, g) evaluates
 // Gauss point g of element `slot`: geometry, F / F-bar, trial b^e and its
 // eigenbasis, the J2 radial return in principal stresses, P = tau F^-T and the
 // two-point tangent A = dP/dFbar built column by column in the eigenbasis of
 // b^e.  The internal force is summed over the element's eight Gauss-point
-// lanes node by node with warp shuffles (FP64) and added into R; the tangent
+// lanes node by node with warp shuffles (FP64); the tangent
 // records (dN/dX, w s A, w s/3 A vec(F), F^-1) go to shared memory in the
 // tangent's type TT (FP32 on the mixed-precision path, where only the tangent
 // is FP32).  The Kirchhoff stress and the elastic/plastic flag are written,
-// and on the commit pass the exponential-map plastic update.  Phase B: the
-// 4 x 24 columns (b,k) of the warp's four element tangents are spread over the
-// 32 lanes; each sums the eight Gauss-point contributions
+// and on the commit pass the exponential-map plastic update.  Phase B, for each
+// component k in turn: lane (slot, b) sums the eight Gauss-point contributions to the
+// column (b, k) of its element's tangent
 //   Ke[:,(b,k)] = sum_g G_g^T (w s A G_g + (w s/3) A vec(F) (g0 - gJ)^T)[:,(b,k)]
-// (lagrangian/src/Elements.jl:470-478 with _fbar_Geff :524-531) and adds them
-// into the 3x3-block CSR tangent in place.  Elements of one color share no
-// node, so the adds need no atomics (lagrangian/src/Assembly.jl:167-188,
-// :370-385).
+// (lagrangian/src/Elements.jl:470-478 with _fbar_Geff :524-531).  Going by k, only a
+// third of A is in shared memory at a time and no lane is idle.
+//
+// What bounds it: instruction issue at the 8 (FP64) or 12 (FP32) warps per SM that its
+// registers allow, with the dependent FP64 arithmetic of phase A in between.  At 64^3,
+// FP32 tangent / FP64: 0.82 / 1.16 ms.  With the whole of A in shared memory (6 warps
+// per SM in FP64), the 96 columns of a warp taken 32 at a time, single-word reads and
+// single multiply-adds: 1.02 / 1.57 ms, 2,480 instructions per element (now 1,640).
+// Three columns per lane at once (FP32): 0.88 ms, its accumulators cost warps.
 //
 // Arithmetic follows the reference kernel element_force_tangent_finite!
 // (Elements.jl:405-494), finite_kinematics (FiniteStrain.jl:148-170),
@@ -37,17 +42,25 @@
 namespace pfem {
 
 constexpr int EPW = 4;                     // elements per warp
-constexpr int GPREC = 24 + 81 + 9 + 9;     // dNdX, w s A, w s/3 A vec(F), F^-1 (TT each)
-constexpr int SLOT_TT = 24 + 8 * GPREC;    // g0, then the 8 Gauss-point records
+// A Gauss point's tangent record (TT each): dN/dX by component, [j][a]; the columns
+// (q, k) of w s A for the k at hand, [q][r] with the rows r = 3 j + i at a stride of 10;
+// w s/3 A vec(F), [r]; F^-1 transposed, [k][j] at a stride of 4.  All parts start on 16
+// bytes; 84 = 20 mod 32 words and 82 = 2 mod 16 double words spread an element's eight
+// points over the banks.
+constexpr int REC_A = 24, REC_AQ = 10, REC_U = REC_A + 32, REC_FI = REC_U + 12;
+template <typename TT>
+constexpr int gprec() { return sizeof(TT) == 4 ? REC_FI + 16 : REC_FI + 14; }
+template <typename TT>
+constexpr int slot_tt() { return 24 + 8 * gprec<TT>(); }  // g0, then the 8 Gauss-point records
 constexpr int WPB = 1;                     // warps per block
 // Shared memory per warp (bytes).  The element's nodal coordinates and
 // displacements (48 doubles) live at the start of the record area until the
 // geometry is formed, then the records overwrite them.
 template <typename TT>
 constexpr int warp_smem_bytes(bool commit) {
-  return commit ? EPW * 48 * 8 : EPW * SLOT_TT * (int)sizeof(TT);
+  return commit ? EPW * 48 * 8 : EPW * slot_tt<TT>() * (int)sizeof(TT);
 }
-static_assert(8 * GPREC * 4 >= 48 * 8, "coordinate scratch must fit in the record area");
+static_assert(8 * gprec<float>() * 4 >= 48 * 8, "coordinate scratch must fit in the record area");
 
 __device__ __forceinline__ double nsgn_x(int a) { return (((a + 1) >> 1) & 1) ? 1.0 : -1.0; }
 __device__ __forceinline__ double nsgn_y(int a) { return ((a >> 1) & 1) ? 1.0 : -1.0; }
@@ -59,6 +72,48 @@ __device__ __forceinline__ void dshape_a(int a, double x, double y, double z, do
   d[0] = 0.125 * xa * (1.0 + ya * y) * (1.0 + za * z);
   d[1] = 0.125 * ya * (1.0 + xa * x) * (1.0 + za * z);
   d[2] = 0.125 * za * (1.0 + xa * x) * (1.0 + ya * y);
+}
+
+// Two floats in one register pair: fma.rn.f32x2 does two of the tangent's
+// multiply-adds per issue slot, each rounded as the single one.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 dup2(float a) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ void split2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+// N (even) consecutive values to or from shared memory, two per access (8-byte aligned
+// floats, 16-byte aligned doubles).
+template <int N, typename TT>
+__device__ __forceinline__ void store_pairs(TT* d, const TT* v) {
+  using V2 = typename std::conditional<std::is_same<TT, float>::value, float2, double2>::type;
+#pragma unroll
+  for (int m = 0; m < N / 2; ++m) {
+    V2 w;
+    w.x = v[2 * m];
+    w.y = v[2 * m + 1];
+    reinterpret_cast<V2*>(d)[m] = w;
+  }
+}
+template <int N, typename TT>
+__device__ __forceinline__ void load_pairs(const TT* s, TT* v) {
+  using V2 = typename std::conditional<std::is_same<TT, float>::value, float2, double2>::type;
+#pragma unroll
+  for (int m = 0; m < N / 2; ++m) {
+    const V2 w = reinterpret_cast<const V2*>(s)[m];
+    v[2 * m] = w.x;
+    v[2 * m + 1] = w.y;
+  }
 }
 
 // ---- saturation (Voce) hardening: yield_stress / yield_slope (Materials.jl:117-127)
@@ -122,15 +177,15 @@ __device__ __forceinline__ T sym_dot(const T* a, const T* b) {
   return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + T(2) * (a[3] * b[3] + a[4] * b[4] + a[5] * b[5]);
 }
 
-// With FP32 tangent records the kernel is occupancy-bound: capping registers
-// for 11 resident one-warp blocks per SM (a little spilling to L1) measured
-// 14 % faster at 64^3 than the unconstrained 222 registers (9 blocks); the
-// FP64 variants lose from the same cap and keep the compiler's choice.
-// The kinematic variant carries more live state and keeps the compiler's choice.
+// With FP32 tangent records registers are capped for 11 resident one-warp blocks per SM
+// (168 registers, 12 blocks, a little spilling to L1); caps for 14 and 16 blocks took
+// 1.05 ms where this takes 0.98 (64^3 assembly).  The FP64 variants lose from a cap and
+// keep the compiler's choice, as does the kinematic variant with its extra state.
 template <typename KT, bool COMMIT, bool FBAR, int HARD>
 __global__ void __launch_bounds__(32 * WPB, (std::is_same<KT, float>::value && !COMMIT && HARD != HARD_KIN) ? 11 : 1)
 element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
   using TT = KT;  // type of the tangent records and of the phase-B arithmetic
+  constexpr int GPREC = gprec<TT>(), SLOT_TT = slot_tt<TT>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = lane >> 3, g = lane & 7;
@@ -290,7 +345,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
   const double e0 = 0.5 * log(bv[0]), e1 = 0.5 * log(bv[1]), e2 = 0.5 * log(bv[2]);
   const double tre = e0 + e1 + e2;
   const double t0 = lam * tre + 2.0 * G * e0, t1 = lam * tre + 2.0 * G * e1, t2 = lam * tre + 2.0 * G * e2;
-  const double pm = (t0 + t1 + t2) / 3.0;
+  const double pm = (t0 + t1 + t2) * (1.0 / 3.0);
   const double s0 = t0 - pm, s1 = t1 - pm, s2 = t2 - pm;
   const double s32 = 1.22474487139158904910;  // sqrt(1.5)
   // Kinematic hardening (finite_stress_update, FiniteStrain.jl:316-324): the
@@ -351,7 +406,8 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       dg = ftr / (3.0 * G + H + m.Hkin);
       g0c = 2.0 * G / (3.0 * G + m.Hkin + H);
     } else {
-      n0 = s0 / nrm; n1 = s1 / nrm; n2 = s2 / nrm;
+      const double inrm = 1.0 / nrm;
+      n0 = s0 * inrm; n1 = s1 * inrm; n2 = s2 * inrm;
       if constexpr (HARD == HARD_VOCE) {
         double Hp;
         dg = voce_dgamma(m, sy0, qtr, an, ftr, &Hp);
@@ -502,9 +558,9 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       const double x0 = d[0] * Ji[0] + d[1] * Ji[3] + d[2] * Ji[6];
       const double x1 = d[0] * Ji[1] + d[1] * Ji[4] + d[2] * Ji[7];
       const double x2 = d[0] * Ji[2] + d[1] * Ji[5] + d[2] * Ji[8];
-      Rg[a * 3 + 0] = (TT)x0;
-      Rg[a * 3 + 1] = (TT)x1;
-      Rg[a * 3 + 2] = (TT)x2;
+      Rg[a] = (TT)x0;
+      Rg[8 + a] = (TT)x1;
+      Rg[16 + a] = (TT)x2;
       double v0 = w * (P[0] * x0 + P[1] * x1 + P[2] * x2);
       double v1 = w * (P[3] * x0 + P[4] * x1 + P[5] * x2);
       double v2 = w * (P[6] * x0 + P[7] * x1 + P[8] * x2);
@@ -534,14 +590,14 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
 #pragma unroll
     for (int A = 0; A < 3; ++A)
 #pragma unroll
-      for (int B = 0; B < 3; ++B) {
-        double v;
-        if (A == B) v = 1.0 / (2.0 * bv[A]);
-        else if (fabs(bv[A] - bv[B]) < 1e-9 * (fabs(bv[A]) + fabs(bv[B]) + 1.0)) v = 1.0 / (bv[A] + bv[B]);
-        else v = (lyv[A] - lyv[B]) / (bv[A] - bv[B]);
+      for (int B = A; B < 3; ++B) {
+        const double sum = bv[A] + bv[B], dif = bv[A] - bv[B];
+        const bool near = A == B || fabs(dif) < 1e-9 * (fabs(bv[A]) + fabs(bv[B]) + 1.0);
+        const double v = (near ? 1.0 : lyv[A] - lyv[B]) / (near ? sum : dif);
         gam[3 * A + B] = (TT)v;
+        gam[3 * B + A] = (TT)v;
       }
-    TT Qt[9], MQ[9], NN[9], FbiT[9], Pt[9], Ft[9];  // MQ = (Cp Fb^T) Q, NN = Q^T Fb^-T
+    TT Qt[9], MQ[9], NN[9], FbiT[9], Pt[9];  // MQ = (Cp Fb^T) Q, NN = Q^T Fb^-T
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -549,7 +605,6 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
         FbiT[3 * i + j] = (TT)Fbi[3 * j + i];
         Qt[3 * i + j] = (TT)Q[3 * i + j];
         Pt[3 * i + j] = (TT)P[3 * i + j];
-        Ft[3 * i + j] = (TT)F[3 * i + j];
       }
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -595,11 +650,34 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       }
     }
     const TT ws_ = (TT)(w * scale);
-    TT* const As = Rg + 24;  // [(j*3+i)*9 + (q*3+p)]
-    TT uacc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    {
+      // w s/3 A vec(F), the F-bar vector, in closed form: along F the elastic strain
+      // changes by I / s, which no flow direction sees (it is deviatoric) and no polar
+      // rotation follows, so dP = (3 K Fbar^-T - P) / s.
+      const double uf = w * (1.0 / 3.0), k3 = 3.0 * lam + 2.0 * G;
+      TT u[REC_AQ], fi[12];
 #pragma unroll
-    for (int col = 0; col < 9; ++col) {
-      const int pp = col % 3, qq = col / 3;
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) u[3 * j + i] = FBAR ? (TT)(uf * (k3 * Fbi[3 * j + i] - P[3 * i + j])) : TT(0);
+      u[9] = TT(0);
+      store_pairs<REC_AQ>(Rg + REC_U, u);
+      // F^-1 of the standard F = scale * Fb^-1 (for gJ = G^T vec(F^-T))
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) fi[4 * k + j] = (TT)(scale * Fbi[3 * j + k]);
+        fi[4 * k + 3] = TT(0);
+      }
+      store_pairs<12>(Rg + REC_FI, fi);
+    }
+    // ---- per k: the three columns (q, k) of A by every Gauss point, then (phase B) the
+    // columns (b, k) of the four element tangents by lane (slot, b) ----
+    const int b = g;
+#pragma unroll
+    for (int pp = 0; pp < 3; ++pp) {
+#pragma unroll
+    for (int qq = 0; qq < 3; ++qq) {
       TT Y[9];
 #pragma unroll
       for (int A = 0; A < 3; ++A)
@@ -661,91 +739,133 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       for (int A = 0; A < 3; ++A)
 #pragma unroll
         for (int j = 0; j < 3; ++j) T[3 * A + j] = dt[3 * A] * NN[j] + dt[3 * A + 1] * NN[3 + j] + dt[3 * A + 2] * NN[6 + j];
-      const TT Fq = Ft[3 * pp + qq];  // standard F for the F-bar vec(F)
+      TT wdP[REC_AQ];
+      wdP[9] = TT(0);
 #pragma unroll
       for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           const TT dP = Qt[3 * i] * T[j] + Qt[3 * i + 1] * T[3 + j] + Qt[3 * i + 2] * T[6 + j] - Pt[3 * i + qq] * FbiT[3 * pp + j];
-          As[(j * 3 + i) * 9 + col] = ws_ * dP;
-          uacc[j * 3 + i] += dP * Fq;
+          wdP[j * 3 + i] = ws_ * dP;
         }
+      store_pairs<REC_AQ>(Rg + REC_A + qq * REC_AQ, wdP);
     }
-    const TT uf = (TT)(w * scale / 3.0);
-#pragma unroll
-    for (int r = 0; r < 9; ++r) Rg[105 + r] = FBAR ? uf * uacc[r] : TT(0);
-    // F^-1 of the standard F = scale * Fb^-1 (for gJ = G^T vec(F^-T))
-#pragma unroll
-    for (int i = 0; i < 9; ++i) Rg[114 + i] = (TT)(scale * Fbi[i]);
     __syncwarp();
-
-  // ---- Phase B: the warp's 4 x 24 Ke columns over 32 lanes, scatter into
-  // the block-CSR tangent ----
+    TT acc[24];  // rows (a, i) of the column
+    const TT g0bk = FBAR ? g0s[3 * b + pp] : TT(0);
+    if constexpr (std::is_same<TT, float>::value) {
+      f32x2 acc2[3][4];  // [i][pair of a]
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) acc2[i][m] = 0ull;
 #pragma unroll 1
-  for (int t = lane; t < EPW * 24; t += 32) {
-    const int s = t / 24, col = t - 24 * s;
-    const long long ls = ((long long)blockIdx.x * WPB + warp) * EPW + s;
-    if (ls >= nlist) continue;
-    const int es = elist[ls];
-    const TT* Ss = wbase + s * SLOT_TT;
-    const int b = col / 3, k = col - 3 * b;
-    TT acc[24];
+      for (int gg = 0; gg < 8; ++gg) {
+        const float* Rr = S + 24 + gg * GPREC;
+        const float db0 = Rr[b], db1 = Rr[8 + b], db2 = Rr[16 + b];
+        f32x2 A[16];  // [q][pair of r] at a stride of 5
 #pragma unroll
-    for (int r = 0; r < 24; ++r) acc[r] = TT(0);
-    const TT g0bk = FBAR ? Ss[col] : TT(0);
+        for (int h = 0; h < 8; ++h) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + REC_A + 4 * h);
+          A[2 * h] = v.x;
+          A[2 * h + 1] = v.y;
+        }
+        f32x2 T2[5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          T2[m] = mul2(A[m], dup2(db0));
+          fma2(T2[m], A[5 + m], dup2(db1));
+          fma2(T2[m], A[10 + m], dup2(db2));
+        }
+        if constexpr (FBAR) {
+          // dg_(b,k) = g0_(b,k) - gJ_(b,k),  gJ_(b,k) = sum_j F^-1[j][k] dNdX[b][j]
+          const float4 fi = *reinterpret_cast<const float4*>(Rr + REC_FI + 4 * pp);
+          const float dg = g0bk - (fi.x * db0 + fi.y * db1 + fi.z * db2);
+#pragma unroll
+          for (int h = 0; h < 3; ++h) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + REC_U + 4 * h);
+            fma2(T2[2 * h], v.x, dup2(dg));
+            if (h < 2) fma2(T2[2 * h + 1], v.y, dup2(dg));
+          }
+        }
+        float T[10];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) split2(T2[m], T[2 * m], T[2 * m + 1]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const ulonglong2 x0 = *reinterpret_cast<const ulonglong2*>(Rr + 8 * j);
+          const ulonglong2 x1 = *reinterpret_cast<const ulonglong2*>(Rr + 8 * j + 4);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const f32x2 t = dup2(T[3 * j + i]);
+            fma2(acc2[i][0], x0.x, t);
+            fma2(acc2[i][1], x0.y, t);
+            fma2(acc2[i][2], x1.x, t);
+            fma2(acc2[i][3], x1.y, t);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) split2(acc2[i][m], acc[6 * m + i], acc[6 * m + 3 + i]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 24; ++r) acc[r] = TT(0);
 #pragma unroll 1
-    for (int gg = 0; gg < 8; ++gg) {
-      const TT* Rr = Ss + 24 + gg * GPREC;
-      const TT* dX = Rr;
-      const TT* A = Rr + 24;
-      const TT* u = Rr + 105;
-      const TT* Fi = Rr + 114;
-      const TT db0 = dX[b * 3], db1 = dX[b * 3 + 1], db2 = dX[b * 3 + 2];
-      // dg_(b,k) = g0_(b,k) - gJ_(b,k),  gJ_(b,k) = sum_j F^-1[j][k] dNdX[b][j]
-      const TT dgbk = FBAR ? (g0bk - (Fi[k] * db0 + Fi[3 + k] * db1 + Fi[6 + k] * db2)) : TT(0);
-      TT T[9];
+      for (int gg = 0; gg < 8; ++gg) {
+        const TT* Rr = S + 24 + gg * GPREC;
+        const TT db0 = Rr[b], db1 = Rr[8 + b], db2 = Rr[16 + b];
+        TT T[REC_AQ], v[REC_AQ];
+        load_pairs<REC_AQ>(Rr + REC_A, v);
 #pragma unroll
-      for (int r = 0; r < 9; ++r)
-        T[r] = A[r * 9 + k] * db0 + A[r * 9 + 3 + k] * db1 + A[r * 9 + 6 + k] * db2 + u[r] * dgbk;
+        for (int r = 0; r < 9; ++r) T[r] = v[r] * db0;
+        load_pairs<REC_AQ>(Rr + REC_A + REC_AQ, v);
 #pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const TT x0 = dX[a * 3], x1 = dX[a * 3 + 1], x2 = dX[a * 3 + 2];
+        for (int r = 0; r < 9; ++r) T[r] += v[r] * db1;
+        load_pairs<REC_AQ>(Rr + REC_A + 2 * REC_AQ, v);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) acc[a * 3 + i] += x0 * T[i] + x1 * T[3 + i] + x2 * T[6 + i];
+        for (int r = 0; r < 9; ++r) T[r] += v[r] * db2;
+        if constexpr (FBAR) {
+          TT fi[4];
+          load_pairs<4>(Rr + REC_FI + 4 * pp, fi);
+          const TT dg = g0bk - (fi[0] * db0 + fi[1] * db1 + fi[2] * db2);
+          load_pairs<REC_AQ>(Rr + REC_U, v);
+#pragma unroll
+          for (int r = 0; r < 9; ++r) T[r] += v[r] * dg;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          TT x[8];
+          load_pairs<8>(Rr + 8 * j, x);
+#pragma unroll
+          for (int a = 0; a < 8; ++a)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) acc[a * 3 + i] += x[a] * T[3 * j + i];
+        }
       }
     }
-    if (p.Kbuf) {
-      // element-ordered: column (b,k) of rows (a,i) at [es][a][i][col]; the 24
-      // lanes of an element write 24 consecutive values per (a,i)
-      KT* kb = p.Kbuf + (long long)es * 576 + col;
+    if (valid) {
+      if (p.Kbuf) {
+        // element-ordered: column (b,k) of rows (a,i) at [e][a][i][(b,k)]
+        KT* kb = p.Kbuf + (long long)e * 576 + 3 * b + pp;
 #pragma unroll
-      for (int a = 0; a < 8; ++a)
+        for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) __stcs(kb + a * 72 + i * 24, (KT)acc[a * 3 + i]);
-      continue;
+          for (int i = 0; i < 3; ++i) __stcs(kb + a * 72 + i * 24, (KT)acc[a * 3 + i]);
+      } else {
+        // in place (colored): the eight target blocks lie in eight different block rows
+        const int* nds = nodes_s[warp][slot];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+          KT* vp = p.Kval + ((long long)p.browptr[nds[a]] + p.rank[(long long)e * 64 + a * 8 + b]) * 9 + pp;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) vp[3 * i] += (KT)acc[a * 3 + i];
+        }
+      }
     }
-    // The eight target blocks lie in eight different block rows, so nothing
-    // aliases: all 24 loads are issued before any store (one memory latency
-    // per column instead of a chain of eight).
-    const int* nds = nodes_s[warp][s];
-    KT* vp[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-      vp[a] = p.Kval + ((long long)p.browptr[nds[a]] + p.rank[(long long)es * 64 + a * 8 + b]) * 9 + k;
-    KT old[24];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      old[a * 3 + 0] = vp[a][0];
-      old[a * 3 + 1] = vp[a][3];
-      old[a * 3 + 2] = vp[a][6];
+    __syncwarp();  // the next k's columns overwrite these
     }
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      vp[a][0] = old[a * 3 + 0] + (KT)acc[a * 3 + 0];
-      vp[a][3] = old[a * 3 + 1] + (KT)acc[a * 3 + 1];
-      vp[a][6] = old[a * 3 + 2] + (KT)acc[a * 3 + 2];
-    }
-  }
   }  // !COMMIT
 }
 
