@@ -813,8 +813,8 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
                                   ctx->dDenseWork, A.coarse_inv, ctx->st);
     CKL();
   } else {
-    CK(pfem::pivot_inverse<T>((int)A.coarse_nnzb, A.lv[L - 1].c_row, A.coarse_cl, A.coarse_val, A.coarse_n, A.coarse_inv,
-                              ctx->st));
+    CK(pfem::pivot_inverse<T>((int)A.coarse_nnzb, A.lv[L - 1].c_row, A.coarse_cl, A.coarse_val, A.coarse_n,
+                              ctx->dDenseWork, A.coarse_inv, ctx->st));
   }
   A.built = true;
   A.version++;

@@ -77,46 +77,69 @@ __global__ void dense_diag_max_kernel(int n, const double* __restrict__ A, doubl
   }
 }
 
-// Dg = A[K,K]^{-1}: in-place Gauss-Jordan on the NB x NB diagonal block in
-// shared memory, one CTA of 1024 threads (four entries each).
-__global__ void __launch_bounds__(1024) gj_diag_kernel(int n, int kb, const double* __restrict__ A,
-                                                       double* __restrict__ Dg, const double* __restrict__ scl) {
-  __shared__ double M[NB][NB + 1];
-  const int t = threadIdx.x;
-  for (int e = t; e < NB * NB; e += 1024) M[e / NB][e % NB] = A[(long long)(kb + e / NB) * n + kb + e % NB];
+// Dg = A[K,K]^{-1}: in-place Gauss-Jordan on the NB x NB diagonal block, one CTA of
+// eight warps with the block in registers: warp w holds the columns w, w + 8, ..., lane
+// l the rows l and l + 32.  What bounds it is the chain of 64 steps, so each has one
+// __syncthreads: the column's warp publishes it as the multipliers, every warp takes the
+// pivot from there.  As in pivot_inverse_kernel a row is divided by its pivot at the
+// end.  19.7 us; with the block in shared memory and five barriers per step 60 us.
+__global__ void __launch_bounds__(256) gj_diag_kernel(int n, int kb, const double* __restrict__ A,
+                                                      double* __restrict__ Dg, const double* __restrict__ scl) {
+  __shared__ double F[2][NB];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double a[8][2];
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) a[m][r] = A[(long long)(kb + lane + 32 * r) * n + kb + w + 8 * m];
   const double floor_abs = 1e-14 * fmax(scl[0], 1e-300);
-  for (int k = 0; k < NB; ++k) {
-    __syncthreads();
-    double piv = M[k][k];
-    if (fabs(piv) < floor_abs) piv = piv >= 0.0 ? floor_abs : -floor_abs;
-    const double ip = 1.0 / piv;
-    __syncthreads();
-    if (t < NB) M[k][t] = (t == k ? 1.0 : M[k][t]) * ip;
-    __syncthreads();
-    double f[4];
-    int ii[4], jj[4];
+  double ips[2] = {1.0, 1.0};  // 1 / pivot of the lane's rows
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = t + q * 1024;
-      ii[q] = e / NB;
-      jj[q] = e % NB;
-      f[q] = M[ii[q]][k];
-    }
-    __syncthreads();
+  for (int m0 = 0; m0 < 8; ++m0) {
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+      const int k = 8 * m0 + q, kl = k & 31;
+      constexpr int HALF = 4;  // k < 32 exactly when m0 < HALF
+      const int kr = m0 < HALF ? 0 : 1;
+      double* const f = F[k & 1];
+      if (w == q) {
+        f[lane] = a[m0][0];
+        f[lane + 32] = a[m0][1];
+      }
+      __syncthreads();
+      double pv = f[k];
+      double f0 = f[lane], f1 = f[lane + 32];
+      double e[8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (ii[q] == k) continue;
-      const double old = jj[q] == k ? 0.0 : M[ii[q]][jj[q]];
-      M[ii[q]][jj[q]] = old - f[q] * M[k][jj[q]];
+      for (int m = 0; m < 8; ++m) e[m] = __shfl_sync(0xffffffffu, a[m][kr], kl);
+      if (fabs(pv) < floor_abs) pv = pv >= 0.0 ? floor_abs : -floor_abs;
+      const double ip = 1.0 / pv;
+      if (lane == kl) {
+        ips[kr] = ip;
+        if (kr == 0) f0 = 0.0; else f1 = 0.0;
+      }
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const double x = e[m] * ip;
+        a[m][0] = fma(-f0, x, a[m][0]);
+        a[m][1] = fma(-f1, x, a[m][1]);
+      }
+      if (w == q) {  // the column becomes the inverse's
+        a[m0][0] = -f0 * ip;
+        a[m0][1] = -f1 * ip;
+        if (lane == kl) a[m0][kr] = 1.0;
+      }
     }
   }
-  __syncthreads();
-  for (int e = t; e < NB * NB; e += 1024) Dg[e] = M[e / NB][e % NB];
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) Dg[(lane + 32 * r) * NB + w + 8 * m] = a[m][r] * ips[r];
 }
 
 // Panel step kb.  CTAs [0, ncb): 64 panel-row columns each, A[K, j] <- Dg A[K, j]
-// for j outside K (the 64 x 64 slab staged in shared memory; thread (column,
-// quarter) computes 16 rows).  CTAs [ncb, ...): C[i, :] = A[i, K] for rows i
+// for j outside K (the 64 x 64 slab staged in shared memory; a thread computes four
+// rows of four columns, 16 apart: eight reads for 16 multiply-adds).  CTAs [ncb, ...): C[i, :] = A[i, K] for rows i
 // outside K, a warp per row.
 __global__ void __launch_bounds__(256) gj_panel_kernel(int n, int kb, int ncb, double* __restrict__ A,
                                                        double* __restrict__ C, const double* __restrict__ Dg) {
@@ -141,19 +164,31 @@ __global__ void __launch_bounds__(256) gj_panel_kernel(int n, int kb, int ncb, d
     V[r][c] = j < n ? A[(long long)(kb + r) * n + j] : 0.0;
   }
   __syncthreads();
-  const int c = t & 63, q = t >> 6, j = j0 + c;
-  if (j >= n) return;
-  double out[16];
+  const int c = t & 15, q = t >> 4;
+  double out[4][4];
 #pragma unroll
-  for (int r = 0; r < 16; ++r) out[r] = 0.0;
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) out[r][u] = 0.0;
 #pragma unroll 8
   for (int s = 0; s < NB; ++s) {
-    const double v = V[s][c];
+    double d[4], v[4];
 #pragma unroll
-    for (int r = 0; r < 16; ++r) out[r] += D[q * 16 + r][s] * v;
+    for (int r = 0; r < 4; ++r) d[r] = D[q * 4 + r][s];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = V[s][c + 16 * u];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) out[r][u] += d[r] * v[u];
   }
 #pragma unroll
-  for (int r = 0; r < 16; ++r) A[(long long)(kb + q * 16 + r) * n + j] = out[r];
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = j0 + c + 16 * u;
+      if (j < n) A[(long long)(kb + q * 4 + r) * n + j] = out[r][u];
+    }
 }
 
 // Trailing update of step kb over TR_ x TC_ tiles; rows of the panel are final.
@@ -217,19 +252,20 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(int n, int kb, double
 // CPW of them, lane l the rows l, l + 32, ...
 //
 // In-place Gauss-Jordan: column c of the identity is never stored.  Rows are not
-// exchanged: step c takes the unused row with the largest |a[., c]| (the lowest such
-// row when equal) and remembers it, and the inverse is written through that
+// exchanged: step c takes the unused row with the largest |a[., c]| (to 11 bits, the
+// lowest such row when equal) and remembers it, and the inverse is written through that
 // permutation.  A pivot row is not divided by its pivot until the end (its later
 // updates are linear in it), so an update is one fused multiply-add per entry, with a
 // multiplier of 0 in the pivot row.  What bounds it is the chain of n steps and their
 // instructions.  A pivot search needs one column only, so the CTA that owns a panel
 // runs the panel's steps by itself (one __syncthreads each), keeping the multipliers
 // of every step in shared memory; one cluster barrier later the other CTAs copy them
-// and apply the whole panel to their own columns without any barrier.  Measured at
-// 162 unknowns (the coarsest level at 8^3 and 64^3): 215 us; with a barrier of
+// (through global memory, W: seven CTAs reading one's shared memory at once took five
+// times as long) and apply the whole panel to their own columns without any barrier.  Measured at
+// 162 unknowns (the coarsest level at 8^3 and 64^3): 173 us; with a barrier of
 // the cluster per step 551 us, dividing at once and selecting the pivot row in every
-// update 286 us; the host's inverse with its two copies took 600-750 us.
-constexpr int PC = 8, PT = 512;  // CTAs of the cluster, threads of a CTA
+// update 286 us, the copies from the owner's shared memory 224 us; the host's inverse with its two copies took 600-750 us.
+constexpr int PC = 8, PT = 256;  // CTAs of the cluster, threads of a CTA
 
 inline int pivot_cols(int n) { return (n + PC - 1) / PC; }
 inline size_t pivot_smem(int n) { return (size_t)2 * pivot_cols(n) * n * sizeof(double); }
@@ -237,7 +273,7 @@ inline size_t pivot_smem(int n) { return (size_t)2 * pivot_cols(n) * n * sizeof(
 template <typename T, int RR, int CPW>
 __global__ void __cluster_dims__(PC, 1, 1) __launch_bounds__(PT)
 pivot_inverse_kernel(int cp, int nnzb, const int* __restrict__ br, const int* __restrict__ cl, const T* __restrict__ val,
-                     int n, T* __restrict__ inv) {
+                     int n, double* W, T* __restrict__ inv) {
   constexpr int NW = PT / 32, CMAX = NW * CPW;
   extern __shared__ __align__(16) double pvm[];
   __shared__ double ipv[2][CMAX];  // 1 / pivot of the own panel's steps, of a copied panel's
@@ -300,65 +336,52 @@ pivot_inverse_kernel(int cp, int nnzb, const int* __restrict__ br, const int* __
   for (int q = 0; q < NW; ++q) scl = fmax(scl, wmax[q]);
   const double floor_abs = 1e-14 * fmax(scl, 1e-300);
   unsigned used = 0;  // of this lane's rows, bit r
-  // Step with multipliers f, pivot row p, 1 / pivot ip on the warp's columns but `skip`.
+  // Step with multipliers f (the pivot row's entry counts as 0), pivot row p, 1 / pivot ip
+  // on the warp's columns but `skip`, which becomes the inverse's.
   auto apply = [&](const double* f, int p, double ip, int skip) {
     const int pr = p >> 5, pl = p & 31;
     double fr[RR], x[CPW];
 #pragma unroll
-    for (int r = 0; r < RR; ++r) fr[r] = lane + 32 * r < n ? f[lane + 32 * r] : 0.0;
+    for (int m = 0; m < CPW; ++m) {
+      double e = a[m][0];
 #pragma unroll
-    for (int r = 0; r < RR; ++r)
-      if (r == pr) {  // the whole CTA takes the same branch
+      for (int r = 1; r < RR; ++r) e = pr == r ? a[m][r] : e;
+      x[m] = __shfl_sync(0xffffffffu, e, pl) * ip;
+    }
 #pragma unroll
-        for (int m = 0; m < CPW; ++m) x[m] = __shfl_sync(0xffffffffu, a[m][r], pl) * ip;
-      }
+    for (int r = 0; r < RR; ++r) {
+      fr[r] = lane + 32 * r < n ? f[lane + 32 * r] : 0.0;
+      if (lane + 32 * r == p) fr[r] = 0.0;
+    }
 #pragma unroll
-    for (int m = 0; m < CPW; ++m)
-      if (m != skip) {
+    for (int m = 0; m < CPW; ++m) {
+      if (m == skip) {
+#pragma unroll
+        for (int r = 0; r < RR; ++r) a[m][r] = lane + 32 * r == p ? 1.0 : -fr[r] * ip;
+      } else {
 #pragma unroll
         for (int r = 0; r < RR; ++r) a[m][r] = fma(-fr[r], x[m], a[m][r]);
       }
+    }
     if (lane == pl) used |= 1u << pr;
   };
-  // The warp that holds step s's column (its m-th) searches it and publishes the step;
-  // the column becomes that of the inverse.
-  auto publish = [&](double (&v)[RR], int s) {
-    // the largest |v| as two 32-bit words (ordered like the number; a NaN is above
-    // all), then the lowest row that has it
-    unsigned hw[RR], hm = 0u, lm = 0u, im = 0xffffffffu;
-    bool on[RR];
+  // The warp that holds step s's column publishes it and its choice of the pivot: the
+  // largest |v| by the upper 23 bits of the number (sign aside: 2^-11 of it; a NaN is
+  // above all) and among equals the lowest row, in one 32-bit maximum.
+  auto publish = [&](const double (&v)[RR], int s) {
+    unsigned key = 0u;
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
-      on[r] = lane + 32 * r < n && !((used >> r) & 1u);
-      hw[r] = (unsigned)__double2hiint(v[r]) & 0x7fffffffu;
-      if (on[r]) hm = max(hm, hw[r]);
+      const int i = lane + 32 * r;
+      const unsigned h = ((unsigned)__double2hiint(v[r]) & 0x7ffffe00u) | (unsigned)(511 - i);
+      if (i < n && !((used >> r) & 1u)) key = max(key, h);
+      if (i < n) {
+        F[(size_t)s * n + i] = v[r];
+        W[(size_t)(j0 + s) * n + i] = v[r];
+      }
     }
-    hm = __reduce_max_sync(0xffffffffu, hm);
-#pragma unroll
-    for (int r = 0; r < RR; ++r)
-      if (on[r] && hw[r] == hm) lm = max(lm, (unsigned)__double2loint(v[r]));
-    lm = __reduce_max_sync(0xffffffffu, lm);
-#pragma unroll
-    for (int r = 0; r < RR; ++r)
-      if (on[r] && hw[r] == hm && (unsigned)__double2loint(v[r]) == lm) im = min(im, (unsigned)(lane + 32 * r));
-    const int p = (int)__reduce_min_sync(0xffffffffu, im), pr = p >> 5, pl = p & 31;
-    double pv = 0.0;
-#pragma unroll
-    for (int r = 0; r < RR; ++r)
-      if (r == pr) pv = __shfl_sync(0xffffffffu, v[r], pl);
-    if (fabs(pv) < floor_abs) pv = (pv >= 0 ? 1.0 : -1.0) * floor_abs;
-    const double ip = 1.0 / pv;
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      const bool here = r == pr && lane == pl;
-      const double f = here ? 0.0 : v[r];
-      if (lane + 32 * r < n) F[(size_t)s * n + lane + 32 * r] = f;
-      v[r] = here ? 1.0 : -f * ip;
-    }
-    if (lane == 0) {
-      ipv[0][s] = ip;
-      prow[0][s] = p;
-    }
+    key = __reduce_max_sync(0xffffffffu, key);
+    if (lane == 0) prow[0][s] = 511 - (int)(key & 511u);
   };
   __syncthreads();  // F and pos have been read
   for (int k = 0; k < PC; ++k) {
@@ -373,17 +396,23 @@ pivot_inverse_kernel(int cp, int nnzb, const int* __restrict__ br, const int* __
             if (m == skip) publish(a[m], s);
         }
         __syncthreads();
-        apply(F + (size_t)s * n, prow[0][s], ipv[0][s], skip);
+        const int p = prow[0][s];
+        double pv = F[(size_t)s * n + p];
+        if (fabs(pv) < floor_abs) pv = (pv >= 0 ? 1.0 : -1.0) * floor_abs;
+        const double ip = 1.0 / pv;
+        if (threadIdx.x == 0) ipv[0][s] = ip;
+        apply(F + (size_t)s * n, p, ip, skip);
       }
     }
     barrier();  // the panel's steps are in its CTA's shared memory
     if (k != rank) {
-      const uint32_t f = remote(F, k), ip = remote(ipv[0], k), pr = remote(prow[0], k);
+      const uint32_t ip = remote(ipv[0], k), pr = remote(prow[0], k);
+      const double* f = W + (size_t)k * cp * n;
       for (int e0 = t; e0 < steps * n; e0 += 8 * PT) {
         double v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-          if (e0 + u * PT < steps * n) v[u] = get(f + 8u * (uint32_t)(e0 + u * PT));
+          if (e0 + u * PT < steps * n) v[u] = __ldcg(f + e0 + u * PT);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
           if (e0 + u * PT < steps * n) G[e0 + u * PT] = v[u];
@@ -461,7 +490,7 @@ void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val,
   const dim3 ug((np + TC_ - 1) / TC_, (np + TR_ - 1) / TR_);
   for (int kb = 0; kb < np; kb += NB) {
     count_launch();
-    gj_diag_kernel<<<1, 1024, 0, st>>>(np, kb, A, Dg, scl);
+    gj_diag_kernel<<<1, 256, 0, st>>>(np, kb, A, Dg, scl);
     count_launch();
     gj_panel_kernel<<<ncb + nrb, 256, panel_sm, st>>>(np, kb, ncb, A, C, Dg);
     count_launch();
@@ -472,25 +501,28 @@ void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val,
 }
 
 template <typename T, int RR, int CPW>
-static cudaError_t pivot_launch(int nnzb, const int* br, const int* cl, const T* val, int n, T* inv, cudaStream_t st) {
+static cudaError_t pivot_launch(int nnzb, const int* br, const int* cl, const T* val, int n, double* work, T* inv, cudaStream_t st) {
   auto* kern = pivot_inverse_kernel<T, RR, CPW>;
   const size_t sm = pivot_smem(n);
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   count_launch();
-  kern<<<PC, PT, sm, st>>>(pivot_cols(n), nnzb, br, cl, val, n, inv);
+  kern<<<PC, PT, sm, st>>>(pivot_cols(n), nnzb, br, cl, val, n, work, inv);
   return cudaGetLastError();
 }
-// Six rows per lane and two columns per warp up to 192 unknowns, ten and three up to
-// kPivotMax.
+// Rows per lane and columns per warp: six and three up to 192 unknowns, seven and four up
+// to 224, ten and five up to kPivotMax.
 template <typename T>
-cudaError_t pivot_inverse(int nnzb, const int* br, const int* cl, const T* val, int n, T* inv, cudaStream_t st) {
-  static_assert(kPivotMax <= 32 * 10 && (kPivotMax + PC - 1) / PC <= 3 * (PT / 32), "rows and columns fit");
-  return n <= 192 ? pivot_launch<T, 6, 2>(nnzb, br, cl, val, n, inv, st)
-                  : pivot_launch<T, 10, 3>(nnzb, br, cl, val, n, inv, st);
+cudaError_t pivot_inverse(int nnzb, const int* br, const int* cl, const T* val, int n, double* work, T* inv,
+                          cudaStream_t st) {
+  static_assert(kPivotMax <= 32 * 10 && (kPivotMax + PC - 1) / PC <= 5 * (PT / 32), "rows and columns fit");
+  if (n <= 192) return pivot_launch<T, 6, 3>(nnzb, br, cl, val, n, work, inv, st);
+  if (n <= 224) return pivot_launch<T, 7, 4>(nnzb, br, cl, val, n, work, inv, st);
+  return pivot_launch<T, 10, 5>(nnzb, br, cl, val, n, work, inv, st);
 }
-template cudaError_t pivot_inverse<float>(int, const int*, const int*, const float*, int, float*, cudaStream_t);
-template cudaError_t pivot_inverse<double>(int, const int*, const int*, const double*, int, double*, cudaStream_t);
+template cudaError_t pivot_inverse<float>(int, const int*, const int*, const float*, int, double*, float*, cudaStream_t);
+template cudaError_t pivot_inverse<double>(int, const int*, const int*, const double*, int, double*, double*,
+                                           cudaStream_t);
 
 template void dense_coarse_inverse<float>(int, const int*, const int*, const float*, int, double*, float*,
                                           cudaStream_t);

@@ -129,11 +129,11 @@ template <typename T> void sa_prolong2(const AmgLevel<T>& v, const T* xc, const 
 // (device rp, cl) and values in, the n x n row-major inverse in precision T out;
 // work holds dense_inverse_work_doubles(n) doubles.
 // Up to kPivotMax unknowns pivot_inverse takes its place: the same with partial
-// pivoting, no work memory.
+// pivoting; work holds dense_inverse_work_doubles(n) doubles as well.
 constexpr int kPivotMax = 300;
 // br, cl: block row and column of each of the nnzb blocks.
-template <typename T> cudaError_t pivot_inverse(int nnzb, const int* br, const int* cl, const T* val, int n, T* inv,
-                                                cudaStream_t st);
+template <typename T> cudaError_t pivot_inverse(int nnzb, const int* br, const int* cl, const T* val, int n,
+                                                double* work, T* inv, cudaStream_t st);
 long long dense_inverse_work_doubles(int n);
 template <typename T> void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val, int n,
                                                 double* work, T* inv, cudaStream_t st);
