@@ -791,6 +791,21 @@ void dense_mv(int n, const T* M, const T* b, T* y, Queue q) {
 }
 
 // ------------------------------------------------------------------ smoothed aggregation
+// Six consecutive values from an address that is 8-byte aligned (float) or
+// 16-byte aligned (double), as three 8- or 16-byte loads: every 6-value row of a
+// bs x 6 transfer block and every 6-vector of a coarse level is.
+template <typename T, bool STREAM>
+__device__ __forceinline__ void load6(const T* p, T* v) {
+  using V2 = typename std::conditional<std::is_same<T, float>::value, float2, double2>::type;
+  const V2* q = reinterpret_cast<const V2*>(p);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const V2 w = STREAM ? __ldcs(q + k) : q[k];
+    v[2 * k] = w.x;
+    v[2 * k + 1] = w.y;
+  }
+}
+
 // P = (I - w D^-1 A) T with the tentative T (one bs x 6 block per fine row).
 // One thread per P block p (row n, aggregate J):
 //   P_p = [J == agg(n)] T_n - w Dinv_n sum_{k in row n, agg(col k) == J} A_k T_col(k)
@@ -815,13 +830,16 @@ __global__ void sa_prolongator_kernel(int nnzP, const int* __restrict__ p_row, c
     const T* A = val + (long long)k * BS * BS;
     const T* Tm = Tb + (long long)col[k] * BS * 6;
 #pragma unroll
-    for (int i = 0; i < BS; ++i)
+    for (int j = 0; j < BS; ++j) {
+      T tv[6];
+      load6<T, false>(Tm + j * 6, tv);
 #pragma unroll
-      for (int j = 0; j < BS; ++j) {
+      for (int i = 0; i < BS; ++i) {
         const T a = A[i * BS + j];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) acc[i][c] += a * Tm[j * 6 + c];
+        for (int c = 0; c < 6; ++c) acc[i][c] += a * tv[c];
       }
+    }
   }
   const T* D = dinv + (long long)n * BS * BS;
   const bool own = p_cl[p] == agg[n];
@@ -870,13 +888,16 @@ __global__ void sa_ap_kernel(int nnzAP, const int* __restrict__ ap_row, const in
     const T* A = val + (long long)k * BS * BS;
     const T* P = pval + (long long)p * BS * 6;
 #pragma unroll
-    for (int i = 0; i < BS; ++i)
+    for (int j = 0; j < BS; ++j) {
+      T pv[6];
+      load6<T, false>(P + j * 6, pv);
 #pragma unroll
-      for (int j = 0; j < BS; ++j) {
+      for (int i = 0; i < BS; ++i) {
         const T a = A[i * BS + j];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) acc[i][c] += a * P[j * 6 + c];
+        for (int c = 0; c < 6; ++c) acc[i][c] += a * pv[c];
       }
+    }
   }
   T* O = apval + (long long)q * BS * 6;
 #pragma unroll
@@ -885,42 +906,59 @@ __global__ void sa_ap_kernel(int nnzAP, const int* __restrict__ ap_row, const in
     for (int c = 0; c < 6; ++c) O[i * 6 + c] = acc[i][c];
 }
 
-// Coarse block c (I, J) = sum_{p in P^T row I} P_p^T AP[row(p), J]   (6 x 6)
-template <typename T, int BS>
-__global__ void sa_rap_kernel(int nnzC, const int* __restrict__ c_row, const int* __restrict__ c_cl,
-                              const int* __restrict__ pt_rp, const int* __restrict__ pt_blk,
-                              const int* __restrict__ p_row, const T* __restrict__ pval,
+// Coarse block c (I, J) = sum_{p in P^T row I} P_p^T AP[row(p), J]   (6 x 6).  LN lanes
+// per block stride over the P^T row (its copy ptval: consecutive lanes read
+// consecutive blocks), each searching its row of AP for J, and add their 36 partial
+// sums by a fixed xor tree.  One thread per block walked the whole row, about 115
+// blocks at level 0: 770 us there at 64^3 and 403 us at level 1, 320 us for the whole of a
+// 23x9x7 mesh; now 634, 58 and 45 us.
+template <typename T, int BS, int LN>
+__global__ void __launch_bounds__(128) sa_rap_kernel(int nnzC, const int* __restrict__ c_row, const int* __restrict__ c_cl,
+                              const int* __restrict__ pt_rp, const int* __restrict__ pt_row,
+                              const T* __restrict__ ptval,
                               const int* __restrict__ ap_rp, const int* __restrict__ ap_cl,
                               const T* __restrict__ apval, T* __restrict__ cval) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nnzC) return;
-  const int I = c_row[c], J = c_cl[c];
+  const long long th = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int c = (int)(th / LN), lane = (int)(th % LN);
+  const bool in = c < nnzC;
+  const int I = in ? c_row[c] : 0, J = in ? c_cl[c] : 0;
   T acc[6][6];
 #pragma unroll
   for (int r = 0; r < 6; ++r)
 #pragma unroll
     for (int q = 0; q < 6; ++q) acc[r][q] = T(0);
-  for (int t = pt_rp[I]; t < pt_rp[I + 1]; ++t) {
-    const int p = pt_blk[t];
-    const int n = p_row[p];
+  const int t1 = in ? pt_rp[I + 1] : 0;
+  for (int t = in ? pt_rp[I] + lane : 0; t < t1; t += LN) {
+    const int n = pt_row[t];
     const int q = find_sorted(ap_cl, ap_rp[n], ap_rp[n + 1], J);
     if (q < 0) continue;
-    const T* P = pval + (long long)p * BS * 6;
+    const T* P = ptval + (long long)t * BS * 6;
     const T* AP = apval + (long long)q * BS * 6;
 #pragma unroll
-    for (int i = 0; i < BS; ++i)
+    for (int i = 0; i < BS; ++i) {
+      T pv[6], av[6];
+      load6<T, false>(P + i * 6, pv);
+      load6<T, false>(AP + i * 6, av);
 #pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        const T pr = P[i * 6 + r];
+      for (int r = 0; r < 6; ++r)
 #pragma unroll
-        for (int q2 = 0; q2 < 6; ++q2) acc[r][q2] += pr * AP[i * 6 + q2];
-      }
+        for (int q2 = 0; q2 < 6; ++q2) acc[r][q2] += pv[r] * av[q2];
+    }
   }
+#pragma unroll
+  for (int r = 0; r < 6; ++r)
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+#pragma unroll
+      for (int o = LN / 2; o > 0; o >>= 1) acc[r][q] += __shfl_xor_sync(0xffffffffu, acc[r][q], o);
+    }
+  if (!in) return;
   T* O = cval + (long long)c * 36;
 #pragma unroll
   for (int r = 0; r < 6; ++r)
 #pragma unroll
-    for (int q = 0; q < 6; ++q) O[r * 6 + q] = acc[r][q];
+    for (int q = 0; q < 6; ++q)
+      if ((r * 6 + q) % LN == lane) O[r * 6 + q] = acc[r][q];
 }
 
 // P^T copy: block t of the aggregate-ordered list is P block pt_blk[t].
@@ -932,21 +970,6 @@ __global__ void sa_transpose_copy_kernel(int nnzP, const int* __restrict__ pt_bl
   const long long t = e / (BS * 6);
   const int q = (int)(e - t * (BS * 6));
   ptval[e] = pval[(long long)pt_blk[t] * (BS * 6) + q];
-}
-
-// Six consecutive values from an address that is 8-byte aligned (float) or
-// 16-byte aligned (double), as three 8- or 16-byte loads: every 6-value row of a
-// bs x 6 transfer block and every 6-vector of a coarse level is.
-template <typename T, bool STREAM>
-__device__ __forceinline__ void load6(const T* p, T* v) {
-  using V2 = typename std::conditional<std::is_same<T, float>::value, float2, double2>::type;
-  const V2* q = reinterpret_cast<const V2*>(p);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const V2 w = STREAM ? __ldcs(q + k) : q[k];
-    v[2 * k] = w.x;
-    v[2 * k + 1] = w.y;
-  }
 }
 
 // Restriction bc = P^T r, WPA warps per aggregate: the lanes stride over the
@@ -1065,36 +1088,22 @@ __global__ void sa_prolong_kernel(int nbrow, const int* __restrict__ p_rp, const
   if (in) x[i] += s;
 }
 
+template <typename T, int BS>
+static void setup_level_t(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st) {
+  launch(st, sa_prolongator_kernel<T, BS>, (v.nnzP + 127) / 128, 128, 0, v.nnzP, v.p_row, v.p_cl, v.A.rowptr, v.A.col, v.A.val,
+         v.pslot, v.agg, v.T, v.dinv, v.co + CO_OMEGA, v.p_val);
+  launch(st, sa_transpose_copy_kernel<T, BS>, (int)(((long long)v.nnzP * BS * 6 + 255) / 256), 256, 0, v.nnzP, v.pt_blk,
+         v.p_val, v.pt_val);
+  launch(st, sa_ap_kernel<T, BS>, (v.nnzAP + 127) / 128, 128, 0, v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
+         v.p_rp, v.p_cl, v.p_val, v.ap_val);
+  constexpr int LN = 8;
+  launch(st, sa_rap_kernel<T, BS, LN>, (int)(((long long)nnzC * LN + 127) / 128), 128, 0, nnzC, v.c_row, v.c_cl, v.pt_rp,
+         v.pt_row, v.pt_val, v.ap_rp, v.ap_cl, v.ap_val, cval);
+}
 template <typename T>
 void sa_setup_level(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st) {
-  const int BSs = v.A.bs;
-  if (BSs == 3) {
-    pfem::count_launch();
-    sa_prolongator_kernel<T, 3><<<(v.nnzP + 127) / 128, 128, 0, st>>>(v.nnzP, v.p_row, v.p_cl, v.A.rowptr, v.A.col,
-                                                                     v.A.val, v.pslot, v.agg, v.T, v.dinv, v.co + CO_OMEGA, v.p_val);
-    pfem::count_launch();
-    sa_ap_kernel<T, 3><<<(v.nnzAP + 127) / 128, 128, 0, st>>>(v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
-                                                             v.p_rp, v.p_cl, v.p_val, v.ap_val);
-    pfem::count_launch();
-    sa_rap_kernel<T, 3><<<(nnzC + 127) / 128, 128, 0, st>>>(nnzC, v.c_row, v.c_cl, v.pt_rp, v.pt_blk, v.p_row, v.p_val,
-                                                           v.ap_rp, v.ap_cl, v.ap_val, cval);
-    pfem::count_launch();
-    sa_transpose_copy_kernel<T, 3><<<(int)(((long long)v.nnzP * 18 + 255) / 256), 256, 0, st>>>(v.nnzP, v.pt_blk,
-                                                                                               v.p_val, v.pt_val);
-  } else {
-    pfem::count_launch();
-    sa_prolongator_kernel<T, 6><<<(v.nnzP + 127) / 128, 128, 0, st>>>(v.nnzP, v.p_row, v.p_cl, v.A.rowptr, v.A.col,
-                                                                     v.A.val, v.pslot, v.agg, v.T, v.dinv, v.co + CO_OMEGA, v.p_val);
-    pfem::count_launch();
-    sa_ap_kernel<T, 6><<<(v.nnzAP + 127) / 128, 128, 0, st>>>(v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
-                                                             v.p_rp, v.p_cl, v.p_val, v.ap_val);
-    pfem::count_launch();
-    sa_rap_kernel<T, 6><<<(nnzC + 127) / 128, 128, 0, st>>>(nnzC, v.c_row, v.c_cl, v.pt_rp, v.pt_blk, v.p_row, v.p_val,
-                                                           v.ap_rp, v.ap_cl, v.ap_val, cval);
-    pfem::count_launch();
-    sa_transpose_copy_kernel<T, 6><<<(int)(((long long)v.nnzP * 36 + 255) / 256), 256, 0, st>>>(v.nnzP, v.pt_blk,
-                                                                                               v.p_val, v.pt_val);
-  }
+  if (v.A.bs == 3) setup_level_t<T, 3>(v, cval, nnzC, st);
+  else setup_level_t<T, 6>(v, cval, nnzC, st);
 }
 // Aggregates below this count get four warps each in the restriction.
 constexpr int kRestrictWideBelow = 4096;
