@@ -35,6 +35,8 @@ struct MlpState {
   bool last_used = false;    // the last prediction kept the learned guess
   int* rows = nullptr;       // batch row indices
   int rows_cap = 0;
+  char* work = nullptr;      // rows of the forward and loss calls, kept between them
+  size_t work_bytes = 0;
 };
 
 size_t mlp_smem_bytes();
