@@ -39,16 +39,17 @@ struct KrylovWork {
   T *rh = nullptr, *v = nullptr, *s = nullptr, *t = nullptr, *ph = nullptr, *sh = nullptr;
   T* sc = nullptr;    // device scalars
   T* part = nullptr;  // reduction partials
-  double* dpart = nullptr;     // the fused PCG body's: r.z, p.q and r.r, kMaxPartials each
-  unsigned* ticket = nullptr;  // zero between launches of cg_xr_fused
+  double* dpart = nullptr;     // the loop bodies' dot products: four of kMaxPartials
+  unsigned* ticket = nullptr;  // zero between launches of cg_xr_fused and bicg_xr
   T* b = nullptr;
   T *xa = nullptr, *b0 = nullptr;  // iterative refinement: accumulated solution, saved right-hand side
 };
 
-// The preconditioned-CG loop captured as one CUDA graph: a prefix (x = 0,
+// The preconditioned CG or BiCGStab loop captured as one CUDA graph: a prefix (x = 0,
 // r = b, |b|) and a conditional WHILE node whose body is one iteration
-// (V-cycle, the p / x / r updates with the dot products inside, |r|); the last kernel's
-// last CTA sets the loop condition from the device-resident residual.  One launch and one host synchronisation per linear solve.
+// (V-cycles, the vector updates with the dot products inside, |r|); the last kernel's
+// last CTA sets the loop condition from the device-resident residual.  One launch and one
+// host synchronisation per linear solve.
 // A set-up writes into the same device arrays, so the graph outlives it; it is
 // captured again when the smoother's degree changes (and, for other degrees than 2,
 // whose coefficients are kernel arguments, after every set-up).  The tolerance and
@@ -151,7 +152,7 @@ struct pfem_ctx {
   Amg<double> amg64;
   KrylovWork<float> kw32;
   KrylovWork<double> kw64;
-  CgGraph cg32, cg64;
+  CgGraph cg32[2], cg64[2];  // [method]
   int tangent_prec = -1;  // precision of the last imposed tangent
   int chain_len = 0;      // the cycle's kernels are being captured as a programmatic
   int* chain = nullptr;   // launch chain: &chain_len meanwhile
@@ -661,11 +662,11 @@ KrylovWork<float>& kw_of<float>(pfem_ctx* c) { return c->kw32; }
 template <>
 KrylovWork<double>& kw_of<double>(pfem_ctx* c) { return c->kw64; }
 template <typename T>
-CgGraph& cg_of(pfem_ctx* c);
+CgGraph& cg_of(pfem_ctx* c, int method);
 template <>
-CgGraph& cg_of<float>(pfem_ctx* c) { return c->cg32; }
+CgGraph& cg_of<float>(pfem_ctx* c, int method) { return c->cg32[method == PFEM_KRYLOV_CG ? 0 : 1]; }
 template <>
-CgGraph& cg_of<double>(pfem_ctx* c) { return c->cg64; }
+CgGraph& cg_of<double>(pfem_ctx* c, int method) { return c->cg64[method == PFEM_KRYLOV_CG ? 0 : 1]; }
 template <typename T>
 T* K_of(pfem_ctx* c);
 template <>
@@ -682,17 +683,6 @@ __global__ void hash_fill_kernel(long long n, float* xf, double* xd) {
     if (xd) xd[i] = v;
   }
 }
-template <typename T>
-__global__ void bicg_finish_kernel(T* sc) {
-  sc[2] = sc[0] / sc[4];
-  sc[3] = sc[5] / sc[6];
-  sc[1] = sc[0];
-}
-template <typename T>
-__global__ void bicg_init_kernel(T* sc) {
-  sc[1] = T(1); sc[2] = T(1); sc[3] = T(1);
-}
-
 // Allocate the device side of the hierarchy for precision T (once).
 template <typename T>
 int amg_alloc(pfem_ctx* ctx) {
@@ -770,7 +760,7 @@ int krylov_alloc(pfem_ctx* ctx) {
   CK(dalloc(ctx, &w.ph, n)); CK(dalloc(ctx, &w.sh, n)); CK(dalloc(ctx, &w.b, n));
   CK(dalloc(ctx, &w.xa, n)); CK(dalloc(ctx, &w.b0, n));
   CK(dalloc(ctx, &w.sc, 16)); CK(dalloc(ctx, &w.part, 2048));
-  CK(dalloc(ctx, &w.dpart, 3 * (size_t)pfem::kMaxPartials));
+  CK(dalloc(ctx, &w.dpart, 4 * (size_t)pfem::kMaxPartials));
   CK(dalloc(ctx, &w.ticket, 1));
   CK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned), ctx->st));
   return PFEM_OK;
@@ -949,10 +939,23 @@ __global__ void cg_graph_init_kernel(cudaGraphConditionalHandle h, const T* __re
   *sc0 = T(1);                  // with p = 0, the first update p = z + (r.z / 1) p gives p = z
   cudaGraphSetConditional(h, (b > 0.0 && isfinite(b)) ? 1u : 0u);
 }
-// Capture (or reuse) the device-side CG loop for the current hierarchy.
+// The same for BiCGStab: rho = |b|^2 is in sc[0] already; with p = v = 0 the first update
+// gives p = r.  A cap below one runs no iteration.
 template <typename T>
-int cg_graph_build(pfem_ctx* ctx) {
-  CgGraph& G = cg_of<T>(ctx);
+__global__ void bicg_graph_init_kernel(cudaGraphConditionalHandle h, const T* __restrict__ bn, T* __restrict__ sc,
+                                       double* __restrict__ ctl, int* __restrict__ state) {
+  const double b = (double)*bn;
+  ctl[2] = ctl[0] * b;
+  state[0] = 0;
+  state[1] = b > 0.0 ? 0 : 1;
+  sc[1] = sc[2] = sc[3] = T(1);
+  cudaGraphSetConditional(h, (b > 0.0 && ctl[1] >= 1.0) ? 1u : 0u);
+}
+// Capture (or reuse) the device-side loop of a method for the current hierarchy.
+template <typename T>
+int cg_graph_build(pfem_ctx* ctx, int method) {
+  CgGraph& G = cg_of<T>(ctx, method);
+  const bool cg = method == PFEM_KRYLOV_CG;
   Amg<T>& A = amg_of<T>(ctx);
   const long long version = A.cheb_degree == 2 ? 0 : A.version;
   if (G.exec && G.degree == A.cheb_degree && G.amg_version == version) return PFEM_OK;
@@ -988,7 +991,14 @@ int cg_graph_build(pfem_ctx* ctx) {
   e = cudaMemcpyAsync(w.r, w.b, n * sizeof(T), cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) return abort_capture(e, "r = b");
   dot<T>(n, w.b, w.b, w.sc + 10, w.part, st, true);
-  blockdiag_apply<T>(K.nbrow, 3, v0.dinv, w.r, v0.r, v0.co + CO_ITH, v0.d, st);
+  if (cg) {
+    blockdiag_apply<T>(K.nbrow, 3, v0.dinv, w.r, v0.r, v0.co + CO_ITH, v0.d, st);
+  } else {
+    e = cudaMemcpyAsync(w.rh, w.b, n * sizeof(T), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return abort_capture(e, "rh = b");
+    fill<T>(n, w.v, T(0), st);
+    dot<T>(n, w.rh, w.r, w.sc + 0, w.part, st, false);
+  }
   cudaStreamCaptureStatus cs;
   const cudaGraphNode_t* deps = nullptr;
   size_t nd = 0;
@@ -997,7 +1007,8 @@ int cg_graph_build(pfem_ctx* ctx) {
   cudaGraphConditionalHandle h;
   e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
   if (e != cudaSuccess) return abort_capture(e, "conditional handle");
-  cg_graph_init_kernel<T><<<1, 1, 0, st>>>(h, w.sc + 10, w.sc + 0, G.ctl, G.state);
+  if (cg) cg_graph_init_kernel<T><<<1, 1, 0, st>>>(h, w.sc + 10, w.sc + 0, G.ctl, G.state);
+  else bicg_graph_init_kernel<T><<<1, 1, 0, st>>>(h, w.sc + 10, w.sc, G.ctl, G.state);
   e = cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &deps, &nd);
   if (e != cudaSuccess) return abort_capture(e, "capture info");
   cudaGraphNodeParams cp = {};
@@ -1011,7 +1022,7 @@ int cg_graph_build(pfem_ctx* ctx) {
   e = cudaStreamUpdateCaptureDependencies(st, &cnode, 1, cudaStreamSetCaptureDependencies);
   if (e != cudaSuccess) return abort_capture(e, "capture dependencies");
   const long long c1 = pfem::launch_counter();
-  // ---- loop body: one PCG iteration ----
+  // ---- loop body: one iteration ----
   body = cp.conditional.phGraph_out[0];
   e = cudaStreamBeginCaptureToGraph(G.body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return abort_capture(e, "body capture");
@@ -1022,23 +1033,34 @@ int cg_graph_build(pfem_ctx* ctx) {
   ctx->chain_len = 0;
   ctx->chain = A.cheb_degree == 2 ? &ctx->chain_len : nullptr;
   const Queue q(bs, ctx->chain);
-  // sc[0] = r.z of the previous iteration, sc[2] = r.z; the dot products are summed
-  // by the kernels whose results they are made of, their final sums by their users
-  double* const part_rz = w.dpart;
-  double* const part_pq = w.dpart + pfem::kMaxPartials;
-  int np_rz = vcycle<T>(ctx, 0, w.r, w.z, true, ctx->chain ? part_rz : nullptr);
-  ctx->st = st;
-  ctx->chain = nullptr;
-  if (np_rz == 0) np_rz = dot_partials_double<T>(n, w.r, w.z, part_rz, q);
-  cg_p_fused<T>(n, part_rz, np_rz, w.sc, w.z, w.p, q);
-  const int np_pq = bsr_spmv<T>(K, w.p, w.q, q, part_pq);
+  double* const part[4] = {w.dpart, w.dpart + pfem::kMaxPartials, w.dpart + 2 * pfem::kMaxPartials,
+                           w.dpart + 3 * pfem::kMaxPartials};
   CgLoop loop;
   loop.h = h;
   loop.ctl = G.ctl;
   loop.state = G.state;
   loop.ticket = w.ticket;
-  loop.part_rr = w.dpart + 2 * pfem::kMaxPartials;
-  cg_xr_fused<T>(K.nbrow, part_pq, np_pq, w.sc, w.p, w.q, w.x, w.r, v0.dinv, v0.co, v0.r, v0.d, loop, q);
+  loop.part_rr = part[2];
+  if (cg) {
+    // sc[0] = r.z of the previous iteration, sc[2] = r.z; the dot products are summed
+    // by the kernels whose results they are made of, their final sums by their users
+    int np_rz = vcycle<T>(ctx, 0, w.r, w.z, true, ctx->chain ? part[0] : nullptr);
+    if (np_rz == 0) np_rz = dot_partials_double<T>(n, w.r, w.z, part[0], q);
+    cg_p_fused<T>(n, part[0], np_rz, w.sc, w.z, w.p, q);
+    const int np_pq = bsr_spmv<T>(K, w.p, w.q, q, part[1]);
+    cg_xr_fused<T>(K.nbrow, part[1], np_pq, w.sc, w.p, w.q, w.x, w.r, v0.dinv, v0.co, v0.r, v0.d, loop, q);
+  } else {
+    bicg_p<T>(K.nbrow, w.sc, w.r, w.v, w.p, v0.dinv, v0.co, v0.r, v0.d, q);
+    vcycle<T>(ctx, 0, w.p, w.ph, true);
+    bsr_spmv<T>(K, w.ph, w.v, q);
+    const int np = dot_partials_double<T>(n, w.rh, w.v, part[0], q);
+    bicg_s<T>(K.nbrow, part[0], np, w.sc, w.r, w.v, w.s, v0.dinv, v0.co, v0.r, v0.d, q);
+    vcycle<T>(ctx, 0, w.s, w.sh, true);
+    bsr_spmv<T>(K, w.sh, w.t, q);
+    bicg_xr<T>(n, w.sc, w.ph, w.sh, w.s, w.t, w.rh, w.x, w.r, part[0], part[1], part[3], loop, q);
+  }
+  ctx->st = st;
+  ctx->chain = nullptr;
   e = cudaStreamEndCapture(bs, &body);
   if (e != cudaSuccess) return abort_capture(e, "body end");
   const long long c2 = pfem::launch_counter();
@@ -1076,72 +1098,28 @@ int read_back(pfem_ctx* ctx) {
 // b and the result x live in kw.b / kw.x.  Returns iterations (>=0) or <0.
 template <typename T>
 int krylov_inner(pfem_ctx* ctx, int method, double rtol, int itmax, int* iters, bool* conv) {
-  Amg<T>& A = amg_of<T>(ctx);
-  KrylovWork<T>& w = kw_of<T>(ctx);
-  const BsrMat<T>& K = A.lv[0].A;
-  const long long n = ctx->ndof;
   cudaStream_t st = ctx->st;
   *iters = 0;
   *conv = false;
-  if (method == PFEM_KRYLOV_CG) {
-    const bool dbg = getenv("PFEM_DEBUG_AMG") != nullptr;
-    auto tg = std::chrono::steady_clock::now();
-    int rc = cg_graph_build<T>(ctx);
-    if (rc) return rc;
-    if (dbg) {
-      const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tg).count();
-      if (ms > 0.05) fprintf(stderr, "cg graph capture + instantiate %.3f ms\n", ms);
-    }
-    CgGraph& G = cg_of<T>(ctx);
-    const double ctl[2] = {rtol, (double)std::max(itmax, 1)};
-    CK(cudaMemcpyAsync(G.ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
-    CK(cudaGraphLaunch(G.exec, st));
-    rc = read_back(ctx);
-    if (rc) return rc;
-    const int* sh = ctx->hBack->cg[std::is_same<T, double>::value ? 1 : 0];
-    *iters = sh[0];
-    *conv = sh[1] != 0;
-    pfem::launch_counter() += G.prefix_kernels + (long long)sh[0] * G.body_kernels;
-    return PFEM_OK;
+  const bool dbg = getenv("PFEM_DEBUG_AMG") != nullptr;
+  auto tg = std::chrono::steady_clock::now();
+  int rc = cg_graph_build<T>(ctx, method);
+  if (rc) return rc;
+  if (dbg) {
+    const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tg).count();
+    if (ms > 0.05) fprintf(stderr, "krylov graph capture + instantiate %.3f ms\n", ms);
   }
-  fill<T>(n, w.x, T(0), st);
-  CK(cudaMemcpyAsync(w.r, w.b, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
-  dot<T>(n, w.b, w.b, w.sc + 10, w.part, st, true);
-  T bn = 0;
-  CK(cudaMemcpyAsync(&bn, w.sc + 10, sizeof(T), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  if (!(bn > 0)) { *conv = true; return PFEM_OK; }
-  const double thr = rtol * (double)bn;
-  {  // BiCGStab: host-driven loop
-    CK(cudaMemcpyAsync(w.rh, w.b, n * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    fill<T>(n, w.v, T(0), st);
-    fill<T>(n, w.p, T(0), st);
-    pfem::count_launch(); bicg_init_kernel<T><<<1, 1, 0, st>>>(w.sc);
-    for (int it = 1; it <= itmax; ++it) {
-      dot<T>(n, w.rh, w.r, w.sc + 0, w.part, st, false);
-      bicg_p<T>(n, w.sc, w.r, w.v, w.p, st);
-      vcycle<T>(ctx, 0, w.p, w.ph);
-      bsr_spmv<T>(K, w.ph, w.v, st);
-      dot<T>(n, w.rh, w.v, w.sc + 4, w.part, st, false);
-      bicg_s<T>(n, w.sc, w.r, w.v, w.s, st);
-      vcycle<T>(ctx, 0, w.s, w.sh);
-      bsr_spmv<T>(K, w.sh, w.t, st);
-      dot<T>(n, w.t, w.s, w.sc + 5, w.part, st, false);
-      dot<T>(n, w.t, w.t, w.sc + 6, w.part, st, false);
-      bicg_xr<T>(n, w.sc, w.ph, w.sh, w.s, w.t, w.x, w.r, st);
-      pfem::count_launch(); bicg_finish_kernel<T><<<1, 1, 0, st>>>(w.sc);
-      // |r| goes to slot 7: slot 3 holds omega for the next iteration's beta
-      dot<T>(n, w.r, w.r, w.sc + 7, w.part, st, true);
-      T rn = 0;
-      CK(cudaMemcpyAsync(&rn, w.sc + 7, sizeof(T), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-      *iters = it;
-      if ((double)rn <= thr) { *conv = true; break; }
-      if (!std::isfinite((double)rn)) break;
-    }
-  }
-  CKL();
-  return read_back(ctx);
+  CgGraph& G = cg_of<T>(ctx, method);
+  const double ctl[2] = {rtol, (double)(method == PFEM_KRYLOV_CG ? std::max(itmax, 1) : itmax)};
+  CK(cudaMemcpyAsync(G.ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, st));
+  CK(cudaGraphLaunch(G.exec, st));
+  rc = read_back(ctx);
+  if (rc) return rc;
+  const int* sh = ctx->hBack->cg[std::is_same<T, double>::value ? 1 : 0];
+  *iters = sh[0];
+  *conv = sh[1] != 0;
+  pfem::launch_counter() += G.prefix_kernels + (long long)sh[0] * G.body_kernels;
+  return PFEM_OK;
 }
 
 // Solve K x = b (kw.b -> kw.x) to relative tolerance rtol.  Below the level a
@@ -1976,7 +1954,7 @@ void pfem_destroy(pfem_ctx* ctx) {
   }
   cudaSetDevice(ctx->device);
   if (ctx->st) cudaStreamSynchronize(ctx->st);
-  for (CgGraph* g : {&ctx->cg32, &ctx->cg64}) {
+  for (CgGraph* g : {&ctx->cg32[0], &ctx->cg32[1], &ctx->cg64[0], &ctx->cg64[1]}) {
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
     if (g->body_stream) cudaStreamDestroy(g->body_stream);

@@ -427,35 +427,6 @@ void axpby(long long n, T a, const T* x, T b, T* y, cudaStream_t st) {
   const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
   if (n > 0) { pfem::count_launch(); axpby_kernel<T><<<blocks, 256, 0, st>>>(n, a, x, b, y); }
 }
-// CG update with device scalars: alpha = num/den;  x += alpha p;  r -= alpha q
-template <typename T>
-__global__ void cg_xr_kernel(long long n, const T* __restrict__ num, const T* __restrict__ den,
-                             const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ x,
-                             T* __restrict__ r) {
-  const T al = *num / *den;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    x[i] += al * p[i];
-    r[i] -= al * q[i];
-  }
-}
-template <typename T>
-void cg_xr(long long n, const T* num, const T* den, const T* p, const T* q, T* x, T* r, cudaStream_t st) {
-  const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
-  pfem::count_launch(); cg_xr_kernel<T><<<blocks, 256, 0, st>>>(n, num, den, p, q, x, r);
-}
-// p = z + (num/den) p
-template <typename T>
-__global__ void cg_p_kernel(long long n, const T* __restrict__ num, const T* __restrict__ den,
-                            const T* __restrict__ z, T* __restrict__ p) {
-  const T be = *num / *den;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    p[i] = z[i] + be * p[i];
-}
-template <typename T>
-void cg_p(long long n, const T* num, const T* den, const T* z, T* p, cudaStream_t st) {
-  const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
-  pfem::count_launch(); cg_p_kernel<T><<<blocks, 256, 0, st>>>(n, num, den, z, p);
-}
 static int fused_update_blocks(long long n) {
   const long long nb = (n + RED_THREADS - 1) / RED_THREADS;
   return (int)(nb < RED_BLOCKS ? (nb > 0 ? nb : 1) : RED_BLOCKS);
@@ -612,59 +583,152 @@ void power_finish(int np, const double* prev, const double* last, T* co, cudaStr
   pfem::count_launch();
   power_finish_kernel<T><<<1, 1024, 0, st>>>(np, prev, last, co);
 }
-// BiCGStab helpers with device scalars s[0..]: see krylov code for layout.
+// ---- BiCGStab updates.  Scalars: sc[0] rho = rh.r, sc[1] rho of the iteration before,
+// sc[2] alpha, sc[3] omega.  A thread per node, as cg_xr_fused; the dot products come as
+// partials in double.  An iteration used to be 78 plain launches from the host with a
+// read-back of |r|, bound by the launches below about 40^3; in the graph with the
+// smoother's starts in its own updates it takes 440 us at 40^3 FP64, 550 before.
 template <typename T>
-__global__ void bicg_p_kernel(long long n, const T* __restrict__ sc, const T* __restrict__ r,
-                              const T* __restrict__ v, T* __restrict__ p) {
-  // beta = (rho_new/rho_old)*(alpha/omega); p = r + beta (p - omega v)
-  const T beta = (sc[0] / sc[1]) * (sc[2] / sc[3]);
-  const T om = sc[3];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    p[i] = r[i] + beta * (p[i] - om * v[i]);
-}
-template <typename T>
-void bicg_p(long long n, const T* sc, const T* r, const T* v, T* p, cudaStream_t st) {
-  const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
-  pfem::count_launch(); bicg_p_kernel<T><<<blocks, 256, 0, st>>>(n, sc, r, v, p);
-}
-// s = r - alpha v  (alpha = sc[0]/sc[4])
-template <typename T>
-__global__ void bicg_s_kernel(long long n, const T* __restrict__ sc, const T* __restrict__ r,
-                              const T* __restrict__ v, T* __restrict__ s) {
-  const T al = sc[0] / sc[4];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    s[i] = r[i] - al * v[i];
-}
-template <typename T>
-void bicg_s(long long n, const T* sc, const T* r, const T* v, T* s, cudaStream_t st) {
-  const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
-  pfem::count_launch(); bicg_s_kernel<T><<<blocks, 256, 0, st>>>(n, sc, r, v, s);
-}
-// x += alpha ph + omega sh;  r = s - omega t  (alpha = sc[0]/sc[4], omega = sc[5]/sc[6])
-template <typename T>
-__global__ void bicg_xr_kernel(long long n, const T* __restrict__ sc, const T* __restrict__ ph,
-                               const T* __restrict__ sh, const T* __restrict__ s, const T* __restrict__ t,
-                               T* __restrict__ x, T* __restrict__ r) {
-  const T al = sc[0] / sc[4];
-  const T om = sc[5] / sc[6];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    x[i] += al * ph[i] + om * sh[i];
-    r[i] = s[i] - om * t[i];
+__device__ __forceinline__ void smoother_start(const T* __restrict__ dinv, T ith, long long n, const T v[3], T* sr,
+                                               T* sd) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    T t = T(0);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) t += dinv[n * 9 + i * 3 + j] * v[j];
+    sr[n * 3 + i] = t;
+    sd[n * 3 + i] = ith * t;
   }
 }
+// beta = (rho / rho_old) (alpha / omega);  p = r + beta (p - omega v)
 template <typename T>
-void bicg_xr(long long n, const T* sc, const T* ph, const T* sh, const T* s, const T* t, T* x, T* r,
-             cudaStream_t st) {
-  const int blocks = (int)std::min<long long>((n + 255) / 256, 4096);
-  pfem::count_launch(); bicg_xr_kernel<T><<<blocks, 256, 0, st>>>(n, sc, ph, sh, s, t, x, r);
+__global__ void __launch_bounds__(256) bicg_p_kernel(int nbrow, const T* sc, const T* r, const T* v, T* p,
+                                                     const T* __restrict__ dinv, const T* __restrict__ co, T* sr,
+                                                     T* sd) {
+  pdl_go();
+  const T ith = co[CO_ITH];
+  pdl_wait();
+  const T beta = (sc[0] / sc[1]) * (sc[2] / sc[3]);
+  const T om = sc[3];
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nbrow; n += gridDim.x * blockDim.x) {
+    T e[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const long long i = (long long)n * 3 + j;
+      e[j] = r[i] + beta * (p[i] - om * v[i]);
+      p[i] = e[j];
+    }
+    smoother_start(dinv, ith, n, e, sr, sd);
+  }
 }
-// scalar bookkeeping: dst[i] = src[j]
+// alpha = rho / sum(part);  s = r - alpha v
 template <typename T>
-__global__ void scalar_copy_kernel(T* dst, const T* src) { *dst = *src; }
+__global__ void __launch_bounds__(256) bicg_s_kernel(int nbrow, const double* part, int np, T* sc, const T* r,
+                                                     const T* v, T* s, const T* __restrict__ dinv,
+                                                     const T* __restrict__ co, T* sr, T* sd) {
+  __shared__ double sh[33];
+  pdl_go();
+  const T ith = co[CO_ITH];
+  pdl_wait();
+  const T al = sc[0] / (T)all_sum_partials(part, np, sh);
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nbrow; n += gridDim.x * blockDim.x) {
+    T e[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const long long i = (long long)n * 3 + j;
+      e[j] = r[i] - al * v[i];
+      s[i] = e[j];
+    }
+    smoother_start(dinv, ith, n, e, sr, sd);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc[2] = al;
+}
+// Partials of t.s and of t.t.
 template <typename T>
-void scalar_copy(T* dst, const T* src, cudaStream_t st) {
-  pfem::count_launch();
-  scalar_copy_kernel<T><<<1, 1, 0, st>>>(dst, src);
+__global__ void __launch_bounds__(256) bicg_dots_kernel(long long n, const T* t, const T* s, double* part_ts,
+                                                        double* part_tt) {
+  __shared__ double sh[32];
+  pdl_go();
+  pdl_wait();
+  double a = 0.0, b = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double ti = (double)t[i];
+    a += ti * (double)s[i];
+    b += ti * ti;
+  }
+  a = block_sum(a, sh);
+  __syncthreads();
+  b = block_sum(b, sh);
+  if (threadIdx.x == 0) {
+    part_ts[blockIdx.x] = a;
+    part_tt[blockIdx.x] = b;
+  }
+}
+// omega = sum(part_ts) / sum(part_tt);  x += alpha ph + omega sh;  r = s - omega t.  The
+// CTA that finishes last adds the shares of r.r and rh.r in their order, leaves the next
+// iteration's scalars and sets the loop's condition.
+template <typename T>
+__global__ void __launch_bounds__(256) bicg_xr_kernel(long long n, const double* part_ts, const double* part_tt,
+                                                      int np, T* sc, const T* ph, const T* sh_, const T* s, const T* t,
+                                                      const T* rh, T* x, T* r, double* part_rho, CgLoop loop) {
+  __shared__ double sh[33];
+  __shared__ bool last;
+  pdl_go();
+  pdl_wait();
+  const T al = sc[2];
+  const T ts = (T)all_sum_partials(part_ts, np, sh);
+  const T om = ts / (T)all_sum_partials(part_tt, np, sh);
+  double rr = 0.0, rho = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    x[i] += al * ph[i] + om * sh_[i];
+    const T e = s[i] - om * t[i];
+    r[i] = e;
+    rr += (double)e * (double)e;
+    rho += (double)rh[i] * (double)e;
+  }
+  __syncthreads();  // sh is free again
+  rr = block_sum(rr, sh);
+  __syncthreads();
+  rho = block_sum(rho, sh);
+  if (threadIdx.x == 0) {
+    loop.part_rr[blockIdx.x] = rr;
+    part_rho[blockIdx.x] = rho;
+    __threadfence();
+    last = atomicInc(loop.ticket, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  rr = all_sum_partials(loop.part_rr, (int)gridDim.x, sh);
+  rho = all_sum_partials(part_rho, (int)gridDim.x, sh);
+  if (threadIdx.x != 0) return;
+  sc[1] = sc[0];
+  sc[0] = (T)rho;
+  sc[3] = om;
+  const double rn = sqrt(rr);
+  const int it = loop.state[0] + 1;
+  const bool conv = rn <= loop.ctl[2];
+  loop.state[0] = it;
+  loop.state[1] = conv ? 1 : 0;
+  cudaGraphSetConditional(loop.h, (!conv && isfinite(rn) && it < (int)loop.ctl[1]) ? 1u : 0u);
+}
+template <typename T>
+void bicg_p(int nbrow, const T* sc, const T* r, const T* v, T* p, const T* dinv, const T* co, T* sr, T* sd, Queue q) {
+  launch(q, bicg_p_kernel<T>, fused_update_blocks(nbrow), RED_THREADS, 0, nbrow, sc, r, v, p, dinv, co, sr, sd);
+}
+template <typename T>
+void bicg_s(int nbrow, const double* part, int np, T* sc, const T* r, const T* v, T* s, const T* dinv, const T* co,
+            T* sr, T* sd, Queue q) {
+  launch(q, bicg_s_kernel<T>, fused_update_blocks(nbrow), RED_THREADS, 0, nbrow, part, np, sc, r, v, s, dinv, co, sr,
+         sd);
+}
+template <typename T>
+void bicg_xr(long long n, T* sc, const T* ph, const T* sh, const T* s, const T* t, const T* rh, T* x, T* r,
+             double* part_ts, double* part_tt, double* part_rho, const CgLoop& loop, Queue q) {
+  const int blocks = fused_update_blocks(n);
+  launch(q, bicg_dots_kernel<T>, blocks, RED_THREADS, 0, n, t, s, part_ts, part_tt);
+  launch(q, bicg_xr_kernel<T>, blocks, RED_THREADS, 0, n, part_ts, part_tt, blocks, sc, ph, sh, s, t, rh, x, r,
+         part_rho, loop);
 }
 
 // precision conversion
@@ -1154,13 +1218,12 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, Queue q)
   template void dot<T>(long long, const T*, const T*, T*, T*, cudaStream_t, bool);                 \
   template void fill<T>(long long, T*, T, cudaStream_t);                                           \
   template void axpby<T>(long long, T, const T*, T, T*, cudaStream_t);                             \
-  template void cg_xr<T>(long long, const T*, const T*, const T*, const T*, T*, T*, cudaStream_t); \
-  template void cg_p<T>(long long, const T*, const T*, const T*, T*, cudaStream_t);                \
-  template void bicg_p<T>(long long, const T*, const T*, const T*, T*, cudaStream_t);              \
-  template void bicg_s<T>(long long, const T*, const T*, const T*, T*, cudaStream_t);              \
-  template void bicg_xr<T>(long long, const T*, const T*, const T*, const T*, const T*, T*, T*,    \
-                           cudaStream_t);                                                          \
-  template void scalar_copy<T>(T*, const T*, cudaStream_t);                                        \
+  template void bicg_p<T>(int, const T*, const T*, const T*, T*, const T*, const T*, T*, T*,       \
+                          Queue);                                                                  \
+  template void bicg_s<T>(int, const double*, int, T*, const T*, const T*, T*, const T*, const T*, \
+                          T*, T*, Queue);                                                          \
+  template void bicg_xr<T>(long long, T*, const T*, const T*, const T*, const T*, const T*, T*,    \
+                           T*, double*, double*, double*, const CgLoop&, Queue);                   \
   template int dot_partials_double<T>(long long, const T*, const T*, double*, const Queue&);       \
   template void cg_p_fused<T>(long long, const double*, int, T*, const T*, T*, Queue);             \
   template void cg_xr_fused<T>(int, const double*, int, T*, const T*, const T*, T*, T*, const T*, const T*, T*, T*, \

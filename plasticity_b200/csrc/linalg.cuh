@@ -91,12 +91,6 @@ template <typename T> void blockdiag_invert(const BsrMat<T>& A, T* dinv, cudaStr
 template <typename T> void dot(long long n, const T* a, const T* b, T* out, T* part, cudaStream_t st, bool take_sqrt);
 template <typename T> void fill(long long n, T* x, T v, cudaStream_t st);
 template <typename T> void axpby(long long n, T a, const T* x, T b, T* y, cudaStream_t st);
-template <typename T> void cg_xr(long long n, const T* num, const T* den, const T* p, const T* q, T* x, T* r, cudaStream_t st);
-template <typename T> void cg_p(long long n, const T* num, const T* den, const T* z, T* p, cudaStream_t st);
-template <typename T> void bicg_p(long long n, const T* sc, const T* r, const T* v, T* p, cudaStream_t st);
-template <typename T> void bicg_s(long long n, const T* sc, const T* r, const T* v, T* s, cudaStream_t st);
-template <typename T> void bicg_xr(long long n, const T* sc, const T* ph, const T* sh, const T* s, const T* t, T* x, T* r, cudaStream_t st);
-template <typename T> void scalar_copy(T* dst, const T* src, cudaStream_t st);
 // PCG updates with the dot products' final sums inside (deterministic):
 // cg_p_fused: rz = sum(part), p = z + (rz / sc[0]) p, sc[2] = rz;
 // cg_xr_fused: alpha = sc[2] / sum(part_pq), x += alpha p, r -= alpha q, sr = Dinv r,
@@ -115,6 +109,17 @@ template <typename T> int dot_partials_double(long long n, const T* a, const T* 
 template <typename T> void cg_p_fused(long long n, const double* part, int np, T* sc, const T* z, T* p, Queue q);
 template <typename T> void cg_xr_fused(int nbrow, const double* part_pq, int np, T* sc, const T* p, const T* q, T* x,
                                        T* r, const T* dinv, const T* co, T* sr, T* sd, const CgLoop& loop, Queue qu);
+// BiCGStab updates, with the smoother's start on p and on s (sr, sd as above):
+// bicg_p: p = r + beta (p - omega v); bicg_s: alpha = sc[0] / sum(part), s = r - alpha v;
+// bicg_xr: omega from the dot products of t with s and itself, x += alpha ph + omega sh,
+// r = s - omega t, the next rho and the loop condition (part_*: kMaxPartials each).
+template <typename T> void bicg_p(int nbrow, const T* sc, const T* r, const T* v, T* p, const T* dinv, const T* co,
+                                  T* sr, T* sd, Queue q);
+template <typename T> void bicg_s(int nbrow, const double* part, int np, T* sc, const T* r, const T* v, T* s,
+                                  const T* dinv, const T* co, T* sr, T* sd, Queue q);
+template <typename T> void bicg_xr(long long n, T* sc, const T* ph, const T* sh, const T* s, const T* t, const T* rh,
+                                   T* x, T* r, double* part_ts, double* part_tt, double* part_rho, const CgLoop& loop,
+                                   Queue q);
 template <typename A, typename B> void convert(long long n, const A* a, B* b, double s, cudaStream_t st);
 template <typename T> void add_to_double(long long n, const T* x, double* U, cudaStream_t st);
 template <typename KT> void impose_dirichlet(const BcDev& bc, long long ndof, double lam, const double* U, KT* K, double* R, double* dg, cudaStream_t st);
