@@ -5,16 +5,15 @@
 // Solver.jl:136-154).  The coarsest operator (6 x 6 blocks, a few thousand
 // unknowns) is expanded to a dense FP64 matrix and inverted in place by blocked
 // Gauss-Jordan elimination; the cycle then applies the inverse as one dense
-// matrix-vector product.  Per panel of NB columns K:
-//   1. diagonal kernel (one CTA): Dg = A[K,K]^{-1} by Gauss-Jordan in shared memory;
-//   2. panel kernel: the panel rows outside the diagonal block, A[K,j] <- Dg A[K,j],
-//      and a copy C = A[i,K] of the panel columns of the other rows;
-//   3. update kernel: A[i, j] -= C[i, :] P[:, j] for every row i outside the panel
-//      (P the scaled panel rows, Dg in the panel's own columns), with the panel's
-//      own columns starting from 0, which turns them into -C Dg; the tile that
-//      holds the diagonal block writes Dg there.
-// Every kernel reads only what the previous one finished writing, and A[K,K] is
-// read only by the diagonal kernel, so no CTA sees a block half replaced.
+// matrix-vector product.  One kernel per panel of NB columns K, over NB x NB tiles; it
+// gets copies of the panel's rows R = A[K, :] and columns C = A[:, K] and the inverse
+// Dg = A[K,K]^{-1}, all made by the kernel before, so a CTA reads from A only the tiles
+// that it writes itself:
+//   P = Dg R[:, j] for its columns j (Dg itself in the panel's own columns),
+//   A[i, j] <- A[i, j] - C[i, :] P outside the panel's rows (0 - C Dg in its columns),
+//   A[K, j] <- P,
+// and it copies what belongs to the next panel.  The CTA with the next diagonal block
+// inverts that before its other tiles: 64 serial steps, which the other CTAs' work hides.
 // No row exchanges: the Galerkin operator of the (Dirichlet-imposed) tangent of a
 // large mesh is close to symmetric positive definite; a pivot below 1e-14 of the
 // largest diagonal entry is replaced by that floor.  Coarsest levels of up to
@@ -27,8 +26,8 @@ namespace pfem {
 namespace {
 
 constexpr int NB = 64;      // panel width
-constexpr int TR_ = 128;    // update tile rows
-constexpr int TC_ = 64;     // update tile columns
+constexpr int PITCH = 68;   // of a tile in shared memory: a half-warp's fragment falls on 16 bank pairs
+constexpr int GTHREADS = 256;
 
 // Dense row-major n x n FP64 matrix from the coarsest level's 6 x 6 blocks.
 template <typename T>
@@ -77,21 +76,20 @@ __global__ void dense_diag_max_kernel(int n, const double* __restrict__ A, doubl
   }
 }
 
-// Dg = A[K,K]^{-1}: in-place Gauss-Jordan on the NB x NB diagonal block, one CTA of
+// Dg = inverse of the NB x NB block at src: in-place Gauss-Jordan by one CTA of
 // eight warps with the block in registers: warp w holds the columns w, w + 8, ..., lane
 // l the rows l and l + 32.  What bounds it is the chain of 64 steps, so each has one
 // __syncthreads: the column's warp publishes it as the multipliers, every warp takes the
 // pivot from there.  As in pivot_inverse_kernel a row is divided by its pivot at the
-// end.  19.7 us; with the block in shared memory and five barriers per step 60 us.
-__global__ void __launch_bounds__(256) gj_diag_kernel(int n, int kb, const double* __restrict__ A,
-                                                      double* __restrict__ Dg, const double* __restrict__ scl) {
-  __shared__ double F[2][NB];
+// end.  19.7 us as a kernel of its own; with the block in shared memory and five
+// barriers per step 60 us.
+__device__ __forceinline__ void gj_invert(const double* src, int ld, double (*F)[NB], const double* scl, double* Dg) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double a[8][2];
 #pragma unroll
   for (int m = 0; m < 8; ++m)
 #pragma unroll
-    for (int r = 0; r < 2; ++r) a[m][r] = A[(long long)(kb + lane + 32 * r) * n + kb + w + 8 * m];
+    for (int r = 0; r < 2; ++r) a[m][r] = src[(long long)(lane + 32 * r) * ld + w + 8 * m];
   const double floor_abs = 1e-14 * fmax(scl[0], 1e-300);
   double ips[2] = {1.0, 1.0};  // 1 / pivot of the lane's rows
 #pragma unroll
@@ -137,112 +135,147 @@ __global__ void __launch_bounds__(256) gj_diag_kernel(int n, int kb, const doubl
     for (int r = 0; r < 2; ++r) Dg[(lane + 32 * r) * NB + w + 8 * m] = a[m][r] * ips[r];
 }
 
-// Panel step kb.  CTAs [0, ncb): 64 panel-row columns each, A[K, j] <- Dg A[K, j]
-// for j outside K (the 64 x 64 slab staged in shared memory; a thread computes four
-// rows of four columns, 16 apart: eight reads for 16 multiply-adds).  CTAs [ncb, ...): C[i, :] = A[i, K] for rows i
-// outside K, a warp per row.
-__global__ void __launch_bounds__(256) gj_panel_kernel(int n, int kb, int ncb, double* __restrict__ A,
-                                                       double* __restrict__ C, const double* __restrict__ Dg) {
-  extern __shared__ __align__(16) double psm[];
-  const int t = threadIdx.x;
-  if ((int)blockIdx.x >= ncb) {
-    const int w = t >> 5, lane = t & 31;
-    const int i = ((int)blockIdx.x - ncb) * 8 + w;
-    if (i < n && (i < kb || i >= kb + NB)) {
-      C[(long long)i * NB + lane] = A[(long long)i * n + kb + lane];
-      C[(long long)i * NB + 32 + lane] = A[(long long)i * n + kb + 32 + lane];
-    }
-    return;
+// A 64 x 64 tile to shared memory, 16 bytes at a time.
+__device__ __forceinline__ void gj_load(double* dst, const double* src, long long ld) {
+  const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll
+  for (int u = 0; u < NB * NB / 2 / GTHREADS; ++u) {
+    const int e = threadIdx.x + u * GTHREADS, r = e / (NB / 2), c = e % (NB / 2) * 2;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d0 + (uint32_t)(r * PITCH + c) * 8u),
+                 "l"(src + r * ld + c) : "memory");
   }
-  const int j0 = (int)blockIdx.x * 64;
-  if (j0 == kb) return;  // the diagonal block's columns: Dg, written by the update kernel
-  double(*D)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(psm);
-  double(*V)[65] = reinterpret_cast<double(*)[65]>(psm + NB * (NB + 1));
-  for (int e = t; e < NB * NB; e += 256) D[e / NB][e % NB] = Dg[e];
-  for (int e = t; e < NB * 64; e += 256) {
-    const int r = e / 64, c = e % 64, j = j0 + c;
-    V[r][c] = j < n ? A[(long long)(kb + r) * n + j] : 0.0;
-  }
+}
+__device__ __forceinline__ void gj_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  const int c = t & 15, q = t >> 4;
-  double out[4][4];
+}
+// acc = X Y of two tiles in shared memory on the FP64 matrix pipe: warp w takes the rows
+// 32 (w % 2) .. and the columns 16 (w / 2) .., as 4 x 2 fragments of 8 x 8.
+__device__ __forceinline__ void gj_mul(const double* X, const double* Y, double (&acc)[4][2][2]) {
+  const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+  const double* x = X + (32 * (w & 1) + g) * PITCH + q;
+  const double* y = Y + q * PITCH + 16 * (w >> 1) + g;
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) out[r][u] = 0.0;
-#pragma unroll 8
-  for (int s = 0; s < NB; ++s) {
-    double d[4], v[4];
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll 4
+  for (int s = 0; s < NB; s += 4) {
+    double xa[4], yb[2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) d[r] = D[q * 4 + r][s];
+    for (int i = 0; i < 4; ++i) xa[i] = x[8 * i * PITCH + s];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = V[s][c + 16 * u];
+    for (int j = 0; j < 2; ++j) yb[j] = y[s * PITCH + 8 * j];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) out[r][u] += d[r] * v[u];
+      for (int j = 0; j < 2; ++j)
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                     : "d"(xa[i]), "d"(yb[j]));
   }
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + c + 16 * u;
-      if (j < n) A[(long long)(kb + q * 4 + r) * n + j] = out[r][u];
-    }
+}
+// Row and column within the tile of fragment (i, j)'s first of two entries.
+__device__ __forceinline__ int gj_row(int i) { return 32 * ((threadIdx.x >> 5) & 1) + 8 * i + ((threadIdx.x & 31) >> 2); }
+__device__ __forceinline__ int gj_col(int j) { return 16 * (threadIdx.x >> 6) + 8 * j + 2 * (threadIdx.x & 3); }
+
+// Copies and the inverse for the first panel; CTA b copies tile b of each.
+__global__ void __launch_bounds__(GTHREADS) gj_start_kernel(int np, const double* __restrict__ A, double* __restrict__ C,
+                                                            double* __restrict__ R, double* __restrict__ Dg,
+                                                            const double* __restrict__ scl) {
+  __shared__ double F[2][NB];
+  const long long t0 = (long long)blockIdx.x * NB;
+  for (int e = threadIdx.x; e < NB * NB; e += GTHREADS) {
+    const int r = e / NB, c = e % NB;
+    R[(long long)r * np + t0 + c] = A[(long long)r * np + t0 + c];
+    C[t0 * NB + e] = A[(t0 + r) * np + c];
+  }
+  if (blockIdx.x == 0) gj_invert(A, np, F, scl, Dg);
 }
 
-// Trailing update of step kb over TR_ x TC_ tiles; rows of the panel are final.
-// Thread (rg, cg) holds rows rg*8 .. +7 and columns cg + 16 b, b < 4.
-__global__ void __launch_bounds__(256, 2) gj_update_kernel(int n, int kb, double* __restrict__ A,
-                                                           const double* __restrict__ C,
-                                                           const double* __restrict__ Dg) {
-  extern __shared__ __align__(16) double usm[];
-  double(*Cs)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(usm);              // TR_ x NB
-  double(*Ps)[TC_ + 1] = reinterpret_cast<double(*)[TC_ + 1]>(usm + TR_ * (NB + 1));  // NB x TC_
-  const int i0 = (int)blockIdx.y * TR_, j0 = (int)blockIdx.x * TC_;
-  const int t = threadIdx.x;
-  for (int e = t; e < TR_ * NB; e += 256) {
-    const int r = e / NB, s = e % NB, i = i0 + r;
-    Cs[r][s] = (i < n && (i < kb || i >= kb + NB)) ? C[(long long)i * NB + s] : 0.0;
+// Step k (the comment at the top).  CTA (j, y): column tile j and every gridDim.y-th row
+// tile, from k + 1 on.  Two CTAs on an SM; the grid is at most that many.  What bounds it
+// is the chain copies -> P -> update -> inverse of one CTA.  A panel at 1440 unknowns
+// takes 32 us; as three kernels (diagonal 20 us, panel rows 22, update 43 with its loads
+// and stores of A one after another) 85 us.  The set-up at 21 x 17 x 13 with it 1.3 ms,
+// 2.0 before; at 40^3 (750 unknowns) 0.75 ms less.
+__global__ void __launch_bounds__(GTHREADS, 2) gj_step_kernel(int np, int k, double* A, const double* C, const double* R,
+                                                              const double* Dg, double* C1, double* R1, double* Dg1,
+                                                              const double* scl) {
+  extern __shared__ __align__(16) double gsm[];
+  __shared__ double F[2][NB];
+  double* const D = gsm;
+  double* const V = gsm + NB * PITCH;
+  double* const Cs = gsm + 2 * NB * PITCH;
+  const int nt = np / NB, jt = (int)blockIdx.x;
+  const long long j0 = (long long)jt * NB;
+  pdl_go();
+  pdl_wait();
+  auto row_tile = [&](int i) { return (k + 1 + i) % nt; };
+  gj_load(D, Dg, NB);
+  if (jt != k) gj_load(V, R + j0, np);
+  const int first = row_tile((int)blockIdx.y);
+  if (first != k) gj_load(Cs, C + (long long)first * NB * NB, NB);
+  gj_wait();
+  double acc[4][2][2];
+  if (jt != k) {
+    gj_mul(D, V, acc);
+    __syncthreads();  // V has been read
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        *reinterpret_cast<double2*>(V + gj_row(i) * PITCH + gj_col(j)) = make_double2(acc[i][j][0], acc[i][j][1]);
+    __syncthreads();
   }
-  const bool diag_cols = j0 == kb;  // TC_ == NB and both are multiples of NB: the panel is one column tile
-  for (int e = t; e < NB * TC_; e += 256) {
-    const int s = e / TC_, c = e % TC_, j = j0 + c;
-    Ps[s][c] = j >= n ? 0.0 : diag_cols ? Dg[s * NB + c] : A[(long long)(kb + s) * n + j];
-  }
-  // the tile holding the diagonal block writes it (no other CTA reads it from A)
-  if (diag_cols && kb >= i0 && kb < i0 + TR_)
-    for (int e = t; e < NB * NB; e += 256) A[(long long)(kb + e / NB) * n + kb + e % NB] = Dg[e];
-  __syncthreads();
-  const int rg = t / 16, cg = t % 16;
-  double acc[8][4];
+  const double* const P = jt != k ? V : D;
+  for (int it = (int)blockIdx.y; it < nt; it += (int)gridDim.y) {
+    const int rt = row_tile(it);
+    const long long i0 = (long long)rt * NB;
+    double2 v[4][2];
+    if (rt == k) {
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-#pragma unroll 4
-  for (int s = 0; s < NB; ++s) {
-    double cv[8], pv[4];
+        for (int j = 0; j < 2; ++j) v[i][j] = *reinterpret_cast<const double2*>(P + gj_row(i) * PITCH + gj_col(j));
+    } else {
 #pragma unroll
-    for (int a = 0; a < 8; ++a) cv[a] = Cs[rg * 8 + a][s];
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) pv[b] = Ps[s][cg + 16 * b];
+        for (int j = 0; j < 2; ++j)
+          v[i][j] = jt == k ? make_double2(0.0, 0.0)
+                            : *reinterpret_cast<const double2*>(A + (i0 + gj_row(i)) * np + j0 + gj_col(j));
+      if (it != (int)blockIdx.y) {
+        __syncthreads();  // Cs has been read
+        gj_load(Cs, C + i0 * NB, NB);
+        gj_wait();
+      }
+      gj_mul(Cs, P, acc);
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] += cv[a] * pv[b];
-  }
+        for (int j = 0; j < 2; ++j) {
+          v[i][j].x -= acc[i][j][0];
+          v[i][j].y -= acc[i][j][1];
+        }
+    }
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int i = i0 + rg * 8 + a;
-    if (i >= n || (i >= kb && i < kb + NB)) continue;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int j = j0 + cg + 16 * b;
-      if (j >= n) continue;
-      double* p = A + (long long)i * n + j;
-      const double old = diag_cols ? 0.0 : *p;
-      *p = old - acc[a][b];
+      for (int j = 0; j < 2; ++j) {
+        const int r = gj_row(i), c = gj_col(j);
+        *reinterpret_cast<double2*>(A + (i0 + r) * np + j0 + c) = v[i][j];
+        if (jt == k + 1) *reinterpret_cast<double2*>(C1 + (i0 + r) * NB + c) = v[i][j];
+        if (rt == k + 1) *reinterpret_cast<double2*>(R1 + (long long)r * np + j0 + c) = v[i][j];
+      }
+    if (rt == k + 1 && jt == k + 1) {  // the next diagonal block
+      __syncthreads();  // Cs has been read
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) *reinterpret_cast<double2*>(Cs + gj_row(i) * PITCH + gj_col(j)) = v[i][j];
+      __syncthreads();
+      gj_invert(Cs, PITCH, F, scl, Dg1);
     }
   }
 }
@@ -456,7 +489,7 @@ __global__ void dense_out_kernel(int n, int np, const double* __restrict__ A, T*
 
 long long dense_inverse_work_doubles(int n) {
   const int np = (n + NB - 1) / NB * NB;
-  return (long long)np * np + (long long)np * NB + NB * NB + 8;
+  return (long long)np * np + 4 * (long long)np * NB + 2 * NB * NB + 8;
 }
 
 // inv (n x n, row-major, precision T) = inverse of the coarsest operator given by
@@ -468,17 +501,13 @@ void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val,
                           cudaStream_t st) {
   const int np = (n + NB - 1) / NB * NB;
   double* A = work;
-  double* C = work + (long long)np * np;
-  double* Dg = C + (long long)np * NB;
-  double* scl = Dg + NB * NB;
-  const size_t panel_sm = (size_t)(NB * (NB + 1) + NB * 65) * sizeof(double);
-  const size_t update_sm = (size_t)(TR_ * (NB + 1) + NB * (TC_ + 1)) * sizeof(double);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(gj_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_sm);
-    cudaFuncSetAttribute(gj_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_sm);
-    attr = true;
-  }
+  const long long slab = (long long)np * NB;
+  double* const C = work + (long long)np * np;  // two each, taken in turn
+  double* const R = C + 2 * slab;
+  double* const Dg = R + 2 * slab;
+  double* const scl = Dg + 2 * NB * NB;
+  const int step_sm = 3 * NB * PITCH * (int)sizeof(double), nt = np / NB;
+  cudaFuncSetAttribute(gj_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, step_sm);
   cudaMemsetAsync(A, 0, (size_t)np * np * sizeof(double), st);
   count_launch();
   bsr6_to_dense_kernel<T><<<1024, 256, 0, st>>>(nbrow, rp, cl, val, np, A);
@@ -486,15 +515,16 @@ void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val,
   dense_fix_rows_kernel<<<(np + 7) / 8, 256, 0, st>>>(np, A);
   count_launch();
   dense_diag_max_kernel<<<1, 1024, 0, st>>>(np, A, scl);
-  const int ncb = np / 64, nrb = (np + 7) / 8;
-  const dim3 ug((np + TC_ - 1) / TC_, (np + TR_ - 1) / TR_);
-  for (int kb = 0; kb < np; kb += NB) {
-    count_launch();
-    gj_diag_kernel<<<1, 256, 0, st>>>(np, kb, A, Dg, scl);
-    count_launch();
-    gj_panel_kernel<<<ncb + nrb, 256, panel_sm, st>>>(np, kb, ncb, A, C, Dg);
-    count_launch();
-    gj_update_kernel<<<ug, 256, update_sm, st>>>(np, kb, A, C, Dg);
+  count_launch();
+  gj_start_kernel<<<nt, GTHREADS, 0, st>>>(np, A, C, R, Dg, scl);
+  // all CTAs run at once, two on an SM, so that the one with the next diagonal block
+  // does not wait for a place
+  const dim3 grid(nt, std::max(1, std::min(nt, 2 * 148 / nt)));
+  int chain = 0;
+  for (int k = 0; k < nt; ++k) {
+    const int a = k & 1, b = a ^ 1;
+    launch(Queue(st, &chain), gj_step_kernel, grid, GTHREADS, step_sm, np, k, A, C + a * slab, R + a * slab,
+           Dg + a * NB * NB, C + b * slab, R + b * slab, Dg + b * NB * NB, scl);
   }
   count_launch();
   dense_out_kernel<T><<<2048, 256, 0, st>>>(n, np, A, inv);

@@ -585,7 +585,7 @@ void power_finish(int np, const double* prev, const double* last, T* co, cudaStr
 }
 // ---- BiCGStab updates.  Scalars: sc[0] rho = rh.r, sc[1] rho of the iteration before,
 // sc[2] alpha, sc[3] omega.  A thread per node, as cg_xr_fused; the dot products come as
-// partials in double.  An iteration used to be 78 plain launches from the host with a
+// partials in double.  An iteration used to be 44 plain launches from the host with a
 // read-back of |r|, bound by the launches below about 40^3; in the graph with the
 // smoother's starts in its own updates it takes 440 us at 40^3 FP64, 550 before.
 template <typename T>

@@ -23,14 +23,14 @@ struct Queue {
   Queue(cudaStream_t s, int* c) : st(s), chain(c) {}
 };
 template <typename... K, typename... A>
-inline void launch(const Queue& q, void (*kern)(K...), int grid, int block, size_t smem, A... args) {
+inline void launch(const Queue& q, void (*kern)(K...), dim3 grid, int block, size_t smem, A... args) {
   count_launch();
-  if (!q.chain || (*q.chain)++ == 0 || grid > kChainGrid) {
+  if (!q.chain || (*q.chain)++ == 0 || grid.x * grid.y > (unsigned)kChainGrid) {
     kern<<<grid, block, smem, q.st>>>(static_cast<K>(args)...);
     return;
   }
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
+  c.gridDim = grid;
   c.blockDim = dim3(block);
   c.dynamicSmemBytes = smem;
   c.stream = q.st;
