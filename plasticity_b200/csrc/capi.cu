@@ -716,15 +716,18 @@ int amg_alloc(pfem_ctx* ctx) {
     std::vector<T> Th(h.T.begin(), h.T.end());
     CK(upload(ctx, &v.T, Th));
     v.nnzP = (int)h.p_cl.size();
-    CK(upload(ctx, &v.p_rp, h.p_rp)); CK(upload(ctx, &v.p_cl, h.p_cl)); CK(upload(ctx, &v.p_row, h.p_row));
+    CK(upload(ctx, &v.p_rp, h.p_rp)); CK(upload(ctx, &v.p_cl, h.p_cl, kCopySlack)); CK(upload(ctx, &v.p_row, h.p_row));
     CK(upload(ctx, &v.pslot, h.pslot)); CK(upload(ctx, &v.pt_rp, h.pt_rp)); CK(upload(ctx, &v.pt_blk, h.pt_blk));
     {
       std::vector<int> ptr_row(h.pt_blk.size());
       for (size_t t = 0; t < h.pt_blk.size(); ++t) ptr_row[t] = h.p_row[h.pt_blk[t]];
-      CK(upload(ctx, &v.pt_row, ptr_row));
+      CK(upload(ctx, &v.pt_row, ptr_row, kCopySlack));
     }
-    CK(dalloc(ctx, &v.p_val, (size_t)v.nnzP * h.bs * 6));
-    CK(dalloc(ctx, &v.pt_val, (size_t)v.nnzP * h.bs * 6));
+    CK(dalloc(ctx, &v.p_val, (size_t)v.nnzP * h.bs * 6, kCopySlack));
+    CK(dalloc(ctx, &v.pt_val, (size_t)v.nnzP * h.bs * 6, kCopySlack));
+    for (int n = 0; n < h.nbrow; n += pfem::kProlongTile)
+      v.p_tile = std::max(v.p_tile, h.p_rp[std::min(h.nbrow, n + pfem::kProlongTile)] - h.p_rp[n]);
+    for (int i = 0; i < h.nagg; ++i) v.pt_max = std::max(v.pt_max, h.pt_rp[i + 1] - h.pt_rp[i]);
     v.nnzAP = (int)h.ap_cl.size();
     CK(upload(ctx, &v.ap_rp, h.ap_rp)); CK(upload(ctx, &v.ap_cl, h.ap_cl)); CK(upload(ctx, &v.ap_row, h.ap_row));
     CK(dalloc(ctx, &v.ap_val, (size_t)v.nnzAP * h.bs * 6));

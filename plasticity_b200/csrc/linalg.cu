@@ -1169,11 +1169,157 @@ void sa_setup_level(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st) {
   if (v.A.bs == 3) setup_level_t<T, 3>(v, cval, nnzC, st);
   else setup_level_t<T, 6>(v, cval, nnzC, st);
 }
+// ---- transfers of the finest level with the blocks streamed through shared memory ----
+// Read straight into registers a lane's 72-byte block costs the L1 a line per lane and
+// load, as the matrix does (spmv_pipe.cuh).  Bytes of a tile's copies: the barrier, the
+// ids, the blocks, each with room for ends rounded out to 16 bytes.
+template <typename T>
+__host__ __device__ inline int stream_vals(int blocks) { return 16 + ((blocks * 4 + 32 + 15) & ~15); }
+template <typename T>
+inline int stream_bytes(int blocks) { return stream_vals<T>(blocks) + blocks * 18 * (int)sizeof(T) + 32; }
+// Blocks t0 .. t1 and their ids; one thread.
+template <typename T>
+__device__ __forceinline__ void stream_issue(unsigned char* sm, int cap, int t0, int t1, const int* ids, const T* vals) {
+  constexpr int VB = 18 * (int)sizeof(T);
+  const uint32_t bar = bulk_smem(sm);
+  const long long ia = ((long long)t0 * 4) & ~15ll, va = ((long long)t0 * VB) & ~15ll;
+  const uint32_t ib = (uint32_t)((((long long)t1 * 4 + 15) & ~15ll) - ia);
+  const uint32_t vb = (uint32_t)((((long long)t1 * VB + 15) & ~15ll) - va);
+  bulk_bar_init(bar, 1);
+  bulk_init_fence();
+  if (t0 == t1) {
+    bulk_expect(bar, 0);
+    return;
+  }
+  bulk_expect(bar, ib + vb);
+  bulk_copy(bar + 16, (const char*)ids + ia, ib, bar);
+  bulk_copy_first(bar + (uint32_t)stream_vals<T>(cap), (const char*)vals + va, vb, bar);
+}
+// sa_restrict_kernel<T, 3, 1, START> with a one-warp CTA per aggregate, its P^T row in
+// shared memory; the sums are added in the same order.
+template <typename T, bool START>
+__global__ void __launch_bounds__(32)
+sa_restrict_stream_kernel(int cap, const int* __restrict__ pt_rp, const int* __restrict__ pt_row,
+                          const T* __restrict__ ptval, const T* r, T* bc, const T* __restrict__ dinv,
+                          const T* __restrict__ co, T* sr, T* sd, int* err) {
+  extern __shared__ __align__(128) unsigned char tsm[];
+  pdl_go();
+  const int I = blockIdx.x, lane = threadIdx.x;
+  const int t0 = pt_rp[I], t1 = pt_rp[I + 1];
+  if (lane == 0) stream_issue<T>(tsm, cap, t0, t1, pt_row, ptval);
+  __syncwarp();
+  T D[6], ith = T(0);
+  if constexpr (START) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j) D[j] = lane < 6 ? dinv[(long long)I * 36 + lane * 6 + j] : T(0);
+    ith = co[CO_ITH];
+  }
+  pdl_wait();
+  if (!__all_sync(0xffffffffu, bulk_bar_wait(bulk_smem(tsm), 0))) {
+    if (lane == 0) atomicExch(err, 1);
+    return;
+  }
+  const int* ids = reinterpret_cast<const int*>(tsm + 16 + (((long long)t0 * 4) & 15));
+  const T* vals = reinterpret_cast<const T*>(tsm + stream_vals<T>(cap) + (((long long)t0 * 18 * (int)sizeof(T)) & 15));
+  T s[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+  for (int t = lane; t < t1 - t0; t += 32) {
+    const T* rv = r + (long long)ids[t] * 3;
+    const T* P = vals + t * 18;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const T rj = rv[j];
+      T pv[6];
+      load6<T, false>(P + j * 6, pv);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) s[c] += pv[c] * rj;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+  if (lane >= 6) return;
+  T out = s[0];
+#pragma unroll
+  for (int c = 1; c < 6; ++c)
+    if (lane == c) out = s[c];
+  bc[(long long)I * 6 + lane] = out;
+  if constexpr (START) {
+    T w = T(0);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) w += D[j] * s[j];
+    sr[(long long)I * 6 + lane] = w;
+    sd[(long long)I * 6 + lane] = ith * w;
+  }
+}
+// sa_prolong_kernel<T, 3> with the P rows of a CTA's 32 nodes in shared memory, a thread
+// per entry; the same sums.
+template <typename T>
+__global__ void __launch_bounds__(3 * kProlongTile)
+sa_prolong_stream_kernel(int nbrow, int cap, const int* __restrict__ p_rp, const int* __restrict__ p_cl,
+                         const T* __restrict__ pval, const T* xc, T* x, int* err) {
+  extern __shared__ __align__(128) unsigned char tsm[];
+  pdl_go();
+  const int n0 = blockIdx.x * kProlongTile, n1 = min(nbrow, n0 + kProlongTile);
+  const int n = n0 + (int)threadIdx.x / 3, j = (int)threadIdx.x % 3;
+  const bool in = n < n1;
+  const int t0 = p_rp[n0];
+  if (threadIdx.x == 0) stream_issue<T>(tsm, cap, t0, p_rp[n1], p_cl, pval);
+  const int p0 = in ? p_rp[n] - t0 : 0, p1 = in ? p_rp[n + 1] - t0 : 0;
+  __syncthreads();
+  pdl_wait();
+  const long long i = (long long)n * 3 + j;
+  const T xi = in ? x[i] : T(0);
+  if (!bulk_bar_wait(bulk_smem(tsm), 0)) {
+    atomicExch(err, 1);
+    return;
+  }
+  const int* ids = reinterpret_cast<const int*>(tsm + 16 + (((long long)t0 * 4) & 15));
+  const T* vals = reinterpret_cast<const T*>(tsm + stream_vals<T>(cap) + (((long long)t0 * 18 * (int)sizeof(T)) & 15));
+  T s = T(0);
+#pragma unroll 4
+  for (int p = p0; p < p1; ++p) {
+    T xv[6], pv[6];
+    load6<T, false>(xc + (long long)ids[p] * 6, xv);
+    load6<T, false>(vals + p * 18 + j * 6, pv);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) s += pv[c] * xv[c];
+  }
+  if (in) x[i] = xi + s;
+}
+// The prolongation streams from as many rows on as the matrix does (kPipeRows3; at 16^3,
+// 4,913 rows, the cycle takes 22.7 us either way).  The restriction streams where the
+// matrix alone fills L2 (126 MB): there it is the early eviction of the streamed blocks,
+// more than the shorter kernel, that counts, as it leaves L2 to the vectors; below, it
+// evicts what would have stayed.  CG iteration, neither / prolongation / both streamed:
+// 139.7 / 137.8 / 140.9 us at 32^3 FP64 (66 MB of matrix), 184 / 184 / 188 at
+// 49 x 37 x 29 FP64 (105 MB), 224.9 / 225.0 / 213.2 at 40^3 FP64 (128 MB), 249 / 245 / 230
+// at 56 x 50 x 48 FP32 (133 MB), 392 / 385 / 377 at 64^3 FP32 (259 MB); both without
+// early eviction 230.9 at 40^3 FP64 and 384 at 64^3.
+constexpr int kStreamSmem = 48 * 1024;  // a tile's most, so that four or more CTAs share an SM
+constexpr long long kMatrixFillsL2 = 120000000;
+template <typename T>
+static bool transfer_streams(const AmgLevel<T>& v, int blocks) {
+  return v.A.bs == 3 && v.A.nbrow >= kPipeRows3 && v.A.err && blocks > 0 && stream_bytes<T>(blocks) <= kStreamSmem;
+}
+template <typename T>
+static bool matrix_fills_l2(const AmgLevel<T>& v) {
+  return v.A.nnzb * 9 * (long long)sizeof(T) > kMatrixFillsL2;
+}
+
 // Aggregates below this count get four warps each in the restriction.
 constexpr int kRestrictWideBelow = 4096;
 
 template <typename T>
 void sa_restrict(const AmgLevel<T>& v, const T* r, T* bc, const AmgLevel<T>* next, Queue q) {
+  if (transfer_streams(v, v.pt_max) && matrix_fills_l2(v)) {
+    auto* kern = next ? sa_restrict_stream_kernel<T, true> : sa_restrict_stream_kernel<T, false>;
+    launch(q, kern, v.nagg, 32, stream_bytes<T>(v.pt_max), v.pt_max, v.pt_rp, v.pt_row, v.pt_val, r, bc,
+           next ? next->dinv : nullptr, next ? next->co : nullptr, next ? next->r : nullptr, next ? next->d : nullptr,
+           v.A.err);
+    return;
+  }
   const bool wide = v.nagg < kRestrictWideBelow;
   const long long warps = (long long)v.nagg * (wide ? 4 : 1);
   const int blocks = (int)((warps + 7) / 8);
@@ -1193,6 +1339,11 @@ static void prolong_launch(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x
 }
 template <typename T>
 void sa_prolong(const AmgLevel<T>& v, const T* xc, T* x, Queue q) {
+  if (transfer_streams(v, v.p_tile)) {
+    launch(q, sa_prolong_stream_kernel<T>, (v.A.nbrow + kProlongTile - 1) / kProlongTile, 3 * kProlongTile,
+           stream_bytes<T>(v.p_tile), v.A.nbrow, v.p_tile, v.p_rp, v.p_cl, v.p_val, xc, x, v.A.err);
+    return;
+  }
   prolong_launch<T>(v, xc, nullptr, x, q);
 }
 template <typename T>

@@ -86,6 +86,8 @@ struct BsrMat {
 // first step of any degree), c1, c2; the prolongator's 4 / (3 rho).
 enum : int { CO_LMAX = 0, CO_ITH = 1, CO_C1 = 2, CO_C2 = 3, CO_OMEGA = 4, CO_COUNT = 8 };
 
+constexpr int kProlongTile = 32;
+
 // One level of smoothed-aggregation AMG.  Every fine block row n belongs to
 // one aggregate agg[n] and carries the tentative bs x 6 block T_n (the six
 // rigid-body modes, orthonormalised per aggregate).  The prolongator is
@@ -107,6 +109,7 @@ struct AmgLevel {
   int *pt_rp = nullptr, *pt_blk = nullptr;  // P^T: P blocks of each aggregate
   int* pt_row = nullptr;  // P^T order: the fine block row of each block
   VT* pt_val = nullptr;   // P^T order: a copy of the P blocks, streamed by the restriction
+  int p_tile = 0, pt_max = 0;  // most blocks of kProlongTile rows of P, of a row of P^T
   int nnzAP = 0;
   int *ap_rp = nullptr, *ap_cl = nullptr, *ap_row = nullptr;
   VT* ap_val = nullptr;
