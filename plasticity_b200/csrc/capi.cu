@@ -72,6 +72,7 @@ struct ReadBack {
   int waits;             // set by a solver kernel whose bounded wait ran out
   int cg[2][2];          // [precision]: iterations, converged
   double scal[2];        // [0] |R|
+  unsigned ticket;       // load_norm_kernel's, zero between its launches
 };
 
 struct HostLevel {
@@ -123,7 +124,7 @@ struct pfem_ctx {
   double* dOut = nullptr;   // 6 x ngp scratch for per-GP results in the caller's layout (lazy)
   int hard = HARD_LINEAR;   // hardening law of the element kernels
   uint8_t* dFlags = nullptr;
-  double *dU = nullptr, *dR = nullptr, *dDg = nullptr, *dUprev = nullptr, *dUprev2 = nullptr;
+  double *dU = nullptr, *dR = nullptr, *dUprev = nullptr, *dUprev2 = nullptr;
   double* dUprev3 = nullptr;
   double bbox_lo[3] = {0, 0, 0}, bbox_ext[3] = {1, 1, 1};
   double *dUtmp = nullptr, *dPart = nullptr;
@@ -1296,10 +1297,12 @@ int residual_system(pfem_ctx* ctx, int prec, double lam, double* rnorm, double* 
   rc = assemble_dev(ctx, prec, false);
   if (rc) return rc;
   CK(cudaEventRecord(ctx->e1, ctx->st));
-  if (prec == PFEM_FP64) impose_dirichlet<double>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK64, ctx->dR, ctx->dDg, ctx->st);
-  else impose_dirichlet<float>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK32, ctx->dR, ctx->dDg, ctx->st);
-  CKL();
-  dot<double>(ctx->ndof, ctx->dR, ctx->dR, ctx->dBack->scal, ctx->dPart, ctx->st, true);
+  if (prec == PFEM_FP64)
+    impose_dirichlet<double>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK64, ctx->dR, ctx->dPart, &ctx->dBack->ticket,
+                             ctx->dBack->scal, ctx->st);
+  else
+    impose_dirichlet<float>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK32, ctx->dR, ctx->dPart, &ctx->dBack->ticket,
+                            ctx->dBack->scal, ctx->st);
   CKL();
   rc = check_status(ctx);  // synchronizes
   *rnorm = ctx->hBack->scal[0];
@@ -1929,7 +1932,6 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
   AL(ctx->dFlags, ctx->ngp);
   AL(ctx->dU, ctx->ndof);
   AL(ctx->dR, ctx->ndof);
-  AL(ctx->dDg, ctx->ndof);
   AL(ctx->dUprev, ctx->ndof);
   AL(ctx->dUprev2, ctx->ndof);
   AL(ctx->dUprev3, ctx->ndof);
@@ -2068,6 +2070,7 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
     CK(h2d(ctx, b.vals, vals.data(), vals.size() * sizeof(double)));
     CK(h2d(ctx, b.ramp, ramp.data(), ramp.size() * sizeof(uint8_t)));
     if (!same_neu) {
+      for (int d : dofs) fn[d] = 0.0;
       CK(h2d(ctx, b.fn, fn.data(), fn.size() * sizeof(double)));
       ctx->neu_dofs_last.assign(neu_dofs, neu_dofs + nneu);
       ctx->neu_vals_last.assign(neu_vals, neu_vals + nneu);
@@ -2080,7 +2083,7 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
     for (int64_t i = 0; i < nneu; ++i) fn[neu_dofs[i] - 1] += neu_vals[i];
   }
   std::vector<uint8_t> isbc(ndof, 0);
-  for (int d : dofs) isbc[d] = 1;
+  for (int d : dofs) { isbc[d] = 1; fn[d] = 0.0; }
   // entries touched by the imposition
   auto blk = [&](int n, int m) -> long long {
     const int* b0 = ctx->bcol.data() + ctx->browptr[n];
@@ -2088,9 +2091,9 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
     return ctx->browptr[n] + (long long)(std::lower_bound(b0, b1, m) - b0);
   };
   std::vector<std::pair<long long, uint8_t>> zl;
-  std::vector<std::tuple<int, int, long long>> rl;  // (row, col, pos)
-  for (int d : dofs) {
-    const int n = d / 3, c = d % 3;
+  std::vector<std::tuple<int, int, long long>> rl;  // (row, index of the column's dof, pos)
+  for (int q = 0; q < (int)dofs.size(); ++q) {
+    const int d = dofs[q], n = d / 3, c = d % 3;
     for (int k = ctx->browptr[n]; k < ctx->browptr[n + 1]; ++k) {
       const int m = ctx->bcol[k];
       for (int j = 0; j < 3; ++j) zl.push_back({(long long)k * 9 + c * 3 + j, (uint8_t)(3 * m + j == d)});
@@ -2098,16 +2101,14 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
       const long long bk = blk(m, n);
       for (int i = 0; i < 3; ++i) {
         const int r = 3 * m + i;
-        const long long pos = bk * 9 + i * 3 + c;
-        zl.push_back({pos, (uint8_t)(r == d)});
-        if (!isbc[r]) rl.emplace_back(r, d, pos);
+        if (!isbc[r]) rl.emplace_back(r, q, bk * 9 + i * 3 + c);
       }
     }
   }
   std::sort(zl.begin(), zl.end());
   zl.erase(std::unique(zl.begin(), zl.end(), [](auto& a, auto& b) { return a.first == b.first; }), zl.end());
   std::sort(rl.begin(), rl.end());
-  std::vector<int> rows, rptr(1, 0), rcol;
+  std::vector<int> rows, rptr(1, 0), rbc;
   std::vector<long long> rpos, zpos;
   std::vector<uint8_t> zone;
   for (size_t i = 0; i < rl.size(); ++i) {
@@ -2117,7 +2118,7 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
       rows.push_back(r);
     }
     rpos.push_back(std::get<2>(rl[i]));
-    rcol.push_back(std::get<1>(rl[i]));
+    rbc.push_back(std::get<1>(rl[i]));
   }
   rptr.push_back((int)rpos.size());
   if (rows.empty()) rptr.assign(1, 0);
@@ -2128,7 +2129,7 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
   ctx->bcs_set = false;
   ctx->bc_dofs.clear();
   dfree(ctx, b.dofs); dfree(ctx, b.vals); dfree(ctx, b.ramp); dfree(ctx, b.fn); dfree(ctx, b.rows);
-  dfree(ctx, b.rptr); dfree(ctx, b.rpos); dfree(ctx, b.rcol); dfree(ctx, b.zpos); dfree(ctx, b.zone);
+  dfree(ctx, b.rptr); dfree(ctx, b.rpos); dfree(ctx, b.rbc); dfree(ctx, b.zpos); dfree(ctx, b.zone);
   b = BcDev();
   b.nbc = (int)dofs.size();
   b.nrows = (int)rows.size();
@@ -2140,7 +2141,7 @@ int pfem_set_bcs(pfem_ctx* ctx, const int64_t* dir_dofs, const double* dir_vals,
   CK(upload(ctx, &b.rows, rows));
   CK(upload(ctx, &b.rptr, rptr));
   CK(upload(ctx, &b.rpos, rpos));
-  CK(upload(ctx, &b.rcol, rcol));
+  CK(upload(ctx, &b.rbc, rbc));
   CK(upload(ctx, &b.zpos, zpos));
   CK(upload(ctx, &b.zone, zone));
   ctx->bc_dofs = dofs;

@@ -755,64 +755,101 @@ void add_to_double(long long n, const T* x, double* U, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ Dirichlet (K3)
-// R -= lambda * Fn  over all dofs, then dg = g(lambda) - U on constrained dofs.
-__global__ void residual_fext_kernel(long long n, double lam, const double* __restrict__ fn,
-                                     double* __restrict__ R) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    R[i] -= lam * fn[i];
-}
-__global__ void bc_dg_kernel(int nbc, const int* __restrict__ dofs, const double* __restrict__ vals,
-                             const uint8_t* __restrict__ ramp, double lam, const double* __restrict__ U,
-                             double* __restrict__ dg) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nbc) return;
-  const int d = dofs[i];
-  const double g = ramp[i] ? lam * vals[i] : vals[i];
-  dg[d] = g - U[d];
-}
-// Free rows touching constrained columns: R[row] += sum_k K[pos_k] * dg[col_k]
-// (impose_dirichlet!, BoundaryConditions.jl:248-256).  One thread per row.
+// With dg = g(lambda) - U on constrained dofs (impose_dirichlet!, BoundaryConditions.jl):
+//   free rows touching constrained columns: R[row] += sum_k K[row, col_k] dg[col_k] and
+//   these entries become 0 (248-256); eight lanes per row, CTAs [0, nb_rows);
+//   the other entries of constrained rows: 0, 1 on the diagonal (259-266);
+//   constrained dofs: R[d] = -dg[d] (269-272).
+// No entry of K or R belongs to two of the three, so they are one launch.  What bounds
+// it is the row's chain of loads: 14.6 us at 57 x 43 x 31 FP64 (34.7 with one entry per
+// lane at a time), where a thread per row took 16.3 us and four more launches the rest.  With
+// load_norm_kernel two launches in place of seven: a residual there 575 -> 552 us.
 template <typename KT>
-__global__ void bc_rhs_kernel(int nrows, const int* __restrict__ rows, const int* __restrict__ ptr,
-                              const long long* __restrict__ pos, const int* __restrict__ cols,
-                              const KT* __restrict__ K, const double* __restrict__ dg,
-                              double* __restrict__ R) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nrows) return;
+__global__ void __launch_bounds__(256) bc_impose_kernel(BcDev bc, int nb_rows, int nb_zero, double lam,
+                                                        const double* __restrict__ U, KT* __restrict__ K,
+                                                        double* __restrict__ R) {
+  auto dg = [&](int k) {
+    const double v = bc.vals[k];
+    return (bc.ramp[k] ? lam * v : v) - U[bc.dofs[k]];
+  };
+  int b = (int)blockIdx.x;
+  if (b < nb_rows) {
+    const int i = b * 32 + ((int)threadIdx.x >> 3), sub = threadIdx.x & 7;
+    const bool in = i < bc.nrows;
+    double s = 0.0;
+    const int e = in ? bc.rptr[i + 1] : 0;
+    // four entries per lane at a time, their loads in flight together
+    for (int k0 = in ? bc.rptr[i] + sub : 0; k0 < e; k0 += 32) {
+      long long pos[4];
+      int c[4];
+      double kv[4], g[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool have = k0 + 8 * u < e;
+        pos[u] = have ? bc.rpos[k0 + 8 * u] : -1;
+        c[u] = have ? bc.rbc[k0 + 8 * u] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        kv[u] = pos[u] >= 0 ? (double)K[pos[u]] : 0.0;
+        g[u] = dg(c[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (pos[u] < 0) continue;
+        s += kv[u] * g[u];
+        K[pos[u]] = KT(0);
+      }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (in && sub == 0) R[bc.rows[i]] += s;
+    return;
+  }
+  b -= nb_rows;
+  if (b < nb_zero) {
+    for (long long i = b * 256ll + threadIdx.x; i < bc.nzero; i += nb_zero * 256ll) K[bc.zpos[i]] = bc.zone[i] ? KT(1) : KT(0);
+    return;
+  }
+  const int k = (b - nb_zero) * 256 + (int)threadIdx.x;
+  if (k < bc.nbc) R[bc.dofs[k]] = -dg(k);
+}
+// R -= lambda Fn (Fn is 0 on constrained dofs), and out = |R|: the CTA that finishes last
+// adds the CTAs' shares in their order.
+__global__ void __launch_bounds__(RED_THREADS) load_norm_kernel(long long n, double lam, const double* __restrict__ fn,
+                                                                double* __restrict__ R, double* part,
+                                                                unsigned* ticket, double* out) {
+  __shared__ double sh[33];
+  __shared__ bool last;
   double s = 0.0;
-  for (int k = ptr[i]; k < ptr[i + 1]; ++k) s += (double)K[pos[k]] * dg[cols[k]];
-  R[rows[i]] += s;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double r = R[i] - lam * fn[i];
+    R[i] = r;
+    s += r * r;
+  }
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s = all_sum_partials(part, (int)gridDim.x, sh);
+  if (threadIdx.x == 0) *out = sqrt(s);
 }
-// Zero constrained rows / columns, unit diagonal (BoundaryConditions.jl:259-266).
 template <typename KT>
-__global__ void bc_zero_kernel(long long n, const long long* __restrict__ pos, const uint8_t* __restrict__ one,
-                               KT* __restrict__ K) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    K[pos[i]] = one[i] ? KT(1) : KT(0);
-}
-// R[d] = -dg[d] (BoundaryConditions.jl:269-272)
-__global__ void bc_set_kernel(int nbc, const int* __restrict__ dofs, const double* __restrict__ dg,
-                              double* __restrict__ R) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nbc) return;
-  R[dofs[i]] = -dg[dofs[i]];
-}
-template <typename KT>
-void impose_dirichlet(const BcDev& bc, long long ndof, double lam, const double* U, KT* K, double* R,
-                      double* dg, cudaStream_t st) {
-  const int b1 = (int)std::min<long long>((ndof + 255) / 256, 4096);
-  pfem::count_launch(); residual_fext_kernel<<<b1, 256, 0, st>>>(ndof, lam, bc.fn, R);
-  if (bc.nbc == 0) return;
-  pfem::count_launch(); bc_dg_kernel<<<(bc.nbc + 255) / 256, 256, 0, st>>>(bc.nbc, bc.dofs, bc.vals, bc.ramp, lam, U, dg);
-  if (bc.nrows > 0) {  // none when every dof is constrained
+void impose_dirichlet(const BcDev& bc, long long ndof, double lam, const double* U, KT* K, double* R, double* part,
+                      unsigned* ticket, double* rnorm, cudaStream_t st) {
+  if (bc.nbc > 0) {
+    const int nb_rows = (bc.nrows + 31) / 32;  // none when every dof is constrained
+    const int nb_zero = (int)std::min<long long>((bc.nzero + 255) / 256, 4096);
     pfem::count_launch();
-    bc_rhs_kernel<KT><<<(bc.nrows + 127) / 128, 128, 0, st>>>(bc.nrows, bc.rows, bc.rptr, bc.rpos, bc.rcol, K, dg, R);
+    bc_impose_kernel<KT><<<nb_rows + nb_zero + (bc.nbc + 255) / 256, 256, 0, st>>>(bc, nb_rows, nb_zero, lam, U, K, R);
   }
-  if (bc.nzero > 0) {
-    const int b2 = (int)std::min<long long>((bc.nzero + 255) / 256, 4096);
-    pfem::count_launch(); bc_zero_kernel<KT><<<b2, 256, 0, st>>>(bc.nzero, bc.zpos, bc.zone, K);
-  }
-  pfem::count_launch(); bc_set_kernel<<<(bc.nbc + 255) / 256, 256, 0, st>>>(bc.nbc, bc.dofs, dg, R);
+  pfem::count_launch();
+  load_norm_kernel<<<fused_update_blocks(ndof), RED_THREADS, 0, st>>>(ndof, lam, bc.fn, R, part, ticket, rnorm);
 }
 // Set U[d] = g(lambda) on constrained dofs (predictors honour the BCs).
 __global__ void bc_apply_kernel(int nbc, const int* __restrict__ dofs, const double* __restrict__ vals,
@@ -1381,7 +1418,7 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, Queue q)
                                const CgLoop&, Queue);                                              \
   template void add_to_double<T>(long long, const T*, double*, cudaStream_t);                      \
   template void impose_dirichlet<T>(const BcDev&, long long, double, const double*, T*, double*,   \
-                                    double*, cudaStream_t);                                        \
+                                      double*, unsigned*, double*, cudaStream_t);                  \
   template void dense_mv<T>(int, const T*, const T*, T*, Queue);                            \
   template void sa_setup_level<T>(const AmgLevel<T>&, T*, int, cudaStream_t);                   \
   template void sa_restrict<T>(const AmgLevel<T>&, const T*, T*, const AmgLevel<T>*, Queue);       \

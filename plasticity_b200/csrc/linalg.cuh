@@ -53,13 +53,13 @@ struct BcDev {
   int* dofs = nullptr;         // 0-based dof
   double* vals = nullptr;
   uint8_t* ramp = nullptr;
-  double* fn = nullptr;        // ndof nodal forces at lambda = 1
+  double* fn = nullptr;        // ndof nodal forces at lambda = 1, 0 on constrained dofs
   int nrows = 0;               // free rows with entries in constrained columns
   int* rows = nullptr;
   int* rptr = nullptr;         // nrows+1
   long long* rpos = nullptr;   // scalar value index into the block-CSR value array
-  int* rcol = nullptr;         // constrained column (dof)
-  long long nzero = 0;         // entries in constrained rows or columns
+  int* rbc = nullptr;          // constrained column (index into dofs)
+  long long nzero = 0;         // entries in constrained rows
   long long* zpos = nullptr;
   uint8_t* zone = nullptr;     // 1 on the diagonal of a constrained row
 };
@@ -122,7 +122,10 @@ template <typename T> void bicg_xr(long long n, T* sc, const T* ph, const T* sh,
                                    Queue q);
 template <typename A, typename B> void convert(long long n, const A* a, B* b, double s, cudaStream_t st);
 template <typename T> void add_to_double(long long n, const T* x, double* U, cudaStream_t st);
-template <typename KT> void impose_dirichlet(const BcDev& bc, long long ndof, double lam, const double* U, KT* K, double* R, double* dg, cudaStream_t st);
+// Impose the constraints on K and R at lambda, subtract the load, *rnorm = |R| (device).
+// part: 2048 doubles; ticket: zero between launches.
+template <typename KT> void impose_dirichlet(const BcDev& bc, long long ndof, double lam, const double* U, KT* K,
+                                             double* R, double* part, unsigned* ticket, double* rnorm, cudaStream_t st);
 void bc_apply(const BcDev& bc, double lam, double* U, cudaStream_t st);
 template <typename T> void dense_mv(int n, const T* M, const T* b, T* y, Queue q);
 template <typename T> void sa_setup_level(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t st);
