@@ -16,8 +16,7 @@ default), sets a displacement that drives most Gauss points plastic (uniform
      W below where a level lies between level 0 and the dense coarse solve)
      outside the graph, so a launch list shows its kernels one by one,
   7. the imposed residual (assembly + Dirichlet imposition kernels) `reps` times,
-  8. `reps` BiCGStab solves (host-driven loop: the Krylov vector and dot kernels
-     run as separate launches, visible to a profiler),
+  8. `reps` BiCGStab solves (a device graph like CG's),
   9. the predictor network's loss and gradient (the backward pass) `reps` times,
   10. four load increments (rows are recorded from the third on), then `reps`
      training steps (backward pass + Adam update) on the recorded rows.
