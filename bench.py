@@ -395,8 +395,8 @@ def main():
         nnzb = M.pattern()[1].size // 9
         by = spmv_bytes(nnzb, M.nn, 3, 4, M.tangent_index_bytes())
         achieved = by / (spmv_ms * 1e-3) / 1e9
-        traffic, traffic_src = ncu_traffic("bsr_spmv_kernel<float,3,0>", by)
-        return {"kernel": "bsr_spmv_kernel<float,3> (level-0 tangent SpMV, FP32 values)", "bound": "hbm",
+        traffic, traffic_src = ncu_traffic("bsr_spmv_pipe_kernel<float,3,0>", by)
+        return {"kernel": "bsr_spmv_pipe_kernel<float,3> (level-0 tangent SpMV, FP32 values)", "bound": "hbm",
                 "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": achieved / pk["hbm_gbs"],
                 "peak_source": ("measured (MEASURED_PEAKS.json hbm_gbs)" if pk_kind == "measured"
                                 else "fallback 6,650 GB/s (no MEASURED_PEAKS.json on this box)"),
