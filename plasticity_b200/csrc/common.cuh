@@ -71,6 +71,11 @@ __device__ __forceinline__ void inv3(const double* a, double* r) {
 // symmetric input, row-major, destroyed).  On exit w holds the eigenvalues
 // and V (row-major) the eigenvectors as columns.  At most `maxsweep` sweeps;
 // each sweep skips rotations whose off-diagonal entry is already zero.
+// t = sign(theta) / (|theta| + sqrt(theta^2 + 1)), theta = d / h.  QUOTIENT: as written;
+// else without the quotient, one division less per rotation.  The two differ in the last
+// bits of a double, but where two eigenvalues are equal the eigenvectors between them are
+// made of such bits, so what is rounded to single precision afterwards keeps one form.
+template <bool QUOTIENT>
 __device__ __forceinline__ void eig3_jacobi(double* a, double* w, double* V) {
 #pragma unroll
   for (int i = 0; i < 9; ++i) V[i] = (i % 4 == 0) ? 1.0 : 0.0;
@@ -85,11 +90,16 @@ __device__ __forceinline__ void eig3_jacobi(double* a, double* w, double* V) {
       const int o = 3 - p - q;
       const double apq = a[3 * p + q];
       if (apq != 0.0) {
-        // t = sign(theta) / (|theta| + sqrt(theta^2 + 1)), theta = d / h, without the
-        // quotient: two divisions and two square roots per rotation
         const double d = a[3 * q + q] - a[3 * p + p], h = 2.0 * apq;
-        const double den = fabs(d) + sqrt(d * d + h * h);
-        const double t = den > 0.0 ? copysign(1.0, d) * h / den : 1.0;  // 0: h^2 underflows beside d = 0
+        double t;
+        if constexpr (QUOTIENT) {
+          const double theta = d / h;
+          if (fabs(theta) > 1e150) t = 0.5 / theta;
+          else t = copysign(1.0, theta) / (fabs(theta) + sqrt(theta * theta + 1.0));
+        } else {
+          const double den = fabs(d) + sqrt(d * d + h * h);
+          t = den > 0.0 ? copysign(1.0, d) * h / den : 1.0;  // 0: h^2 underflows beside d = 0
+        }
         // not rsqrt: it makes the rotations less orthogonal (the residual's error against
         // 64 bits grows by an eighth) for 2.5 % of the element kernel
         const double c = 1.0 / sqrt(t * t + 1.0);

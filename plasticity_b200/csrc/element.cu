@@ -13,15 +13,20 @@
 // component k in turn: lane (slot, b) sums the eight Gauss-point contributions to the
 // column (b, k) of its element's tangent
 //   Ke[:,(b,k)] = sum_g G_g^T (w s A G_g + (w s/3) A vec(F) (g0 - gJ)^T)[:,(b,k)]
-// (lagrangian/src/Elements.jl:470-478 with _fbar_Geff :524-531).  Going by k, only a
-// third of A is in shared memory at a time and no lane is idle.
+// (lagrangian/src/Elements.jl:470-478 with _fbar_Geff :524-531), and no lane is idle.
+// FP64: only the third of A that a k needs is in shared memory at a time.  FP32: all of
+// it, because the order of the single-precision sums is fixed: every column of A adds to
+// A vec(F) in the order of the columns, and a point's three products are added to each
+// other before they are added to the entry.  The solution of a linear system can depend
+// on one rounding of the tangent by hundreds of roundings (a slender box clamped at one
+// end), so another order is another result.
 //
-// What bounds it: instruction issue at the 8 (FP64) or 12 (FP32) warps per SM that its
-// registers allow, with the dependent FP64 arithmetic of phase A in between.  At 64^3,
-// FP32 tangent / FP64: 0.82 / 1.16 ms.  With the whole of A in shared memory (6 warps
-// per SM in FP64), the 96 columns of a warp taken 32 at a time, single-word reads and
-// single multiply-adds: 1.02 / 1.57 ms, 2,480 instructions per element (now 1,640).
-// Three columns per lane at once (FP32): 0.88 ms, its accumulators cost warps.
+// What bounds it: the latency of dependent arithmetic, FP64 in phase A, at the 8 (FP64) or
+// 12 (FP32) warps per SM that its registers and shared memory allow.  One residual call
+// at 64^3 with FP32 tangent 1.28 ms, at 57 x 43 x 31 FP64 0.55 ms; with the 96 columns of
+// a warp taken 32 at a time, single-word reads and single multiply-adds 1.37 and 0.66 ms.
+// FP32 with the record spread over 19 KB per warp, which leaves L1 less, 1.38 ms; by k as
+// in FP64 with the products added one by one 1.19 ms, but other results.
 //
 // Arithmetic follows the reference kernel element_force_tangent_finite!
 // (Elements.jl:405-494), finite_kinematics (FiniteStrain.jl:148-170),
@@ -42,14 +47,19 @@
 namespace pfem {
 
 constexpr int EPW = 4;                     // elements per warp
-// A Gauss point's tangent record (TT each): dN/dX by component, [j][a]; the columns
-// (q, k) of w s A for the k at hand, [q][r] with the rows r = 3 j + i at a stride of 10;
-// w s/3 A vec(F), [r]; F^-1 transposed, [k][j] at a stride of 4.  All parts start on 16
-// bytes; 84 = 20 mod 32 words and 82 = 2 mod 16 double words spread an element's eight
-// points over the banks.
-constexpr int REC_A = 24, REC_AQ = 10, REC_U = REC_A + 32, REC_FI = REC_U + 12;
+// A Gauss point's tangent record (TT each).  dN/dX by component, [j][a].  The columns
+// (q, k) of w s A, [q][r] with the rows r = 3 j + i at a stride of 10: of all k in FP32
+// (at a stride of 32), of the k at hand in FP64.  w s/3 A vec(F), [r], and F^-1 are in
+// FP64 parts of their own, F^-1 transposed, [k][j] at a stride of 4; in FP32 they fill the
+// gaps: F^-1_qk is row 9 of column (q, k), the first three pairs of the F-bar vector end
+// the three k, its last three entries the record.  All parts start on 16 bytes; 124 = 28
+// mod 32 words and 82 = 2 mod 16 double words spread an element's points over the banks.
+constexpr int REC_A = 24, REC_AQ = 10, REC_AK = 32, REC_UK = 30;
 template <typename TT>
-constexpr int gprec() { return sizeof(TT) == 4 ? REC_FI + 16 : REC_FI + 14; }
+constexpr int rec_u() { return REC_A + (sizeof(TT) == 4 ? 3 : 1) * REC_AK; }
+constexpr int REC_FI = rec_u<double>() + 12;
+template <typename TT>
+constexpr int gprec() { return sizeof(TT) == 4 ? rec_u<TT>() + 4 : REC_FI + 14; }
 template <typename TT>
 constexpr int slot_tt() { return 24 + 8 * gprec<TT>(); }  // g0, then the 8 Gauss-point records
 constexpr int WPB = 1;                     // warps per block
@@ -75,7 +85,8 @@ __device__ __forceinline__ void dshape_a(int a, double x, double y, double z, do
 }
 
 // Two floats in one register pair: fma.rn.f32x2 does two of the tangent's
-// multiply-adds per issue slot, each rounded as the single one.
+// multiply-adds per issue slot, each rounded as the single one.  In a sum of three
+// products the middle one is rounded, then the first and the last are added.
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 dup2(float a) {
   f32x2 r;
@@ -86,6 +97,11 @@ __device__ __forceinline__ void split2(f32x2 v, float& a, float& b) { asm("mov.b
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) {
@@ -185,7 +201,8 @@ template <typename KT, bool COMMIT, bool FBAR, int HARD>
 __global__ void __launch_bounds__(32 * WPB, (std::is_same<KT, float>::value && !COMMIT && HARD != HARD_KIN) ? 11 : 1)
 element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
   using TT = KT;  // type of the tangent records and of the phase-B arithmetic
-  constexpr int GPREC = gprec<TT>(), SLOT_TT = slot_tt<TT>();
+  constexpr int GPREC = gprec<TT>(), SLOT_TT = slot_tt<TT>(), REC_U = rec_u<TT>();
+  constexpr bool kQuot = COMMIT || std::is_same<TT, float>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = lane >> 3, g = lane & 7;
@@ -336,7 +353,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
     for (int i = 0; i < 9; ++i) Q[i] = (i % 4 == 0) ? 1.0 : 0.0;
     bv[0] = bv[1] = bv[2] = 1.0;
   } else {
-    eig3_jacobi(be, bv, Q);
+    eig3_jacobi<kQuot>(be, bv, Q);
   }
   // ---- return_map on principal values (Materials.jl:159-250) ----
   const double G = m.G, lam = m.lam, H = m.Hiso;
@@ -363,7 +380,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
 #pragma unroll
       for (int j = 0; j < 3; ++j) Cm[3 * i + j] = Fb[i] * Fb[j] + Fb[3 + i] * Fb[3 + j] + Fb[6 + i] * Fb[6 + j];
     double lc[3];
-    eig3_jacobi(Cm, lc, Vu);
+    eig3_jacobi<kQuot>(Cm, lc, Vu);
     double imu[3];
 #pragma unroll
     for (int A = 0; A < 3; ++A) {
@@ -474,7 +491,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
                           -2.0 * c * nh6[3], -2.0 * c * nh6[4], -2.0 * c * nh6[5]};
     double E2[9], w2[3], V2[9];
     unpack_sym(ee, E2);
-    eig3_jacobi(E2, w2, V2);
+    eig3_jacobi<kQuot>(E2, w2, V2);
     double FQ[9], T[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -650,34 +667,8 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       }
     }
     const TT ws_ = (TT)(w * scale);
-    {
-      // w s/3 A vec(F), the F-bar vector, in closed form: along F the elastic strain
-      // changes by I / s, which no flow direction sees (it is deviatoric) and no polar
-      // rotation follows, so dP = (3 K Fbar^-T - P) / s.
-      const double uf = w * (1.0 / 3.0), k3 = 3.0 * lam + 2.0 * G;
-      TT u[REC_AQ], fi[12];
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) u[3 * j + i] = FBAR ? (TT)(uf * (k3 * Fbi[3 * j + i] - P[3 * i + j])) : TT(0);
-      u[9] = TT(0);
-      store_pairs<REC_AQ>(Rg + REC_U, u);
-      // F^-1 of the standard F = scale * Fb^-1 (for gJ = G^T vec(F^-T))
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) fi[4 * k + j] = (TT)(scale * Fbi[3 * j + k]);
-        fi[4 * k + 3] = TT(0);
-      }
-      store_pairs<12>(Rg + REC_FI, fi);
-    }
-    // ---- per k: the three columns (q, k) of A by every Gauss point, then (phase B) the
-    // columns (b, k) of the four element tangents by lane (slot, b) ----
-    const int b = g;
-#pragma unroll
-    for (int pp = 0; pp < 3; ++pp) {
-#pragma unroll
-    for (int qq = 0; qq < 3; ++qq) {
+    // Column (q, p) of A: dP / dFbar_pq, [3 j + i].
+    auto column = [&](const int pp, const int qq, TT* dP) {
       TT Y[9];
 #pragma unroll
       for (int A = 0; A < 3; ++A)
@@ -739,18 +730,23 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       for (int A = 0; A < 3; ++A)
 #pragma unroll
         for (int j = 0; j < 3; ++j) T[3 * A + j] = dt[3 * A] * NN[j] + dt[3 * A + 1] * NN[3 + j] + dt[3 * A + 2] * NN[6 + j];
-      TT wdP[REC_AQ];
-      wdP[9] = TT(0);
 #pragma unroll
       for (int j = 0; j < 3; ++j)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const TT dP = Qt[3 * i] * T[j] + Qt[3 * i + 1] * T[3 + j] + Qt[3 * i + 2] * T[6 + j] - Pt[3 * i + qq] * FbiT[3 * pp + j];
-          wdP[j * 3 + i] = ws_ * dP;
-        }
-      store_pairs<REC_AQ>(Rg + REC_A + qq * REC_AQ, wdP);
-    }
-    __syncwarp();
+        for (int i = 0; i < 3; ++i)
+          dP[j * 3 + i] = Qt[3 * i] * T[j] + Qt[3 * i + 1] * T[3 + j] + Qt[3 * i + 2] * T[6 + j] - Pt[3 * i + qq] * FbiT[3 * pp + j];
+    };
+    auto keep = [&](const int at, const int qq, const TT* dP, const TT row9) {
+      TT wdP[REC_AQ];
+#pragma unroll
+      for (int r = 0; r < 9; ++r) wdP[r] = ws_ * dP[r];
+      wdP[9] = row9;
+      store_pairs<REC_AQ>(Rg + REC_A + at * REC_AK + qq * REC_AQ, wdP);
+    };
+    // Phase B for component k = pp: the columns (b, k) of the four element tangents by lane
+    // (slot, b).
+    const int b = g;
+    auto tangent = [&](const int pp) {
     TT acc[24];  // rows (a, i) of the column
     const TT g0bk = FBAR ? g0s[3 * b + pp] : TT(0);
     if constexpr (std::is_same<TT, float>::value) {
@@ -763,45 +759,53 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       for (int gg = 0; gg < 8; ++gg) {
         const float* Rr = S + 24 + gg * GPREC;
         const float db0 = Rr[b], db1 = Rr[8 + b], db2 = Rr[16 + b];
-        f32x2 A[16];  // [q][pair of r] at a stride of 5
+        f32x2 A[16];  // [q][pair of r] at a stride of 5; the last pair is not A's
 #pragma unroll
         for (int h = 0; h < 8; ++h) {
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + REC_A + 4 * h);
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + REC_A + pp * REC_AK + 4 * h);
           A[2 * h] = v.x;
           A[2 * h + 1] = v.y;
         }
         f32x2 T2[5];
 #pragma unroll
         for (int m = 0; m < 5; ++m) {
-          T2[m] = mul2(A[m], dup2(db0));
-          fma2(T2[m], A[5 + m], dup2(db1));
+          T2[m] = mul2(A[5 + m], dup2(db1));
+          fma2(T2[m], A[m], dup2(db0));
           fma2(T2[m], A[10 + m], dup2(db2));
         }
         if constexpr (FBAR) {
-          // dg_(b,k) = g0_(b,k) - gJ_(b,k),  gJ_(b,k) = sum_j F^-1[j][k] dNdX[b][j]
-          const float4 fi = *reinterpret_cast<const float4*>(Rr + REC_FI + 4 * pp);
-          const float dg = g0bk - (fi.x * db0 + fi.y * db1 + fi.z * db2);
+          // dg_(b,k) = g0_(b,k) - gJ_(b,k),  gJ_(b,k) = sum_j F^-1[j][k] dNdX[b][j]: row 9
+          float t8, gj;
+          split2(T2[4], t8, gj);
+          const f32x2 dg = dup2(g0bk - gj);
 #pragma unroll
-          for (int h = 0; h < 3; ++h) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + REC_U + 4 * h);
-            fma2(T2[2 * h], v.x, dup2(dg));
-            if (h < 2) fma2(T2[2 * h + 1], v.y, dup2(dg));
-          }
+          for (int h = 0; h < 3; ++h)
+            fma2(T2[h], *reinterpret_cast<const f32x2*>(Rr + REC_A + h * REC_AK + REC_UK), dg);
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + REC_U);
+          fma2(T2[3], v.x, dg);
+          fma2(T2[4], v.y, dg);
         }
         float T[10];
 #pragma unroll
         for (int m = 0; m < 5; ++m) split2(T2[m], T[2 * m], T[2 * m + 1]);
+        f32x2 x[3][4];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const ulonglong2 x0 = *reinterpret_cast<const ulonglong2*>(Rr + 8 * j);
-          const ulonglong2 x1 = *reinterpret_cast<const ulonglong2*>(Rr + 8 * j + 4);
+        for (int j = 0; j < 3; ++j)
 #pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            const f32x2 t = dup2(T[3 * j + i]);
-            fma2(acc2[i][0], x0.x, t);
-            fma2(acc2[i][1], x0.y, t);
-            fma2(acc2[i][2], x1.x, t);
-            fma2(acc2[i][3], x1.y, t);
+          for (int h = 0; h < 2; ++h) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Rr + 8 * j + 4 * h);
+            x[j][2 * h] = v.x;
+            x[j][2 * h + 1] = v.y;
+          }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const f32x2 t0 = dup2(T[i]), t1 = dup2(T[3 + i]), t2 = dup2(T[6 + i]);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            f32x2 v = mul2(x[1][m], t1);
+            fma2(v, x[0][m], t0);
+            fma2(v, x[2][m], t2);
+            acc2[i][m] = add2(acc2[i][m], v);
           }
         }
       }
@@ -864,7 +868,66 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
         }
       }
     }
-    __syncwarp();  // the next k's columns overwrite these
+    };
+    if constexpr (std::is_same<TT, float>::value) {
+      TT u[REC_AQ];
+#pragma unroll
+      for (int r = 0; r < REC_AQ; ++r) u[r] = TT(0);
+#pragma unroll
+      for (int qq = 0; qq < 3; ++qq)
+#pragma unroll
+        for (int pp = 0; pp < 3; ++pp) {
+          TT dP[9];
+          column(pp, qq, dP);
+          keep(pp, qq, dP, (TT)(scale * Fbi[3 * qq + pp]));
+          if constexpr (FBAR) {
+            const TT Fq = (TT)F[3 * pp + qq];  // standard F for the F-bar vec(F)
+#pragma unroll
+            for (int r = 0; r < 9; ++r) u[r] += dP[r] * Fq;
+          }
+        }
+      const TT uf = (TT)(w * scale / 3.0);
+#pragma unroll
+      for (int r = 0; r < 9; ++r) u[r] = uf * u[r];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) store_pairs<2>(Rg + REC_A + h * REC_AK + REC_UK, u + 2 * h);
+      store_pairs<4>(Rg + REC_U, u + 6);
+      __syncwarp();
+#pragma unroll 1
+      for (int pp = 0; pp < 3; ++pp) tangent(pp);
+    } else {
+      // w s/3 A vec(F), the F-bar vector, in closed form: along F the elastic strain
+      // changes by I / s, which no flow direction sees (it is deviatoric) and no polar
+      // rotation follows, so dP = (3 K Fbar^-T - P) / s.
+      const double uf = w * (1.0 / 3.0), k3 = 3.0 * lam + 2.0 * G;
+      TT u[REC_AQ];
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) u[3 * j + i] = FBAR ? (TT)(uf * (k3 * Fbi[3 * j + i] - P[3 * i + j])) : TT(0);
+      u[9] = TT(0);
+      store_pairs<REC_AQ>(Rg + REC_U, u);
+      // F^-1 of the standard F = scale * Fb^-1 (for gJ = G^T vec(F^-T))
+      TT fi[12];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) fi[4 * k + j] = (TT)(scale * Fbi[3 * j + k]);
+        fi[4 * k + 3] = TT(0);
+      }
+      store_pairs<12>(Rg + REC_FI, fi);
+#pragma unroll
+      for (int pp = 0; pp < 3; ++pp) {
+#pragma unroll
+        for (int qq = 0; qq < 3; ++qq) {
+          TT dP[9];
+          column(pp, qq, dP);
+          keep(0, qq, dP, TT(0));
+        }
+        __syncwarp();
+        tangent(pp);
+        __syncwarp();  // the next k's columns overwrite these
+      }
     }
   }  // !COMMIT
 }
