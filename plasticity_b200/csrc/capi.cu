@@ -675,13 +675,13 @@ float* K_of<float>(pfem_ctx* c) { return c->dK32; }
 template <>
 double* K_of<double>(pfem_ctx* c) { return c->dK64; }
 
-__global__ void hash_fill_kernel(long long n, float* xf, double* xd) {
+template <typename T>
+__global__ void hash_fill_kernel(long long n, T* x, T* one) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *one = T(1);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     unsigned long long h = (unsigned long long)i * 0x9E3779B97F4A7C15ull;
     h ^= h >> 29; h *= 0xBF58476D1CE4E5B9ull; h ^= h >> 32;
-    const double v = 0.5 + (double)(h & 0xFFFFFF) / (double)0x1000000;
-    if (xf) xf[i] = (float)v;
-    if (xd) xd[i] = v;
+    x[i] = (T)(0.5 + (double)(h & 0xFFFFFF) / (double)0x1000000);
   }
 }
 // Allocate the device side of the hierarchy for precision T (once).
@@ -804,24 +804,17 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
     AmgLevel<T>& v = A.lv[l];
     blockdiag_invert<T>(v.A, v.dinv, ctx->st);
     CKL();
-    // Power iteration on D^-1 A, 12 steps, each one pass over the matrix; the iterate is
-    // rescaled every second step only (a spectral radius of 1e18 still fits single
-    // precision), and the estimate is the ratio of the last two norms.
+    // Power iteration on D^-1 A: 12 steps, each one pass over the matrix on the iterate
+    // scaled to length 1 and the norm of the result, the estimate at the end.
     const long long n = (long long)v.A.nbrow * v.A.bs;
-    pfem::count_launch(); hash_fill_kernel<<<256, 256, 0, ctx->st>>>(n, std::is_same<T, float>::value ? (float*)v.d : nullptr,
-                                               std::is_same<T, double>::value ? (double*)v.d : nullptr);
+    KrylovWork<T>& w = kw_of<T>(ctx);
+    pfem::count_launch(); hash_fill_kernel<T><<<256, 256, 0, ctx->st>>>(n, v.d, v.co + CO_INV);
     for (int it = 1; it <= 12; ++it) {
       const T* from = it % 2 ? v.d : v.r;
       T* to = it % 2 ? v.r : v.d;
-      bsr_power_step<T>(v.A, v.dinv, from, to, ctx->st);
-      if (it % 2 == 0 && it < 12) {
-        const int np = norm2_partials<T>(n, to, ctx->dPart, ctx->st);
-        scale_by_norm<T>(n, ctx->dPart, np, to, ctx->st);
-      }
+      bsr_power_step<T>(v.A, v.dinv, from, to, v.co, ctx->st);
+      power_norm<T>(n, to, w.part, w.ticket, it == 12, v.co, ctx->st);
     }
-    const int np = norm2_partials<T>(n, v.r, ctx->dPart, ctx->st);
-    norm2_partials<T>(n, v.d, ctx->dPart + 1024, ctx->st);
-    power_finish<T>(np, ctx->dPart, ctx->dPart + 1024, v.co, ctx->st);
     CKL();
     // smoothed prolongator and Galerkin operator of the next level
     T* cval = (l + 1 < L) ? A.lv[l + 1].A.val : A.coarse_val;

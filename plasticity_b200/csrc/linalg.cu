@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(128) bsr_spmv_kernel(int nbrow, const int* __r
 #pragma unroll
   for (int j = 0; j < BS; ++j) D[j] = (MODE >= 2 && own) ? a.dinv[(long long)row * (BS * BS) + lane * BS + j] : T(0);
   const T c1 = MODE == 3 || MODE == 4 ? a.co[CO_C1] : MODE == 5 || MODE == 7 ? a.co[CO_ITH] : T(0);
-  const T c2 = MODE == 3 || MODE == 4 ? a.co[CO_C2] : T(0);
+  const T c2 = MODE == 3 || MODE == 4 ? a.co[CO_C2] : MODE == 6 ? a.co[CO_INV] : T(0);
   pdl_wait();
   T bi = T(0), yi = T(0), xi = T(0), oi = T(0);
   if (own) {
@@ -115,7 +115,10 @@ __global__ void __launch_bounds__(128) bsr_spmv_kernel(int nbrow, const int* __r
   while (k < e) {
     T xv[BS];
 #pragma unroll
-    for (int j = 0; j < BS; ++j) xv[j] = a.x[(long long)c * BS + j];
+    for (int j = 0; j < BS; ++j) {
+      xv[j] = a.x[(long long)c * BS + j];
+      if (MODE == 6) xv[j] *= c2;
+    }
 #pragma unroll
     for (int i = 0; i < BS; ++i)
 #pragma unroll
@@ -285,9 +288,9 @@ void bsr_residual_start(const BsrMat<T>& A, const T* dinv, const T* x, const T* 
   spmv_launch<T, 7>(A, a, q);
 }
 template <typename T>
-void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, cudaStream_t st) {
+void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, const T* co, cudaStream_t st) {
   SpmvVec<T> a;
-  a.x = x; a.y = y; a.dinv = dinv;
+  a.x = x; a.y = y; a.dinv = dinv; a.co = co;
   spmv_launch<T, 6>(A, a, st);
 }
 
@@ -522,51 +525,52 @@ void cg_xr_fused(int nbrow, const double* part_pq, int np, T* sc, const T* p, co
          co, sr, sd, loop);
 }
 
-// ---- power iteration: squared norms in double (an iterate may be as large as its type
-// allows), kNormBlocks partials at most ----
-constexpr int kNormBlocks = 1024;
-static int norm_blocks(long long n) {
-  return (int)std::min<long long>(std::max<long long>((n + RED_THREADS - 1) / RED_THREADS, 1), kNormBlocks);
-}
+// The sum of np partials (at most 2048) in the order in which sum_final_kernel adds them,
+// by a CTA of 256 threads, each for four of that one's: to every thread.
 template <typename T>
-__global__ void norm2_partials_kernel(long long n, const T* __restrict__ v, double* __restrict__ part) {
-  __shared__ double sh[32];
-  double s = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    s += (double)v[i] * (double)v[i];
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-template <typename T>
-int norm2_partials(long long n, const T* v, double* part, cudaStream_t st) {
-  const int blocks = norm_blocks(n);
-  pfem::count_launch();
-  norm2_partials_kernel<T><<<blocks, RED_THREADS, 0, st>>>(n, v, part);
-  return blocks;
-}
-// v /= sqrt(sum(part))
-template <typename T>
-__global__ void scale_by_norm_kernel(long long n, const double* __restrict__ part, int np, T* __restrict__ v) {
-  __shared__ double sh[33];
-  const double inv = 1.0 / sqrt(all_sum_partials(part, np, sh));
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    v[i] = (T)((double)v[i] * inv);
-}
-template <typename T>
-void scale_by_norm(long long n, const double* part, int np, T* v, cudaStream_t st) {
-  pfem::count_launch();
-  scale_by_norm_kernel<T><<<norm_blocks(n), RED_THREADS, 0, st>>>(n, part, np, v);
-}
-// A level's scalars from the last two iterates' squared norms (np partials each).
-template <typename T>
-__global__ void power_finish_kernel(int np, const double* __restrict__ prev, const double* __restrict__ last,
-                                    T* __restrict__ co) {
-  __shared__ double sh[33];
-  const double a = all_sum_partials(prev, np, sh);
+__device__ __forceinline__ T sum_as_final(const T* part, int np, T* sh) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    T v = T(0);
+    for (int i = threadIdx.x + q * RED_THREADS; i < np; i += 1024) v += part[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (l == 0) sh[w + 8 * q] = v;
+  }
   __syncthreads();
-  const double b = all_sum_partials(last, np, sh);
+  T v = sh[l];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();  // sh may be written again
+  return v;
+}
+// ---- power iteration.  The norm of an iterate in the matrix's type, in dot's order; its
+// reciprocal goes to co[CO_INV], where the next step's product reads it: the scaled
+// iterate is never stored, and a step is two launches.  FP32 coarse levels see the last
+// bit of the estimate through the prolongator, so the order is kept. ----
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS) power_norm_kernel(long long n, const T* __restrict__ v, T* part,
+                                                                 unsigned* ticket, bool finish, T* co) {
+  __shared__ T sh[32];
+  __shared__ bool last;
+  T s = T(0);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    s += v[i] * v[i];
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const T norm = sqrt(sum_as_final(part, (int)gridDim.x, sh));
   if (threadIdx.x != 0) return;
-  const double lm = sqrt(b / a);
+  co[CO_INV] = T(1) / norm;
+  if (!finish) return;
+  const double lm = (double)norm;
   const T lmax = (T)(1.1 * lm);
   const double lmx = (double)lmax, lmn = lmx / 30.0;
   const double th = 0.5 * (lmx + lmn), de = 0.5 * (lmx - lmn);
@@ -579,9 +583,9 @@ __global__ void power_finish_kernel(int np, const double* __restrict__ prev, con
   co[CO_OMEGA] = T(4.0 / (3.0 * lm));
 }
 template <typename T>
-void power_finish(int np, const double* prev, const double* last, T* co, cudaStream_t st) {
+void power_norm(long long n, const T* v, T* part, unsigned* ticket, bool finish, T* co, cudaStream_t st) {
   pfem::count_launch();
-  power_finish_kernel<T><<<1, 1024, 0, st>>>(np, prev, last, co);
+  power_norm_kernel<T><<<fused_update_blocks(n), RED_THREADS, 0, st>>>(n, v, part, ticket, finish, co);
 }
 // ---- BiCGStab updates.  Scalars: sc[0] rho = rh.r, sc[1] rho of the iteration before,
 // sc[2] alpha, sc[3] omega.  A thread per node, as cg_xr_fused; the dot products come as
@@ -1397,10 +1401,8 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, Queue q)
                             double*);                                                              \
   template void bsr_residual_precond<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, const T*, Queue); \
   template void bsr_residual_start<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, T*, const T*, Queue); \
-  template void bsr_power_step<T>(const BsrMat<T>&, const T*, const T*, T*, cudaStream_t);         \
-  template int norm2_partials<T>(long long, const T*, double*, cudaStream_t);                      \
-  template void scale_by_norm<T>(long long, const double*, int, T*, cudaStream_t);                 \
-  template void power_finish<T>(int, const double*, const double*, T*, cudaStream_t);              \
+  template void bsr_power_step<T>(const BsrMat<T>&, const T*, const T*, T*, const T*, cudaStream_t); \
+  template void power_norm<T>(long long, const T*, T*, unsigned*, bool, T*, cudaStream_t);         \
   template void blockdiag_apply<T>(int, int, const T*, const T*, T*, const T*, T*, Queue);         \
   template void blockdiag_invert<T>(const BsrMat<T>&, T*, cudaStream_t);                           \
   template void dot<T>(long long, const T*, const T*, T*, T*, cudaStream_t, bool);                 \

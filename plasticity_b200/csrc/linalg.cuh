@@ -79,12 +79,12 @@ template <typename T> void bsr_residual_precond(const BsrMat<T>& A, const T* din
 // res = b - A x, r = Dinv res, d = co[CO_ITH] r: a residual and the smoother's start on it.
 template <typename T> void bsr_residual_start(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* res, T* r,
                                               T* d, const T* co, Queue q);
-// Power iteration: y = Dinv A x; the partials of |v|^2 (at most 1024, count returned);
-// v /= sqrt(sum(part)); a level's scalars from the last two iterates' squared norms.
-template <typename T> void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, cudaStream_t st);
-template <typename T> int norm2_partials(long long n, const T* v, double* part, cudaStream_t st);
-template <typename T> void scale_by_norm(long long n, const double* part, int np, T* v, cudaStream_t st);
-template <typename T> void power_finish(int np, const double* prev, const double* last, T* co, cudaStream_t st);
+// Power iteration: y = Dinv A (co[CO_INV] x); co[CO_INV] = 1 / |v|, with finish also the
+// level's other scalars from |v|.  part: 2048; ticket: zero between launches.
+template <typename T> void bsr_power_step(const BsrMat<T>& A, const T* dinv, const T* x, T* y, const T* co,
+                                          cudaStream_t st);
+template <typename T> void power_norm(long long n, const T* v, T* part, unsigned* ticket, bool finish, T* co,
+                                      cudaStream_t st);
 // r = Dinv v, d = *scale r (scale on the device).
 template <typename T> void blockdiag_apply(int nbrow, int bs, const T* dinv, const T* v, T* r, const T* scale, T* d, Queue q);
 template <typename T> void blockdiag_invert(const BsrMat<T>& A, T* dinv, cudaStream_t st);

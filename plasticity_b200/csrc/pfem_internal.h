@@ -83,8 +83,9 @@ struct BsrMat {
 
 // Scalars of a level's set-up: the spectral radius estimate of D^-1 A (x 1.1); of the
 // degree-2 Chebyshev smoother on [lmax/30, lmax]: 1 / th (th the interval's centre, the
-// first step of any degree), c1, c2; the prolongator's 4 / (3 rho).
-enum : int { CO_LMAX = 0, CO_ITH = 1, CO_C1 = 2, CO_C2 = 3, CO_OMEGA = 4, CO_COUNT = 8 };
+// first step of any degree), c1, c2; the prolongator's 4 / (3 rho); the power iteration's
+// 1 / |iterate|.
+enum : int { CO_LMAX = 0, CO_ITH = 1, CO_C1 = 2, CO_C2 = 3, CO_OMEGA = 4, CO_INV = 5, CO_COUNT = 8 };
 
 constexpr int kProlongTile = 32;
 

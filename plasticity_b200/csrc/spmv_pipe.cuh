@@ -27,11 +27,11 @@ namespace pfem {
 
 // What an SpMV works on, and what it does with a row's sum v = (A x), by mode:
 //   0: y = v   1: y = b - v   2: y -= Dinv v, xo += x   3: xo = c2 x + c1 (y - Dinv v)
-//   4: as 3, added to xo      5: y = Dinv (b - v), xo = y / th      6: y = Dinv v
+//   4: as 3, added to xo      5: y = Dinv (b - v), xo = y / th      6: y = Dinv v, x scaled
 //   7: z = b - v, y = Dinv z, xo = y / th
 // 2 is a Chebyshev step on x = d; 3 and 4 the degree-2 smoother in one pass (x = d0,
 // y = r0); 5 its start on a residual, 7 the same with the residual kept; 6 a step of
-// the power iteration.  1 / th, c1 and c2 are the level's scalars co.  Vectors that
+// the power iteration, on x / |x|.  1 / th, c1 and c2 are the level's scalars co.  Vectors that
 // earlier kernels of a programmatic launch chain write are not __restrict__ const: such
 // a load could be served by the read-only path while they are still being written.
 template <typename T>
@@ -125,7 +125,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
   __syncwarp();
   uint32_t phase = 0;
   const T c1 = MODE == 3 || MODE == 4 ? a.co[CO_C1] : MODE == 5 || MODE == 7 ? a.co[CO_ITH] : T(0);
-  const T c2 = MODE == 3 || MODE == 4 ? a.co[CO_C2] : T(0);
+  const T c2 = MODE == 3 || MODE == 4 ? a.co[CO_C2] : MODE == 6 ? a.co[CO_INV] : T(0);
   double dot = 0.0;
   pdl_wait();  // the first tile is on its way
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
@@ -174,7 +174,10 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           const bool in = q < len;
           const long long c = in ? (C16 ? row + (int)cs16[q] : cs[q]) : 0;
 #pragma unroll
-          for (int j = 0; j < 3; ++j) xv[m][j] = in ? a.x[c * 3 + j] : T(0);
+          for (int j = 0; j < 3; ++j) {
+            xv[m][j] = in ? a.x[c * 3 + j] : T(0);
+            if (MODE == 6) xv[m][j] *= c2;
+          }
         }
 #pragma unroll
         for (int m = 0; m < NP; ++m) {
@@ -277,7 +280,10 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           const bool in = q < b1;
           const long long c = in ? cs[q] : 0;
 #pragma unroll
-          for (int j = 0; j < BS; ++j) xv[h][j] = in ? a.x[c * BS + j] : T(0);
+          for (int j = 0; j < BS; ++j) {
+            xv[h][j] = in ? a.x[c * BS + j] : T(0);
+            if (MODE == 6) xv[h][j] *= c2;
+          }
         }
         T acc[BS];
 #pragma unroll

@@ -62,7 +62,7 @@ def tangent(element, hard, field):
 
 def hierarchy():
     """The prolongator of the tangent and its Galerkin operator."""
-    M, U = model((6, 5, 4), "small", "linear", 0)
+    M, U = model((8, 5, 3), "small", "linear", 0)
     M.set_displacement(U)
     _, R = M.residual(1.0, precision="mixed")
     M.linear_solve(-R, rtol=0.5, precision="mixed")

@@ -27,3 +27,7 @@ def test_tangent(kept, i):
     K = G.tangent(*G.TANGENTS[i])
     assert np.mean(K != kept["tangent_%d" % i]) <= RARE
 
+
+def test_hierarchy(kept):
+    P, _ = G.hierarchy()
+    assert np.mean((P != kept["prolongator"])[P != 0]) <= RARE
