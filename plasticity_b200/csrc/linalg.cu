@@ -1066,6 +1066,75 @@ __global__ void __launch_bounds__(128) sa_rap_kernel(int nnzC, const int* __rest
       if ((r * 6 + q) % LN == lane) O[r * 6 + q] = acc[r][q];
 }
 
+// The same for FP32 in the order of the P^T row, as one thread per block would add it: the
+// coarse operator's small eigenvalues are what is left of terms hundreds of times larger,
+// so in FP32 another order is another operator, and the solution of a slender box moves
+// with it.  What the LN lanes of a block find is taken in turn, lane r with the six entries
+// of row r.  Set-up with this / with the kernel above, FP32: 0.40 / 0.40 ms at 8^3, 1.01 /
+// 1.03 at 80 x 16 x 16, 1.57 / 1.54 at 40^3, 3.90 / 3.68 at 64^3; one at a time 0.45, 1.13,
+// 1.58 and 3.89; 16 lanes 0.39, 1.04, 1.63 and 4.31.  (FP64 2.23 / 2.07 ms at 40^3.)
+template <typename T, int BS, int LN>
+__global__ void __launch_bounds__(128) sa_rap_ordered_kernel(int nnzC, const int* __restrict__ c_row, const int* __restrict__ c_cl,
+                              const int* __restrict__ pt_rp, const int* __restrict__ pt_row,
+                              const T* __restrict__ ptval,
+                              const int* __restrict__ ap_rp, const int* __restrict__ ap_cl,
+                              const T* __restrict__ apval, T* __restrict__ cval) {
+  static_assert(LN >= 6 && 32 % LN == 0, "a lane per row of the block");
+  constexpr int AT = BS == 3 ? 4 : 2;
+  const long long th = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int c = (int)(th / LN), lane = threadIdx.x % LN, base = (threadIdx.x & 31) - lane;
+  const bool in = c < nnzC;
+  const int I = in ? c_row[c] : 0, J = in ? c_cl[c] : 0;
+  const int r = min(lane, 5);
+  T acc[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) acc[q] = T(0);
+  const int t1 = in ? pt_rp[I + 1] : 0;
+  int t = in ? pt_rp[I] + lane : 0;
+  while (__any_sync(0xffffffffu, t - lane < t1)) {  // whole warps, for the shuffles
+    int q = -1;
+    if (t < t1) {
+      const int n = pt_row[t];
+      q = find_sorted(ap_cl, ap_rp[n], ap_rp[n + 1], J);
+    }
+    unsigned m = (__ballot_sync(0xffffffffu, q >= 0) >> base) & ((1u << (LN - 1)) * 2u - 1u);
+    while (__any_sync(0xffffffffu, m != 0u)) {
+      // AT of them at a time, their loads in flight together
+      T p[AT][BS], av[AT][BS][6];
+      bool have[AT];
+#pragma unroll
+      for (int e = 0; e < AT; ++e) {
+        have[e] = m != 0u;
+        const int u = m ? __ffs(m) - 1 : 0;
+        m &= m - 1u;
+        const int qu = __shfl_sync(0xffffffffu, q, base + u);
+        if (have[e]) {
+          const T* P = ptval + (long long)(t - lane + u) * BS * 6 + r;
+          const T* AP = apval + (long long)qu * BS * 6;
+#pragma unroll
+          for (int i = 0; i < BS; ++i) {
+            p[e][i] = P[i * 6];
+            load6<T, false>(AP + i * 6, av[e][i]);
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < AT; ++e)
+        if (have[e]) {
+#pragma unroll
+          for (int i = 0; i < BS; ++i)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) acc[k] += p[e][i] * av[e][i][k];
+        }
+    }
+    t += LN;
+  }
+  if (!in || lane >= 6) return;
+  T* O = cval + (long long)c * 36 + r * 6;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) O[k] = acc[k];
+}
+
 // P^T copy: block t of the aggregate-ordered list is P block pt_blk[t].
 template <typename T, int BS>
 __global__ void sa_transpose_copy_kernel(int nnzP, const int* __restrict__ pt_blk, const T* __restrict__ pval,
@@ -1202,7 +1271,11 @@ static void setup_level_t(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t 
   launch(st, sa_ap_kernel<T, BS>, (v.nnzAP + 127) / 128, 128, 0, v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
          v.p_rp, v.p_cl, v.p_val, v.ap_val);
   constexpr int LN = 8;
-  launch(st, sa_rap_kernel<T, BS, LN>, (int)(((long long)nnzC * LN + 127) / 128), 128, 0, nnzC, v.c_row, v.c_cl, v.pt_rp,
+  auto* rap = [] {
+    if constexpr (std::is_same<T, float>::value) return &sa_rap_ordered_kernel<T, BS, LN>;
+    else return &sa_rap_kernel<T, BS, LN>;
+  }();
+  launch(st, rap, (int)(((long long)nnzC * LN + 127) / 128), 128, 0, nnzC, v.c_row, v.c_cl, v.pt_rp,
          v.pt_row, v.pt_val, v.ap_rp, v.ap_cl, v.ap_val, cval);
 }
 template <typename T>

@@ -29,5 +29,7 @@ def test_tangent(kept, i):
 
 
 def test_hierarchy(kept):
-    P, _ = G.hierarchy()
+    P, A = G.hierarchy()
     assert np.mean((P != kept["prolongator"])[P != 0]) <= RARE
+    assert np.mean((A != kept["galerkin"])[A != 0]) <= RARE
+
