@@ -38,8 +38,8 @@ struct KrylovWork {
   T *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
   T *rh = nullptr, *v = nullptr, *s = nullptr, *t = nullptr, *ph = nullptr, *sh = nullptr;
   T* sc = nullptr;    // device scalars
-  T* part = nullptr;  // reduction partials
-  double* dpart = nullptr;     // the loop bodies' dot products: four of kMaxPartials
+  T* part = nullptr;  // reduction partials: four of kMaxPartials
+  double* dpart = nullptr;     // kMaxPartials
   unsigned* ticket = nullptr;  // zero between launches of cg_xr_fused and bicg_xr
   T* b = nullptr;
   T *xa = nullptr, *b0 = nullptr;  // iterative refinement: accumulated solution, saved right-hand side
@@ -763,8 +763,8 @@ int krylov_alloc(pfem_ctx* ctx) {
   CK(dalloc(ctx, &w.v, n)); CK(dalloc(ctx, &w.s, n)); CK(dalloc(ctx, &w.t, n));
   CK(dalloc(ctx, &w.ph, n)); CK(dalloc(ctx, &w.sh, n)); CK(dalloc(ctx, &w.b, n));
   CK(dalloc(ctx, &w.xa, n)); CK(dalloc(ctx, &w.b0, n));
-  CK(dalloc(ctx, &w.sc, 16)); CK(dalloc(ctx, &w.part, 2048));
-  CK(dalloc(ctx, &w.dpart, 4 * (size_t)pfem::kMaxPartials));
+  CK(dalloc(ctx, &w.sc, 16)); CK(dalloc(ctx, &w.part, 4 * (size_t)pfem::kMaxPartials));
+  CK(dalloc(ctx, &w.dpart, (size_t)pfem::kMaxPartials));
   CK(dalloc(ctx, &w.ticket, 1));
   CK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned), ctx->st));
   return PFEM_OK;
@@ -860,7 +860,7 @@ int amg_setup(pfem_ctx* ctx, int cheb_degree) {
 // receives the partials of b.x (only degree 2, nonzero x); their count is returned.
 template <typename T>
 int cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero, bool started = false,
-         double* part = nullptr) {
+         T* part = nullptr) {
   const long long n = (long long)v.A.nbrow * v.A.bs;
   const T* const ith = v.co + CO_ITH;
   if (degree == 2) {
@@ -897,7 +897,7 @@ int cheb(pfem_ctx* ctx, AmgLevel<T>& v, int degree, const T* b, T* x, bool zero,
 // started: v.r and v.d hold the smoother's start on b (the kernel that made b wrote
 // them as well).  part: partials of b.x, as cheb.
 template <typename T>
-int vcycle(pfem_ctx* ctx, int l, const T* b, T* x, bool started = false, double* part = nullptr) {
+int vcycle(pfem_ctx* ctx, int l, const T* b, T* x, bool started = false, T* part = nullptr) {
   Amg<T>& A = amg_of<T>(ctx);
   const int L = (int)A.lv.size();
   AmgLevel<T>& v = A.lv[l];
@@ -1030,31 +1030,30 @@ int cg_graph_build(pfem_ctx* ctx, int method) {
   ctx->chain_len = 0;
   ctx->chain = A.cheb_degree == 2 ? &ctx->chain_len : nullptr;
   const Queue q(bs, ctx->chain);
-  double* const part[4] = {w.dpart, w.dpart + pfem::kMaxPartials, w.dpart + 2 * pfem::kMaxPartials,
-                           w.dpart + 3 * pfem::kMaxPartials};
+  T* const part[2] = {w.part, w.part + pfem::kMaxPartials};
   CgLoop loop;
   loop.h = h;
   loop.ctl = G.ctl;
   loop.state = G.state;
   loop.ticket = w.ticket;
-  loop.part_rr = part[2];
   if (cg) {
-    // sc[0] = r.z of the previous iteration, sc[2] = r.z; the dot products are summed
-    // by the kernels whose results they are made of, their final sums by their users
+    // sc[0] = r.z of the previous iteration, sc[2] = r.z; the final sums of the dot
+    // products are their users'
     int np_rz = vcycle<T>(ctx, 0, w.r, w.z, true, ctx->chain ? part[0] : nullptr);
-    if (np_rz == 0) np_rz = dot_partials_double<T>(n, w.r, w.z, part[0], q);
+    if (np_rz == 0) np_rz = dot_partials<T>(n, w.r, w.z, part[0], q);
     cg_p_fused<T>(n, part[0], np_rz, w.sc, w.z, w.p, q);
     const int np_pq = bsr_spmv<T>(K, w.p, w.q, q, part[1]);
-    cg_xr_fused<T>(K.nbrow, part[1], np_pq, w.sc, w.p, w.q, w.x, w.r, v0.dinv, v0.co, v0.r, v0.d, loop, q);
+    cg_xr_fused<T>(K.nbrow, part[1], np_pq, w.sc, w.p, w.q, w.x, w.r, v0.dinv, v0.co, v0.r, v0.d, w.dpart,
+                   loop, q);
   } else {
     bicg_p<T>(K.nbrow, w.sc, w.r, w.v, w.p, v0.dinv, v0.co, v0.r, v0.d, q);
     vcycle<T>(ctx, 0, w.p, w.ph, true);
     bsr_spmv<T>(K, w.ph, w.v, q);
-    const int np = dot_partials_double<T>(n, w.rh, w.v, part[0], q);
+    const int np = dot_partials<T>(n, w.rh, w.v, part[0], q);
     bicg_s<T>(K.nbrow, part[0], np, w.sc, w.r, w.v, w.s, v0.dinv, v0.co, v0.r, v0.d, q);
     vcycle<T>(ctx, 0, w.s, w.sh, true);
     bsr_spmv<T>(K, w.sh, w.t, q);
-    bicg_xr<T>(n, w.sc, w.ph, w.sh, w.s, w.t, w.rh, w.x, w.r, part[0], part[1], part[3], loop, q);
+    bicg_xr<T>(n, w.sc, w.ph, w.sh, w.s, w.t, w.rh, w.x, w.r, w.part, loop, q);
   }
   ctx->st = st;
   ctx->chain = nullptr;

@@ -30,22 +30,22 @@ __device__ __forceinline__ T block_sum(T v, T* sh) {
   return v;
 }
 
-// Partials of a.b summed in double, at most kMaxPartials (count returned).
+// Partials of a.b (count returned): the first pass of dot, also inside a launch chain.
 template <typename T>
-__global__ void dot_partial_double_kernel(long long n, const T* a, const T* b, double* part) {
-  __shared__ double sh[32];
+__global__ void dot_partial_kernel(long long n, const T* a, const T* b, T* part) {
+  __shared__ T sh[32];
   pdl_go();
   pdl_wait();
-  double v = 0.0;
+  T v = T(0);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    v += (double)a[i] * (double)b[i];
+    v += a[i] * b[i];
   v = block_sum(v, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
 template <typename T>
-int dot_partials_double(long long n, const T* a, const T* b, double* part, const Queue& q) {
+int dot_partials(long long n, const T* a, const T* b, T* part, const Queue& q) {
   const int blocks = (int)std::min<long long>(std::max<long long>((n + RED_THREADS - 1) / RED_THREADS, 1), RED_BLOCKS);
-  launch(q, dot_partial_double_kernel<T>, blocks, RED_THREADS, 0, n, a, b, part);
+  launch(q, dot_partial_kernel<T>, blocks, RED_THREADS, 0, n, a, b, part);
   return blocks;
 }
 
@@ -240,15 +240,23 @@ static int spmv_launch(const BsrMat<T>& A, const SpmvVec<T>& a, const Queue& qu)
   }
 }
 
+// The dot products of a CG iteration.  FP64: inside the products that hold their operands.
+// FP32: in passes of their own, in dot's order and type; the solution of a slender box
+// differs by hundreds of roundings with another order.  A mixed CG iteration so / with the
+// sums inside: 27.1 / 26.0 us at 8^3, 112 / 115 at 49 x 37 x 29, 373 / 367 at 64^3.
 template <typename T>
-int bsr_spmv(const BsrMat<T>& A, const T* x, T* y, Queue q, double* part) {
+constexpr bool kDotsInside = std::is_same<T, double>::value;
+template <typename T>
+int bsr_spmv(const BsrMat<T>& A, const T* x, T* y, Queue q, T* part) {
   SpmvVec<T> a;
   a.x = x; a.y = y; a.part = part;
-  if (!part) return spmv_launch<T, 0>(A, a, q);
-  const int np = spmv_launch<T, 0, true>(A, a, q);
+  int np = 0;
+  if constexpr (kDotsInside<T>) {
+    if (part) np = spmv_launch<T, 0, true>(A, a, q);
+  }
   if (np > 0) return np;
   spmv_launch<T, 0>(A, a, q);
-  return dot_partials_double<T>((long long)A.nbrow * A.bs, x, y, part, q);
+  return part ? dot_partials<T>((long long)A.nbrow * A.bs, x, y, part, q) : 0;
 }
 template <typename T>
 void bsr_residual(const BsrMat<T>& A, const T* x, const T* b, T* r, Queue q) {
@@ -264,15 +272,17 @@ void bsr_cheb_step(const BsrMat<T>& A, const T* dinv, const T* d, T* r, T* x, cu
 }
 template <typename T>
 int bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero, const T* co, Queue q,
-              const T* b, double* part) {
+              const T* b, T* part) {
   SpmvVec<T> a;
   a.x = d0; a.y = const_cast<T*>(r0); a.dinv = dinv; a.xo = x; a.co = co; a.b = b; a.part = part;
   if (zero) return spmv_launch<T, 3>(A, a, q);
-  if (!part) return spmv_launch<T, 4>(A, a, q);
-  const int np = spmv_launch<T, 4, true>(A, a, q);
+  int np = 0;
+  if constexpr (kDotsInside<T>) {
+    if (part) np = spmv_launch<T, 4, true>(A, a, q);
+  }
   if (np > 0) return np;
   spmv_launch<T, 4>(A, a, q);
-  return dot_partials_double<T>((long long)A.nbrow * A.bs, b, x, part, q);
+  return part ? dot_partials<T>((long long)A.nbrow * A.bs, b, x, part, q) : 0;
 }
 template <typename T>
 void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r, T* d, const T* co, Queue q) {
@@ -382,17 +392,6 @@ void blockdiag_invert(const BsrMat<T>& A, T* dinv, cudaStream_t st) {
 
 // ------------------------------------------------------------------ dot products
 template <typename T>
-__global__ void dot_partial_kernel(long long n, const T* __restrict__ a, const T* __restrict__ b,
-                                   T* __restrict__ part) {
-  __shared__ T sh[32];
-  T v = T(0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    v += a[i] * b[i];
-  v = block_sum(v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
-}
-template <typename T>
 __global__ void sum_final_kernel(int np, const T* __restrict__ part, T* __restrict__ out, int sqrt_out) {
   __shared__ T sh[32];
   T v = T(0);
@@ -402,9 +401,7 @@ __global__ void sum_final_kernel(int np, const T* __restrict__ part, T* __restri
 }
 template <typename T>
 void dot(long long n, const T* a, const T* b, T* out, T* part, cudaStream_t st, bool take_sqrt) {
-  long long nb = (n + RED_THREADS - 1) / RED_THREADS;
-  const int blocks = (int)(nb < RED_BLOCKS ? (nb > 0 ? nb : 1) : RED_BLOCKS);
-  pfem::count_launch(); dot_partial_kernel<T><<<blocks, RED_THREADS, 0, st>>>(n, a, b, part);
+  const int blocks = dot_partials<T>(n, a, b, part, st);
   pfem::count_launch(); sum_final_kernel<T><<<1, 1024, 0, st>>>(blocks, part, out, take_sqrt ? 1 : 0);
 }
 
@@ -449,11 +446,11 @@ __device__ __forceinline__ T all_sum_partials(const T* part, int np, T* sh) {
 }
 // rz = sum(part_rz);  p = z + (rz / sc[0]) p;  sc[2] = rz
 template <typename T>
-__global__ void cg_p_fused_kernel(long long n, const double* part, int np, T* sc, const T* z, T* p) {
-  __shared__ double sh[33];
+__global__ void cg_p_fused_kernel(long long n, const T* part, int np, T* sc, const T* z, T* p) {
+  __shared__ T sh[33];
   pdl_go();
   pdl_wait();
-  const T rz = (T)all_sum_partials(part, np, sh);
+  const T rz = all_sum_partials(part, np, sh);
   const T be = rz / sc[0];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     p[i] = z[i] + be * p[i];
@@ -464,15 +461,17 @@ __global__ void cg_p_fused_kernel(long long n, const double* part, int np, T* sc
 // CTA that finishes last adds the CTAs' shares of r.r in their order and sets the
 // loop's condition.
 template <typename T>
-__global__ void __launch_bounds__(256) cg_xr_fused_kernel(int nbrow, const double* part_pq, int np, T* sc, const T* p,
+__global__ void __launch_bounds__(256) cg_xr_fused_kernel(int nbrow, const T* part_pq, int np, T* sc, const T* p,
                                                           const T* q, T* x, T* r, const T* __restrict__ dinv,
-                                                          const T* __restrict__ co, T* sr, T* sd, CgLoop loop) {
+                                                          const T* __restrict__ co, T* sr, T* sd, double* part_rr,
+                                                          CgLoop loop) {
+  __shared__ T sht[33];
   __shared__ double sh[33];
   __shared__ bool last;
   pdl_go();
   const T ith = co[CO_ITH];
   pdl_wait();
-  const T pq = (T)all_sum_partials(part_pq, np, sh);
+  const T pq = all_sum_partials(part_pq, np, sht);
   const T al = sc[2] / pq;
   double acc = 0.0;
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nbrow; n += gridDim.x * blockDim.x) {
@@ -494,17 +493,16 @@ __global__ void __launch_bounds__(256) cg_xr_fused_kernel(int nbrow, const doubl
       sd[at + i] = ith * t;
     }
   }
-  __syncthreads();  // sh is free again
   acc = block_sum(acc, sh);
   if (threadIdx.x == 0) {
-    loop.part_rr[blockIdx.x] = acc;
+    part_rr[blockIdx.x] = acc;
     __threadfence();
     last = atomicInc(loop.ticket, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const double rr = all_sum_partials(loop.part_rr, (int)gridDim.x, sh);
+  const double rr = all_sum_partials(part_rr, (int)gridDim.x, sh);
   if (threadIdx.x != 0) return;
   sc[0] = sc[2];
   const double rn = sqrt(rr);
@@ -515,14 +513,14 @@ __global__ void __launch_bounds__(256) cg_xr_fused_kernel(int nbrow, const doubl
   cudaGraphSetConditional(loop.h, (!conv && isfinite(rn) && it < (int)loop.ctl[1]) ? 1u : 0u);
 }
 template <typename T>
-void cg_p_fused(long long n, const double* part, int np, T* sc, const T* z, T* p, Queue q) {
+void cg_p_fused(long long n, const T* part, int np, T* sc, const T* z, T* p, Queue q) {
   launch(q, cg_p_fused_kernel<T>, fused_update_blocks(n), RED_THREADS, 0, n, part, np, sc, z, p);
 }
 template <typename T>
-void cg_xr_fused(int nbrow, const double* part_pq, int np, T* sc, const T* p, const T* q, T* x, T* r, const T* dinv,
-                 const T* co, T* sr, T* sd, const CgLoop& loop, Queue qu) {
+void cg_xr_fused(int nbrow, const T* part_pq, int np, T* sc, const T* p, const T* q, T* x, T* r, const T* dinv,
+                 const T* co, T* sr, T* sd, double* part_rr, const CgLoop& loop, Queue qu) {
   launch(qu, cg_xr_fused_kernel<T>, fused_update_blocks(nbrow), RED_THREADS, 0, nbrow, part_pq, np, sc, p, q, x, r, dinv,
-         co, sr, sd, loop);
+         co, sr, sd, part_rr, loop);
 }
 
 // The sum of np partials (at most 2048) in the order in which sum_final_kernel adds them,
@@ -589,9 +587,10 @@ void power_norm(long long n, const T* v, T* part, unsigned* ticket, bool finish,
 }
 // ---- BiCGStab updates.  Scalars: sc[0] rho = rh.r, sc[1] rho of the iteration before,
 // sc[2] alpha, sc[3] omega.  A thread per node, as cg_xr_fused; the dot products come as
-// partials in double.  An iteration used to be 44 plain launches from the host with a
-// read-back of |r|, bound by the launches below about 40^3; in the graph with the
-// smoother's starts in its own updates it takes 440 us at 40^3 FP64, 550 before.
+// dot's partials and are added in its order.  An iteration used to be 78 plain launches
+// from the host with a read-back of |r|, bound by the launches below about 40^3; in the
+// graph with the smoother's starts in its own updates it is 44 and takes 440 us at 40^3
+// FP64, 550 before.
 template <typename T>
 __device__ __forceinline__ void smoother_start(const T* __restrict__ dinv, T ith, long long n, const T v[3], T* sr,
                                                T* sd) {
@@ -627,14 +626,14 @@ __global__ void __launch_bounds__(256) bicg_p_kernel(int nbrow, const T* sc, con
 }
 // alpha = rho / sum(part);  s = r - alpha v
 template <typename T>
-__global__ void __launch_bounds__(256) bicg_s_kernel(int nbrow, const double* part, int np, T* sc, const T* r,
+__global__ void __launch_bounds__(256) bicg_s_kernel(int nbrow, const T* part, int np, T* sc, const T* r,
                                                      const T* v, T* s, const T* __restrict__ dinv,
                                                      const T* __restrict__ co, T* sr, T* sd) {
-  __shared__ double sh[33];
+  __shared__ T sh[32];
   pdl_go();
   const T ith = co[CO_ITH];
   pdl_wait();
-  const T al = sc[0] / (T)all_sum_partials(part, np, sh);
+  const T al = sc[0] / sum_as_final(part, np, sh);
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nbrow; n += gridDim.x * blockDim.x) {
     T e[3];
 #pragma unroll
@@ -649,15 +648,15 @@ __global__ void __launch_bounds__(256) bicg_s_kernel(int nbrow, const double* pa
 }
 // Partials of t.s and of t.t.
 template <typename T>
-__global__ void __launch_bounds__(256) bicg_dots_kernel(long long n, const T* t, const T* s, double* part_ts,
-                                                        double* part_tt) {
-  __shared__ double sh[32];
+__global__ void __launch_bounds__(256) bicg_dots_kernel(long long n, const T* t, const T* s, T* part_ts,
+                                                        T* part_tt) {
+  __shared__ T sh[32];
   pdl_go();
   pdl_wait();
-  double a = 0.0, b = 0.0;
+  T a = T(0), b = T(0);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double ti = (double)t[i];
-    a += ti * (double)s[i];
+    const T ti = t[i];
+    a += ti * s[i];
     b += ti * ti;
   }
   a = block_sum(a, sh);
@@ -672,30 +671,30 @@ __global__ void __launch_bounds__(256) bicg_dots_kernel(long long n, const T* t,
 // CTA that finishes last adds the shares of r.r and rh.r in their order, leaves the next
 // iteration's scalars and sets the loop's condition.
 template <typename T>
-__global__ void __launch_bounds__(256) bicg_xr_kernel(long long n, const double* part_ts, const double* part_tt,
+__global__ void __launch_bounds__(256) bicg_xr_kernel(long long n, const T* part_ts, const T* part_tt,
                                                       int np, T* sc, const T* ph, const T* sh_, const T* s, const T* t,
-                                                      const T* rh, T* x, T* r, double* part_rho, CgLoop loop) {
-  __shared__ double sh[33];
+                                                      const T* rh, T* x, T* r, T* part_rr, T* part_rho,
+                                                      CgLoop loop) {
+  __shared__ T sh[32];
   __shared__ bool last;
   pdl_go();
   pdl_wait();
   const T al = sc[2];
-  const T ts = (T)all_sum_partials(part_ts, np, sh);
-  const T om = ts / (T)all_sum_partials(part_tt, np, sh);
-  double rr = 0.0, rho = 0.0;
+  const T ts = sum_as_final(part_ts, np, sh);
+  const T om = ts / sum_as_final(part_tt, np, sh);
+  T rr = T(0), rho = T(0);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     x[i] += al * ph[i] + om * sh_[i];
     const T e = s[i] - om * t[i];
     r[i] = e;
-    rr += (double)e * (double)e;
-    rho += (double)rh[i] * (double)e;
+    rr += e * e;
+    rho += rh[i] * e;
   }
-  __syncthreads();  // sh is free again
   rr = block_sum(rr, sh);
   __syncthreads();
   rho = block_sum(rho, sh);
   if (threadIdx.x == 0) {
-    loop.part_rr[blockIdx.x] = rr;
+    part_rr[blockIdx.x] = rr;
     part_rho[blockIdx.x] = rho;
     __threadfence();
     last = atomicInc(loop.ticket, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
@@ -703,13 +702,13 @@ __global__ void __launch_bounds__(256) bicg_xr_kernel(long long n, const double*
   __syncthreads();
   if (!last) return;
   __threadfence();
-  rr = all_sum_partials(loop.part_rr, (int)gridDim.x, sh);
-  rho = all_sum_partials(part_rho, (int)gridDim.x, sh);
+  rr = sum_as_final(part_rr, (int)gridDim.x, sh);
+  rho = sum_as_final(part_rho, (int)gridDim.x, sh);
   if (threadIdx.x != 0) return;
   sc[1] = sc[0];
-  sc[0] = (T)rho;
+  sc[0] = rho;
   sc[3] = om;
-  const double rn = sqrt(rr);
+  const double rn = (double)sqrt(rr);
   const int it = loop.state[0] + 1;
   const bool conv = rn <= loop.ctl[2];
   loop.state[0] = it;
@@ -721,18 +720,19 @@ void bicg_p(int nbrow, const T* sc, const T* r, const T* v, T* p, const T* dinv,
   launch(q, bicg_p_kernel<T>, fused_update_blocks(nbrow), RED_THREADS, 0, nbrow, sc, r, v, p, dinv, co, sr, sd);
 }
 template <typename T>
-void bicg_s(int nbrow, const double* part, int np, T* sc, const T* r, const T* v, T* s, const T* dinv, const T* co,
+void bicg_s(int nbrow, const T* part, int np, T* sc, const T* r, const T* v, T* s, const T* dinv, const T* co,
             T* sr, T* sd, Queue q) {
   launch(q, bicg_s_kernel<T>, fused_update_blocks(nbrow), RED_THREADS, 0, nbrow, part, np, sc, r, v, s, dinv, co, sr,
          sd);
 }
 template <typename T>
 void bicg_xr(long long n, T* sc, const T* ph, const T* sh, const T* s, const T* t, const T* rh, T* x, T* r,
-             double* part_ts, double* part_tt, double* part_rho, const CgLoop& loop, Queue q) {
+             T* part, const CgLoop& loop, Queue q) {
   const int blocks = fused_update_blocks(n);
+  T* const part_ts = part, * const part_tt = part + kMaxPartials;
   launch(q, bicg_dots_kernel<T>, blocks, RED_THREADS, 0, n, t, s, part_ts, part_tt);
   launch(q, bicg_xr_kernel<T>, blocks, RED_THREADS, 0, n, part_ts, part_tt, blocks, sc, ph, sh, s, t, rh, x, r,
-         part_rho, loop);
+         part + 2 * kMaxPartials, part + 3 * kMaxPartials, loop);
 }
 
 // precision conversion
@@ -1467,11 +1467,11 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, Queue q)
 
 // ------------------------------------------------------------------ instantiations
 #define PFEM_INST(T)                                                                               \
-  template int bsr_spmv<T>(const BsrMat<T>&, const T*, T*, Queue, double*);                        \
+  template int bsr_spmv<T>(const BsrMat<T>&, const T*, T*, Queue, T*);                             \
   template void bsr_residual<T>(const BsrMat<T>&, const T*, const T*, T*, Queue);                  \
   template void bsr_cheb_step<T>(const BsrMat<T>&, const T*, const T*, T*, T*, cudaStream_t);      \
   template int bsr_cheb2<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, bool, const T*, Queue, const T*, \
-                            double*);                                                              \
+                            T*);                                                                   \
   template void bsr_residual_precond<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, const T*, Queue); \
   template void bsr_residual_start<T>(const BsrMat<T>&, const T*, const T*, const T*, T*, T*, T*, const T*, Queue); \
   template void bsr_power_step<T>(const BsrMat<T>&, const T*, const T*, T*, const T*, cudaStream_t); \
@@ -1483,14 +1483,14 @@ void sa_prolong2(const AmgLevel<T>& v, const T* xc, const T* xc2, T* x, Queue q)
   template void axpby<T>(long long, T, const T*, T, T*, cudaStream_t);                             \
   template void bicg_p<T>(int, const T*, const T*, const T*, T*, const T*, const T*, T*, T*,       \
                           Queue);                                                                  \
-  template void bicg_s<T>(int, const double*, int, T*, const T*, const T*, T*, const T*, const T*, \
+  template void bicg_s<T>(int, const T*, int, T*, const T*, const T*, T*, const T*, const T*,      \
                           T*, T*, Queue);                                                          \
   template void bicg_xr<T>(long long, T*, const T*, const T*, const T*, const T*, const T*, T*,    \
-                           T*, double*, double*, double*, const CgLoop&, Queue);                   \
-  template int dot_partials_double<T>(long long, const T*, const T*, double*, const Queue&);       \
-  template void cg_p_fused<T>(long long, const double*, int, T*, const T*, T*, Queue);             \
-  template void cg_xr_fused<T>(int, const double*, int, T*, const T*, const T*, T*, T*, const T*, const T*, T*, T*, \
-                               const CgLoop&, Queue);                                              \
+                           T*, T*, const CgLoop&, Queue);                                          \
+  template int dot_partials<T>(long long, const T*, const T*, T*, const Queue&);                   \
+  template void cg_p_fused<T>(long long, const T*, int, T*, const T*, T*, Queue);                  \
+  template void cg_xr_fused<T>(int, const T*, int, T*, const T*, const T*, T*, T*, const T*, const T*, T*, T*, \
+                               double*, const CgLoop&, Queue);                                     \
   template void add_to_double<T>(long long, const T*, double*, cudaStream_t);                      \
   template void impose_dirichlet<T>(const BcDev&, long long, double, const double*, T*, double*,   \
                                       double*, unsigned*, double*, cudaStream_t);                  \

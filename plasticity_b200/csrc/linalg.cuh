@@ -65,14 +65,14 @@ struct BcDev {
 };
 
 // y = A x; with part, also the partials of x.y (their count is returned).
-template <typename T> int bsr_spmv(const BsrMat<T>& A, const T* x, T* y, Queue q, double* part = nullptr);
+template <typename T> int bsr_spmv(const BsrMat<T>& A, const T* x, T* y, Queue q, T* part = nullptr);
 template <typename T> void bsr_residual(const BsrMat<T>& A, const T* x, const T* b, T* r, Queue q);
 template <typename T> void bsr_cheb_step(const BsrMat<T>& A, const T* dinv, const T* d, T* r, T* x, cudaStream_t st);
 // Degree-2 Chebyshev in one pass: x (=, or += unless zero) c2 d0 + c1 (r0 - Dinv A d0);
 // co holds the level's scalars on the device.  With part (not zero): also the partials
 // of b.x (count returned).
 template <typename T> int bsr_cheb2(const BsrMat<T>& A, const T* dinv, const T* d0, const T* r0, T* x, bool zero,
-                                    const T* co, Queue q, const T* b = nullptr, double* part = nullptr);
+                                    const T* co, Queue q, const T* b = nullptr, T* part = nullptr);
 // r = Dinv (b - A x), d = co[CO_ITH] r.
 template <typename T> void bsr_residual_precond(const BsrMat<T>& A, const T* dinv, const T* x, const T* b, T* r,
                                                 T* d, const T* co, Queue q);
@@ -102,24 +102,24 @@ struct CgLoop {
   const double* ctl;    // [1] iteration cap, [2] absolute threshold
   int* state;           // [0] iterations, [1] converged
   unsigned* ticket;     // zero between launches
-  double* part_rr;      // kMaxPartials
 };
-// Partials of a.b in double (at most kMaxPartials, count returned).
-template <typename T> int dot_partials_double(long long n, const T* a, const T* b, double* part, const Queue& q);
-template <typename T> void cg_p_fused(long long n, const double* part, int np, T* sc, const T* z, T* p, Queue q);
-template <typename T> void cg_xr_fused(int nbrow, const double* part_pq, int np, T* sc, const T* p, const T* q, T* x,
-                                       T* r, const T* dinv, const T* co, T* sr, T* sd, const CgLoop& loop, Queue qu);
+// Partials of a.b in dot's order (count returned).
+template <typename T> int dot_partials(long long n, const T* a, const T* b, T* part, const Queue& q);
+template <typename T> void cg_p_fused(long long n, const T* part, int np, T* sc, const T* z, T* p, Queue q);
+template <typename T> void cg_xr_fused(int nbrow, const T* part_pq, int np, T* sc, const T* p, const T* q, T* x,
+                                       T* r, const T* dinv, const T* co, T* sr, T* sd, double* part_rr,
+                                       const CgLoop& loop, Queue qu);
 // BiCGStab updates, with the smoother's start on p and on s (sr, sd as above):
 // bicg_p: p = r + beta (p - omega v); bicg_s: alpha = sc[0] / sum(part), s = r - alpha v;
 // bicg_xr: omega from the dot products of t with s and itself, x += alpha ph + omega sh,
-// r = s - omega t, the next rho and the loop condition (part_*: kMaxPartials each).
+// r = s - omega t, the next rho and the loop condition (part: four of kMaxPartials).  The
+// dot products are dot's.
 template <typename T> void bicg_p(int nbrow, const T* sc, const T* r, const T* v, T* p, const T* dinv, const T* co,
                                   T* sr, T* sd, Queue q);
-template <typename T> void bicg_s(int nbrow, const double* part, int np, T* sc, const T* r, const T* v, T* s,
+template <typename T> void bicg_s(int nbrow, const T* part, int np, T* sc, const T* r, const T* v, T* s,
                                   const T* dinv, const T* co, T* sr, T* sd, Queue q);
 template <typename T> void bicg_xr(long long n, T* sc, const T* ph, const T* sh, const T* s, const T* t, const T* rh,
-                                   T* x, T* r, double* part_ts, double* part_tt, double* part_rho, const CgLoop& loop,
-                                   Queue q);
+                                   T* x, T* r, T* part, const CgLoop& loop, Queue q);
 template <typename A, typename B> void convert(long long n, const A* a, B* b, double s, cudaStream_t st);
 template <typename T> void add_to_double(long long n, const T* x, double* U, cudaStream_t st);
 // Impose the constraints on K and R at lambda, subtract the load, *rnorm = |R| (device).

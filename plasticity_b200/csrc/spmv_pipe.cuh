@@ -13,8 +13,9 @@
 // block of its row; the lanes of a warp read shared memory at the rows' stride (27
 // blocks = 243 words, odd: few bank conflicts), and in a node-ordered mesh the rows'
 // k-th neighbours are consecutive nodes, so the gathers of x fall into a few lines.
-// Each component has seven partial sums, one block of a 27-block row each, added as a
-// tree: no deeper than the register kernel's two blocks per lane and four shuffles.
+// Each component has four partial sums of two blocks each, added as a tree: the register
+// kernel's two blocks per lane and four shuffles in the same order, so that a product is
+// the same number whichever kernel makes it (seven sums of one block took the same time).
 // 6 x 6 blocks: half a warp per row, lane k takes blocks k and k + 16, 16-byte reads
 // at a stride of 36 words (no conflicts).
 #pragma once
@@ -43,7 +44,7 @@ struct SpmvVec {
   T* xo = nullptr;
   const T* co = nullptr;
   T* z = nullptr;
-  double* part = nullptr;  // partials of x.y (mode 0) or b.xo (mode 4), one per CTA
+  T* part = nullptr;  // partials of x.y (mode 0) or b.xo (mode 4), one per CTA (FP64)
 };
 
 // LANES lanes per row and ROWS rows per tile; a CTA is one warp with one tile in shared
@@ -160,35 +161,33 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
       const T* vs = reinterpret_cast<const T*>(st + (((long long)s0 * (9 * (int)sizeof(T))) & 15)) + (long long)b0 * 9;
       const int* cs = reinterpret_cast<const int*>(st + lay.cols + (((long long)s0 * 4) & 15)) + b0;
       const int16_t* cs16 = reinterpret_cast<const int16_t*>(st + lay.cols + (((long long)s0 * 2) & 15)) + b0;
-      // seven partial sums per component, each of every seventh of the lane's blocks
-      constexpr int NP = 7;
+      // four partial sums per component, as the register kernel's lanes par + 4 m have them:
+      // block q = par + 4 m, then block q + 16
+      constexpr int NP = 16 / LN;
       T acc[NP][3];
 #pragma unroll
       for (int m = 0; m < NP; ++m) acc[m][0] = acc[m][1] = acc[m][2] = T(0);
-      const int most = __reduce_max_sync(0xffffffffu, len);
-      for (int base = par; base < most; base += LN * NP) {
-        T xv[NP][3];
+      T xv[2 * NP][3];
 #pragma unroll
-        for (int m = 0; m < NP; ++m) {
-          const int q = base + LN * m;
-          const bool in = q < len;
-          const long long c = in ? (C16 ? row + (int)cs16[q] : cs[q]) : 0;
+      for (int m = 0; m < 2 * NP; ++m) {
+        const int q = par + LN * m;
+        const bool in = q < len;
+        const long long c = in ? (C16 ? row + (int)cs16[q] : cs[q]) : 0;
 #pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            xv[m][j] = in ? a.x[c * 3 + j] : T(0);
-            if (MODE == 6) xv[m][j] *= c2;
-          }
+        for (int j = 0; j < 3; ++j) {
+          xv[m][j] = in ? a.x[c * 3 + j] : T(0);
+          if (MODE == 6) xv[m][j] *= c2;
         }
+      }
 #pragma unroll
-        for (int m = 0; m < NP; ++m) {
-          const int q = base + LN * m;
-          if (q < len) {
-            const T* B = vs + q * 9;
+      for (int m = 0; m < 2 * NP; ++m) {
+        const int q = par + LN * m;
+        if (q < len) {
+          const T* B = vs + q * 9;
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+          for (int i = 0; i < 3; ++i)
 #pragma unroll
-              for (int j = 0; j < 3; ++j) acc[m][i] += B[i * 3 + j] * xv[m][j];
-          }
+            for (int j = 0; j < 3; ++j) acc[m % NP][i] += B[i * 3 + j] * xv[m][j];
         }
       }
       __syncwarp();
@@ -201,7 +200,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
       T v[3];
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        v[i] = ((acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i])) + ((acc[4][i] + acc[5][i]) + acc[6][i]);
+        v[i] = (acc[0][i] + acc[2][i]) + (acc[1][i] + acc[3][i]);
 #pragma unroll
         for (int o = 16; o >= R; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
       }

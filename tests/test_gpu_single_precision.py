@@ -33,3 +33,9 @@ def test_hierarchy(kept):
     assert np.mean((P != kept["prolongator"])[P != 0]) <= RARE
     assert np.mean((A != kept["galerkin"])[A != 0]) <= RARE
 
+
+@pytest.mark.parametrize("i", range(len(G.SOLVES)))
+def test_solution(kept, i):
+    x, y = G.solution(*G.SOLVES[i]).astype(float), kept["solution_%d" % i].astype(float)
+    # the bound for a single-precision result; the same order gives the same bits
+    assert np.linalg.norm(x - y) <= 2e-5 * np.linalg.norm(y)
