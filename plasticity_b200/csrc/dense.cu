@@ -530,14 +530,18 @@ void dense_coarse_inverse(int nbrow, const int* rp, const int* cl, const T* val,
   dense_out_kernel<T><<<2048, 256, 0, st>>>(n, np, A, inv);
 }
 
-template <typename T, int RR, int CPW>
+// NMAX: the largest size of the instantiation, whose shared memory is the kernel's limit
+// for every launch of it (the limit is the process's: with a launch's own size in it, another
+// context's launch in between could meet a smaller one).
+template <typename T, int RR, int CPW, int NMAX>
 static cudaError_t pivot_launch(int nnzb, const int* br, const int* cl, const T* val, int n, double* work, T* inv, cudaStream_t st) {
   auto* kern = pivot_inverse_kernel<T, RR, CPW>;
-  const size_t sm = pivot_smem(n);
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  static_assert(NMAX <= 32 * RR && (NMAX + PC - 1) / PC <= CPW * (PT / 32), "rows and columns fit");
+  const cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pivot_smem(NMAX));
   if (e != cudaSuccess) return e;
   count_launch();
-  kern<<<PC, PT, sm, st>>>(pivot_cols(n), nnzb, br, cl, val, n, work, inv);
+  kern<<<PC, PT, pivot_smem(n), st>>>(pivot_cols(n), nnzb, br, cl, val, n, work, inv);
   return cudaGetLastError();
 }
 // Rows per lane and columns per warp: six and three up to 192 unknowns, seven and four up
@@ -545,10 +549,9 @@ static cudaError_t pivot_launch(int nnzb, const int* br, const int* cl, const T*
 template <typename T>
 cudaError_t pivot_inverse(int nnzb, const int* br, const int* cl, const T* val, int n, double* work, T* inv,
                           cudaStream_t st) {
-  static_assert(kPivotMax <= 32 * 10 && (kPivotMax + PC - 1) / PC <= 5 * (PT / 32), "rows and columns fit");
-  if (n <= 192) return pivot_launch<T, 6, 3>(nnzb, br, cl, val, n, work, inv, st);
-  if (n <= 224) return pivot_launch<T, 7, 4>(nnzb, br, cl, val, n, work, inv, st);
-  return pivot_launch<T, 10, 5>(nnzb, br, cl, val, n, work, inv, st);
+  if (n <= 192) return pivot_launch<T, 6, 3, 192>(nnzb, br, cl, val, n, work, inv, st);
+  if (n <= 224) return pivot_launch<T, 7, 4, 224>(nnzb, br, cl, val, n, work, inv, st);
+  return pivot_launch<T, 10, 5, kPivotMax>(nnzb, br, cl, val, n, work, inv, st);
 }
 template cudaError_t pivot_inverse<float>(int, const int*, const int*, const float*, int, double*, float*, cudaStream_t);
 template cudaError_t pivot_inverse<double>(int, const int*, const int*, const double*, int, double*, double*,

@@ -1465,8 +1465,11 @@ void launch_gather_rows(int nn, const int* nptr, const int* nel, const uint8_t* 
                                                                   err);
     return;
   }
-  if (sm > 48 * 1024)  // rows longer than a hex mesh's 27 blocks (the 8-bit rank table caps them at 256)
-    cudaFuncSetAttribute(gather_rows_kernel<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // rows longer than a hex mesh's 27 blocks; the 8-bit rank table caps them at 256, and the
+  // limit is set for those, as it is the process's and not this launch's
+  if (sm > 48 * 1024)
+    cudaFuncSetAttribute(gather_rows_kernel<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(WARPS * 256 * 9 * sizeof(KT)));
   pfem::count_launch();
   gather_rows_kernel<KT><<<blocks, 32 * WARPS, sm, st>>>(nn, nptr, nel, nloc, browptr, rank, Kbuf, Fbuf, Kval, R,
                                                         maxlen);

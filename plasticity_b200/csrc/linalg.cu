@@ -181,8 +181,7 @@ __global__ void __launch_bounds__(128) bsr_spmv_kernel(int nbrow, const int* __r
 template <typename T, int BS, int MODE, bool C16, bool DOT>
 static int pipe_launch_t(const BsrMat<T>& A, const SpmvVec<T>& a, const Queue& qu) {
   auto* kern = bsr_spmv_pipe_kernel<T, BS, MODE, C16, DOT>;
-  const int sm = pipe_smem_bytes<T, BS>(A.max_row, C16);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  const int sm = pipe_smem_bytes<T, BS>(A.max_row, C16);  // at most 38 KB: no limit to raise
   int dev = 0, sms = 148, per = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -204,7 +203,7 @@ template <typename T>
 static bool spmv_streams(const BsrMat<T>& A) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(A.val) | reinterpret_cast<uintptr_t>(A.rowptr) |
                        (A.bs == 3 && A.col16 ? reinterpret_cast<uintptr_t>(A.col16) : reinterpret_cast<uintptr_t>(A.col));
-  return A.nbrow >= (A.bs == 3 ? kPipeRows3 : kPipeRows6) && A.max_row >= 1 && A.max_row <= 32 && A.err && !(at & 15);
+  return A.nbrow >= (A.bs == 3 ? kPipeRows3 : kPipeRows6) && A.max_row >= 1 && A.max_row <= kPipeMaxRow && A.err && !(at & 15);
 }
 
 // DOT (3 x 3 blocks): returns the number of partials, 0 when there would be too many.

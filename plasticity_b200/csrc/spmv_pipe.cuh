@@ -68,19 +68,24 @@ struct PipeLay {
   int cols, rows, bytes;
 };
 template <typename T, int BS>
-__host__ __device__ inline PipeLay pipe_lay(int max_row, bool c16) {
+__host__ __device__ constexpr PipeLay pipe_lay(int max_row, bool c16) {
   constexpr int R = PipeShape<T, BS>::ROWS;
-  PipeLay l;
+  PipeLay l = {};
   l.cols = (R * max_row * BS * BS * (int)sizeof(T) + 32 + 15) & ~15;
   l.rows = l.cols + ((R * max_row * (c16 ? 2 : 4) + 32 + 15) & ~15);
   l.bytes = l.rows + R * 4 + 16;
   return l;
 }
 constexpr int kPipeHead = 16;  // the barrier, in front of the tile
+constexpr int kPipeMaxRow = 32;  // blocks of a row that two passes of 16 lanes take
 template <typename T, int BS>
-inline int pipe_smem_bytes(int max_row, bool c16) {
+constexpr int pipe_smem_bytes(int max_row, bool c16) {
   return kPipeHead + pipe_lay<T, BS>(max_row, c16).bytes;
 }
+// Without cudaFuncAttributeMaxDynamicSharedMemorySize, which is the process's and not the
+// launch's: a context that set it for its rows would take it from another one's launch.
+static_assert(pipe_smem_bytes<double, 6>(kPipeMaxRow, false) <= 48 * 1024 &&
+                  pipe_smem_bytes<double, 3>(kPipeMaxRow, false) <= 48 * 1024, "a tile needs no attribute");
 
 // Start the copies of tile t (rows t R .., blocks s0 .. s1); one lane.
 template <typename T, int BS, bool C16>
