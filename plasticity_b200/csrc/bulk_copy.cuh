@@ -17,9 +17,8 @@ __device__ __forceinline__ void bulk_init_fence() {
 }
 // This thread's accesses of shared memory before the copies that follow.
 __device__ __forceinline__ void bulk_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// False when the phase has not completed within the limit.
-__device__ __forceinline__ bool bulk_bar_wait(uint32_t bar, uint32_t phase) {
-  for (long long it = 0; it < kBulkWaitLimit; ++it) {
+__device__ __forceinline__ bool bulk_bar_poll(uint32_t bar, uint32_t phase, long long polls) {
+  for (long long it = 0; it < polls; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -29,6 +28,16 @@ __device__ __forceinline__ bool bulk_bar_wait(uint32_t bar, uint32_t phase) {
         : "memory");
     if (done) return true;
   }
+  return false;
+}
+// False, with *err set, when the phase has not completed within the limit.  Its copies may
+// still be on their way then, into shared memory that is another CTA's once this one has
+// left, so they get the limit once more before the caller is told.
+__device__ __forceinline__ bool bulk_bar_wait(uint32_t bar, uint32_t phase, int* err, long long polls = kBulkWaitLimit,
+                                              long long drain = kBulkWaitLimit) {
+  if (bulk_bar_poll(bar, phase, polls)) return true;
+  atomicExch(err, 1);
+  bulk_bar_poll(bar, phase, drain);
   return false;
 }
 __device__ __forceinline__ void bulk_expect(uint32_t bar, uint32_t bytes) {

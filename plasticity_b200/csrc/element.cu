@@ -1405,10 +1405,9 @@ __global__ void __launch_bounds__(32 * GS_WARPS) gather_rows_stream_kernel(
     GatherStage<KT>& S = stage[warp][s];
     if (lane < 24) S.f[lane] = fv;
     if (nqa > 0) {
-      if (!__all_sync(0xffffffffu, bulk_bar_wait(bar + 8 * s, (phase >> s) & 1u))) {
-        // report it, and leave only when the other half's copies have landed as well
-        if (lane == 0) atomicExch(err, 1);
-        if (a + step < nn && nqb > 0) bulk_bar_wait(bar + 8 * (s ^ 1), (phase >> (s ^ 1)) & 1u);
+      if (!__all_sync(0xffffffffu, bulk_bar_wait(bar + 8 * s, (phase >> s) & 1u, err))) {
+        // leave only when the other half's copies have landed as well
+        if (a + step < nn && nqb > 0) bulk_bar_wait(bar + 8 * (s ^ 1), (phase >> (s ^ 1)) & 1u, err);
         return;
       }
       phase ^= 1u << s;

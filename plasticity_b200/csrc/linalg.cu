@@ -1328,10 +1328,7 @@ sa_restrict_stream_kernel(int cap, const int* __restrict__ pt_rp, const int* __r
     ith = co[CO_ITH];
   }
   pdl_wait();
-  if (!__all_sync(0xffffffffu, bulk_bar_wait(bulk_smem(tsm), 0))) {
-    if (lane == 0) atomicExch(err, 1);
-    return;
-  }
+  if (!__all_sync(0xffffffffu, bulk_bar_wait(bulk_smem(tsm), 0, err))) return;
   const int* ids = reinterpret_cast<const int*>(tsm + 16 + (((long long)t0 * 4) & 15));
   const T* vals = reinterpret_cast<const T*>(tsm + stream_vals<T>(cap) + (((long long)t0 * 18 * (int)sizeof(T)) & 15));
   T s[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
@@ -1384,10 +1381,7 @@ sa_prolong_stream_kernel(int nbrow, int cap, const int* __restrict__ p_rp, const
   pdl_wait();
   const long long i = (long long)n * 3 + j;
   const T xi = in ? x[i] : T(0);
-  if (!bulk_bar_wait(bulk_smem(tsm), 0)) {
-    atomicExch(err, 1);
-    return;
-  }
+  if (!bulk_bar_wait(bulk_smem(tsm), 0, err)) return;
   const int* ids = reinterpret_cast<const int*>(tsm + 16 + (((long long)t0 * 4) & 15));
   const T* vals = reinterpret_cast<const T*>(tsm + stream_vals<T>(cap) + (((long long)t0 * 18 * (int)sizeof(T)) & 15));
   T s = T(0);

@@ -156,10 +156,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           for (int i = 0; i < 9; ++i) D[i] = a.dinv[(long long)row * 9 + i];
         }
       }
-      if (!__all_sync(0xffffffffu, bulk_bar_wait(bar, phase))) {
-        if (lane == 0) atomicExch(err, 1);
-        return;
-      }
+      if (!__all_sync(0xffffffffu, bulk_bar_wait(bar, phase, err))) return;
       const int* rp = reinterpret_cast<const int*>(st + lay.rows);
       const int s0 = rp[0];
       const int b0 = ok ? rp[rl] - s0 : 0, len = ok ? rp[rl + 1] - s0 - b0 : 0;
@@ -269,7 +266,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           }
         }
         if (!waited) {
-          waited = __all_sync(0xffffffffu, bulk_bar_wait(bar, phase));
+          waited = __all_sync(0xffffffffu, bulk_bar_wait(bar, phase, err));
           if (!waited) break;
         }
         const int* rp = reinterpret_cast<const int*>(st + lay.rows);
@@ -347,10 +344,7 @@ bsr_spmv_pipe_kernel(int nbrow, int ntiles, int max_row, const int* __restrict__
           a.xo[at] = MODE == 3 ? upd : oi + upd;
         }
       }
-      if (!waited) {
-        if (lane == 0) atomicExch(err, 1);
-        return;
-      }
+      if (!waited) return;
       __syncwarp();
       if (lane == 0 && t + (int)gridDim.x < ntiles) {
         const int tn = t + gridDim.x, tf = tn + gridDim.x;
