@@ -1081,12 +1081,14 @@ int cg_graph_build(pfem_ctx* ctx, int method) {
 }
 
 // Bring ReadBack to the host (synchronizes); an error when a solver kernel gave up
-// waiting for its own copies.
+// waiting for its own copies, whose results are then not to be built on.
 int read_back(pfem_ctx* ctx) {
   CK(cudaMemcpyAsync(ctx->hBack, ctx->dBack, sizeof(ReadBack), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   if (!ctx->hBack->waits) return PFEM_OK;
   CK(cudaMemsetAsync(&ctx->dBack->waits, 0, sizeof(int), ctx->st));
+  ctx->tangent_prec = -1;
+  ctx->amg32.built = ctx->amg64.built = false;
   return fail(ctx, PFEM_ERR_CUDA, "a solver kernel's wait for its copies timed out");
 }
 
@@ -1160,7 +1162,8 @@ int krylov(pfem_ctx* ctx, int method, double rtol, int itmax, int* iters, bool* 
     dot<T>(n, w.b, w.b, w.sc + 12, w.part, st, true);
     T r = 0;
     CK(cudaMemcpyAsync(&r, w.sc + 12, sizeof(T), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    rc = read_back(ctx);  // the residual is a streamed product: its norm counts only if that is whole
+    if (rc) return rc;
     rn = (double)r;
     if (!std::isfinite(rn)) break;
     if (rn <= target) {
@@ -1296,12 +1299,12 @@ int residual_system(pfem_ctx* ctx, int prec, double lam, double* rnorm, double* 
     impose_dirichlet<float>(ctx->bc, ctx->ndof, lam, ctx->dU, ctx->dK32, ctx->dR, ctx->dPart, &ctx->dBack->ticket,
                             ctx->dBack->scal, ctx->st);
   CKL();
+  ctx->tangent_prec = prec;
   rc = check_status(ctx);  // synchronizes
   *rnorm = ctx->hBack->scal[0];
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx->e0, ctx->e1);
   if (t_asm) *t_asm += ms;
-  ctx->tangent_prec = prec;
   return rc;
 }
 
