@@ -23,7 +23,7 @@
 //
 // What bounds it: the latency of dependent arithmetic, FP64 in phase A, at the 8 (FP64) or
 // 12 (FP32) warps per SM that its registers and shared memory allow.  One residual call
-// at 64^3 with FP32 tangent 1.28 ms, at 57 x 43 x 31 FP64 0.55 ms; with the 96 columns of
+// at 64^3 with FP32 tangent 1.26 ms, at 57 x 43 x 31 FP64 0.55 ms; with the 96 columns of
 // a warp taken 32 at a time, single-word reads and single multiply-adds 1.37 and 0.66 ms.
 // FP32 with the record spread over 19 KB per warp, which leaves L1 less, 1.38 ms; by k as
 // in FP64 with the products added one by one 1.19 ms, but other results.
@@ -743,12 +743,10 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       wdP[9] = row9;
       store_pairs<REC_AQ>(Rg + REC_A + at * REC_AK + qq * REC_AQ, wdP);
     };
-    // Phase B for component k = pp: the columns (b, k) of the four element tangents by lane
-    // (slot, b).
-    const int b = g;
-    auto tangent = [&](const int pp) {
+    // Phase B: column (b, k = pp) of the tangent of the element in slot sl (ce, at Ss).
+    auto tangent = [&](const TT* Ss, const int sl, const int ce, const bool cvalid, const int b, const int pp) {
     TT acc[24];  // rows (a, i) of the column
-    const TT g0bk = FBAR ? g0s[3 * b + pp] : TT(0);
+    const TT g0bk = FBAR ? Ss[3 * b + pp] : TT(0);
     if constexpr (std::is_same<TT, float>::value) {
       f32x2 acc2[3][4];  // [i][pair of a]
 #pragma unroll
@@ -757,7 +755,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
         for (int m = 0; m < 4; ++m) acc2[i][m] = 0ull;
 #pragma unroll 1
       for (int gg = 0; gg < 8; ++gg) {
-        const float* Rr = S + 24 + gg * GPREC;
+        const float* Rr = Ss + 24 + gg * GPREC;
         const float db0 = Rr[b], db1 = Rr[8 + b], db2 = Rr[16 + b];
         f32x2 A[16];  // [q][pair of r] at a stride of 5; the last pair is not A's
 #pragma unroll
@@ -818,7 +816,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       for (int r = 0; r < 24; ++r) acc[r] = TT(0);
 #pragma unroll 1
       for (int gg = 0; gg < 8; ++gg) {
-        const TT* Rr = S + 24 + gg * GPREC;
+        const TT* Rr = Ss + 24 + gg * GPREC;
         const TT db0 = Rr[b], db1 = Rr[8 + b], db2 = Rr[16 + b];
         TT T[REC_AQ], v[REC_AQ];
         load_pairs<REC_AQ>(Rr + REC_A, v);
@@ -849,23 +847,31 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
         }
       }
     }
-    if (valid) {
+    if (cvalid) {
       if (p.Kbuf) {
         // element-ordered: column (b,k) of rows (a,i) at [e][a][i][(b,k)]
-        KT* kb = p.Kbuf + (long long)e * 576 + 3 * b + pp;
+        KT* kb = p.Kbuf + (long long)ce * 576 + 3 * b + pp;
 #pragma unroll
         for (int a = 0; a < 8; ++a)
 #pragma unroll
           for (int i = 0; i < 3; ++i) __stcs(kb + a * 72 + i * 24, (KT)acc[a * 3 + i]);
       } else {
-        // in place (colored): the eight target blocks lie in eight different block rows
-        const int* nds = nodes_s[warp][slot];
+        // in place (colored): the eight target blocks lie in eight different block rows, so
+        // all 24 loads are issued before any store (one memory latency per column; entry by
+        // entry 2.47 ms at 64^3 FP64, so 2.02)
+        const int* nds = nodes_s[warp][sl];
+        KT* vp[8];
+        KT old[24];
 #pragma unroll
         for (int a = 0; a < 8; ++a) {
-          KT* vp = p.Kval + ((long long)p.browptr[nds[a]] + p.rank[(long long)e * 64 + a * 8 + b]) * 9 + pp;
+          vp[a] = p.Kval + ((long long)p.browptr[nds[a]] + p.rank[(long long)ce * 64 + a * 8 + b]) * 9 + pp;
 #pragma unroll
-          for (int i = 0; i < 3; ++i) vp[3 * i] += (KT)acc[a * 3 + i];
+          for (int i = 0; i < 3; ++i) old[a * 3 + i] = vp[a][3 * i];
         }
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) vp[a][3 * i] = old[a * 3 + i] + (KT)acc[a * 3 + i];
       }
     }
     };
@@ -893,8 +899,22 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
       for (int h = 0; h < 3; ++h) store_pairs<2>(Rg + REC_A + h * REC_AK + REC_UK, u + 2 * h);
       store_pairs<4>(Rg + REC_U, u + 6);
       __syncwarp();
+      // Element-ordered: k after k, lane (slot, b).  In place: the warp's 96 columns 32 at a
+      // time, so that neighbouring lanes have neighbouring entries of K (64^3: 1.80 ms k
+      // after k).
 #pragma unroll 1
-      for (int pp = 0; pp < 3; ++pp) tangent(pp);
+      for (int r = 0; r < 3; ++r) {
+        int sl = slot, cb = g, k = r, ce = e, cv = valid;
+        if (!p.Kbuf) {
+          const int t = lane + 32 * r, col = t % 24;
+          sl = t / 24;
+          cb = col / 3;
+          k = col - 3 * cb;
+          ce = __shfl_sync(0xffffffffu, e, 8 * sl);
+          cv = __shfl_sync(0xffffffffu, (int)valid, 8 * sl);
+        }
+        tangent(wbase + sl * SLOT_TT, sl, ce, cv != 0, cb, k);
+      }
     } else {
       // w s/3 A vec(F), the F-bar vector, in closed form: along F the elastic strain
       // changes by I / s, which no flow direction sees (it is deviatoric) and no polar
@@ -925,7 +945,7 @@ element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
           keep(0, qq, dP, TT(0));
         }
         __syncwarp();
-        tangent(pp);
+        tangent(S, slot, e, valid, g, pp);
         __syncwarp();  // the next k's columns overwrite these
       }
     }
