@@ -65,8 +65,10 @@ struct CgGraph {
   long long prefix_kernels = 0, body_kernels = 0;
 };
 
-// What the host reads back after a residual or a linear solve, in one copy to a
-// page-locked mirror (each small copy to pageable memory costs about 9 us).
+// What the host reads back after a residual or a linear solve, in one copy (each small one
+// costs about 9 us).  Its mirror is ordinary memory: page-locked, a copy took 2 us less,
+// but a context 2.7 ms more to make (cudaMallocHost and what follows from it; 1.4 ms in
+// all at 8^3) and 0.4 ms to take down.
 struct ReadBack {
   DevStatus status;      // first inverted Gauss point of the last assembly
   int waits;             // set by a solver kernel whose bounded wait ran out
@@ -141,7 +143,8 @@ struct pfem_ctx {
   float* dKbuf32 = nullptr;
   double* dKbuf64 = nullptr;
   double* dFbuf = nullptr;
-  ReadBack *dBack = nullptr, *hBack = nullptr;
+  ReadBack* dBack = nullptr;
+  ReadBack hBack = {};
   // boundary conditions
   bool bcs_set = false;
   BcDev bc;
@@ -1083,9 +1086,9 @@ int cg_graph_build(pfem_ctx* ctx, int method) {
 // Bring ReadBack to the host (synchronizes); an error when a solver kernel gave up
 // waiting for its own copies, whose results are then not to be built on.
 int read_back(pfem_ctx* ctx) {
-  CK(cudaMemcpyAsync(ctx->hBack, ctx->dBack, sizeof(ReadBack), cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaMemcpyAsync(&ctx->hBack, ctx->dBack, sizeof(ReadBack), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
-  if (!ctx->hBack->waits) return PFEM_OK;
+  if (!ctx->hBack.waits) return PFEM_OK;
   CK(cudaMemsetAsync(&ctx->dBack->waits, 0, sizeof(int), ctx->st));
   ctx->tangent_prec = -1;
   ctx->amg32.built = ctx->amg64.built = false;
@@ -1113,7 +1116,7 @@ int krylov_inner(pfem_ctx* ctx, int method, double rtol, int itmax, int* iters, 
   CK(cudaGraphLaunch(G.exec, st));
   rc = read_back(ctx);
   if (rc) return rc;
-  const int* sh = ctx->hBack->cg[std::is_same<T, double>::value ? 1 : 0];
+  const int* sh = ctx->hBack.cg[std::is_same<T, double>::value ? 1 : 0];
   *iters = sh[0];
   *conv = sh[1] != 0;
   pfem::launch_counter() += G.prefix_kernels + (long long)sh[0] * G.body_kernels;
@@ -1273,7 +1276,7 @@ int ensure_tangent(pfem_ctx* ctx, int prec) {
 int check_status(pfem_ctx* ctx) {
   int rc = read_back(ctx);
   if (rc) return rc;
-  const DevStatus& s = ctx->hBack->status;
+  const DevStatus& s = ctx->hBack.status;
   if (s.code) {
     char buf[256];
     snprintf(buf, sizeof(buf),
@@ -1301,7 +1304,7 @@ int residual_system(pfem_ctx* ctx, int prec, double lam, double* rnorm, double* 
   CKL();
   ctx->tangent_prec = prec;
   rc = check_status(ctx);  // synchronizes
-  *rnorm = ctx->hBack->scal[0];
+  *rnorm = ctx->hBack.scal[0];
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx->e0, ctx->e1);
   if (t_asm) *t_asm += ms;
@@ -1933,8 +1936,7 @@ int pfem_create(pfem_ctx** out, const double* nodes, int64_t nn, const int64_t* 
   AL(ctx->dUtmp, ctx->ndof);
   AL(ctx->dPart, 2048);
   AL(ctx->dBack, 1);
-  if ((ce = cudaMallocHost((void**)&ctx->hBack, sizeof(ReadBack))) != cudaSuccess ||
-      (ce = cudaMemsetAsync(ctx->dBack, 0, sizeof(ReadBack), ctx->st)) != cudaSuccess) {
+  if ((ce = cudaMemsetAsync(ctx->dBack, 0, sizeof(ReadBack), ctx->st)) != cudaSuccess) {
     pfem_set_cuda_error(ce, "ReadBack", __FILE__, __LINE__);
     return bail(PFEM_ERR_CUDA);
   }
@@ -1960,7 +1962,6 @@ void pfem_destroy(pfem_ctx* ctx) {
     if (g->body_stream) cudaStreamDestroy(g->body_stream);
   }
   for (void* p : ctx->allocs) cudaFree(p);
-  if (ctx->hBack) cudaFreeHost(ctx->hBack);
   if (ctx->e0) cudaEventDestroy(ctx->e0);
   if (ctx->e1) cudaEventDestroy(ctx->e1);
   if (ctx->t0) cudaEventDestroy(ctx->t0);
