@@ -1190,13 +1190,19 @@ int assemble_dev(pfem_ctx* ctx, int prec, bool commit) {
   const bool small = ctx->kind == PFEM_HEX8_SMALL;
   CK(cudaMemsetAsync(&ctx->dBack->status, 0, sizeof(DevStatus), st));
   if (commit) {
-    ElemArgs<double> a{};
-    a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
-    a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
-    a.R = ctx->dR; a.Kval = ctx->dK64; a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
-    a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
-    if (small) launch_element_small<double>(a, ctx->dAllElems, (int)ctx->ne, true, ctx->hard, st);
-    else launch_element_color<double>(a, ctx->dAllElems, (int)ctx->ne, true, fbar, ctx->hard, st);
+    // no tangent here, but the type picks the rotations of the principal axes, and a state
+    // should come from those that the tangents and forces of its path use
+    auto update = [&](auto a) {
+      using KT = typename std::remove_pointer<decltype(a.Kval)>::type;
+      a.X = ctx->dX; a.elem = ctx->dElem; a.U = ctx->dU; a.cpi = ctx->dCpi; a.alpha = ctx->dAlpha;
+      a.epsp = ctx->dEpsp; a.beta = ctx->dBeta; a.sigy0_e = ctx->dSigy; a.tau = ctx->dTau; a.flags = ctx->dFlags;
+      a.R = ctx->dR; a.Kval = K_of<KT>(ctx); a.browptr = ctx->dBrowptr; a.rank = ctx->dRank;
+      a.ngp = ctx->ngp; a.mat = ctx->mat; a.status = &ctx->dBack->status;
+      if (small) launch_element_small<KT>(a, ctx->dAllElems, (int)ctx->ne, true, ctx->hard, st);
+      else launch_element_color<KT>(a, ctx->dAllElems, (int)ctx->ne, true, fbar, ctx->hard, st);
+    };
+    if (prec == PFEM_FP64) update(ElemArgs<double>{});
+    else update(ElemArgs<float>{});
     CKL();
     return PFEM_OK;
   }
@@ -1495,8 +1501,8 @@ int newton_dev(pfem_ctx* ctx, double lam, const pfem_solve_opts* o, int* iters, 
   return PFEM_OK;
 }
 
-int commit_dev(pfem_ctx* ctx) {
-  int rc = assemble_dev(ctx, PFEM_FP64, true);
+int commit_dev(pfem_ctx* ctx, int prec) {
+  int rc = assemble_dev(ctx, prec, true);
   if (rc) return rc;
   return check_status(ctx);
 }
@@ -2238,7 +2244,7 @@ int pfem_assemble(pfem_ctx* ctx, const double* U, int32_t commit, int32_t precis
   if (rc) return rc;
   const int prec = precision == PFEM_MIXED ? PFEM_MIXED : PFEM_FP64;
   if (commit) {
-    rc = commit_dev(ctx);
+    rc = commit_dev(ctx, PFEM_MIXED);  // the caller may go on in either precision
     if (rc) return rc;
   } else {
     rc = ensure_tangent(ctx, prec);
@@ -2445,7 +2451,7 @@ int pfem_newton(pfem_ctx* ctx, double lambda, const pfem_solve_opts* o, int32_t*
   if (krylov_hist) std::copy(kh.begin(), kh.end(), krylov_hist);
   if (rc) return rc;
   if (!conv) return fail(ctx, PFEM_ERR_NOT_CONVERGED, "load step did not converge");
-  rc = commit_dev(ctx);
+  rc = commit_dev(ctx, o->precision);
   if (rc) return rc;
   return step_end(ctx, lambda);
 }
@@ -2505,7 +2511,7 @@ int pfem_solve(pfem_ctx* ctx, const pfem_solve_opts* o, pfem_solve_result* res, 
       const bool soft = rc == PFEM_ERR_NOT_CONVERGED || rc == PFEM_ERR_INVERTED_ELEMENT;
       if (rc && !soft) return rc;
       if (rc == PFEM_OK && conv) {
-        rc = commit_dev(ctx);
+        rc = commit_dev(ctx, o->precision);
         if (rc) return rc;
         rc = step_end(ctx, lam);
         if (rc) return rc;

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * WPB, (std::is_same<KT, float>::value && !
 element_color_kernel(ElemArgs<KT> p, const int* __restrict__ elist, int nlist) {
   using TT = KT;  // type of the tangent records and of the phase-B arithmetic
   constexpr int GPREC = gprec<TT>(), SLOT_TT = slot_tt<TT>(), REC_U = rec_u<TT>();
-  constexpr bool kQuot = COMMIT || std::is_same<TT, float>::value;
+  constexpr bool kQuot = std::is_same<TT, float>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = lane >> 3, g = lane & 7;
