@@ -1065,13 +1065,13 @@ __global__ void __launch_bounds__(128) sa_rap_kernel(int nnzC, const int* __rest
       if ((r * 6 + q) % LN == lane) O[r * 6 + q] = acc[r][q];
 }
 
-// The same for FP32 in the order of the P^T row, as one thread per block would add it: the
+// The same for FP32 in the order of the P^T row, as one thread per block adds it: the
 // coarse operator's small eigenvalues are what is left of terms hundreds of times larger,
 // so in FP32 another order is another operator, and the solution of a slender box moves
 // with it.  What the LN lanes of a block find is taken in turn, lane r with the six entries
 // of row r.  Set-up with this / with the kernel above, FP32: 0.40 / 0.40 ms at 8^3, 1.01 /
-// 1.03 at 80 x 16 x 16, 1.57 / 1.54 at 40^3, 3.90 / 3.68 at 64^3; one at a time 0.45, 1.13,
-// 1.58 and 3.89; 16 lanes 0.39, 1.04, 1.63 and 4.31.  (FP64 2.23 / 2.07 ms at 40^3.)
+// 1.03 at 80 x 16 x 16, 1.57 / 1.54 at 40^3; one at a time 0.45, 1.13 and 1.58; 16 lanes
+// 0.39, 1.04 and 1.63.  (FP64 2.23 / 2.07 ms at 40^3.)
 template <typename T, int BS, int LN>
 __global__ void __launch_bounds__(128) sa_rap_ordered_kernel(int nnzC, const int* __restrict__ c_row, const int* __restrict__ c_cl,
                               const int* __restrict__ pt_rp, const int* __restrict__ pt_row,
@@ -1269,12 +1269,17 @@ static void setup_level_t(const AmgLevel<T>& v, T* cval, int nnzC, cudaStream_t 
          v.p_val, v.pt_val);
   launch(st, sa_ap_kernel<T, BS>, (v.nnzAP + 127) / 128, 128, 0, v.nnzAP, v.ap_row, v.ap_cl, v.A.rowptr, v.A.col, v.A.val,
          v.p_rp, v.p_cl, v.p_val, v.ap_val);
+  // FP32: a thread per block where those fill the chip (set-up with one / with eight lanes
+  // per block: 0.61 / 0.39 ms at 8^3, 1.67 / 1.60 at 40^3, 2.82 / 2.85 at 52^3 with 140,608
+  // blocks, 3.54 / 3.94 at 64^3 with 262,144); both add in the order of the P^T row.
+  constexpr int kRapOneThread = 150000;
+  const bool one = std::is_same<T, float>::value && nnzC >= kRapOneThread;
   constexpr int LN = 8;
-  auto* rap = [] {
-    if constexpr (std::is_same<T, float>::value) return &sa_rap_ordered_kernel<T, BS, LN>;
+  auto* rap = [one] {
+    if constexpr (std::is_same<T, float>::value) return one ? &sa_rap_kernel<T, BS, 1> : &sa_rap_ordered_kernel<T, BS, LN>;
     else return &sa_rap_kernel<T, BS, LN>;
   }();
-  launch(st, rap, (int)(((long long)nnzC * LN + 127) / 128), 128, 0, nnzC, v.c_row, v.c_cl, v.pt_rp,
+  launch(st, rap, (int)(((long long)nnzC * (one ? 1 : LN) + 127) / 128), 128, 0, nnzC, v.c_row, v.c_cl, v.pt_rp,
          v.pt_row, v.pt_val, v.ap_rp, v.ap_cl, v.ap_val, cval);
 }
 template <typename T>

@@ -27,11 +27,13 @@ TANGENTS = [("finite_fbar", "linear", "noise"), ("finite_fbar", "linear", "equal
             ("finite", "voce", "noise")]
 
 # box, element, hardening, pulled along, method, every how many entries are kept: around
-# the row limits of the streamed products (8192 block rows, 4096 of 6 x 6) and transfers
+# the row limits of the streamed products (8192 block rows, 4096 of 6 x 6) and transfers, and
+# with more coarse blocks (157,300 in the last) than eight lanes each are given
 SOLVES = [((13, 7, 7), "finite_fbar", "linear", 0, "cg", 1), ((20, 8, 8), "small", "linear", 0, "cg", 3),
           ((30, 8, 6), "finite", "linear", 0, "cg", 3), ((35, 25, 40), "finite_fbar", "linear", 2, "cg", 19),
           ((41, 21, 30), "finite", "voce", 0, "cg", 19), ((50, 50, 50), "finite_fbar", "linear", 0, "cg", 97),
-          ((14, 10, 9), "finite_fbar", "linear", 0, "bicgstab", 1), ((27, 20, 25), "small", "linear", 0, "bicgstab", 19)]
+          ((14, 10, 9), "finite_fbar", "linear", 0, "bicgstab", 1), ((27, 20, 25), "small", "linear", 0, "bicgstab", 19),
+          ((56, 54, 52), "finite", "linear", 2, "cg", 97)]
 
 
 def model(n, element, hard, axis, seed=3):
