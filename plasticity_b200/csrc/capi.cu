@@ -520,8 +520,9 @@ void mgs_qr(int m, std::vector<double>& A, double R[36]) {
 // constrained aggregates leave coarse rows that are nearly dependent)
 // and applied as one dense matrix-vector product per cycle.  The inverse costs
 // n^3 at every rebuild: at 64^3 a 3,072-unknown dense level 2 saves a W-cycle's
-// two visits to it (about 100 us per cycle) but adds about 11 ms per rebuild,
-// so by default the hierarchy goes one level further there (162 unknowns).
+// two visits to it (a CG iteration of 368 us instead of 375) but adds 3.6 ms per rebuild
+// (7.5 ms mixed, 9.4 ms FP64), so by default the hierarchy goes one level further there
+// (162 unknowns).
 // PFEM_COARSE_DENSE_MAX overrides the bound.
 constexpr long long kCoarseDenseMax = 1500;
 // The adaptive AMG policy charges a rebuild this many Krylov iterations.

@@ -22,7 +22,8 @@
 // end), so another order is another result.
 //
 // What bounds it: the latency of dependent arithmetic, FP64 in phase A, at the 8 (FP64) or
-// 12 (FP32) warps per SM that its registers and shared memory allow.  One residual call
+// 12 (FP32) warps per SM that its registers and shared memory allow: the FP64 pipe is 52
+// and 24 % busy, and 38 and 46 % of the issue slots are taken (40^3).  One residual call
 // at 64^3 with FP32 tangent 1.26 ms, at 57 x 43 x 31 FP64 0.55 ms; with the 96 columns of
 // a warp taken 32 at a time, single-word reads and single multiply-adds 1.37 and 0.66 ms.
 // FP32 with the record spread over 19 KB per warp, which leaves L1 less, 1.38 ms; by k as
@@ -194,8 +195,8 @@ __device__ __forceinline__ T sym_dot(const T* a, const T* b) {
 }
 
 // With FP32 tangent records registers are capped for 11 resident one-warp blocks per SM
-// (168 registers, 12 blocks, a little spilling to L1); caps for 14 and 16 blocks took
-// 1.05 ms where this takes 0.98 (64^3 assembly).  The FP64 variants lose from a cap and
+// (168 registers, 12 blocks, a little spilling to L1): without the cap (244 registers, 8
+// blocks) a residual call at 64^3 takes 4 % more.  The FP64 variants lose from a cap and
 // keep the compiler's choice, as does the kinematic variant with its extra state.
 template <typename KT, bool COMMIT, bool FBAR, int HARD>
 __global__ void __launch_bounds__(32 * WPB, (std::is_same<KT, float>::value && !COMMIT && HARD != HARD_KIN) ? 11 : 1)

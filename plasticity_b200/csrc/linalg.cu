@@ -586,10 +586,10 @@ void power_norm(long long n, const T* v, T* part, unsigned* ticket, bool finish,
 }
 // ---- BiCGStab updates.  Scalars: sc[0] rho = rh.r, sc[1] rho of the iteration before,
 // sc[2] alpha, sc[3] omega.  A thread per node, as cg_xr_fused; the dot products come as
-// dot's partials and are added in its order.  An iteration used to be 78 plain launches
+// dot's partials and are added in its order.  An iteration used to be 44 plain launches
 // from the host with a read-back of |r|, bound by the launches below about 40^3; in the
-// graph with the smoother's starts in its own updates it is 44 and takes 440 us at 40^3
-// FP64, 550 before.
+// graph with the smoother's starts in its own updates it takes 410 us at 40^3 FP64, 550
+// before.
 template <typename T>
 __device__ __forceinline__ void smoother_start(const T* __restrict__ dinv, T ith, long long n, const T v[3], T* sr,
                                                T* sd) {
@@ -1015,7 +1015,7 @@ __global__ void sa_ap_kernel(int nnzAP, const int* __restrict__ ap_row, const in
 // consecutive blocks), each searching its row of AP for J, and add their 36 partial
 // sums by a fixed xor tree.  One thread per block walked the whole row, about 115
 // blocks at level 0: 770 us there at 64^3 and 403 us at level 1, 320 us for the whole of a
-// 23x9x7 mesh; now 634, 58 and 45 us.
+// 23x9x7 mesh; so 634, 58 and 45 us (FP32).
 template <typename T, int BS, int LN>
 __global__ void __launch_bounds__(128) sa_rap_kernel(int nnzC, const int* __restrict__ c_row, const int* __restrict__ c_cl,
                               const int* __restrict__ pt_rp, const int* __restrict__ pt_row,

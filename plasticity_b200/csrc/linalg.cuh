@@ -14,7 +14,7 @@ namespace pfem {
 // are launched the plain way: their CTAs would take the slots of the running kernel's
 // last ones and wait there.  The cycle in its graph, plain / all chained / this rule:
 // 18.6 / 16.5 / 15.6 us at 8^3, 68 / 72 / 64 at 32^3, 104 / 109 / 100 at 40^3,
-// 337 / 356 / 325 at 64^3.
+// 337 / 356 / 325 at 64^3 (before the transfers there were streamed: 293 since).
 constexpr int kChainGrid = 4 * 148;
 struct Queue {
   cudaStream_t st = nullptr;

@@ -50,7 +50,7 @@ struct SpmvVec {
 // LANES lanes per row and ROWS rows per tile; a CTA is one warp with one tile in shared
 // memory (8 rows of 27 blocks: 8 KB float, 16 KB double; 4 rows of 6 x 6: 15 KB), so
 // that 13 to 24 of them share an SM and the copies of some overlap the arithmetic of
-// the others.  Measured at 64^3, FP32, per pass over 281 MB: 44.0 us (6.4 TB/s; the
+// the others.  Measured at 64^3, FP32, per pass over 281 MB: 42.6 us (6.6 TB/s; the
 // register kernel 59.8); one warp with two stages 49.2, two warps with two stages
 // 50.5, a producer lane feeding eight half-warp-per-row warps through four stages
 // 51.4.  FP64 79.0 us (103.1).  Two lanes per row: the same at 64^3, 14 % slower at
